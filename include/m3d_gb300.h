@@ -123,10 +123,15 @@ typedef struct m3d_params {
                                  as the reference, 1 Eisenstat split form (staged rows) for batches
                                  without a right-hand side that gets the gradient-space term (those
                                  always run the right-preconditioned form) */
-    int gradcorr;             /* 1: the mixed-precision inner solve adds a gradient-space term
-                                 G (i omega L)^-1 G^T (one multigrid V-cycle on the divergence-
-                                 correction Laplacian L) to the SSOR preconditioner of the
-                                 right-hand sides with f <= gradcorr_fmax; needs div_correction.
+    int gradcorr;             /* 1: the mixed-precision inner solve of right-hand sides with
+                                 f <= gradcorr_fmax is preconditioned by geometric multigrid on the
+                                 uniform grids under the octree (edge and node cycles, damped Jacobi
+                                 smoothing), where every leaf is at level 2 or finer and the levels
+                                 span at most 4; on other meshes, and with a setting of the SSOR sweeps
+                                 or of the aggregation cycle other than its default (ssor_relax,
+                                 coop_sweep, sweep_rows, gradcorr_presmooth), by SSOR plus a
+                                 gradient-space term G (i omega L)^-1 G^T (one multigrid V-cycle on
+                                 the divergence-correction Laplacian L); needs div_correction.
                                  Batches with such a right-hand side run the right-preconditioned
                                  form.  0: SSOR alone (the reference's preconditioner) */
     double gradcorr_fmax;     /* Hz */

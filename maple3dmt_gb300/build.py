@@ -23,8 +23,8 @@ LIB = os.path.join(LIB_DIR, "libm3d_gb300.so")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 HOST_SRCS = ["host/octree_build.cpp", "host/mesh_capi.cpp", "host/layout.cpp", "host/layout_capi.cpp", "host/amg.cpp",
-             "host/regularization.cpp"]
-CUDA_SRCS = ["cuda/krylov.cu", "cuda/physics.cu", "cuda/gradcorr.cu", "cuda/regularization.cu", "cuda/dot.cu",
+             "host/regularization.cpp", "host/edgemg.cpp"]
+CUDA_SRCS = ["cuda/krylov.cu", "cuda/physics.cu", "cuda/gradcorr.cu", "cuda/edgemg.cu", "cuda/regularization.cu", "cuda/dot.cu",
              "cuda/learned.cu", "solver.cu", "learned_solver.cu", "capi.cu", "noalloc.cu", "learned_capi.cu"]
 
 

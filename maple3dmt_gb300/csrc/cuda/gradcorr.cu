@@ -358,6 +358,18 @@ GcRowTerm gc_row_term(const GcDev& g, const BatchView& B) {
 }
 
 template <int K>
+void gc_restrict_edges_k(const GcDev& g, const float2* in, cudaStream_t s, long long* launches) {
+    k_gc_restrict_edges<K><<<gc_grid((long)g.nn * K), kGcBlock, 0, s>>>(g, in, 0);
+    gc_check(launches);
+}
+
+template <int K>
+void gc_smooth0_k(const GcDev& g, const float2* t, float2* out, cudaStream_t s, long long* launches) {
+    k_gc_smooth0<K><<<gc_grid((long)g.nn * K), kGcBlock, 0, s>>>(g, t, out);
+    gc_check(launches);
+}
+
+template <int K>
 void gc_apply_k(const GcDev& g, int n_rows, const float2* in, cudaStream_t s, long long* launches,
                 KernelTimer* timer) {
     const int nl = g.n_levels;
@@ -713,6 +725,15 @@ template long long dc_poisson_mixed_k<2>(const GcDev&, int, DcWork, RedScratch, 
 template long long dc_poisson_mixed_k<4>(const GcDev&, int, DcWork, RedScratch, cudaStream_t, long long*);
 template long long dc_poisson_mixed_k<8>(const GcDev&, int, DcWork, RedScratch, cudaStream_t, long long*);
 template long long dc_poisson_mixed_k<16>(const GcDev&, int, DcWork, RedScratch, cudaStream_t, long long*);
+
+template void gc_restrict_edges_k<2>(const GcDev&, const float2*, cudaStream_t, long long*);
+template void gc_smooth0_k<2>(const GcDev&, const float2*, float2*, cudaStream_t, long long*);
+template void gc_restrict_edges_k<4>(const GcDev&, const float2*, cudaStream_t, long long*);
+template void gc_smooth0_k<4>(const GcDev&, const float2*, float2*, cudaStream_t, long long*);
+template void gc_restrict_edges_k<8>(const GcDev&, const float2*, cudaStream_t, long long*);
+template void gc_smooth0_k<8>(const GcDev&, const float2*, float2*, cudaStream_t, long long*);
+template void gc_restrict_edges_k<16>(const GcDev&, const float2*, cudaStream_t, long long*);
+template void gc_smooth0_k<16>(const GcDev&, const float2*, float2*, cudaStream_t, long long*);
 
 template void gc_apply_k<2>(const GcDev&, int, const float2*, cudaStream_t, long long*, KernelTimer*);
 template void gc_apply_k<4>(const GcDev&, int, const float2*, cudaStream_t, long long*, KernelTimer*);

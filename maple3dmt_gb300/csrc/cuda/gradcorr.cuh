@@ -98,6 +98,13 @@ template <int K>
 void gc_apply_k(const GcDev& g, int n_rows, const float2* in, cudaStream_t s, long long* launches,
                 KernelTimer* timer);
 
+// The two octree-level steps of a node cycle that the geometric multigrid
+// (edgemg.cuh) shares: g.lv[0].b = G~^T in, and out = t + omega D^-1 (b - L t).
+template <int K>
+void gc_restrict_edges_k(const GcDev& g, const float2* in, cudaStream_t s, long long* launches);
+template <int K>
+void gc_smooth0_k(const GcDev& g, const float2* t, float2* out, cudaStream_t s, long long* launches);
+
 // Solves L phi = divJ for the right-hand sides of w with cg_run set (the
 // PCG stage of divcorr_poisson_, forward_solver_fv.cpp:668-710): FP64
 // iterative refinement around FP32 PCG solves preconditioned by the FP32

@@ -1,6 +1,7 @@
 // Batched SSOR-BiCGStab kernels.  See krylov.cuh for what they restate.
 #include "krylov.cuh"
 
+#include "edgemg.cuh"
 #include "gradcorr.cuh"
 
 #include <algorithm>
@@ -161,6 +162,18 @@ __device__ __forceinline__ float2 inv_c(float2 d) {
     return make_float2(d.x / n, -d.y / n);
 }
 
+// w / d of the Jacobi step kSpmvSmooth, d = S + i m: the damping w goes from
+// kSmoothDamping on rows of the curl-curl part to 1 where the mass part
+// outweighs it -- such a row is all but decoupled and the step solves it
+template <class C> __device__ __forceinline__ C smooth_scale(C d) {
+    const auto s = d.x * d.x, m = d.y * d.y, r = 1 / (s + m);   // s + m squared leaves the FP32 range
+    const auto w = (kSmoothDamping * s + m) * r * r;
+    C z;
+    z.x = w * d.x;
+    z.y = -w * d.y;
+    return z;
+}
+
 // ---------------------------------------------------------------------------
 // Scalar recurrences of BiCGStabSolver::solve (src/forward/bicgstab.cpp),
 // run by thread k < K of the last block of each reduction.
@@ -289,8 +302,8 @@ __global__ void __launch_bounds__(kBlock) k_spmv(OpView<R> A, DiagView<R> D, Bat
                                                  RedScratch rs) {
     using C = cplx<R>;
     constexpr int RPW = Rpw<K>::v;
-    constexpr int NQ = (MODE == kSpmvAp) ? 1 : (MODE == kSpmvAs || MODE == kSpmvTrueRes) ? 2 : 3;
-    constexpr bool REDUCE = MODE != kSpmvPlain;
+    constexpr int NQ = (MODE == kSpmvAp || MODE == kSpmvSmooth) ? 1 : (MODE == kSpmvAs || MODE == kSpmvTrueRes) ? 2 : 3;
+    constexpr bool REDUCE = MODE != kSpmvPlain && MODE != kSpmvSmooth;
     const int lane = threadIdx.x & 31;
     const int rhs = lane % K, sub = lane / K;
     const long wg = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -323,7 +336,9 @@ __global__ void __launch_bounds__(kBlock) k_spmv(OpView<R> A, DiagView<R> D, Bat
             accR[0].x += bv.x * bv.x + bv.y * bv.y;
             accR[1].x += rv.x * rv.x + rv.y * rv.y;
             accR[2] = cadd(accR[2], cjmul(rv, rv));
-        } else {  // kSpmvTrueRes
+        } else if (MODE == kSpmvSmooth) {
+            y[i] = cadd(x[i], cmul(csub(aux[i], yv), smooth_scale(d)));
+        } else if (MODE == kSpmvTrueRes) {
             const C bv = aux[i];
             const C rv = csub(bv, yv);
             y[i] = rv;
@@ -410,8 +425,8 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
     using C = cplx<R>;
     using Sh = StagedShape<K>;
     constexpr int RPW = Rpw<K>::v;
-    constexpr int NQ = (MODE == kSpmvAp) ? 1 : (MODE == kSpmvAs || MODE == kSpmvTrueRes) ? 2 : 3;
-    constexpr bool REDUCE = MODE != kSpmvPlain;
+    constexpr int NQ = (MODE == kSpmvAp || MODE == kSpmvSmooth) ? 1 : (MODE == kSpmvAs || MODE == kSpmvTrueRes) ? 2 : 3;
+    constexpr bool REDUCE = MODE != kSpmvPlain && MODE != kSpmvSmooth;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rhs = lane % K;
     const int lr0 = warp * RPW + lane / K;
@@ -449,7 +464,9 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
                 accR[0].x += av.x * av.x + av.y * av.y;
                 accR[1].x += rv.x * rv.x + rv.y * rv.y;
                 accR[2] = cadd(accR[2], cjmul(rv, rv));
-            } else {  // kSpmvTrueRes
+            } else if (MODE == kSpmvSmooth) {
+                y[i] = cadd(xi, cmul(csub(av, yv), smooth_scale(d)));
+            } else if (MODE == kSpmvTrueRes) {
                 const C rv = csub(av, yv);
                 y[i] = rv;
                 accR[0].x += rv.x * rv.x + rv.y * rv.y;
@@ -768,8 +785,12 @@ void spmv_staged(const KrylovCtx<R>& c, int mode, const cplx<R>* x, cplx<R>* y, 
     const int sb = c.seg.stage_spmv;
     // reducing modes: every block must reach the reduction, so the grid stays
     // within the partial-sum scratch
-    const int cap = (mode == kSpmvPlain) ? (1 << 20) : c.red.max_blocks;
+    const int cap = (mode == kSpmvPlain || mode == kSpmvSmooth) ? (1 << 20) : c.red.max_blocks;
     switch (mode) {
+        case kSpmvSmooth:
+            launch_staged(k_spmv_st<R, K, kSpmvSmooth>, NT, sb, ns, cap, c.stream, c.seg, ns, c.D, c.B, x, y, aux,
+                          aux_out, st, c.red);
+            break;
         case kSpmvPlain:
             launch_staged(k_spmv_st<R, K, kSpmvPlain>, NT, sb, ns, cap, c.stream, c.seg, ns, c.D, c.B, x, y, aux,
                           aux_out, st, c.red);
@@ -798,7 +819,7 @@ void spmv_k(const KrylovCtx<R>& c, int mode, const cplx<R>* x, cplx<R>* y, const
             cplx<R>* aux_out, BicgState* st) {
     const long warps = (long)c.A.n_pad / Rpw<K>::v;
     int grid;
-    if (mode == kSpmvPlain) {
+    if (mode == kSpmvPlain || mode == kSpmvSmooth) {
         grid = blocks_for(warps, kWarpsPerBlock, 1 << 20);
     } else {
         grid = c.grid_spmv;
@@ -816,6 +837,9 @@ void spmv_k(const KrylovCtx<R>& c, int mode, const cplx<R>* x, cplx<R>* y, const
     switch (mode) {
         case kSpmvPlain:
             k_spmv<R, K, kSpmvPlain><<<grid, kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red);
+            break;
+        case kSpmvSmooth:
+            k_spmv<R, K, kSpmvSmooth><<<grid, kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red);
             break;
         case kSpmvAp: {
             auto kf = k_spmv<R, K, kSpmvAp>;
@@ -1001,6 +1025,23 @@ void gc_term(const KrylovCtx<R>& c, const cplx<R>* in) {
     }
 }
 
+// out = B in: the geometric multigrid preconditioner (edgemg.cuh), or SSOR
+// plus the gradient-space term: V-cycle first, added by the backward sweep.
+template <class R, int K>
+void precond_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out) {
+    if constexpr (std::is_same<R, float>::value) {
+        if (c.emg) {
+            emg_coarse_k<K>(c, in, y);
+            spmv_k<R, K>(c, kSpmvSmooth, y, out, in, nullptr, nullptr);
+            return;
+        }
+    }
+    GcRowTerm gt;
+    if (c.gc) gt = gc_row_term(*c.gc, c.B);
+    gc_term<R, K>(c, in);
+    ssor_k<R, K>(c, in, y, out, gt);
+}
+
 template <class R, int K>
 void iteration_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* st) {
     const long n = (long)c.n_pad * K;
@@ -1010,19 +1051,13 @@ void iteration_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* st) {
     k_update_p<R, K><<<gv, kBlock, 0, c.stream>>>(n, v.r, v.p, v.v, st);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);
-    // the gradient-space term: V-cycle first, added to the preconditioned
-    // vector by the backward sweep
-    GcRowTerm gt;
-    if (c.gc) gt = gc_row_term(*c.gc, c.B);
-    gc_term<R, K>(c, v.p);
-    ssor_k<R, K>(c, v.p, v.y, v.ph, gt);
+    precond_k<R, K>(c, v.p, v.y, v.ph);
     spmv_k<R, K>(c, kSpmvAp, v.ph, v.v, v.r0, nullptr, st);
     th = c.timer ? c.timer->begin(kClsVec, 3 * vb, K) : -1;
     k_update_s<R, K><<<wave_grid(k_update_s<R, K>, gv), kBlock, 0, c.stream>>>(n, v.r, v.v, v.s, st, c.red);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);
-    gc_term<R, K>(c, v.s);
-    ssor_k<R, K>(c, v.s, v.y, v.sh, gt);
+    precond_k<R, K>(c, v.s, v.y, v.sh);
     spmv_k<R, K>(c, kSpmvAs, v.sh, v.t, v.s, nullptr, st);
     th = c.timer ? c.timer->begin(kClsVec, 8 * vb, K) : -1;
     k_update_xr<R, K><<<wave_grid(k_update_xr<R, K>, gv), kBlock, 0, c.stream>>>(n, v.x, v.r, v.r0, v.ph, v.sh, v.s, v.t, st, c.red);
@@ -1403,13 +1438,7 @@ void ssor_apply(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* o
 // sweep) -- the right preconditioner of one half iteration of iteration_k.
 template <class R>
 void precond_apply(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out) {
-#define CALL(K)                                  \
-    {                                            \
-        GcRowTerm gt;                            \
-        if (c.gc) gt = gc_row_term(*c.gc, c.B);  \
-        gc_term<R, K>(c, in);                    \
-        ssor_k<R, K>(c, in, y, out, gt);         \
-    }
+#define CALL(K) precond_k<R, K>(c, in, y, out)
     M3D_DISPATCH_K(c.B.K, CALL)
 #undef CALL
 }

@@ -129,6 +129,7 @@ struct KernelTimer {
 };
 
 struct GcDev;   // gradient-space correction of the preconditioner (gradcorr.cuh)
+struct EmgDev;  // geometric multigrid preconditioner (edgemg.cuh)
 
 // Everything one launch of the batched solver needs.
 template <class R>
@@ -160,6 +161,9 @@ struct KrylovCtx {
     // right-preconditioned form only (complex FP32): when set, each SSOR
     // apply is followed by the gradient-space term of the preconditioner
     const GcDev* gc = nullptr;
+    // complex FP32 with gc: when set, the preconditioner is the geometric
+    // multigrid one instead of SSOR plus the gradient-space term
+    const EmgDev* emg = nullptr;
     // when set, the V-cycle runs on gc_stream, forked after the p / s update
     // and joined before the backward sweep, overlapping the forward sweep
     cudaStream_t gc_stream = nullptr;
@@ -185,7 +189,10 @@ enum SpmvMode : int {
     kSpmvAs = 2,       // t = A s_hat, (t, t), (t, s) -> omega
     kSpmvInit = 3,     // r = b - A x, r0 = r, |b|, |r|, (r0, r) -> start
     kSpmvTrueRes = 4,  // y = b - A x, |y| / |b| -> true_res
+    kSpmvSmooth = 6,   // y = x + w (b - A x) / d: one damped Jacobi step (w = kSmoothDamping)
 };
+
+constexpr float kSmoothDamping = 0.4f;
 
 // Host launchers (explicit instantiations for R in {double, float}).
 template <class R>

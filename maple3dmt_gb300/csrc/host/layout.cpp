@@ -159,7 +159,7 @@ void build_layout(const LeafInput& in, HostLayout& L) {
     L.ne = ne;
 
     // ---- faces (staggered_grid.cpp:128-224) ----
-    std::vector<double> fx, fy, fz;
+    std::vector<double>&fx = L.fx, &fy = L.fy, &fz = L.fz;
     std::vector<int>& fnorm = L.fnorm;
     std::vector<int>& fcm = L.fcm;
     std::vector<int>& fcp = L.fcp;

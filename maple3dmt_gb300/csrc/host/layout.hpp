@@ -42,6 +42,7 @@ struct HostLayout {
     std::vector<char> dead;              // dead (coarse hanging) edges
     std::vector<std::array<int, 3>> hp;  // hanging pairs: coarse, child1, child2
     // faces
+    std::vector<double> fx, fy, fz;      // face centres
     std::vector<double> farea, fdual;
     std::vector<int> fnorm, fcm, fcp;    // normal direction, minus / plus cell (after the hanging fix-up)
     std::vector<char> dead_f;

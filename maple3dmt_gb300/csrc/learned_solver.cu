@@ -588,7 +588,7 @@ BatchResult GpuSolver::solve_batch_fgmres(int K, const int* fmap, double2* b, do
                 const double om = 2.0 * kPi * fz_freqs[fmap[k]];
                 use_gc |= om > 0.0 && om <= gc.omega_max;
             }
-    if (use_gc) attach_gc(c32);
+    if (use_gc) attach_gc(c32, false);
     const bool learned = P.learned_period > 0 && net && net_trained;
     const long n = (long)n_pad * K;
     const long ld = n;

@@ -232,6 +232,7 @@ void GpuSolver::free_all() {
     dfree(dc.lap_diag); dfree(dc.lap_off); dfree(dc.jac_inv); dfree(dc.st);
     dfree(dc.lap_seg); dfree(d_lap_work); dfree(d_lap_qpos);
     free_amg();
+    free_emg();
     amg_host = AmgHierarchy{};
     a0_pos_q.clear();
     a0_pos_d.clear();
@@ -536,6 +537,8 @@ void GpuSolver::setup(const m3d_leaves* lv, const m3d_params* params) {
     }
     h_inc_ptr = inc_ptr;
     h_inc_other = inc_other;
+    node_free.assign(nn, 0);
+    for (int v = 0; v < nn; ++v) node_free[v] = !node_bc[v];
 
     // upload
     md.ne = ne; md.n_pad = n_pad; md.nc = L.nc; md.nn = nn; md.n_slices = n_slices;
@@ -591,8 +594,67 @@ void GpuSolver::setup(const m3d_leaves* lv, const m3d_params* params) {
     d_states = dalloc<BicgState>(dev::kMaxRhs);
     d_states2 = dalloc<BicgState>(dev::kMaxRhs);
     sigma_h.assign(L.nc, 0.0);
+    if (want_emg()) build_emg();
     sync();
     ready = true;
+}
+
+// Uniform grids, transfers and face weights of the geometric multigrid
+// preconditioner (host/edgemg.cpp), once per mesh; work vectors for up to
+// 16 right-hand sides.  Meshes outside its rule keep emg_ok = false.
+void GpuSolver::build_emg() {
+    std::vector<char> free(L.ne);
+    for (int e = 0; e < L.ne; ++e) free[e] = !(flags_ref[e] & kFlagConstrained);
+    EmgHost H;
+    emg_build(L, free, node_free, iperm, n_pad, P.air_z_threshold, H);
+    if (!H.ok) return;
+    auto up = [&](const auto& v) {
+        auto* p = dupload(v, stream);
+        emg_mem.push_back((void*)p);
+        return p;
+    };
+    auto zeros = [&](size_t n) {
+        float2* p = dalloc_zero<float2>(n, stream);
+        emg_mem.push_back((void*)p);
+        return p;
+    };
+    emg.n_levels = (int)H.lv.size();
+    emg.gap = H.gap;
+    for (int l = 0; l < emg.n_levels; ++l) {
+        const EmgHostLevel& h = H.lv[l];
+        EmgLevel& g = emg.lv[l];
+        g.n = h.n;
+        for (int a = 0; a < 3; ++a) g.h[a] = (float)h.h[a];
+        g.ph = h.planes_h;
+        g.pv = h.planes_v;
+        g.pn = h.planes_n;
+        g.w = up(h.w);
+        const size_t ne = (size_t)emg_edges(h.n), nn = (size_t)(h.n + 1) * (h.n + 1) * (h.n + 1);
+        g.me = dalloc_zero<float>(ne, stream);
+        emg_mem.push_back((void*)g.me);
+        for (float2** q : {&g.b, &g.x, &g.y}) *q = zeros(ne * dev::kMaxRhs);
+        for (float2** q : {&g.nb, &g.ny, &g.nt}) *q = zeros(nn * dev::kMaxRhs);
+    }
+    emg.p_base = up(H.p_base);
+    emg.p_code = up(H.p_code);
+    emg.r_ptr = up(H.r_ptr);
+    emg.r_row = up(H.r_row);
+    emg.r_w = up(H.r_w);
+    emg.n_base = up(H.n_base);
+    emg.n_code = up(H.n_code);
+    emg.nr_ptr = up(H.nr_ptr);
+    emg.nr_node = up(H.nr_node);
+    emg.nr_w = up(H.nr_w);
+    sync();
+    emg_ok = true;
+}
+
+void GpuSolver::free_emg() {
+    if (stream) cudaStreamSynchronize(stream);
+    for (void* p : emg_mem) cudaFree(p);
+    emg_mem.clear();
+    emg = EmgDev{};
+    emg_ok = false;
 }
 
 void GpuSolver::set_sigma(const double* sigma, int n) {
@@ -751,6 +813,7 @@ void GpuSolver::ensure_sigma_device() {
         ++launches;
         lap_built = true;
         if (want_amg()) build_amg();
+        if (emg_ok) emg_set_mass(emg, d_Me, stream, &launches);
     }
 }
 
@@ -843,10 +906,13 @@ void GpuSolver::build_gc() {
     gc_ok = true;
 }
 
-// The gradient-space term on a FP32 batch context; with gradcorr_overlap its
-// V-cycles run on the side stream, overlapping the forward SSOR sweeps.
-void GpuSolver::attach_gc(KrylovCtx<float>& c) {
+// The preconditioner of a FP32 batch context beyond plain SSOR: the
+// geometric multigrid one where the mesh has it, else the gradient-space
+// term.  With gradcorr_overlap the node cycles run on the side stream, beside
+// the edge cycle or the forward SSOR sweeps.
+void GpuSolver::attach_gc(KrylovCtx<float>& c, bool multigrid) {
     c.gc = &gc;
+    c.emg = multigrid && emg_ok ? &emg : nullptr;
     if (P.gradcorr_overlap == 1) {
         c.gc_stream = gc_stream;
         c.gc_fork = gc_fork;
@@ -1397,7 +1463,9 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
     std::vector<int> run = active;
     std::vector<double> prev(K, 1e300), scale(K, 0.0);
     std::vector<BicgState> hs(K);
-    const int chunk = 10;
+    // the multigrid preconditioner; a step that does not reduce the residual
+    // with it is run again with SSOR
+    bool multigrid = emg_ok;
     const int max_steps = 2 + std::max(0, P.max_refinements) * 4;
     auto pow2_at_least = [](int n) { int k = 2; while (k < n) k *= 2; return k; };
     auto launch_grid = [](long n) { return (int)((n + 255) / 256); };
@@ -1424,7 +1492,8 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
                 R.status[k] = kBreakdown;
                 continue;
             }
-            if (rel > 0.9 * prev[k] || R.iters[k] >= maxiter || step == max_steps) {
+            if (rel > 0.9 * prev[k] && multigrid) multigrid = false;
+            else if (rel > 0.9 * prev[k] || R.iters[k] >= maxiter || step == max_steps) {
                 run[k] = 0;
                 if (R.status[k] == kInactive || R.status[k] == kConverged) R.status[k] = kMaxIter;
                 continue;
@@ -1460,6 +1529,9 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
                     const double om = 2.0 * kPi * fz_freqs[fmap[lanes[j]]];
                     use_gc |= om > 0.0 && om <= gc.omega_max;
                 }
+        // iterations between polls of the device's status: a multigrid solve
+        // converges in 10 to 20 iterations, which ten at a time would overrun
+        const int chunk = use_gc && multigrid ? 2 : 10;
         const bool eis = !use_gc && P.ssor_form == 1 && P.row_kernels == kRowsStaged && P.ssor_relax == 1.0;
         // residual replacement needs the untransformed residual of the
         // right-preconditioned form
@@ -1516,7 +1588,7 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
         }
         cuda_ok(cudaMemcpyAsync(d_states, ls.data(), sizeof(BicgState) * Kc, cudaMemcpyHostToDevice, stream), "states");
         KrylovCtx<float> c32 = kctx32(Kc, fm.data());
-        if (use_gc) attach_gc(c32);
+        if (use_gc) attach_gc(c32, multigrid);
         if (eis) eis_init(c32, cur, d_states);
         else bicg_init(c32, cur, d_states);
         int it = 0;
@@ -1599,7 +1671,7 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
                 std::swap(cur_cap, other_cap);
                 Kc = Kn;
                 c32 = kctx32(Kc, fm.data());
-                if (use_gc) attach_gc(c32);
+                if (use_gc) attach_gc(c32, multigrid);
                 chunks_of_shape = 0;
             }
             auto body = [&]() {

@@ -16,6 +16,7 @@
 #include "host/layout.hpp"
 #include "cuda/krylov.cuh"
 #include "cuda/physics.cuh"
+#include "cuda/edgemg.cuh"
 #include "cuda/gradcorr.cuh"
 #include "cuda/regularization.cuh"
 #include "cuda/learned.cuh"
@@ -190,9 +191,22 @@ private:
     bool gc_ok = false;
     std::vector<void*> gc_mem;
     void build_gc();
+    // geometric multigrid preconditioner of the FP32 inner solve
+    EmgDev emg{};
+    bool emg_ok = false;
+    std::vector<void*> emg_mem;
+    std::vector<char> node_free;        // not a Dirichlet node of the divergence correction
+    void build_emg();
+    void free_emg();
+    // the default preconditioner; a setting of the SSOR sweeps or of the
+    // aggregation cycle of the gradient-space term asks for those
+    bool want_emg() const {
+        return P.precision == 1 && P.gradcorr == 1 && P.gradcorr_presmooth == 0 && P.ssor_relax == 1.0 &&
+               P.coop_sweep == 0 && P.sweep_rows == 0;
+    }
     cudaStream_t gc_stream = nullptr;
     cudaEvent_t gc_fork = nullptr, gc_join = nullptr;
-    void attach_gc(KrylovCtx<float>& c);
+    void attach_gc(KrylovCtx<float>& c, bool multigrid = true);
     bool want_amg() const {
         return P.divcorr_precond == 1 || (P.precision == 1 && (P.gradcorr == 1 || P.divcorr_mixed == 1));
     }
