@@ -156,9 +156,12 @@ __device__ bool grid_reduce(const double2 (&acc)[KT][NQ], int rhs0, RedScratch r
 // summed by a fixed set of threads, then in a fixed order).  Deterministic
 // for a fixed launch shape.  Returns true in the last block, where
 // out[q * K + k] (shared, NQ*K entries) holds the totals.
-template <int NQ, int K, int NT = kBlock>
-__device__ bool grid_reduce_lanes(double2 (&acc)[NQ], RedScratch rs, double2* out) {
-    static_assert(K >= 1 && K <= 32 && (K & (K - 1)) == 0, "K must be a power of two <= 32");
+//
+// LPT: neighbouring right-hand sides per thread (lane l works on LPT (l % (K /
+// LPT)) and the next ones), acc[j] for the j-th of them.
+template <int NQ, int K, int NT, int LPT>
+__device__ bool grid_reduce_multi(double2 (&acc)[LPT][NQ], RedScratch rs, double2* out) {
+    static_assert(K >= LPT && K <= 32 && (K & (K - 1)) == 0, "K must be a power of two <= 32");
     static_assert(NT % 32 == 0 && NT >= 32, "block size must be whole warps");
     constexpr int PK = NQ * K;
     constexpr int NW = NT / 32;
@@ -167,12 +170,16 @@ __device__ bool grid_reduce_lanes(double2 (&acc)[NQ], RedScratch rs, double2* ou
     __shared__ bool am_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int off = 16; off >= K; off >>= 1)
+    for (int off = 16; off >= K / LPT; off >>= 1)
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) acc[q] = cadd(acc[q], shfl_xor(acc[q], off));
-    if (lane < K)
+        for (int j = 0; j < LPT; ++j)
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) sm[warp][q * K + lane] = acc[q];
+            for (int q = 0; q < NQ; ++q) acc[j][q] = cadd(acc[j][q], shfl_xor(acc[j][q], off));
+    if (lane < K / LPT)
+#pragma unroll
+        for (int j = 0; j < LPT; ++j)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) sm[warp][q * K + lane * LPT + j] = acc[j][q];
     __syncthreads();
     if (threadIdx.x < PK) {
         double2 s = make_double2(0.0, 0.0);
@@ -190,13 +197,24 @@ __device__ bool grid_reduce_lanes(double2 (&acc)[NQ], RedScratch rs, double2* ou
     __threadfence();
     constexpr int CH = NT / PK > 0 ? NT / PK : 1;   // threads per total
     const int p = threadIdx.x % PK, j = threadIdx.x / PK;
+    // eight loads in flight: one at a time, the last block's walk over the
+    // partials was 10 us of every reducing kernel
     double2 s = make_double2(0.0, 0.0);
     if (j < CH)
-        for (int b = j; b < (int)gridDim.x; b += CH) s = cadd(s, __ldcg(&rs.partial[(size_t)b * PK + p]));
+        for (int b = j; b < (int)gridDim.x; b += 8 * CH) {
+            double2 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                v[u] = b + u * CH < (int)gridDim.x ? __ldcg(&rs.partial[(size_t)(b + u * CH) * PK + p])
+                                                   : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s = cadd(s, v[u]);
+        }
     chunk[threadIdx.x] = s;
     __syncthreads();
     if (threadIdx.x < PK) {
         double2 t = make_double2(0.0, 0.0);
+#pragma unroll 8
         for (int jj = 0; jj < CH; ++jj) t = cadd(t, chunk[jj * PK + threadIdx.x]);
         out[threadIdx.x] = t;
         rs.final_[threadIdx.x] = t;
@@ -204,6 +222,21 @@ __device__ bool grid_reduce_lanes(double2 (&acc)[NQ], RedScratch rs, double2* ou
     if (threadIdx.x == 0) *rs.counter = 0u;
     __syncthreads();
     return true;
+}
+
+// Blocks of a reducing vector kernel over n elements: one resident wave at
+// most, and at least four elements a thread -- on small vectors the walk over
+// more partials costs more than the extra blocks save.
+template <class F>
+inline int reduce_grid(F* kernel, int cap, long n) {
+    const long b = (n + 4 * kBlock - 1) / (4 * kBlock);
+    const int w = wave_grid(kernel, cap);
+    return (int)(b < 1 ? 1 : b < w ? b : w);
+}
+
+template <int NQ, int K, int NT = kBlock>
+__device__ __forceinline__ bool grid_reduce_lanes(double2 (&acc)[NQ], RedScratch rs, double2* out) {
+    return grid_reduce_multi<NQ, K, NT, 1>(*reinterpret_cast<double2(*)[1][NQ]>(&acc), rs, out);
 }
 
 }  // namespace dev

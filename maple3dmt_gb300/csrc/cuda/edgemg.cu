@@ -12,6 +12,8 @@ using namespace dev;
 namespace {
 
 constexpr int kNT = 256;
+constexpr int kLongRow = 24;    // transfer rows longer than this (two levels of refinement) are summed by a block
+constexpr int kLongNT = 128;
 
 template <int D> using Dir = std::integral_constant<int, D>;   // direction tag
 
@@ -226,6 +228,7 @@ __global__ void __launch_bounds__(kNT) k_restrict0(EmgDev g, Omegas om, const fl
         float4 s = vz<float4>(), x = vz<float4>();
         if (edge_free<D>(L, i, j, k)) {
             const int q0 = __ldg(&g.r_ptr[c]), q1 = __ldg(&g.r_ptr[c + 1]);
+            if (q1 - q0 > kLongRow) return;   // k_restrict0_long
             for (int q = q0; q < q1; q += 4) {
                 float w[4];
                 float4 v[4];
@@ -243,6 +246,42 @@ __global__ void __launch_bounds__(kNT) k_restrict0(EmgDev g, Omegas om, const fl
         f4(L.b)[(size_t)c * H + h] = s;
         f4(L.x)[(size_t)c * H + h] = x;
     });
+}
+
+// Sum of w_q v[idx_q] over one long transfer row by a block of kLongNT threads
+// (lanes H, the entries dealt out to the rest); the total on the first H.
+template <int H>
+__device__ __forceinline__ float4 long_row(const int* __restrict__ idx, const float* __restrict__ w, int q0, int q1,
+                                           const float4* __restrict__ v) {
+    constexpr int G = kLongNT / H;
+    __shared__ float4 part[kLongNT];
+    const int h = threadIdx.x % H, g = threadIdx.x / H;
+    float4 s = vz<float4>();
+    for (int q = q0 + g; q < q1; q += G) s = s + __ldg(&w[q]) * v[(size_t)__ldg(&idx[q]) * H + h];
+    part[threadIdx.x] = s;
+    __syncthreads();
+    for (int o = G / 2; o > 0; o >>= 1) {
+        if (g < o) part[threadIdx.x] = part[threadIdx.x] + part[threadIdx.x + o * H];
+        __syncthreads();
+    }
+    return part[threadIdx.x];
+}
+
+// The rows of P^T with more than kLongRow entries: coarse edges inside a
+// refinement of two or three levels collect up to 196 or 1800 octree edges,
+// which one thread after another made 50 us on the 157 k-edge mesh.
+template <int K>
+__global__ void __launch_bounds__(kLongNT) k_restrict0_long(EmgDev g, Omegas om, const float4* __restrict__ r) {
+    constexpr int H = K / 2;
+    const EmgLevel& L = g.lv[0];
+    const int c = g.r_long[blockIdx.x], n = L.n, h = threadIdx.x % H;
+    const float4 s = long_row<H>(g.r_row, g.r_w, g.r_ptr[c], g.r_ptr[c + 1], r);
+    if (threadIdx.x >= H) return;
+    const int per = n * (n + 1) * (n + 1), D = c / per, q = c % per;
+    const int nx = D == 0 ? n : n + 1, ny = D == 1 ? n : n + 1, i = q % nx, j = q / nx % ny, k = q / (nx * ny);
+    const float S = D == 0 ? edge_diag<0>(L, i, j, k) : D == 1 ? edge_diag<1>(L, i, j, k) : edge_diag<2>(L, i, j, k);
+    f4(L.b)[(size_t)c * H + h] = s;
+    f4(L.x)[(size_t)c * H + h] = idiag(om_of(om, h, (float4*)nullptr), kEmgEdge, S, __ldg(&L.me[c]), s);
 }
 
 // y = b - A x
@@ -336,104 +375,174 @@ __global__ void __launch_bounds__(kNT) k_smooth(EmgLevel L, Omegas om) {
 // The grids of at most kEmgBottom cells per side: one block per right-hand
 // side runs their whole cycle, vectors in shared memory (a launch per step
 // would cost more than the steps: 2 k edges).  Reads b and x of the first such
-// level, or restricts them itself from the finer level's y; writes its y.
-constexpr int kBottomNT = 512;
-constexpr int kBottomEdges = 3 * kEmgBottom * (kEmgBottom + 1) * (kEmgBottom + 1);
+// level, writes its y.  The coarsest grid's Jacobi steps keep each edge's
+// stencil in registers: twelve weights and positions, one edge per thread.
+constexpr int kBottomNT = 1024;
 constexpr int kCoarsestSteps = 12;
 
-template <class F> __device__ __forceinline__ void each_bottom(const EmgLevel& L, const F& f) {
+template <class F> __device__ __forceinline__ void with_edge(const EmgLevel& L, int t, const F& f) {
     const int n = L.n, per = n * (n + 1) * (n + 1);
-    for (int t = threadIdx.x; t < 3 * per; t += kBottomNT) {
-        if (t < per) {
-            const int i = t % n, j = t / n % (n + 1), k = t / (n * (n + 1));
-            if (edge_free<0>(L, i, j, k)) f(Dir<0>{}, i, j, k, t);
-        } else if (t < 2 * per) {
-            const int q = t - per, i = q % (n + 1), j = q / (n + 1) % n, k = q / (n * (n + 1));
-            if (edge_free<1>(L, i, j, k)) f(Dir<1>{}, i, j, k, t);
-        } else {
-            const int q = t - 2 * per, i = q % (n + 1), j = q / (n + 1) % (n + 1), k = q / ((n + 1) * (n + 1));
-            if (edge_free<2>(L, i, j, k)) f(Dir<2>{}, i, j, k, t);
-        }
+    if (t < per) {
+        const int i = t % n, j = t / n % (n + 1), k = t / (n * (n + 1));
+        if (edge_free<0>(L, i, j, k)) f(Dir<0>{}, i, j, k);
+    } else if (t < 2 * per) {
+        const int q = t - per, i = q % (n + 1), j = q / (n + 1) % n, k = q / (n * (n + 1));
+        if (edge_free<1>(L, i, j, k)) f(Dir<1>{}, i, j, k);
+    } else if (t < 3 * per) {
+        const int q = t - 2 * per, i = q % (n + 1), j = q / (n + 1) % (n + 1), k = q / ((n + 1) * (n + 1));
+        if (edge_free<2>(L, i, j, k)) f(Dir<2>{}, i, j, k);
     }
+}
+
+// positions and weights of the twelve neighbours of an edge, as curl_row sums them
+template <int D>
+__device__ __forceinline__ void curl_stencil(const EmgLevel& L, int i, int j, int k, int (&at)[12], float (&w)[12],
+                                             float& S) {
+    const int n = L.n;
+    S = 0.0f;
+    auto dir = [&](auto tag, int o) {
+        constexpr int A = decltype(tag)::value, B = 3 - D - A;
+        constexpr int ai = A == 0, aj = A == 1, ak = A == 2, di = D == 0, dj = D == 1, dk = D == 2;
+        const float hd = L.h[D], ha = L.h[A];
+        const float wp = __ldg(&L.w[fid<B>(n, i, j, k)]), wm = __ldg(&L.w[fid<B>(n, i - ai, j - aj, k - ak)]);
+        at[o] = eid<D>(n, i + ai, j + aj, k + ak);
+        at[o + 1] = eid<D>(n, i - ai, j - aj, k - ak);
+        at[o + 2] = eid<A>(n, i + di, j + dj, k + dk);
+        at[o + 3] = eid<A>(n, i, j, k);
+        at[o + 4] = eid<A>(n, i - ai + di, j - aj + dj, k - ak + dk);
+        at[o + 5] = eid<A>(n, i - ai, j - aj, k - ak);
+        w[o] = -hd * hd * wp;
+        w[o + 1] = -hd * hd * wm;
+        w[o + 2] = hd * ha * wp;
+        w[o + 3] = -hd * ha * wp;
+        w[o + 4] = -hd * ha * wm;
+        w[o + 5] = hd * ha * wm;
+        S += hd * hd * (wp + wm);
+    };
+    dir(Dir<D == 0 ? 1 : 0>{}, 0);
+    dir(Dir<D == 2 ? 1 : 2>{}, 6);
 }
 
 __global__ void __launch_bounds__(kBottomNT) k_bottom(EmgDev g, int l0, int K, Omegas oms) {
     extern __shared__ float2 sm[];
-    const int lane = blockIdx.x;
+    const int lane = blockIdx.x, tid = threadIdx.x;
     const Om<float2> om{oms.v[lane]};
     const int nl = g.n_levels;
-    // two vectors (x and a second one) and the right-hand side per level
-    float2* vec[2][3];
-    {
-        float2* p = sm;
-        for (int l = l0; l < nl; ++l) {
-            const int ne = 3 * g.lv[l].n * (g.lv[l].n + 1) * (g.lv[l].n + 1);
-            for (int q = 0; q < 3; ++q) { vec[l - l0][q] = p; p += ne; }
-        }
-        for (float2* z = sm + threadIdx.x; z < p; z += kBottomNT) *z = make_float2(0.f, 0.f);
-    }
-    __syncthreads();
-    {
-        const EmgLevel& L = g.lv[l0];
-        float2 *b = vec[0][0], *x = vec[0][1];
-        each_bottom(L, [&](auto, int, int, int, int e) {
-            b[e] = L.b[(size_t)e * K + lane];
-            x[e] = L.x[(size_t)e * K + lane];
-        });
-        __syncthreads();
-    }
-    auto step = [&](const EmgLevel& L, const float2* b, const float2* x, float2* out, bool resid) {
-        each_bottom(L, [&](auto tag, int i, int j, int k, int e) {
-            constexpr int D = decltype(tag)::value;
-            const float m = __ldg(&L.me[e]);
-            float S;
-            const float2 ax = curl_row<D, float2>(L, i, j, k, x[e], [&](int q) { return x[q]; }, S);
-            const float2 r = b[e] - ax - imass(om, m, x[e]);
-            out[e] = resid ? r : x[e] + idiag(om, kEmgEdge, S, m, r);
-        });
-        __syncthreads();
-    };
     const bool two = l0 + 1 < nl;
     const EmgLevel& L = g.lv[l0];
     const EmgLevel& C = g.lv[nl - 1];
+    const int nL = 3 * L.n * (L.n + 1) * (L.n + 1), nC = 3 * C.n * (C.n + 1) * (C.n + 1);
+    // b, x and a third vector per level (the levels' own b, x: zero on edges that are not free)
+    float2 *b = sm, *x = sm + nL, *y = sm + 2 * nL;
+    float2 *cb = two ? sm + 3 * nL : b, *cx = two ? cb + nC : x, *cy = two ? cx + nC : y;
+    for (int e = tid; e < nL; e += kBottomNT) {
+        b[e] = L.b[(size_t)e * K + lane];
+        x[e] = L.x[(size_t)e * K + lane];
+        y[e] = make_float2(0.f, 0.f);
+    }
+    if (two)
+        for (int e = tid; e < nC; e += kBottomNT) cx[e] = cy[e] = make_float2(0.f, 0.f);
+    // the coarsest grid's stencil (at most 300 edges, one per thread)
+    int at[12];
+    float w[12], S = 0.0f, m = 0.0f;
+    bool mine = false;
+    with_edge(C, tid, [&](auto tag, int i, int j, int k) {
+        curl_stencil<decltype(tag)::value>(C, i, j, k, at, w, S);
+        m = __ldg(&C.me[tid]);
+        mine = true;
+    });
+    __syncthreads();
+    auto step = [&](const float2* in, float2* out, bool resid) {
+        for (int e = tid; e < nL; e += kBottomNT)
+            with_edge(L, e, [&](auto tag, int i, int j, int k) {
+                const float me = __ldg(&L.me[e]);
+                float d;
+                const float2 ax = curl_row<decltype(tag)::value, float2>(L, i, j, k, in[e],
+                                                                         [&](int q) { return in[q]; }, d);
+                const float2 r = b[e] - ax - imass(om, me, in[e]);
+                out[e] = resid ? r : in[e] + idiag(om, kEmgEdge, d, me, r);
+            });
+        __syncthreads();
+    };
     if (two) {
-        step(L, vec[0][0], vec[0][1], vec[0][2], true);
-        float2 *b = vec[1][0], *x = vec[1][1];
-        each_bottom(C, [&](auto tag, int i, int j, int k, int e) {
-            constexpr int D = decltype(tag)::value;
-            const float2 s = gather_edge<D, float2>(L.n, i, j, k, [&](int q) { return vec[0][2][q]; });
-            b[e] = s;
-            x[e] = idiag(om, kEmgEdge, edge_diag<D>(C, i, j, k), __ldg(&C.me[e]), s);
-        });
+        step(x, y, true);
+        if (mine)
+            with_edge(C, tid, [&](auto tag, int i, int j, int k) {
+                const float2 s = gather_edge<decltype(tag)::value, float2>(L.n, i, j, k, [&](int q) { return y[q]; });
+                cb[tid] = s;
+                cx[tid] = idiag(om, kEmgEdge, S, m, s);
+            });
         __syncthreads();
     }
-    // coarsest grid: Jacobi steps
-    const int c = two ? 1 : 0;
-    for (int q = 0; q < kCoarsestSteps; q += 2) {
-        step(C, vec[c][0], vec[c][1], vec[c][2], false);
-        step(C, vec[c][0], vec[c][2], vec[c][1], false);
-    }
-    float2* y = vec[c][1];
-    if (two) {
-        float2* x = vec[0][1];
-        each_bottom(L, [&](auto tag, int i, int j, int k, int e) {
-            constexpr int D = decltype(tag)::value;
-            x[e] = x[e] + interp_edge<D, float2>(C.n, i, j, k, [&](int q) { return vec[1][1][q]; });
-        });
+    const float2 bb = mine ? cb[tid] : make_float2(0.f, 0.f);
+    for (int q = 0; q < kCoarsestSteps; ++q) {
+        const float2* in = q & 1 ? cy : cx;
+        if (mine) {
+            const float2 xc = in[tid];
+            float2 ax = S * xc;
+#pragma unroll
+            for (int u = 0; u < 12; ++u) ax = ax + w[u] * in[at[u]];
+            (q & 1 ? cx : cy)[tid] = xc + idiag(om, kEmgEdge, S, m, bb - ax - imass(om, m, xc));
+        }
         __syncthreads();
-        step(L, vec[0][0], x, vec[0][2], false);
-        y = vec[0][2];
+    }
+    const float2* out = cx;
+    if (two) {
+        for (int e = tid; e < nL; e += kBottomNT)
+            with_edge(L, e, [&](auto tag, int i, int j, int k) {
+                x[e] = x[e] + interp_edge<decltype(tag)::value, float2>(C.n, i, j, k, [&](int q) { return cx[q]; });
+            });
+        __syncthreads();
+        // y holds the residual on free edges only, which the step overwrites
+        step(x, y, false);
+        out = y;
     }
     // every edge: the finer level's interpolation reads the zeros too
-    for (int e = threadIdx.x; e < 3 * L.n * (L.n + 1) * (L.n + 1); e += kBottomNT) L.y[(size_t)e * K + lane] = y[e];
+    for (int e = tid; e < nL; e += kBottomNT) L.y[(size_t)e * K + lane] = out[e];
 }
 
 // ---------------------------------------------------------------------------
-// node cycle (V(0,1))
+// node cycle: V(0,1) in the edge preconditioner, the symmetric V(1,1) (PRE) in
+// the divergence correction's PCG
 // ---------------------------------------------------------------------------
 
-// nb0 = Pn^T b from the octree nodes
-template <int K>
+// Laplacian row on a uniform grid: six edges, coarse edge masses over h^2
+template <class V, class At>
+__device__ __forceinline__ V lap_row(const EmgLevel& L, int i, int j, int k, V xc, const At& at, float& d) {
+    const int n = L.n;
+    V s = vz<V>();
+    d = 0.0f;
+    auto put = [&](int e, int v, float ih2) {
+        const float m = __ldg(&L.me[e]) * ih2;
+        s = s + m * (xc - at(v));
+        d += m;
+    };
+    const float a = 1.0f / (L.h[0] * L.h[0]), b = 1.0f / (L.h[1] * L.h[1]), c = 1.0f / (L.h[2] * L.h[2]);
+    put(eid<0>(n, i - 1, j, k), nid(n, i - 1, j, k), a);
+    put(eid<0>(n, i, j, k), nid(n, i + 1, j, k), a);
+    put(eid<1>(n, i, j - 1, k), nid(n, i, j - 1, k), b);
+    put(eid<1>(n, i, j, k), nid(n, i, j + 1, k), b);
+    put(eid<2>(n, i, j, k - 1), nid(n, i, j, k - 1), c);
+    put(eid<2>(n, i, j, k), nid(n, i, j, k + 1), c);
+    return s;
+}
+
+// diagonal of the node Laplacian on a uniform grid
+__device__ __forceinline__ float lap_diag(const EmgLevel& L, int i, int j, int k) {
+    const int n = L.n;
+    return (__ldg(&L.me[eid<0>(n, i - 1, j, k)]) + __ldg(&L.me[eid<0>(n, i, j, k)])) / (L.h[0] * L.h[0]) +
+           (__ldg(&L.me[eid<1>(n, i, j - 1, k)]) + __ldg(&L.me[eid<1>(n, i, j, k)])) / (L.h[1] * L.h[1]) +
+           (__ldg(&L.me[eid<2>(n, i, j, k - 1)]) + __ldg(&L.me[eid<2>(n, i, j, k)])) / (L.h[2] * L.h[2]);
+}
+
+// w b / diag, the pre-smoothed iterate of the V(1,1) cycle
+template <class V> __device__ __forceinline__ V node_pre(const EmgLevel& L, int i, int j, int k, V b) {
+    const float d = node_free(L, i, j, k) ? lap_diag(L, i, j, k) : 0.0f;
+    return d > 0.0f ? (kEmgNode / d) * b : vz<V>();
+}
+
+// nb0 = Pn^T b from the octree nodes; PRE: nt0 = w nb0 / diag
+template <int K, bool PRE>
 __global__ void __launch_bounds__(kNT) k_node_restrict0(EmgDev g, const float4* __restrict__ b) {
     constexpr int H = K / 2;
     const EmgLevel& L = g.lv[0];
@@ -441,6 +550,7 @@ __global__ void __launch_bounds__(kNT) k_node_restrict0(EmgDev g, const float4* 
         const int c = nid(L.n, i, j, k);
         float4 s = vz<float4>();
         const int q0 = __ldg(&g.nr_ptr[c]), q1 = __ldg(&g.nr_ptr[c + 1]);
+        if (q1 - q0 > kLongRow) return;   // k_node_restrict0_long
         for (int q = q0; q < q1; q += 4) {
             float w[4];
             float4 v[4];
@@ -454,8 +564,37 @@ __global__ void __launch_bounds__(kNT) k_node_restrict0(EmgDev g, const float4* 
             for (int u = 0; u < 4; ++u) s = s + w[u] * v[u];
         }
         f4(L.nb)[(size_t)c * H + h] = s;
+        if (PRE) f4(L.nt)[(size_t)c * H + h] = node_pre(L, i, j, k, s);
     });
 }
+
+template <int K, bool PRE>
+__global__ void __launch_bounds__(kLongNT) k_node_restrict0_long(EmgDev g, const float4* __restrict__ b) {
+    constexpr int H = K / 2;
+    const EmgLevel& L = g.lv[0];
+    const int c = g.nr_long[blockIdx.x], n1 = L.n + 1, h = threadIdx.x % H;
+    const float4 s = long_row<H>(g.nr_node, g.nr_w, g.nr_ptr[c], g.nr_ptr[c + 1], b);
+    if (threadIdx.x >= H) return;
+    f4(L.nb)[(size_t)c * H + h] = s;
+    if (PRE) f4(L.nt)[(size_t)c * H + h] = node_pre(L, c % n1, c / n1 % n1, c / (n1 * n1), s);
+}
+
+// ny = nb - L nt
+template <int K>
+__global__ void __launch_bounds__(kNT) k_node_resid(EmgLevel L) {
+    constexpr int H = K / 2;
+    each_node<H>(L, [&](int i, int j, int k, int h) {
+        const size_t c = (size_t)nid(L.n, i, j, k) * H + h;
+        float4 v = vz<float4>();
+        if (node_free(L, i, j, k)) {
+            const float4* t = f4(L.nt);
+            float d;
+            v = f4(L.nb)[c] - lap_row<float4>(L, i, j, k, t[c], [&](int q) { return t[(size_t)q * H + h]; }, d);
+        }
+        f4(L.ny)[c] = v;
+    });
+}
+
 
 template <class V, class At>
 __device__ __forceinline__ V gather_node(int n, int I, int J, int Kk, const At& at) {
@@ -480,20 +619,24 @@ __device__ __forceinline__ V interp_node(int n, int i, int j, int k, const At& a
     return ((oi ? 0.5f : 1.0f) * (oj ? 0.5f : 1.0f) * (ok ? 0.5f : 1.0f)) * s;
 }
 
-template <int K>
+// nb = Pn^T of the finer level's right-hand side, or (PRE) of its residual in
+// ny, with nt = w nb / diag
+template <int K, bool PRE>
 __global__ void __launch_bounds__(kNT) k_node_restrict(EmgLevel F, EmgLevel L) {
     constexpr int H = K / 2;
     each_node<H>(L, [&](int i, int j, int k, int h) {
         float4 s = vz<float4>();
-        const float4* b = f4(F.nb);
+        const float4* b = f4(PRE ? F.ny : F.nb);
         if (node_free(L, i, j, k))
             s = gather_node<float4>(F.n, i, j, k, [&](int v) { return b[(size_t)v * H + h]; });
-        f4(L.nb)[(size_t)nid(L.n, i, j, k) * H + h] = s;
+        const size_t c = (size_t)nid(L.n, i, j, k) * H + h;
+        f4(L.nb)[c] = s;
+        if (PRE) f4(L.nt)[c] = node_pre(L, i, j, k, s);
     });
 }
 
-// t = Pn y_coarse
-template <int K>
+// nt = Pn y_coarse, or (PRE) nt += Pn y_coarse
+template <int K, bool PRE>
 __global__ void __launch_bounds__(kNT) k_node_prolong(EmgLevel L, EmgLevel C) {
     constexpr int H = K / 2;
     each_node<H>(L, [&](int i, int j, int k, int h) {
@@ -501,29 +644,9 @@ __global__ void __launch_bounds__(kNT) k_node_prolong(EmgLevel L, EmgLevel C) {
         const float4* y = f4(C.ny);
         if (node_free(L, i, j, k))
             s = interp_node<float4>(C.n, i, j, k, [&](int v) { return y[(size_t)v * H + h]; });
-        f4(L.nt)[(size_t)nid(L.n, i, j, k) * H + h] = s;
+        const size_t c = (size_t)nid(L.n, i, j, k) * H + h;
+        f4(L.nt)[c] = PRE ? f4(L.nt)[c] + s : s;
     });
-}
-
-// Laplacian row on a uniform grid: six edges, coarse edge masses over h^2
-template <class V, class At>
-__device__ __forceinline__ V lap_row(const EmgLevel& L, int i, int j, int k, V xc, const At& at, float& d) {
-    const int n = L.n;
-    V s = vz<V>();
-    d = 0.0f;
-    auto put = [&](int e, int v, float ih2) {
-        const float m = __ldg(&L.me[e]) * ih2;
-        s = s + m * (xc - at(v));
-        d += m;
-    };
-    const float a = 1.0f / (L.h[0] * L.h[0]), b = 1.0f / (L.h[1] * L.h[1]), c = 1.0f / (L.h[2] * L.h[2]);
-    put(eid<0>(n, i - 1, j, k), nid(n, i - 1, j, k), a);
-    put(eid<0>(n, i, j, k), nid(n, i + 1, j, k), a);
-    put(eid<1>(n, i, j - 1, k), nid(n, i, j - 1, k), b);
-    put(eid<1>(n, i, j, k), nid(n, i, j + 1, k), b);
-    put(eid<2>(n, i, j, k - 1), nid(n, i, j, k - 1), c);
-    put(eid<2>(n, i, j, k), nid(n, i, j, k + 1), c);
-    return s;
 }
 
 // ny = t + w (nb - L t) / diag
@@ -544,61 +667,75 @@ __global__ void __launch_bounds__(kNT) k_node_smooth(EmgLevel L) {
     });
 }
 
+template <bool PRE>
 __global__ void __launch_bounds__(kBottomNT) k_node_bottom(EmgDev g, int l0, int K) {
     constexpr int kN = (kEmgBottom + 1) * (kEmgBottom + 1) * (kEmgBottom + 1);
-    __shared__ float2 vec[2][3][kN];
-    const int lane = blockIdx.x, nl = g.n_levels;
-    for (int t = threadIdx.x; t < 2 * 3 * kN; t += kBottomNT) (&vec[0][0][0])[t] = make_float2(0.f, 0.f);
-    __syncthreads();
-    auto each = [&](const EmgLevel& L, const auto& f) {
-        const int n1 = L.n + 1;
-        for (int t = threadIdx.x; t < n1 * n1 * n1; t += kBottomNT) {
-            const int i = t % n1, j = t / n1 % n1, k = t / (n1 * n1);
-            if (node_free(L, i, j, k)) f(i, j, k, t);
-        }
-        __syncthreads();
-    };
+    constexpr int kNc = 5 * 5 * 5;
+    static_assert(kN <= kBottomNT, "one node per thread");
+    __shared__ float2 b[kN], x[kN], y[kN], cb[kNc], cx[kNc], cy[kNc];
+    const int lane = blockIdx.x, tid = threadIdx.x, nl = g.n_levels;
     const bool two = l0 + 1 < nl;
     const EmgLevel& L = g.lv[l0];
     const EmgLevel& C = g.lv[nl - 1];
-    const int c = two ? 1 : 0;
-    each(L, [&](int, int, int, int t) { vec[0][0][t] = L.nb[(size_t)t * K + lane]; });
-    if (two)
-        each(C, [&](int i, int j, int k, int t) {
-            vec[1][0][t] = gather_node<float2>(L.n, i, j, k, [&](int q) { return vec[0][0][q]; });
-        });
-    auto smooth = [&](const EmgLevel& M, const float2* b, const float2* x, float2* out) {
-        each(M, [&](int i, int j, int k, int t) {
-            float d;
-            const float2 lx = lap_row<float2>(M, i, j, k, x[t], [&](int q) { return x[q]; }, d);
-            out[t] = d > 0.0f ? x[t] + (kEmgNode / d) * (b[t] - lx) : x[t];
-        });
+    const int nL = (L.n + 1) * (L.n + 1) * (L.n + 1);
+    const int i = tid % (L.n + 1), j = tid / (L.n + 1) % (L.n + 1), k = tid / ((L.n + 1) * (L.n + 1));
+    const int ci = tid % 5, cj = tid / 5 % 5, ck = tid / 25;   // two: the coarsest grid has 4 cells per side
+    const bool in = tid < nL && node_free(L, i, j, k);
+    const bool cin = two && tid < kNc && node_free(C, ci, cj, ck);
+    if (tid < nL) {
+        b[tid] = in ? L.nb[(size_t)tid * K + lane] : make_float2(0.f, 0.f);
+        x[tid] = y[tid] = make_float2(0.f, 0.f);
+    }
+    if (tid < kNc) cb[tid] = cx[tid] = cy[tid] = make_float2(0.f, 0.f);
+    __syncthreads();
+    auto jacobi = [&](const EmgLevel& M, bool on, int a, int c, int d, const float2* rhs, const float2* v, float2* out) {
+        if (on) {
+            float dg;
+            const float2 lv = lap_row<float2>(M, a, c, d, v[tid], [&](int q) { return v[q]; }, dg);
+            out[tid] = dg > 0.0f ? v[tid] + (kEmgNode / dg) * (rhs[tid] - lv) : v[tid];
+        }
+        __syncthreads();
     };
-    for (int q = 0; q < kCoarsestSteps; q += 2) {   // from zero
-        smooth(C, vec[c][0], vec[c][1], vec[c][2]);
-        smooth(C, vec[c][0], vec[c][2], vec[c][1]);
+    const float2* rc = b;   // what the coarsest grid gets
+    if (two && PRE) {
+        if (in) x[tid] = node_pre(L, i, j, k, b[tid]);
+        __syncthreads();
+        if (in) {
+            float dg;
+            y[tid] = b[tid] - lap_row<float2>(L, i, j, k, x[tid], [&](int q) { return x[q]; }, dg);
+        }
+        __syncthreads();
+        rc = y;
     }
-    const float2* y = vec[c][1];
     if (two) {
-        each(L, [&](int i, int j, int k, int t) {
-            vec[0][1][t] = interp_node<float2>(C.n, i, j, k, [&](int q) { return vec[1][1][q]; });
-        });
-        smooth(L, vec[0][0], vec[0][1], vec[0][2]);
-        y = vec[0][2];
+        if (cin) cb[tid] = gather_node<float2>(L.n, ci, cj, ck, [&](int q) { return rc[q]; });
+        __syncthreads();
+        for (int q = 0; q < kCoarsestSteps; q += 2) {   // from zero
+            jacobi(C, cin, ci, cj, ck, cb, cx, cy);
+            jacobi(C, cin, ci, cj, ck, cb, cy, cx);
+        }
+        if (in) x[tid] = x[tid] + interp_node<float2>(C.n, i, j, k, [&](int q) { return cx[q]; });
+        __syncthreads();
+        jacobi(L, in, i, j, k, b, x, y);
+    } else {
+        for (int q = 0; q < kCoarsestSteps; q += 2) {
+            jacobi(L, in, i, j, k, b, x, y);
+            jacobi(L, in, i, j, k, b, y, x);
+        }
     }
-    const int nn = (L.n + 1) * (L.n + 1) * (L.n + 1);
-    for (int t = threadIdx.x; t < nn; t += kBottomNT) L.ny[(size_t)t * K + lane] = y[t];
+    if (tid < nL) L.ny[(size_t)tid * K + lane] = two ? y[tid] : x[tid];
 }
 
-// t = Pn ny0 on the octree nodes (0 on Dirichlet nodes)
+// t = Pn ny0 on the octree nodes (0 on Dirichlet nodes), plus x if given
 template <int K>
-__global__ void __launch_bounds__(kNT) k_node_prolong0(EmgDev g, int nn, float4* __restrict__ out) {
+__global__ void __launch_bounds__(kNT) k_node_prolong0(EmgDev g, int nn, const float4* __restrict__ x,
+                                                       float4* __restrict__ out) {
     constexpr int H = K / 2;
     const long i = (long)blockIdx.x * kNT + threadIdx.x;
     if (i >= (long)nn * H) return;
     const int v = (int)(i / H), h = (int)(i % H);
     const int base = __ldg(&g.n_base[v]);
-    float4 s = vz<float4>();
+    float4 s = x ? x[i] : vz<float4>();
     if (base >= 0) {
         const unsigned code = __ldg(&g.n_code[v]);
         const float u = 1.0f / (float)(1 << g.gap);
@@ -671,6 +808,10 @@ void edge_cycle(const EmgDev& g, const Omegas& om, const float2* r, cudaStream_t
     const int l0 = bottom_level(g);
     k_restrict0<K><<<edge_grid<K>(g.lv[0]), kNT, 0, s>>>(g, om, f4(r));
     ck(launches);
+    if (g.n_r_long) {
+        k_restrict0_long<K><<<g.n_r_long, kLongNT, 0, s>>>(g, om, f4(r));
+        ck(launches);
+    }
     for (int l = 0; l < l0; ++l) {
         k_resid<K><<<edge_grid<K>(g.lv[l]), kNT, 0, s>>>(g.lv[l], om);
         ck(launches);
@@ -689,30 +830,51 @@ void edge_cycle(const EmgDev& g, const Omegas& om, const float2* r, cudaStream_t
     }
 }
 
-template <int K>
-void node_cycle(const EmgDev& g, const GcDev& gc, const float2* r, cudaStream_t s, long long* launches) {
+// the uniform grids' part of a node cycle, from octree node vector b to ny of level 0
+template <int K, bool PRE>
+void node_grids(const EmgDev& g, const float2* b, cudaStream_t s, long long* launches) {
     const int l0 = bottom_level(g);
-    gc_restrict_edges_k<K>(gc, r, s, launches);
-    k_node_restrict0<K><<<node_grid<K>(g.lv[0]), kNT, 0, s>>>(g, f4(gc.lv[0].b));
+    k_node_restrict0<K, PRE><<<node_grid<K>(g.lv[0]), kNT, 0, s>>>(g, f4(b));
     ck(launches);
-    for (int l = 0; l < l0; ++l) {
-        k_node_restrict<K><<<node_grid<K>(g.lv[l + 1]), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
+    if (g.n_nr_long) {
+        k_node_restrict0_long<K, PRE><<<g.n_nr_long, kLongNT, 0, s>>>(g, f4(b));
         ck(launches);
     }
-    k_node_bottom<<<K, kBottomNT, 0, s>>>(g, l0, K);
+    for (int l = 0; l < l0; ++l) {
+        if (PRE) {
+            k_node_resid<K><<<node_grid<K>(g.lv[l]), kNT, 0, s>>>(g.lv[l]);
+            ck(launches);
+        }
+        k_node_restrict<K, PRE><<<node_grid<K>(g.lv[l + 1]), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
+        ck(launches);
+    }
+    k_node_bottom<PRE><<<K, kBottomNT, 0, s>>>(g, l0, K);
     ck(launches);
     for (int l = l0 - 1; l >= 0; --l) {
-        k_node_prolong<K><<<node_grid<K>(g.lv[l]), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
+        k_node_prolong<K, PRE><<<node_grid<K>(g.lv[l]), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
         ck(launches);
         k_node_smooth<K><<<node_grid<K>(g.lv[l]), kNT, 0, s>>>(g.lv[l]);
         ck(launches);
     }
-    k_node_prolong0<K><<<grid1((long)gc.nn * (K / 2)), kNT, 0, s>>>(g, gc.nn, f4(gc.lv[0].y));
+}
+
+template <int K>
+void node_cycle(const EmgDev& g, const GcDev& gc, const float2* r, cudaStream_t s, long long* launches) {
+    gc_restrict_edges_k<K>(gc, r, s, launches);
+    node_grids<K, false>(g, gc.lv[0].b, s, launches);
+    k_node_prolong0<K><<<grid1((long)gc.nn * (K / 2)), kNT, 0, s>>>(g, gc.nn, nullptr, f4(gc.lv[0].y));
     ck(launches);
     gc_smooth0_k<K>(gc, gc.lv[0].y, gc.out0, s, launches);
 }
 
 }  // namespace
+
+std::vector<int> emg_long_rows(const std::vector<int>& ptr) {
+    std::vector<int> rows;
+    for (size_t c = 0; c + 1 < ptr.size(); ++c)
+        if (ptr[c + 1] - ptr[c] > kLongRow) rows.push_back((int)c);
+    return rows;
+}
 
 void emg_set_mass(const EmgDev& g, const double* Me, cudaStream_t s, long long* launches) {
     const int n = (int)emg_edges(g.lv[0].n);
@@ -746,12 +908,25 @@ void emg_coarse_k(const KrylovCtx<float>& c, const float2* r, float2* z0) {
     }
     edge_cycle<K>(g, om, r, c.stream, c.launches);
     if (c.gc_stream) cudaStreamWaitEvent(c.stream, c.gc_join, 0);
-    const long n = (long)c.n_pad * (K / 2);
+    const long n = (long)c.n_rows_pad * (K / 2);
     k_combine<K><<<grid1(n), kNT, 0, c.stream>>>(g, gc_row_term(gc, c.B), c.D, om, n, f4(r), f4(z0));
     ck(c.launches);
     if (c.timer) c.timer->end(th);
 }
 
+template <int K>
+void emg_node_precond_k(const EmgDev& g, const GcDev& gc, float2* z, cudaStream_t s, long long* launches) {
+    gc_presmooth0_k<K>(gc, s, launches);   // x = omega D^-1 b, y = b - L x
+    node_grids<K, true>(g, gc.lv[0].y, s, launches);
+    k_node_prolong0<K><<<grid1((long)gc.nn * (K / 2)), kNT, 0, s>>>(g, gc.nn, f4(gc.lv[0].x), f4(gc.lv[0].y));
+    ck(launches);
+    gc_smooth0_k<K>(gc, gc.lv[0].y, z, s, launches);
+}
+
+template void emg_node_precond_k<2>(const EmgDev&, const GcDev&, float2*, cudaStream_t, long long*);
+template void emg_node_precond_k<4>(const EmgDev&, const GcDev&, float2*, cudaStream_t, long long*);
+template void emg_node_precond_k<8>(const EmgDev&, const GcDev&, float2*, cudaStream_t, long long*);
+template void emg_node_precond_k<16>(const EmgDev&, const GcDev&, float2*, cudaStream_t, long long*);
 template void emg_coarse_k<2>(const KrylovCtx<float>&, const float2*, float2*);
 template void emg_coarse_k<4>(const KrylovCtx<float>&, const float2*, float2*);
 template void emg_coarse_k<8>(const KrylovCtx<float>&, const float2*, float2*);

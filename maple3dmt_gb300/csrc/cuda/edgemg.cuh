@@ -58,7 +58,13 @@ struct EmgDev {
     const unsigned* n_code = nullptr;
     const int *nr_ptr = nullptr, *nr_node = nullptr;
     const float* nr_w = nullptr;
+    // transfer rows that a block sums each (emg_long_rows)
+    const int *r_long = nullptr, *nr_long = nullptr;
+    int n_r_long = 0, n_nr_long = 0;
 };
+
+// The rows of a transfer (CSR row pointers) that take a block each.
+std::vector<int> emg_long_rows(const std::vector<int>& ptr);
 
 // Coarse edge masses for the current conductivity (Me per permuted row).
 void emg_set_mass(const EmgDev& g, const double* Me, cudaStream_t s, long long* launches);
@@ -67,5 +73,10 @@ void emg_set_mass(const EmgDev& g, const double* Me, cudaStream_t s, long long* 
 // c.gc_stream when set (forked and joined here); r, z0 [n_pad][K].
 template <int K>
 void emg_coarse_k(const KrylovCtx<float>& c, const float2* r, float2* z0);
+
+// z = V(1,1) of gc.lv[0].b for the divergence-correction Laplacian: octree
+// nodes, then the uniform node grids; symmetric, so PCG can use it.
+template <int K>
+void emg_node_precond_k(const EmgDev& g, const GcDev& gc, float2* z, cudaStream_t s, long long* launches);
 
 }  // namespace m3d

@@ -1,6 +1,8 @@
 // Gradient-space correction kernels (see gradcorr.cuh).
 #include "gradcorr.cuh"
 
+#include "edgemg.cuh"
+
 #include <algorithm>
 #include <stdexcept>
 #include <vector>
@@ -53,7 +55,7 @@ __global__ void k_gc_pack0(GcDev g) {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= g.nn) return;
     g.lap_diag32[v] = (float)g.lap_diag[v];
-    g.lv[0].dinv32[v] = (float)g.lv[0].dinv[v];
+    g.lv[0].dinv32[v] = (float)g.jac_inv[v];
     for (int q = g.inc_ptr[v]; q < g.inc_ptr[v + 1]; ++q)
         g.lap_pk[q] = make_int2(g.inc_other[q], __float_as_int((float)g.lap_off[q]));
 }
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(kGcBlock) k_gc_pre0(GcDev g) {
     const GcLevel& L = g.lv[0];
     const long n = (long)g.nn * K;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const float sc = g.omega * (float)__ldg(&L.dinv[i / K]);
+        const float sc = g.omega * __ldg(&L.dinv32[i / K]);
         const float2 b = L.b[i];
         L.x[i] = f2(sc * b.x, sc * b.y);
     }
@@ -366,6 +368,15 @@ void gc_restrict_edges_k(const GcDev& g, const float2* in, cudaStream_t s, long 
 template <int K>
 void gc_smooth0_k(const GcDev& g, const float2* t, float2* out, cudaStream_t s, long long* launches) {
     k_gc_smooth0<K><<<gc_grid((long)g.nn * K), kGcBlock, 0, s>>>(g, t, out);
+    gc_check(launches);
+}
+
+template <int K>
+void gc_presmooth0_k(const GcDev& g, cudaStream_t s, long long* launches) {
+    const int grid = gc_grid((long)g.nn * K);
+    k_gc_pre0<K><<<grid, kGcBlock, 0, s>>>(g);
+    gc_check(launches);
+    k_gc_resid<K, true><<<grid, kGcBlock, 0, s>>>(g, g.lv[0]);
     gc_check(launches);
 }
 
@@ -663,14 +674,21 @@ long long dc_poisson_mixed_k(const GcDev& g, int nn, DcWork w, RedScratch red, c
     long long launches = 0;
     const int cap = red.max_blocks;
     const int g_n = gc_grid((long)nn * K);
-    const int g_norm = wave_grid(k_dcm_norm<K>, cap, kGcBlock), g_first = wave_grid(k_dcm_first<K>, cap, kGcBlock);
-    const int g_ap = wave_grid(k_dcm_ap<K>, cap, kGcBlock), g_up = wave_grid(k_dcm_update<K>, cap, kGcBlock);
-    const int g_rz = wave_grid(k_dcm_rz<K>, cap, kGcBlock);
-    constexpr int kMaxRef = 8, kCap = 400, kPoll = 8;
+    const long n = (long)nn * K;
+    const int g_norm = reduce_grid(k_dcm_norm<K>, cap, n), g_first = reduce_grid(k_dcm_first<K>, cap, n);
+    const int g_ap = reduce_grid(k_dcm_ap<K>, cap, n), g_up = reduce_grid(k_dcm_update<K>, cap, n);
+    const int g_rz = reduce_grid(k_dcm_rz<K>, cap, n);
+    constexpr int kMaxRef = 8, kCap = 400;
+    // iterations between polls: the geometric cycle needs about ten in all
+    const int kPoll = g.emg ? 4 : 8;
     // V(1,1) cycle on the FP32 residual, into z
     GcDev gv = g;
     gv.lv[0].b = g.dc_r;
     auto precondition = [&]() {
+        if (g.emg) {
+            emg_node_precond_k<K>(*g.emg, gv, g.dc_z, s, &launches);
+            return;
+        }
         k_gc_pre0<K><<<g_n, kGcBlock, 0, s>>>(gv);
         gc_check(&launches);
         vcycle_k<K>(gv, gv.n_levels > 1 ? 1 : 0, g.dc_z, s, &launches);
@@ -726,12 +744,16 @@ template long long dc_poisson_mixed_k<4>(const GcDev&, int, DcWork, RedScratch, 
 template long long dc_poisson_mixed_k<8>(const GcDev&, int, DcWork, RedScratch, cudaStream_t, long long*);
 template long long dc_poisson_mixed_k<16>(const GcDev&, int, DcWork, RedScratch, cudaStream_t, long long*);
 
+template void gc_presmooth0_k<2>(const GcDev&, cudaStream_t, long long*);
 template void gc_restrict_edges_k<2>(const GcDev&, const float2*, cudaStream_t, long long*);
 template void gc_smooth0_k<2>(const GcDev&, const float2*, float2*, cudaStream_t, long long*);
+template void gc_presmooth0_k<4>(const GcDev&, cudaStream_t, long long*);
 template void gc_restrict_edges_k<4>(const GcDev&, const float2*, cudaStream_t, long long*);
 template void gc_smooth0_k<4>(const GcDev&, const float2*, float2*, cudaStream_t, long long*);
+template void gc_presmooth0_k<8>(const GcDev&, cudaStream_t, long long*);
 template void gc_restrict_edges_k<8>(const GcDev&, const float2*, cudaStream_t, long long*);
 template void gc_smooth0_k<8>(const GcDev&, const float2*, float2*, cudaStream_t, long long*);
+template void gc_presmooth0_k<16>(const GcDev&, cudaStream_t, long long*);
 template void gc_restrict_edges_k<16>(const GcDev&, const float2*, cudaStream_t, long long*);
 template void gc_smooth0_k<16>(const GcDev&, const float2*, float2*, cudaStream_t, long long*);
 

@@ -39,6 +39,8 @@
 
 namespace m3d {
 
+struct EmgDev;   // geometric multigrid (edgemg.cuh)
+
 struct GcLevel {
     int n = 0;
     const int *ptr = nullptr, *col = nullptr;   // A_l in CSR (levels >= 1)
@@ -84,6 +86,10 @@ struct GcDev {
     // FP32 PCG work of the mixed-precision divergence-correction solve, [nn][kMaxRhs]
     float2 *dc_x = nullptr, *dc_r = nullptr, *dc_z = nullptr, *dc_p = nullptr, *dc_ap = nullptr;
     GcPcgState* dc_st = nullptr;          // [kMaxRhs]
+    // when set, the PCG's preconditioner is the geometric node cycle, and only
+    // level 0 of this structure is filled in (n_levels = 1)
+    const EmgDev* emg = nullptr;
+    const double* jac_inv = nullptr;      // [nn] inverse diagonal of the Laplacian
 };
 
 // Masked FP32 restriction / prolongation weights (once per mesh).
@@ -98,12 +104,15 @@ template <int K>
 void gc_apply_k(const GcDev& g, int n_rows, const float2* in, cudaStream_t s, long long* launches,
                 KernelTimer* timer);
 
-// The two octree-level steps of a node cycle that the geometric multigrid
+// The octree-level steps of a node cycle that the geometric multigrid
 // (edgemg.cuh) shares: g.lv[0].b = G~^T in, and out = t + omega D^-1 (b - L t).
 template <int K>
 void gc_restrict_edges_k(const GcDev& g, const float2* in, cudaStream_t s, long long* launches);
 template <int K>
 void gc_smooth0_k(const GcDev& g, const float2* t, float2* out, cudaStream_t s, long long* launches);
+// g.lv[0].x = omega D^-1 b, g.lv[0].y = b - L x
+template <int K>
+void gc_presmooth0_k(const GcDev& g, cudaStream_t s, long long* launches);
 
 // Solves L phi = divJ for the right-hand sides of w with cg_run set (the
 // PCG stage of divcorr_poisson_, forward_solver_fv.cpp:668-710): FP64

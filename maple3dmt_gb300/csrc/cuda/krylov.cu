@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(kBlock) k_spmv(OpView<R> A, DiagView<R> D, Bat
                                                  const cplx<R>* __restrict__ x, cplx<R>* __restrict__ y,
                                                  const cplx<R>* __restrict__ aux,
                                                  cplx<R>* __restrict__ aux_out, BicgState* st,
-                                                 RedScratch rs) {
+                                                 RedScratch rs, int n_rows_pad) {
     using C = cplx<R>;
     constexpr int RPW = Rpw<K>::v;
     constexpr int NQ = (MODE == kSpmvAp || MODE == kSpmvSmooth) ? 1 : (MODE == kSpmvAs || MODE == kSpmvTrueRes) ? 2 : 3;
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kBlock) k_spmv(OpView<R> A, DiagView<R> D, Bat
     C accR[NQ];   // per-thread partial sums in the working precision
 #pragma unroll
     for (int q = 0; q < NQ; ++q) accR[q] = cm<R>(0, 0);
-    const long groups = A.n_pad / RPW;
+    const long groups = n_rows_pad / RPW;
     for (long t = wg; t < groups; t += W) {
         const int row = (int)(t * RPW) + sub;
         const C s = row_dot<R, K>(A, A.rp[row], A.rp[row + 1], x, rhs);
@@ -363,7 +363,8 @@ __global__ void __launch_bounds__(kBlock) k_spmv(OpView<R> A, DiagView<R> D, Bat
     }
 }
 
-// SSOR forward sweep over the 32-row slices of one colour (list[0..count)):
+// SSOR forward sweep over the sweep slices of one colour (list: 32 row numbers
+// of each of the count slices):
 //   y_i = (in_i - sum_{j in earlier colours} a_ij y_j) / d_i      (ssor.h:58-66)
 // Gathered rows belong to other colours, which this launch does not write.
 template <class R, int K>
@@ -380,7 +381,7 @@ __global__ void __launch_bounds__(kBlock) k_ssor_fwd(OpView<R> A, DiagView<R> D,
     const long tasks = (long)count * GPS;
     const R om = (R)B.omega[rhs];
     for (long t = wg; t < tasks; t += W) {
-        const int row = list[t / GPS] * kSlice + (int)(t % GPS) * RPW + sub;
+        const int row = list[(t / GPS) * kSlice + (t % GPS) * RPW + sub];
         const C s = row_dot<R, K>(A, A.rp[row], A.rs[row], y, rhs);
         const size_t i = (size_t)row * K + rhs;
         y[i] = cmul(csub(in[i], s), cscale(inv_c(diag_of(D, row, om)), (R)B.relax));
@@ -403,7 +404,7 @@ __global__ void __launch_bounds__(kBlock) k_ssor_bwd(OpView<R> A, DiagView<R> D,
     const long tasks = (long)count * GPS;
     const R om = (R)B.omega[rhs];
     for (long t = wg; t < tasks; t += W) {
-        const int row = list[t / GPS] * kSlice + (int)(t % GPS) * RPW + sub;
+        const int row = list[(t / GPS) * kSlice + (t % GPS) * RPW + sub];
         const C s = row_dot<R, K>(A, A.rs[row], A.rp[row + 1], out, rhs);
         const size_t i = (size_t)row * K + rhs;
         out[i] = csub(y[i], cmul(s, cscale(inv_c(diag_of(D, row, om)), (R)B.relax)));
@@ -414,72 +415,155 @@ __global__ void __launch_bounds__(kBlock) k_ssor_bwd(OpView<R> A, DiagView<R> D,
 // Slice-staged row kernels (segments of staged.cuh in shared memory).
 // ---------------------------------------------------------------------------
 
-// SpMV over slice-staged rows, same modes and reductions as k_spmv.
+// Launch shape of the row-staged SpMV: a thread works on one row and, in
+// complex FP32, on two neighbouring right-hand sides (16-byte gathers: half
+// the load instructions of one right-hand side per thread); 256 threads cover
+// ROWS rows a pass, a stage holds T slices = PASSES passes.
+template <class R, int K> struct SpmvShape {
+    static constexpr int NT = 256;
+    static constexpr int LPT = sizeof(R) == 4 ? 2 : 1;
+    static constexpr int TPR = K / LPT;              // threads per row
+    static constexpr int ROWS = NT / TPR;
+    static constexpr int T = ROWS >= 128 ? ROWS / 32 : ROWS >= 64 ? 4 : ROWS >= 32 ? 2 : 1;
+    static constexpr int PASSES = T * kSlice / ROWS;
+    static constexpr int LOG_T = T == 1 ? 0 : T == 2 ? 1 : T == 4 ? 2 : T == 8 ? 3 : 4;
+    // 24 resident warps of complex FP32 (85 registers, twelve gathers in
+    // flight per thread), 16 of FP64
+    static constexpr int MIN_BLOCKS = sizeof(R) == 4 ? 3 : 2;
+};
+
+// The LPT right-hand sides of one thread.
+template <class R, int LPT> struct alignas(LPT * 2 * sizeof(R)) CVec {
+    cplx<R> v[LPT];
+};
+
+// SpMV over row segments, same modes and reductions as k_spmv.  The rows are
+// in the octree's cell order and every block owns a contiguous range of them,
+// so most gathers hit the SM's L1 (see tile_pipeline): at K = 8 on the
+// 1.7 M-edge mesh the pass over colour-sorted slices dealt out to the blocks
+// in turn took 200 us, bound by L2 gathers (13 rows of 64 bytes per row).
 template <class R, int K, int MODE>
-__global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) k_spmv_st(SegView<R> S, long n_slices, DiagView<R> D,
-                                                                BatchView B, const cplx<R>* __restrict__ x,
-                                                                cplx<R>* __restrict__ y,
-                                                                const cplx<R>* __restrict__ aux,
-                                                                cplx<R>* __restrict__ aux_out, BicgState* st,
-                                                                RedScratch rs) {
+__global__ void __launch_bounds__(SpmvShape<R, K>::NT, SpmvShape<R, K>::MIN_BLOCKS)
+    k_spmv_st(SegView<R> S, int n_slices, DiagView<R> D, BatchView B, const cplx<R>* __restrict__ x,
+              cplx<R>* __restrict__ y, const cplx<R>* __restrict__ aux, cplx<R>* __restrict__ aux_out, BicgState* st,
+              RedScratch rs) {
     using C = cplx<R>;
-    using Sh = StagedShape<K>;
-    constexpr int RPW = Rpw<K>::v;
+    using Sh = SpmvShape<R, K>;
+    using V = CVec<R, Sh::LPT>;
     constexpr int NQ = (MODE == kSpmvAp || MODE == kSpmvSmooth) ? 1 : (MODE == kSpmvAs || MODE == kSpmvTrueRes) ? 2 : 3;
     constexpr bool REDUCE = MODE != kSpmvPlain && MODE != kSpmvSmooth;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int rhs = lane % K;
-    const int lr0 = warp * RPW + lane / K;
-    const R om = (R)B.omega[rhs];
-    C accR[NQ];
+    const int h = threadIdx.x % Sh::TPR, r0 = threadIdx.x / Sh::TPR;
+    const V* xv = reinterpret_cast<const V*>(x);
+    R om[Sh::LPT];
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) accR[q] = cm<R>(0, 0);
-    slice_pipeline<3>(S.seg, S.work_nat, n_slices, S.stage_spmv, S.err, [&](const SegItem& it, const unsigned char* base) {
-        SegRows<R> lo, up;
-        lo.bind(base);
-        up.bind(base + (size_t)it.lo_len * 16);
+    for (int j = 0; j < Sh::LPT; ++j) om[j] = (R)B.omega[h * Sh::LPT + j];
+    C accR[Sh::LPT][NQ];   // per-thread partial sums in the working precision
+#pragma unroll
+    for (int j = 0; j < Sh::LPT; ++j)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) accR[j][q] = cm<R>(0, 0);
+    tile_pipeline<Sh::T>(S.row_seg, S.row_off, n_slices, S.stage_row[Sh::LOG_T], S.err,
+                         [&](int tile, const unsigned char* base) {
+        const int s0 = tile * Sh::T, a0 = __ldg(&S.row_off[s0]);
 #pragma unroll
         for (int ps = 0; ps < Sh::PASSES; ++ps) {
-            const int lr = ps * Sh::ROWS_PER_PASS + lr0;
-            const int row = it.slice * kSlice + lr;
-            const size_t i = (size_t)row * K + rhs;
-            const C xi = x[i];
-            const C av = (MODE != kSpmvPlain) ? aux[i] : cm<R>(0, 0);
-            const C d = diag_of(D, row, om);
-            const C s = seg_row_dot_lu<R, K>(lo, up, lr, x, rhs);
-            const C yv = cadd(s, cmul(d, xi));
-            if (MODE == kSpmvPlain) {
-                y[i] = yv;
-            } else if (MODE == kSpmvAp) {
-                y[i] = yv;
-                accR[0] = cadd(accR[0], cjmul(av, yv));
-            } else if (MODE == kSpmvAs) {
-                y[i] = yv;
-                accR[0].x += yv.x * yv.x + yv.y * yv.y;
-                accR[1] = cadd(accR[1], cjmul(yv, av));
-            } else if (MODE == kSpmvInit) {
-                const C rv = csub(av, yv);
-                y[i] = rv;
-                aux_out[i] = rv;
-                accR[0].x += av.x * av.x + av.y * av.y;
-                accR[1].x += rv.x * rv.x + rv.y * rv.y;
-                accR[2] = cadd(accR[2], cjmul(rv, rv));
-            } else if (MODE == kSpmvSmooth) {
-                y[i] = cadd(xi, cmul(csub(av, yv), smooth_scale(d)));
-            } else if (MODE == kSpmvTrueRes) {
-                const C rv = csub(av, yv);
-                y[i] = rv;
-                accR[0].x += rv.x * rv.x + rv.y * rv.y;
-                accR[1].x += av.x * av.x + av.y * av.y;
+            const int lr = ps * Sh::ROWS + r0, sl = s0 + lr / kSlice;
+            if (sl >= n_slices) continue;
+            SegRows<R> A;
+            A.bind(base + (size_t)(__ldg(&S.row_off[sl]) - a0) * 16);
+            const int row = s0 * kSlice + lr;
+            const size_t i = (size_t)row * Sh::TPR + h;
+            const V xi = xv[i];
+            V av{};
+            if (MODE != kSpmvPlain) av = reinterpret_cast<const V*>(aux)[i];
+            const cplx<R> dm = D.sm[row];
+            V s{};
+            int k = A.begin_of(lr % kSlice);
+            const int e = A.end[lr % kSlice];
+            // whole rows of twelve entries (76 % of the rows) with all their
+            // gathers in flight, other lengths four at a time
+            if (k + 12 <= e) {
+                V g[12];
+#pragma unroll
+                for (int u = 0; u < 12; u += 4) {
+                    const int4 c = *reinterpret_cast<const int4*>(A.col + k + u);
+                    g[u] = xv[(size_t)c.x * Sh::TPR + h];
+                    g[u + 1] = xv[(size_t)c.y * Sh::TPR + h];
+                    g[u + 2] = xv[(size_t)c.z * Sh::TPR + h];
+                    g[u + 3] = xv[(size_t)c.w * Sh::TPR + h];
+                }
+#pragma unroll
+                for (int u = 0; u < 12; u += 4) {
+                    R a[4];
+                    lds4(A.val + k + u, a);
+#pragma unroll
+                    for (int w = 0; w < 4; ++w)
+#pragma unroll
+                        for (int j = 0; j < Sh::LPT; ++j) {
+                            s.v[j].x += a[w] * g[u + w].v[j].x;
+                            s.v[j].y += a[w] * g[u + w].v[j].y;
+                        }
+                }
+                k += 12;
             }
+            for (; k < e; k += 4) {
+                const int4 c = *reinterpret_cast<const int4*>(A.col + k);
+                R a[4];
+                lds4(A.val + k, a);
+                const V g[4] = {xv[(size_t)c.x * Sh::TPR + h], xv[(size_t)c.y * Sh::TPR + h],
+                                xv[(size_t)c.z * Sh::TPR + h], xv[(size_t)c.w * Sh::TPR + h]};
+#pragma unroll
+                for (int w = 0; w < 4; ++w)
+#pragma unroll
+                    for (int j = 0; j < Sh::LPT; ++j) {
+                        s.v[j].x += a[w] * g[w].v[j].x;
+                        s.v[j].y += a[w] * g[w].v[j].y;
+                    }
+            }
+            V out{}, out2{};
+#pragma unroll
+            for (int j = 0; j < Sh::LPT; ++j) {
+                const C d = cm<R>(dm.x, om[j] * dm.y);
+                const C yv = cadd(s.v[j], cmul(d, xi.v[j]));
+                const C a = av.v[j];
+                if constexpr (MODE == kSpmvPlain) {
+                    out.v[j] = yv;
+                } else if constexpr (MODE == kSpmvAp) {
+                    out.v[j] = yv;
+                    accR[j][0] = cadd(accR[j][0], cjmul(a, yv));
+                } else if constexpr (MODE == kSpmvAs) {
+                    out.v[j] = yv;
+                    accR[j][0].x += yv.x * yv.x + yv.y * yv.y;
+                    accR[j][1] = cadd(accR[j][1], cjmul(yv, a));
+                } else if constexpr (MODE == kSpmvInit) {
+                    const C rv = csub(a, yv);
+                    out.v[j] = rv;
+                    out2.v[j] = rv;
+                    accR[j][0].x += a.x * a.x + a.y * a.y;
+                    accR[j][1].x += rv.x * rv.x + rv.y * rv.y;
+                    accR[j][2] = cadd(accR[j][2], cjmul(rv, rv));
+                } else if constexpr (MODE == kSpmvSmooth) {
+                    out.v[j] = cadd(xi.v[j], cmul(csub(a, yv), smooth_scale(d)));
+                } else {  // kSpmvTrueRes
+                    const C rv = csub(a, yv);
+                    out.v[j] = rv;
+                    accR[j][0].x += rv.x * rv.x + rv.y * rv.y;
+                    accR[j][1].x += a.x * a.x + a.y * a.y;
+                }
+            }
+            reinterpret_cast<V*>(y)[i] = out;
+            if constexpr (MODE == kSpmvInit) reinterpret_cast<V*>(aux_out)[i] = out2;
         }
     });
     if (!REDUCE) return;
-    double2 acc[NQ];
+    double2 acc[Sh::LPT][NQ];
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) acc[q] = to_d(accR[q]);
+    for (int j = 0; j < Sh::LPT; ++j)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) acc[j][q] = to_d(accR[j][q]);
     __shared__ double2 out[NQ * K];
-    if (grid_reduce_lanes<NQ, K, Sh::NT>(acc, rs, out)) {
+    __syncthreads();
+    if (grid_reduce_multi<NQ, K, Sh::NT, Sh::LPT>(acc, rs, out)) {
         if (threadIdx.x < K) {
             BicgState T = st[threadIdx.x];
             if (MODE == kSpmvAp) ep_r0v(T, out, threadIdx.x, K);
@@ -494,9 +578,9 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
 // SSOR forward sweep of one colour over slice-staged lower parts
 // (ssor.h:58-66); items work_col[0..count) of the colour.
 template <class R, int K>
-__device__ __forceinline__ void ssor_fwd_rows(const SegItem& it, const unsigned char* base, const DiagView<R>& D,
-                                              R om, R rx, int rhs, int lr0, const cplx<R>* __restrict__ in,
-                                              cplx<R>* y) {
+__device__ __forceinline__ void ssor_fwd_rows(const SegItem& it, const unsigned char* base,
+                                              const int* __restrict__ rows, const DiagView<R>& D, R om, R rx, int rhs,
+                                              int lr0, const cplx<R>* __restrict__ in, cplx<R>* y) {
     using C = cplx<R>;
     using Sh = StagedShape<K>;
     SegRows<R> lo;
@@ -507,7 +591,7 @@ __device__ __forceinline__ void ssor_fwd_rows(const SegItem& it, const unsigned 
 #pragma unroll
     for (int ps = 0; ps < Sh::PASSES; ++ps) {
         const int lr = ps * Sh::ROWS_PER_PASS + lr0;
-        const int row = it.slice * kSlice + lr;
+        const int row = __ldg(&rows[it.slice * kSlice + lr]);
         const size_t i = (size_t)row * K + rhs;
         const C iv = in[i];
         const C d = diag_of(D, row, om);
@@ -527,7 +611,7 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
     const int lr0 = warp * RPW + lane / K;
     const R om = (R)B.omega[rhs];
     slice_pipeline<1>(S.seg, work, count, S.stage_lo, S.err, [&](const SegItem& it, const unsigned char* base) {
-        ssor_fwd_rows<R, K>(it, base, D, om, (R)B.relax, rhs, lr0, in, y);
+        ssor_fwd_rows<R, K>(it, base, S.rows, D, om, (R)B.relax, rhs, lr0, in, y);
     });
 }
 
@@ -537,9 +621,9 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
 // forward result, read once per row before it is replaced) and gathers the
 // later colours' w from there.
 template <class R, int K, bool GC>
-__device__ __forceinline__ void ssor_bwd_rows(const SegItem& it, const unsigned char* base, const DiagView<R>& D,
-                                              R om, R rx, int rhs, int lr0, cplx<R>* y, cplx<R>* out,
-                                              const GcRowTerm& gt) {
+__device__ __forceinline__ void ssor_bwd_rows(const SegItem& it, const unsigned char* base,
+                                              const int* __restrict__ rows, const DiagView<R>& D, R om, R rx, int rhs,
+                                              int lr0, cplx<R>* y, cplx<R>* out, const GcRowTerm& gt) {
     using C = cplx<R>;
     using Sh = StagedShape<K>;
     constexpr int NP = Sh::PASSES;
@@ -547,11 +631,14 @@ __device__ __forceinline__ void ssor_bwd_rows(const SegItem& it, const unsigned 
     up.bind(base);
     // every pass's loads (the term's node indices first, the row gathers, then
     // the node values) are issued before the first row is written
+    int rw[NP];
+#pragma unroll
+    for (int ps = 0; ps < NP; ++ps) rw[ps] = __ldg(&rows[it.slice * kSlice + ps * Sh::ROWS_PER_PASS + lr0]);
     int n0[NP], n1[NP];
     if (GC) {
 #pragma unroll
         for (int ps = 0; ps < NP; ++ps) {
-            const int row = it.slice * kSlice + ps * Sh::ROWS_PER_PASS + lr0;
+            const int row = rw[ps];
             n0[ps] = __ldg(&gt.e_node[2 * row]);
             n1[ps] = __ldg(&gt.e_node[2 * row + 1]);
         }
@@ -561,7 +648,7 @@ __device__ __forceinline__ void ssor_bwd_rows(const SegItem& it, const unsigned 
 #pragma unroll
     for (int ps = 0; ps < NP; ++ps) {
         const int lr = ps * Sh::ROWS_PER_PASS + lr0;
-        const int row = it.slice * kSlice + lr;
+        const int row = rw[ps];
         yv[ps] = y[(size_t)row * K + rhs];
         dv[ps] = diag_of(D, row, om);
         h[ps].load(up.col, up.val, up.begin_of(lr), up.end[lr], GC ? y : out, rhs);
@@ -573,7 +660,7 @@ __device__ __forceinline__ void ssor_bwd_rows(const SegItem& it, const unsigned 
         g0[ps] = g1[ps] = 0.0f;
         ya[ps] = yb[ps] = make_float2(0.0f, 0.0f);
         if (GC) {
-            const int row = it.slice * kSlice + ps * Sh::ROWS_PER_PASS + lr0;
+            const int row = rw[ps];
             g0[ps] = __ldg(&gt.e_g[2 * row]);
             g1[ps] = __ldg(&gt.e_g[2 * row + 1]);
             ya[ps] = gt.ya[(size_t)n0[ps] * K + rhs];
@@ -583,7 +670,7 @@ __device__ __forceinline__ void ssor_bwd_rows(const SegItem& it, const unsigned 
 #pragma unroll
     for (int ps = 0; ps < NP; ++ps) {
         const int lr = ps * Sh::ROWS_PER_PASS + lr0;
-        const int row = it.slice * kSlice + lr;
+        const int row = rw[ps];
         const size_t i = (size_t)row * K + rhs;
         C s = h[ps].sum(cm<R>(0, 0));
         const int b = up.begin_of(lr) + 8, e = up.end[lr];
@@ -611,7 +698,7 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
     const int lr0 = warp * RPW + lane / K;
     const R om = (R)B.omega[rhs];
     slice_pipeline<2>(S.seg, work, count, S.stage_up, S.err, [&](const SegItem& it, const unsigned char* base) {
-        ssor_bwd_rows<R, K, GC>(it, base, D, om, (R)B.relax, rhs, lr0, y, out, gt);
+        ssor_bwd_rows<R, K, GC>(it, base, S.rows, D, om, (R)B.relax, rhs, lr0, y, out, gt);
     });
 }
 
@@ -633,7 +720,7 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
         const int s0 = gptr[g], s1 = gptr[g + 1];
         slice_pipeline<1>(S.seg, work + s0, s1 - s0, S.stage_lo, S.err,
                           [&](const SegItem& it, const unsigned char* base) {
-                              ssor_fwd_rows<R, K>(it, base, D, om, (R)B.relax, rhs, lr0, in, y);
+                              ssor_fwd_rows<R, K>(it, base, S.rows, D, om, (R)B.relax, rhs, lr0, in, y);
                           });
     }
 }
@@ -652,7 +739,7 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
         const int s0 = gptr[g], s1 = gptr[g + 1];
         slice_pipeline<2>(S.seg, work + s0, s1 - s0, S.stage_up, S.err,
                           [&](const SegItem& it, const unsigned char* base) {
-                              ssor_bwd_rows<R, K, GC>(it, base, D, om, (R)B.relax, rhs, lr0, y, out, gt);
+                              ssor_bwd_rows<R, K, GC>(it, base, S.rows, D, om, (R)B.relax, rhs, lr0, y, out, gt);
                           });
     }
 }
@@ -777,47 +864,35 @@ double matrix_bytes(const KrylovCtx<R>& c) {
     return (double)c.nnz * (sizeof(R) + 4) + 4.0 * ((double)c.n_rows + 1) + (double)c.n_rows * sizeof(cplx<R>);
 }
 
+template <class R, int K, int MODE>
+void spmv_staged_mode(const KrylovCtx<R>& c, const cplx<R>* x, cplx<R>* y, const cplx<R>* aux, cplx<R>* aux_out,
+                      BicgState* st) {
+    using Sh = SpmvShape<R, K>;
+    const int ns = c.n_rows_pad / kSlice;
+    // reducing modes: every block must reach the reduction, so the grid stays
+    // within the partial-sum scratch
+    const int cap = (MODE == kSpmvPlain || MODE == kSpmvSmooth) ? (1 << 20) : c.red.max_blocks;
+    launch_staged(k_spmv_st<R, K, MODE>, Sh::NT, c.seg.stage_row[Sh::LOG_T], (ns + Sh::T - 1) / Sh::T, cap, c.stream,
+                  c.seg, ns, c.D, c.B, x, y, aux, aux_out, st, c.red);
+}
+
 template <class R, int K>
 void spmv_staged(const KrylovCtx<R>& c, int mode, const cplx<R>* x, cplx<R>* y, const cplx<R>* aux,
                  cplx<R>* aux_out, BicgState* st) {
-    constexpr int NT = StagedShape<K>::NT;
-    const long ns = c.n_pad / kSlice;
-    const int sb = c.seg.stage_spmv;
-    // reducing modes: every block must reach the reduction, so the grid stays
-    // within the partial-sum scratch
-    const int cap = (mode == kSpmvPlain || mode == kSpmvSmooth) ? (1 << 20) : c.red.max_blocks;
     switch (mode) {
-        case kSpmvSmooth:
-            launch_staged(k_spmv_st<R, K, kSpmvSmooth>, NT, sb, ns, cap, c.stream, c.seg, ns, c.D, c.B, x, y, aux,
-                          aux_out, st, c.red);
-            break;
-        case kSpmvPlain:
-            launch_staged(k_spmv_st<R, K, kSpmvPlain>, NT, sb, ns, cap, c.stream, c.seg, ns, c.D, c.B, x, y, aux,
-                          aux_out, st, c.red);
-            break;
-        case kSpmvAp:
-            launch_staged(k_spmv_st<R, K, kSpmvAp>, NT, sb, ns, cap, c.stream, c.seg, ns, c.D, c.B, x, y, aux,
-                          aux_out, st, c.red);
-            break;
-        case kSpmvAs:
-            launch_staged(k_spmv_st<R, K, kSpmvAs>, NT, sb, ns, cap, c.stream, c.seg, ns, c.D, c.B, x, y, aux,
-                          aux_out, st, c.red);
-            break;
-        case kSpmvInit:
-            launch_staged(k_spmv_st<R, K, kSpmvInit>, NT, sb, ns, cap, c.stream, c.seg, ns, c.D, c.B, x, y, aux,
-                          aux_out, st, c.red);
-            break;
-        default:
-            launch_staged(k_spmv_st<R, K, kSpmvTrueRes>, NT, sb, ns, cap, c.stream, c.seg, ns, c.D, c.B, x, y, aux,
-                          aux_out, st, c.red);
-            break;
+        case kSpmvPlain: spmv_staged_mode<R, K, kSpmvPlain>(c, x, y, aux, aux_out, st); break;
+        case kSpmvAp: spmv_staged_mode<R, K, kSpmvAp>(c, x, y, aux, aux_out, st); break;
+        case kSpmvAs: spmv_staged_mode<R, K, kSpmvAs>(c, x, y, aux, aux_out, st); break;
+        case kSpmvInit: spmv_staged_mode<R, K, kSpmvInit>(c, x, y, aux, aux_out, st); break;
+        case kSpmvSmooth: spmv_staged_mode<R, K, kSpmvSmooth>(c, x, y, aux, aux_out, st); break;
+        default: spmv_staged_mode<R, K, kSpmvTrueRes>(c, x, y, aux, aux_out, st); break;
     }
 }
 
 template <class R, int K>
 void spmv_k(const KrylovCtx<R>& c, int mode, const cplx<R>* x, cplx<R>* y, const cplx<R>* aux,
             cplx<R>* aux_out, BicgState* st) {
-    const long warps = (long)c.A.n_pad / Rpw<K>::v;
+    const long warps = (long)c.n_rows_pad / Rpw<K>::v;
     int grid;
     if (mode == kSpmvPlain || mode == kSpmvSmooth) {
         grid = blocks_for(warps, kWarpsPerBlock, 1 << 20);
@@ -836,29 +911,35 @@ void spmv_k(const KrylovCtx<R>& c, int mode, const cplx<R>* x, cplx<R>* y, const
     }
     switch (mode) {
         case kSpmvPlain:
-            k_spmv<R, K, kSpmvPlain><<<grid, kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red);
+            k_spmv<R, K, kSpmvPlain><<<grid, kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red,
+                                                      c.n_rows_pad);
             break;
         case kSpmvSmooth:
-            k_spmv<R, K, kSpmvSmooth><<<grid, kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red);
+            k_spmv<R, K, kSpmvSmooth><<<grid, kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red,
+                                                      c.n_rows_pad);
             break;
         case kSpmvAp: {
             auto kf = k_spmv<R, K, kSpmvAp>;
-            kf<<<wave_grid(kf, cap), kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red);
+            kf<<<wave_grid(kf, cap), kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red,
+                                                      c.n_rows_pad);
             break;
         }
         case kSpmvAs: {
             auto kf = k_spmv<R, K, kSpmvAs>;
-            kf<<<wave_grid(kf, cap), kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red);
+            kf<<<wave_grid(kf, cap), kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red,
+                                                      c.n_rows_pad);
             break;
         }
         case kSpmvInit: {
             auto kf = k_spmv<R, K, kSpmvInit>;
-            kf<<<wave_grid(kf, cap), kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red);
+            kf<<<wave_grid(kf, cap), kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red,
+                                                      c.n_rows_pad);
             break;
         }
         default: {
             auto kf = k_spmv<R, K, kSpmvTrueRes>;
-            kf<<<wave_grid(kf, cap), kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red);
+            kf<<<wave_grid(kf, cap), kBlock, 0, c.stream>>>(c.A, c.D, c.B, x, y, aux, aux_out, st, c.red,
+                                                      c.n_rows_pad);
             break;
         }
     }
@@ -988,7 +1069,7 @@ void ssor_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out, 
         const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
         if (s1 <= s0) continue;
         const int grid = blocks_for((long)(s1 - s0) * G, kWarpsPerBlock, 1 << 20);
-        k_ssor_fwd<R, K><<<grid, kBlock, 0, c.stream>>>(c.A, c.D, c.B, c.colour_list + s0, s1 - s0, in, y);
+        k_ssor_fwd<R, K><<<grid, kBlock, 0, c.stream>>>(c.A, c.D, c.B, c.sweep_rows + (size_t)s0 * kSlice, s1 - s0, in, y);
         check_launch(c.launches);
     }
     wait_join();
@@ -996,11 +1077,11 @@ void ssor_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out, 
         const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
         if (s1 <= s0) continue;
         const int grid = blocks_for((long)(s1 - s0) * G, kWarpsPerBlock, 1 << 20);
-        k_ssor_bwd<R, K><<<grid, kBlock, 0, c.stream>>>(c.A, c.D, c.B, c.colour_list + s0, s1 - s0, y, out);
+        k_ssor_bwd<R, K><<<grid, kBlock, 0, c.stream>>>(c.A, c.D, c.B, c.sweep_rows + (size_t)s0 * kSlice, s1 - s0, y, out);
         check_launch(c.launches);
     }
     if (gt.ya) {   // CSR rows: the gradient-space term in a pass of its own
-        const long n = (long)c.n_pad * K;
+        const long n = (long)c.n_rows_pad * K;
         k_add_gc_term<R, K><<<blocks_for(n, kBlock, 1 << 20), kBlock, 0, c.stream>>>(n, out, gt);
         check_launch(c.launches);
     }
@@ -1044,23 +1125,23 @@ void precond_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* ou
 
 template <class R, int K>
 void iteration_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* st) {
-    const long n = (long)c.n_pad * K;
+    const long n = (long)c.n_rows_pad * K;
     const int gv = c.grid_vec;
     const double vb = (double)c.n_rows * K * sizeof(cplx<R>);
     int th = c.timer ? c.timer->begin(kClsVec, 4 * vb, K) : -1;
-    k_update_p<R, K><<<gv, kBlock, 0, c.stream>>>(n, v.r, v.p, v.v, st);
+    k_update_p<R, K><<<blocks_for(n, 2 * kBlock, gv), kBlock, 0, c.stream>>>(n, v.r, v.p, v.v, st);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);
     precond_k<R, K>(c, v.p, v.y, v.ph);
     spmv_k<R, K>(c, kSpmvAp, v.ph, v.v, v.r0, nullptr, st);
     th = c.timer ? c.timer->begin(kClsVec, 3 * vb, K) : -1;
-    k_update_s<R, K><<<wave_grid(k_update_s<R, K>, gv), kBlock, 0, c.stream>>>(n, v.r, v.v, v.s, st, c.red);
+    k_update_s<R, K><<<reduce_grid(k_update_s<R, K>, gv, n), kBlock, 0, c.stream>>>(n, v.r, v.v, v.s, st, c.red);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);
     precond_k<R, K>(c, v.s, v.y, v.sh);
     spmv_k<R, K>(c, kSpmvAs, v.sh, v.t, v.s, nullptr, st);
     th = c.timer ? c.timer->begin(kClsVec, 8 * vb, K) : -1;
-    k_update_xr<R, K><<<wave_grid(k_update_xr<R, K>, gv), kBlock, 0, c.stream>>>(n, v.x, v.r, v.r0, v.ph, v.sh, v.s, v.t, st, c.red);
+    k_update_xr<R, K><<<reduce_grid(k_update_xr<R, K>, gv, n), kBlock, 0, c.stream>>>(n, v.x, v.r, v.r0, v.ph, v.sh, v.s, v.t, st, c.red);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);
 }
@@ -1135,7 +1216,7 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v)
 #pragma unroll
         for (int ps = 0; ps < Sh::PASSES; ++ps) {
             const int lr = ps * Sh::ROWS_PER_PASS + lr0;
-            const int row = it.slice * kSlice + lr;
+            const int row = __ldg(&S.rows[it.slice * kSlice + lr]);
             const size_t i = (size_t)row * K + rhs;
             C z;
             if (FUSE == 1) {
@@ -1187,7 +1268,7 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v)
 #pragma unroll
         for (int ps = 0; ps < Sh::PASSES; ++ps) {
             const int lr = ps * Sh::ROWS_PER_PASS + lr0;
-            const int row = it.slice * kSlice + lr;
+            const int row = __ldg(&S.rows[it.slice * kSlice + lr]);
             const size_t i = (size_t)row * K + rhs;
             const C zv = z[i], wv = w[i];
             const C d = diag_of(D, row, om);
@@ -1365,7 +1446,7 @@ void eis_init_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* st) {
                       c.seg.work_col + s0, s1 - s0, c.D, c.B, (const cplx<R>*)v.b, v.y);
         check_launch(c.launches);
     }
-    const long n = (long)c.n_pad * K;
+    const long n = (long)c.n_rows_pad * K;
     k_eis_init<R, K><<<wave_grid(k_eis_init<R, K>, c.grid_vec), kBlock, 0, c.stream>>>(n, c.D, c.B, v.y, v.r, v.r0,
                                                                                     st, c.red);
     check_launch(c.launches);
@@ -1373,7 +1454,7 @@ void eis_init_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* st) {
 
 template <class R, int K>
 void eis_iteration_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* st) {
-    const long n = (long)c.n_pad * K;
+    const long n = (long)c.n_rows_pad * K;
     const int gv = c.grid_vec;
     const double vb = (double)c.n_rows * K * sizeof(cplx<R>);
     // p update + v = A_hat p: matrix once, r, p (read, write), v (read, write), w (write, read), y
@@ -1386,7 +1467,7 @@ void eis_iteration_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* s
     eis_apply_k<R, K, 2, kEisAsS>(c, nullptr, v.s, v.r, v.v, st, v.ph, v.y, v.t, v.s);
     if (c.timer) c.timer->end(th);
     th = c.timer ? c.timer->begin(kClsVec, 8 * vb, K) : -1;
-    k_update_xr<R, K><<<wave_grid(k_update_xr<R, K>, gv), kBlock, 0, c.stream>>>(n, v.x, v.r, v.r0, v.p, v.s, v.s,
+    k_update_xr<R, K><<<reduce_grid(k_update_xr<R, K>, gv, n), kBlock, 0, c.stream>>>(n, v.x, v.r, v.r0, v.p, v.s, v.s,
                                                                               v.t, st, c.red);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);

@@ -42,7 +42,7 @@ struct BicgState {
 
 enum : int { kRunning = 0, kConverged = 1, kBreakdown = 2, kMaxIter = 3, kInactive = 9 };
 
-// Off-diagonal part in "split CSR": rows in the solver's permuted order, each
+// Off-diagonal part in "split CSR": rows in the solver's order, each
 // row holding its lower entries (columns in earlier colours) in
 // [rp[i], rs[i]) and its upper entries in [rs[i], rp[i+1]).
 template <class R>
@@ -137,9 +137,10 @@ struct KrylovCtx {
     OpView<R> A;
     DiagView<R> D;
     BatchView B;
-    std::vector<int> colour_ptr;     // [n_colours + 1] ranges of colour_list per colour
-    const int* colour_list;          // device: 32-row slice ids grouped by colour, memory order inside
-    int n_pad;
+    std::vector<int> colour_ptr;     // [n_colours + 1] ranges of sweep slices per colour
+    const int* sweep_rows;           // device: 32 row numbers per sweep slice, slices grouped by colour
+    int n_rows_pad;                  // rows the products and vector kernels run over: all, or the free rows
+                                     // (the first ones) in the FP32 inner solve
     int grid_vec;     // blocks for vector kernels with reductions
     int grid_spmv;    // blocks for SpMV kernels with reductions
     dev::RedScratch red;

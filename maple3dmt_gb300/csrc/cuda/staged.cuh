@@ -1,7 +1,6 @@
-// Slice-staged operator rows: the off-diagonal matrix, split into its lower
-// (earlier colour) and upper parts, is stored per 32-row slice as a
-// contiguous segment that one bulk asynchronous copy (cp.async.bulk, the
-// TMA engine's 1-D mode) moves into shared memory:
+// Matrix rows staged in shared memory by bulk asynchronous copies
+// (cp.async.bulk, the TMA engine's 1-D mode).  A segment holds the
+// off-diagonal entries of 32 rows:
 //
 //   segment = [uint16 end[32]]                 row r owns entries [end[r-1], end[r])
 //             [int32 col[n]]
@@ -10,11 +9,18 @@
 // with every row padded to a multiple of four entries (padding entries point
 // at the row itself with value 0), so rows start on 16-byte boundaries and
 // are read four entries at a time, and every segment starts and ends on a
-// 16-byte boundary.  A slice's work item
-// (int4) is {slice, lower offset, upper offset, (lower length << 16) | upper
-// length}, offsets and lengths in 16-byte units.  Kernels keep two segments in
-// flight per block (double buffering on two mbarriers): the next slice's
-// matrix stream arrives while the current slice's gathers run.
+// 16-byte boundary.  Two sets exist per precision:
+//
+//  * row segments (SpMV): slice s holds rows 32 s .. 32 s + 31 with all their
+//    entries, segments one after another, so neighbouring slices are one copy;
+//  * sweep segments (SSOR): a sweep slice holds 32 rows of one colour, named
+//    by its list of row numbers, with a lower (earlier colour) and an upper
+//    segment.  Its work item (int4) is {slice, lower offset, upper offset,
+//    (lower length << 16) | upper length}, offsets and lengths in 16-byte units.
+//
+// Kernels keep two stages in flight per block (double buffering on two
+// mbarriers): the next stage's matrix stream arrives while the current one's
+// gathers run.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -38,13 +44,16 @@ constexpr unsigned kTestConsumeNoWait = 1u << 31;
 
 template <class R>
 struct SegView {
-    const unsigned char* seg;   // all segments of one precision
-    const int4* work_nat;       // [n_slices] natural slice order (SpMV)
-    const int4* work_col;       // colour sweep order (slices of colour c at colour_ptr[c])
-    int stage_spmv;             // bytes of the largest lower + upper segment pair
-    int stage_lo;               // bytes of the largest lower segment
-    int stage_up;               // bytes of the largest upper segment
-    unsigned* err;              // device flag, kErrCopyTimeout on a barrier timeout
+    using Real = R;
+    const unsigned char* row_seg = nullptr;   // row segments
+    const int* row_off = nullptr;             // [n_slices + 1] their offsets, 16-byte units
+    int stage_row[5] = {};      // bytes of the largest run of 1, 2, 4, 8, 16 neighbouring row segments
+    const unsigned char* seg = nullptr;       // sweep segments (null until a sweep is asked for)
+    const int4* work_col = nullptr;           // sweep order (sweep slices of group g at colour_ptr[g])
+    const int* rows = nullptr;                // [sweep slices][32] row numbers (-1: none)
+    int stage_lo = 0;           // bytes of the largest lower segment
+    int stage_up = 0;           // bytes of the largest upper segment
+    unsigned* err = nullptr;    // device flag, kErrCopyTimeout on a barrier timeout
 };
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
@@ -247,6 +256,59 @@ __device__ __forceinline__ void slice_pipeline(const unsigned char* __restrict__
     }
 }
 
+// The same for row segments: block b owns the tiles (T slices, one copy each)
+// [n b / grid, n (b + 1) / grid) and runs them in order.  A contiguous range
+// keeps a block on neighbouring rows, whose gathers hit its SM's L1: on the
+// benchmark mesh half of a row's columns lie within 13 rows of it and three
+// quarters within 86.
+template <int T, class Body>
+__device__ __forceinline__ void tile_pipeline(const unsigned char* __restrict__ seg, const int* __restrict__ off,
+                                              int n_slices, int stage_bytes, unsigned* err, Body body) {
+    extern __shared__ __align__(128) unsigned char dsm[];
+    __shared__ __align__(8) uint64_t bar[2];
+    __shared__ int no_wait;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_mbar_init();
+        no_wait = (*reinterpret_cast<volatile unsigned*>(err) & kTestConsumeNoWait) != 0;
+    }
+    __syncthreads();
+    const long n_tiles = (n_slices + T - 1) / T;
+    const int t0 = (int)(n_tiles * blockIdx.x / gridDim.x), t1 = (int)(n_tiles * (blockIdx.x + 1) / gridDim.x);
+    auto issue = [&](int t, int stg) {   // thread 0 only
+        const int s0 = t * T, s1 = min(s0 + T, n_slices);
+        const int a = __ldg(&off[s0]);
+        const unsigned bytes = (unsigned)(__ldg(&off[s1]) - a) * 16u;
+        mbar_expect_tx(&bar[stg], bytes);
+        bulk_g2s(dsm + (size_t)stg * stage_bytes, seg + (size_t)a * 16, bytes, &bar[stg]);
+    };
+    auto wait_stage = [&](int stg, unsigned parity) {
+        return no_wait ? mbar_test_wait(&bar[stg], parity) : mbar_wait_bounded(&bar[stg], parity);
+    };
+    if (t0 >= t1) return;   // uniform: the whole block has no tile
+    if (threadIdx.x == 0) issue(t0, 0);
+    bool fail = __syncthreads_or(!wait_stage(0, 0u)) != 0;
+    for (int t = t0, k = 0;; ++t, ++k) {
+        const int stg = k & 1;
+        if (fail) {   // as in slice_pipeline
+            if (threadIdx.x == 0) {
+                atomicOr(err, kErrCopyTimeout);
+                mbar_wait_bounded(&bar[stg], (unsigned)(k >> 1) & 1u);
+            }
+            __syncthreads();
+            return;
+        }
+        if (threadIdx.x == 0 && t + 1 < t1) {
+            fence_proxy_async_smem();
+            issue(t + 1, stg ^ 1);
+        }
+        body(t, dsm + (size_t)stg * stage_bytes);
+        if (t + 1 >= t1) return;
+        fail = __syncthreads_or(!wait_stage(stg ^ 1, (unsigned)((k + 1) >> 1) & 1u)) != 0;
+    }
+}
+
 // Barrier over all blocks of a cooperative launch (every block resident):
 // an arrival counter and a generation word in global memory, the wait
 // bounded by kWaitCycles; a timeout sets kErrCopyTimeout in *err and lets the
@@ -358,47 +420,6 @@ __device__ __forceinline__ cplx<R> seg_row_dot(const int* __restrict__ col, cons
 #pragma unroll
         for (int u = 0; u < 4; ++u) { s.x += a1[u] * x[4 + u].x; s.y += a1[u] * x[4 + u].y; }
     }
-    return s;
-}
-
-// Lower and upper parts of one staged row: the first (up to) eight entries of
-// each part are gathered in one round, longer rows continue part by part.
-template <class R, int K>
-__device__ __forceinline__ cplx<R> seg_row_dot_lu(const SegRows<R>& lo, const SegRows<R>& up, int r,
-                                                  const cplx<R>* __restrict__ v, int rhs) {
-    using C = cplx<R>;
-    const int bl = lo.begin_of(r), el = lo.end[r];
-    const int bu = up.begin_of(r), eu = up.end[r];
-    const bool on[4] = {bl < el, bl + 4 < el, bu < eu, bu + 4 < eu};
-    const int at[4] = {bl, bl + 4, bu, bu + 4};
-    R a[4][4];
-    C x[16];
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        const SegRows<R>& P = g < 2 ? lo : up;
-        if (on[g]) {
-            const int4 c = *reinterpret_cast<const int4*>(P.col + at[g]);
-            lds4(P.val + at[g], a[g]);
-            x[4 * g + 0] = v[(size_t)c.x * K + rhs];
-            x[4 * g + 1] = v[(size_t)c.y * K + rhs];
-            x[4 * g + 2] = v[(size_t)c.z * K + rhs];
-            x[4 * g + 3] = v[(size_t)c.w * K + rhs];
-        } else {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) { a[g][u] = (R)0; x[4 * g + u] = cm<R>(0, 0); }
-        }
-    }
-    C s = cm<R>(0, 0);
-#pragma unroll
-    for (int g = 0; g < 2; ++g)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) { s.x += a[g][u] * x[4 * g + u].x; s.y += a[g][u] * x[4 * g + u].y; }
-    if (bl + 8 < el) s = seg_row_dot<R, K>(lo.col, lo.val, bl + 8, el, v, rhs, s);
-#pragma unroll
-    for (int g = 2; g < 4; ++g)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) { s.x += a[g][u] * x[4 * g + u].x; s.y += a[g][u] * x[4 * g + u].y; }
-    if (bu + 8 < eu) s = seg_row_dot<R, K>(up.col, up.val, bu + 8, eu, v, rhs, s);
     return s;
 }
 

@@ -574,13 +574,14 @@ void GpuSolver::fg_mdot(const float2* V, int nv, const float2* w, int K, std::ve
 
 BatchResult GpuSolver::solve_batch_fgmres(int K, const int* fmap, double2* b, double2* x,
                                           const std::vector<int>& active, double tol, int maxiter) {
+    ensure_sweeps(seg32);
     using cd = std::complex<double>;
     const int m = std::max(2, std::min(P.fgmres_m > 0 ? P.fgmres_m : 20, kFgMaxV - 1));
     ensure_vecs(K);
     ensure_vecs32(K);
     ensure_fgmres(K, m);
     const KrylovCtx<double> c64 = kctx(K, fmap);
-    KrylovCtx<float> c32 = kctx32(K, fmap);
+    KrylovCtx<float> c32 = kctx32(K, fmap, false);
     bool use_gc = false;
     if (gc_ok && P.gradcorr == 1 && gc.omega_max > 0.0)
         for (int k = 0; k < K; ++k)

@@ -64,6 +64,13 @@ __global__ void k_zero_col(double2* x, int K, int k, int n_pad) {
     if (r < n_pad) x[(size_t)r * K + k] = make_double2(0.0, 0.0);
 }
 
+// x = b on the identity rows of the lanes of `on`
+struct LaneMask { bool v[dev::kMaxRhs]; };
+__global__ void k_identity_rows(double2* __restrict__ x, const double2* __restrict__ b, int K, long n, LaneMask on) {
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && on.v[i % K]) x[i] = b[i];
+}
+
 // b32 = y64 / scale[k] (scale 0: column left at zero)
 __global__ void k_to_f32_scaled(const double2* __restrict__ y, float2* __restrict__ b,
                                 const double* __restrict__ scale, int K, long n) {
@@ -210,9 +217,11 @@ void GpuSolver::free_all() {
     dfree(md.inc_ptr); dfree(md.inc_edge); dfree(md.inc_other); dfree(md.inc_gv); dfree(md.inc_gw);
     dfree(md.node_bc); dfree(md.e_node); dfree(md.e_g); dfree(md.cell_ptr); dfree(md.cell_edge);
     dfree(d_op_rp); dfree(d_op_rs); dfree(d_col); dfree(d_val); dfree(d_val32);
-    dfree(d_seg64); dfree(d_seg32); dfree(d_work64); dfree(d_work32); dfree(d_seg_err);
+    dfree(d_row_seg64); dfree(d_row_seg32); dfree(d_row_off64); dfree(d_row_off32); dfree(d_seg_err);
+    for (void* p : sweep_mem) cudaFree(p);
+    sweep_mem.clear();
     seg64 = dev::SegView<double>{}; seg32 = dev::SegView<float>{};
-    dfree(d_colour_list); dfree(d_colour_ptr); dfree(d_gridbar);
+    dfree(d_sweep_rows); dfree(d_colour_ptr); dfree(d_gridbar);
     dfree(d_src_wr); dfree(d_src_g); src_ns = -1;
     dfree(d_sigma); dfree(d_Me); dfree(d_me_dc);
     dfree(d_diag); dfree(d_diag32); dfree(d_omegas);
@@ -353,82 +362,55 @@ void GpuSolver::setup(const m3d_leaves* lv, const m3d_params* params) {
     }
     const int n_col = *std::max_element(colour.begin(), colour.end()) + 1;
 
-    // Permutation: the reference order (cell by cell along the Morton curve)
-    // is cut into blocks of kRowBlock edges; inside a block rows are grouped by
-    // colour (reference order kept within a group) and each group is padded to
-    // whole slices.  A row's neighbours then sit in the same block or the next
-    // one, so gathers stay inside a small, cache-resident window, while each
-    // SSOR colour sweep walks its slice list across all blocks.
-    //
-    // Sweep groups: with sweep_rows > 0 the reference order is also cut into
-    // super-blocks of about sweep_rows edges, and the SSOR ordering becomes
-    // (super-block, colour): a sweep runs every colour of one super-block
-    // before the next one, so the rows it gathers stay in L2 while the
-    // super-block is swept.  A group (super-block, colour) is what a colour
-    // was: independent rows, one sweep step.  sweep_rows = 0: one super-block.
-    constexpr int kRowBlock = 16384;
-    const int blocks_per_sb = P.sweep_rows > 0 ? std::max(1, P.sweep_rows / kRowBlock) : (1 << 30);
-    const int n_sb = (int)(((long)(ne + kRowBlock - 1) / kRowBlock + blocks_per_sb - 1) / blocks_per_sb);
-    auto group_of = [&](int e) { return (e / kRowBlock / blocks_per_sb) * n_col + colour[e]; };
-    const int n_grp = n_sb * n_col;
+    // Row order: the free rows in reference order (cell by cell along the
+    // Morton curve), then the identity rows of the eliminated system (boundary
+    // and air edges, dead hanging edges: a sixth to a third of all), each part
+    // padded to whole slices.  A row's neighbours sit a few rows away, so
+    // gathers hit L1, and the FP32 inner solve runs over the free rows alone.
     perm.clear();
-    std::vector<std::vector<int>> slices_of(n_grp);
-    {
-        std::vector<std::vector<int>> byc(n_col);
-        for (int b0 = 0; b0 < ne; b0 += kRowBlock) {
-            for (auto& v : byc) v.clear();
-            for (int e = b0; e < std::min(ne, b0 + kRowBlock); ++e) byc[colour[e]].push_back(e);
-            const int g0 = (b0 / kRowBlock / blocks_per_sb) * n_col;
-            for (int c = 0; c < n_col; ++c) {
-                if (byc[c].empty()) continue;
-                const int s0 = (int)(perm.size() / dev::kSlice);
-                for (int e : byc[c]) perm.push_back(e);
-                while (perm.size() % dev::kSlice) perm.push_back(-1);
-                const int s1 = (int)(perm.size() / dev::kSlice);
-                for (int s = s0; s < s1; ++s) slices_of[g0 + c].push_back(s);
-            }
-        }
-    }
-    colour_ptr.assign(1, 0);
-    colour_list.clear();
-    for (int g = 0; g < n_grp; ++g) {
-        if (slices_of[g].empty()) continue;
-        colour_list.insert(colour_list.end(), slices_of[g].begin(), slices_of[g].end());
-        colour_ptr.push_back((int)colour_list.size());
+    for (int part = 0; part < 2; ++part) {
+        for (int e = 0; e < ne; ++e)
+            if (free_row(e) == (part == 0)) perm.push_back(e);
+        // at least one padding row in the end: sweep slices are filled up with it
+        do perm.push_back(-1);
+        while (perm.size() % dev::kSlice);
+        if (part == 0) n_free = (int)perm.size();
     }
     n_pad = (int)perm.size();
     n_slices = n_pad / dev::kSlice;
     iperm.assign(ne, -1);
     for (int r = 0; r < n_pad; ++r) if (perm[r] >= 0) iperm[perm[r]] = r;
 
-    // Split CSR of the free-free off-diagonal part in permuted row order:
-    // lower (earlier sweep group) entries, then upper, each in reference
-    // column order.
-    std::vector<int> op_rp(n_pad + 1, 0), op_rs(n_pad, 0), ecol;
-    std::vector<double> eval;
+    // SSOR sweep groups: a group's rows are independent (one colour), swept by
+    // one launch over its sweep slices, which list 32 rows each.  With
+    // sweep_rows > 0 the reference order is also cut into super-blocks of about
+    // sweep_rows edges, and the SSOR ordering becomes (super-block, colour): a
+    // sweep runs every colour of one super-block before the next one, so the
+    // rows it gathers stay in L2 while the super-block is swept.
+    // sweep_rows = 0: one super-block.
+    constexpr int kRowBlock = 16384;
+    const int blocks_per_sb = P.sweep_rows > 0 ? std::max(1, P.sweep_rows / kRowBlock) : (1 << 30);
+    const int n_sb = (int)(((long)(ne + kRowBlock - 1) / kRowBlock + blocks_per_sb - 1) / blocks_per_sb);
+    edge_group.resize(ne);
+    for (int e = 0; e < ne; ++e) edge_group[e] = (e / kRowBlock / blocks_per_sb) * n_col + colour[e];
     {
-        ecol.reserve((size_t)L.s_idx.size());
-        eval.reserve((size_t)L.s_idx.size());
-        std::vector<int> up_c;
-        std::vector<double> up_v;
-        for (int r = 0; r < n_pad; ++r) {
-            const int e = perm[r];
-            up_c.clear(); up_v.clear();
-            if (e >= 0 && free_row(e))
-                for (int k = L.s_ptr[e]; k < L.s_ptr[e + 1]; ++k) {
-                    const int j = L.s_idx[k];
-                    if (j == e || !free_row(j)) continue;
-                    if (group_of(j) < group_of(e)) { ecol.push_back(iperm[j]); eval.push_back(L.s_val[k]); }
-                    else { up_c.push_back(iperm[j]); up_v.push_back(L.s_val[k]); }
-                }
-            op_rs[r] = (int)ecol.size();
-            ecol.insert(ecol.end(), up_c.begin(), up_c.end());
-            eval.insert(eval.end(), up_v.begin(), up_v.end());
-            op_rp[r + 1] = (int)ecol.size();
-            if (ecol.size() > 2000000000UL) throw std::runtime_error("mesh too large for 32-bit row pointers");
+        std::vector<std::vector<int>> rows_of((size_t)n_sb * n_col);
+        for (int r = 0; r < n_pad; ++r)
+            if (perm[r] >= 0) rows_of[edge_group[perm[r]]].push_back(r);
+        colour_ptr.assign(1, 0);
+        sweep_rows.clear();
+        for (auto& rows : rows_of) {
+            if (rows.empty()) continue;
+            sweep_rows.insert(sweep_rows.end(), rows.begin(), rows.end());
+            sweep_rows.resize((sweep_rows.size() + dev::kSlice - 1) / dev::kSlice * dev::kSlice, n_pad - 1);
+            colour_ptr.push_back((int)(sweep_rows.size() / dev::kSlice));
         }
-        nnz_off = (long)ecol.size();
     }
+
+    std::vector<int> op_rp, op_rs, ecol;
+    std::vector<double> eval;
+    split_csr(op_rp, op_rs, ecol, eval);
+    nnz_off = (long)ecol.size();
 
     // Per permuted row data.
     std::vector<unsigned char> flags(n_pad, kFlagPad);
@@ -566,10 +548,10 @@ void GpuSolver::setup(const m3d_leaves* lv, const m3d_params* params) {
     }
     d_op_rp = dupload(op_rp, stream); d_op_rs = dupload(op_rs, stream);
     d_col = dupload(ecol, stream); d_val = dupload(eval, stream);
-    d_colour_list = dupload(colour_list, stream);
+    d_sweep_rows = dupload(sweep_rows, stream);
     d_colour_ptr = dupload(colour_ptr, stream);
     d_gridbar = dalloc_zero<unsigned>(2, stream);
-    build_segments(op_rp, op_rs, ecol, eval);
+    build_row_segments(op_rp, ecol, eval);
     {
         std::vector<float> ev32(eval.begin(), eval.end());
         d_val32 = dupload(ev32, stream);
@@ -595,8 +577,47 @@ void GpuSolver::setup(const m3d_leaves* lv, const m3d_params* params) {
     d_states2 = dalloc<BicgState>(dev::kMaxRhs);
     sigma_h.assign(L.nc, 0.0);
     if (want_emg()) build_emg();
+    if (P.precision == 0) ensure_sweeps(seg64);
+    else if (!emg_ok || P.krylov == 1) ensure_sweeps(seg32);
     sync();
     ready = true;
+}
+
+// Split CSR of the free-free off-diagonal part in row order: lower (earlier
+// sweep group) entries, then upper, each in reference column order.
+void GpuSolver::split_csr(std::vector<int>& rp, std::vector<int>& rs, std::vector<int>& col,
+                          std::vector<double>& val) const {
+    rp.assign(n_pad + 1, 0);
+    rs.assign(n_pad, 0);
+    col.clear();
+    val.clear();
+    col.reserve(L.s_idx.size());
+    val.reserve(L.s_idx.size());
+    auto free_row = [&](int e) { return !(flags_ref[e] & kFlagConstrained); };
+    std::vector<int> up_c;
+    std::vector<double> up_v;
+    for (int r = 0; r < n_pad; ++r) {
+        const int e = perm[r];
+        up_c.clear();
+        up_v.clear();
+        if (e >= 0 && free_row(e))
+            for (int k = L.s_ptr[e]; k < L.s_ptr[e + 1]; ++k) {
+                const int j = L.s_idx[k];
+                if (j == e || !free_row(j)) continue;
+                if (edge_group[j] < edge_group[e]) {
+                    col.push_back(iperm[j]);
+                    val.push_back(L.s_val[k]);
+                } else {
+                    up_c.push_back(iperm[j]);
+                    up_v.push_back(L.s_val[k]);
+                }
+            }
+        rs[r] = (int)col.size();
+        col.insert(col.end(), up_c.begin(), up_c.end());
+        val.insert(val.end(), up_v.begin(), up_v.end());
+        rp[r + 1] = (int)col.size();
+        if (col.size() > 2000000000UL) throw std::runtime_error("mesh too large for 32-bit row pointers");
+    }
 }
 
 // Uniform grids, transfers and face weights of the geometric multigrid
@@ -645,6 +666,11 @@ void GpuSolver::build_emg() {
     emg.nr_ptr = up(H.nr_ptr);
     emg.nr_node = up(H.nr_node);
     emg.nr_w = up(H.nr_w);
+    const std::vector<int> rl = emg_long_rows(H.r_ptr), nl = emg_long_rows(H.nr_ptr);
+    emg.n_r_long = (int)rl.size();
+    emg.n_nr_long = (int)nl.size();
+    emg.r_long = up(rl);
+    emg.nr_long = up(nl);
     sync();
     emg_ok = true;
 }
@@ -812,9 +838,50 @@ void GpuSolver::ensure_sigma_device() {
         phys::dc_build_laplacian(md, d_me_dc, dc, stream);
         ++launches;
         lap_built = true;
-        if (want_amg()) build_amg();
-        if (emg_ok) emg_set_mass(emg, d_Me, stream, &launches);
+        if (emg_ok) {
+            // the geometric grids need the coarse masses and the level-0 copy
+            // alone; the aggregation hierarchy only where something else asks
+            emg_set_mass(emg, d_Me, stream, &launches);
+            amg_stale = true;
+            if (!gc_ok) {
+                build_gc0();
+            } else {
+                gc_pack_level0(gc, stream);
+                ++launches;
+            }
+            if (P.divcorr_precond == 1 && P.divcorr_mixed == 0) need_amg();
+        } else if (want_amg()) {
+            build_amg();
+        }
     }
+}
+
+// The aggregation hierarchy for the current conductivity on a mesh with
+// geometric grids: the FP64 PCG and the gradient-space term of SSOR use it.
+void GpuSolver::need_amg() {
+    if (!emg_ok || !amg_stale) return;
+    build_amg();
+    amg_stale = false;
+    if (!gc_ok) build_gc0();   // no hierarchy on this mesh
+}
+
+// The part of build_gc that the geometric multigrid uses: octree-node vectors,
+// the packed Laplacian and the FP32 PCG's work.
+void GpuSolver::build_gc0() {
+    if (P.precision != 1) return;
+    gc = GcDev{};
+    gc_common();
+    gc.n_levels = 1;
+    GcLevel& g = gc.lv[0];
+    g.n = L.nn;
+    for (float2** q : {&g.b, &g.x, &g.y}) {
+        *q = dalloc_zero<float2>((size_t)L.nn * dev::kMaxRhs, stream);
+        gc_mem.push_back((void*)*q);
+    }
+    gc_pack_level0(gc, stream);
+    ++launches;
+    sync();
+    gc_ok = true;
 }
 
 void GpuSolver::free_amg() {
@@ -829,42 +896,62 @@ void GpuSolver::free_amg() {
     gc_ok = false;
 }
 
-// Gradient-space correction over the device hierarchy just built: level 0
-// reads the divergence-correction Laplacian through the node incidence, the
-// coarser levels the hierarchy's CSR operators (both refreshed in place for
-// a new conductivity); FP32 work vectors for up to 16 right-hand sides.
-void GpuSolver::build_gc() {
-    if (!amg_ok || P.precision != 1 || (P.gradcorr != 1 && P.divcorr_mixed != 1)) return;
+// Level-0 data of the node cycles: transfer weights, the packed FP32
+// Laplacian, the result vector, the FP32 PCG's work, the side stream.
+void GpuSolver::gc_common() {
     auto zeros2 = [&](size_t n) {
         float2* p = dalloc_zero<float2>(n, stream);
         gc_mem.push_back((void*)p);
         return p;
     };
+    auto alloc = [&](auto*& p, size_t n) {
+        p = dalloc<std::remove_reference_t<decltype(*p)>>(std::max<size_t>(1, n));
+        gc_mem.push_back((void*)p);
+    };
     const long n_inc = (long)h_inc_other.size();
-    float* inc_g = dalloc<float>((size_t)std::max<long>(1, n_inc));
-    gc_mem.push_back((void*)inc_g);
-    float* e_g = dalloc<float>(2 * (size_t)n_pad);
-    gc_mem.push_back((void*)e_g);
+    float *inc_g, *e_g;
+    alloc(inc_g, (size_t)n_inc);
+    alloc(e_g, 2 * (size_t)n_pad);
     gc_weights(md, inc_g, e_g, stream);
     ++launches;
-    gc.n_levels = amg.n_levels;
     gc.nn = L.nn;
     gc.inc_ptr = md.inc_ptr;
     gc.inc_other = md.inc_other;
     gc.inc_edge = md.inc_edge;
     gc.lap_off = dc.lap_off;
     gc.lap_diag = dc.lap_diag;
+    gc.jac_inv = dc.jac_inv;
     gc.inc_g = inc_g;
-    int2* pk = dalloc<int2>((size_t)std::max<long>(1, n_inc));
-    gc_mem.push_back((void*)pk);
-    float* d32 = dalloc<float>((size_t)L.nn);
-    gc_mem.push_back((void*)d32);
-    gc.lap_pk = pk;
-    gc.lap_diag32 = d32;
-    float* dv32 = dalloc<float>((size_t)L.nn);
-    gc_mem.push_back((void*)dv32);
+    alloc(gc.lap_pk, (size_t)n_inc);
+    alloc(gc.lap_diag32, (size_t)L.nn);
+    alloc(gc.lv[0].dinv32, (size_t)L.nn);
     gc.e_node = md.e_node;
     gc.e_g = e_g;
+    gc.out0 = zeros2((size_t)L.nn * dev::kMaxRhs);
+    if (P.divcorr_mixed == 1) {
+        for (float2** q : {&gc.dc_x, &gc.dc_r, &gc.dc_z, &gc.dc_p, &gc.dc_ap}) *q = zeros2((size_t)L.nn * dev::kMaxRhs);
+        GcPcgState* st = dalloc_zero<GcPcgState>(dev::kMaxRhs, stream);
+        gc_mem.push_back((void*)st);
+        gc.dc_st = st;
+    }
+    gc.omega_max = P.gradcorr == 1 ? 2.0 * kPi * P.gradcorr_fmax : 0.0;
+    gc.inc_entries = n_inc;
+    gc.emg = emg_ok ? &emg : nullptr;
+    if (!gc_stream) {
+        cuda_ok(cudaStreamCreateWithFlags(&gc_stream, cudaStreamNonBlocking), "stream");
+        cuda_ok(cudaEventCreateWithFlags(&gc_fork, cudaEventDisableTiming), "event");
+        cuda_ok(cudaEventCreateWithFlags(&gc_join, cudaEventDisableTiming), "event");
+    }
+}
+
+// Gradient-space correction over the device hierarchy just built: level 0
+// reads the divergence-correction Laplacian through the node incidence, the
+// coarser levels the hierarchy's CSR operators (both refreshed in place for
+// a new conductivity); FP32 work vectors for up to 16 right-hand sides.
+void GpuSolver::build_gc() {
+    if (!amg_ok || P.precision != 1 || (P.gradcorr != 1 && P.divcorr_mixed != 1)) return;
+    gc_common();
+    gc.n_levels = amg.n_levels;
     for (int l = 0; l < amg.n_levels; ++l) {
         const phys::AmgLevelDev& a = amg.lv[l];
         GcLevel& g = gc.lv[l];
@@ -873,35 +960,20 @@ void GpuSolver::build_gc() {
         g.col = a.col;
         g.val = a.val;
         g.dinv = a.dinv;
-        if (l == 0) g.dinv32 = dv32;
         g.agg = a.agg;
         g.rptr = a.rptr;
         g.rcol = a.rcol;
-        const size_t n = (size_t)a.n * dev::kMaxRhs;
-        g.b = zeros2(n);
-        g.x = zeros2(n);
-        g.y = zeros2(n);
-    }
-    gc.out0 = zeros2((size_t)L.nn * dev::kMaxRhs);
-    if (P.divcorr_mixed == 1) {
-        for (float2** q : {&gc.dc_x, &gc.dc_r, &gc.dc_z, &gc.dc_p, &gc.dc_ap}) *q = zeros2((size_t)L.nn * dev::kMaxRhs);
-        GcPcgState* st = dalloc_zero<GcPcgState>(dev::kMaxRhs, stream);
-        gc_mem.push_back((void*)st);
-        gc.dc_st = st;
+        for (float2** q : {&g.b, &g.x, &g.y}) {
+            *q = dalloc_zero<float2>((size_t)a.n * dev::kMaxRhs, stream);
+            gc_mem.push_back((void*)*q);
+        }
     }
     gc.n_coarse = amg.n_coarse;
     gc.coarse_inv = amg.coarse_inv;
     gc.omega = (float)amg.omega;
     gc.presmooth = P.gradcorr_presmooth;
-    gc.omega_max = P.gradcorr == 1 ? 2.0 * kPi * P.gradcorr_fmax : 0.0;
-    gc.inc_entries = n_inc;
     gc_pack_level0(gc, stream);
     ++launches;
-    if (!gc_stream) {
-        cuda_ok(cudaStreamCreateWithFlags(&gc_stream, cudaStreamNonBlocking), "stream");
-        cuda_ok(cudaEventCreateWithFlags(&gc_fork, cudaEventDisableTiming), "event");
-        cuda_ok(cudaEventCreateWithFlags(&gc_join, cudaEventDisableTiming), "event");
-    }
     sync();
     gc_ok = true;
 }
@@ -911,8 +983,12 @@ void GpuSolver::build_gc() {
 // term.  With gradcorr_overlap the node cycles run on the side stream, beside
 // the edge cycle or the forward SSOR sweeps.
 void GpuSolver::attach_gc(KrylovCtx<float>& c, bool multigrid) {
-    c.gc = &gc;
     c.emg = multigrid && emg_ok ? &emg : nullptr;
+    if (!c.emg) {
+        need_amg();
+        if (!amg_ok) return;
+    }
+    c.gc = &gc;
     if (P.gradcorr_overlap == 1) {
         c.gc_stream = gc_stream;
         c.gc_fork = gc_fork;
@@ -1076,8 +1152,8 @@ KrylovCtx<double> GpuSolver::kctx(int K, const int* fmap) const {
         c.B.omega[k] = (k < K && c.B.fmap[k] < (int)fz_freqs.size()) ? 2.0 * kPi * fz_freqs[c.B.fmap[k]] : 0.0;
     }
     c.colour_ptr = colour_ptr;
-    c.colour_list = d_colour_list;
-    c.n_pad = n_pad;
+    c.sweep_rows = d_sweep_rows;
+    c.n_rows_pad = n_pad;
     c.grid_vec = red.max_blocks;
     c.grid_spmv = std::max(2, red.max_blocks / 2);
     c.red = red;
@@ -1139,6 +1215,7 @@ void GpuSolver::factorize(const std::vector<double>& freqs) {
 BatchResult GpuSolver::solve_batch(int K, const int* fmap, double2* b, double2* x, const std::vector<int>& active,
                                    double tol, int maxiter) {
     ensure_vecs(K);
+    ensure_sweeps(seg64);
     KrylovCtx<double> c = kctx(K, fmap);
     KrylovVecs<double> v = kv;
     v.b = b;
@@ -1241,7 +1318,7 @@ void GpuSolver::ensure_vecs32b(int K) {
     kv32b_K = K;
 }
 
-KrylovCtx<float> GpuSolver::kctx32(int K, const int* fmap) const {
+KrylovCtx<float> GpuSolver::kctx32(int K, const int* fmap, bool free_rows) const {
     const KrylovCtx<double> c = kctx(K, fmap);
     KrylovCtx<float> f;
     f.A = OpView<float>{d_op_rp, d_op_rs, d_col, d_val32, n_pad};
@@ -1249,8 +1326,8 @@ KrylovCtx<float> GpuSolver::kctx32(int K, const int* fmap) const {
     f.B = c.B;
     f.B.relax = P.ssor_relax;   // the FP64 context keeps the reference's 1
     f.colour_ptr = c.colour_ptr;
-    f.colour_list = c.colour_list;
-    f.n_pad = c.n_pad;
+    f.sweep_rows = c.sweep_rows;
+    f.n_rows_pad = free_rows ? n_free : n_pad;
     f.grid_vec = c.grid_vec;
     f.grid_spmv = c.grid_spmv;
     f.red = c.red;
@@ -1302,76 +1379,110 @@ void GpuSolver::set_test_consume_no_wait(bool on) {
     sync();
 }
 
-// Slice segments (staged.cuh) of the split operator for both precisions:
-// per 32-row slice a lower and an upper segment, each [uint16 row ends]
-// [int32 columns] [values], every row padded to a multiple of four entries,
-// 16-byte aligned, and one work item per slice in natural and in
-// colour-sweep order.
-void GpuSolver::build_segments(const std::vector<int>& op_rp, const std::vector<int>& op_rs,
-                               const std::vector<int>& ecol, const std::vector<double>& eval) {
-    const int ns = n_slices;
-    auto build = [&](auto tag, std::vector<unsigned char>& buf, std::vector<int4>& work, int& st_lo, int& st_up,
-                     int& st_spmv) {
-        using R = decltype(tag);
-        buf.clear();
-        work.assign((size_t)ns, make_int4(0, 0, 0, 0));
-        st_lo = st_up = st_spmv = 0;
-        auto put = [&](int s, bool upper) -> std::pair<long, int> {
-            const long off = (long)buf.size();
-            uint16_t end[dev::kSlice];
-            std::vector<int> cols;
-            std::vector<R> vals;
-            for (int r = 0; r < dev::kSlice; ++r) {
-                const int row = s * dev::kSlice + r;
-                const int b = upper ? op_rs[row] : op_rp[row];
-                const int e = upper ? op_rp[row + 1] : op_rs[row];
-                for (int k = b; k < e; ++k) { cols.push_back(ecol[k]); vals.push_back((R)eval[k]); }
-                // pad the row to whole groups of four with zero entries on the
-                // row itself (a finite value times zero)
-                while (cols.size() % 4) { cols.push_back(row); vals.push_back((R)0); }
-                if (cols.size() > 65535) throw std::runtime_error("slice segment too large");
-                end[r] = (uint16_t)cols.size();
-            }
-            const size_t n = cols.size();
-            const size_t n4 = (n + 3) & ~(size_t)3;
-            const size_t per = 16 / sizeof(R);
-            const size_t nv = (n + per - 1) / per * per;
-            const size_t bytes = dev::kSegHeader + 4 * n4 + sizeof(R) * nv;
-            buf.resize(off + bytes, 0);
-            std::memcpy(buf.data() + off, end, sizeof(end));
-            std::memcpy(buf.data() + off + dev::kSegHeader, cols.data(), 4 * n);
-            std::memcpy(buf.data() + off + dev::kSegHeader + 4 * n4, vals.data(), sizeof(R) * n);
-            if ((long)(bytes / 16) > 65535) throw std::runtime_error("slice segment too large");
-            return {off / 16, (int)(bytes / 16)};
-        };
-        for (int s = 0; s < ns; ++s) {
-            const auto lo = put(s, false);
-            const auto up = put(s, true);
-            if (lo.first > 2000000000L || up.first > 2000000000L) throw std::runtime_error("mesh too large for segments");
-            work[s] = make_int4(s, (int)lo.first, (int)up.first, (lo.second << 16) | up.second);
-            st_lo = std::max(st_lo, lo.second * 16);
-            st_up = std::max(st_up, up.second * 16);
-            st_spmv = std::max(st_spmv, (lo.second + up.second) * 16);
-        }
-        std::vector<int4> wc(colour_list.size());
-        for (size_t i = 0; i < colour_list.size(); ++i) wc[i] = work[colour_list[i]];
-        work.insert(work.end(), wc.begin(), wc.end());
-    };
-    std::vector<unsigned char> b64, b32;
-    std::vector<int4> w64, w32;
-    int l64, u64, s64, l32, u32, s32;
-    build(double(0), b64, w64, l64, u64, s64);
-    build(float(0), b32, w32, l32, u32, s32);
-    d_seg64 = dupload(b64, stream);
-    d_seg32 = dupload(b32, stream);
-    d_work64 = dupload(w64, stream);
-    d_work32 = dupload(w32, stream);
+namespace {
+
+// Appends one segment (staged.cuh): entries [begin(r), end(r)) of up to 32
+// rows, padded to whole groups of four with zero entries on the row itself (a
+// finite value times zero).  Returns its offset and length in 16-byte units.
+template <class R, class Rows>
+std::pair<long, int> put_segment(std::vector<unsigned char>& buf, const std::vector<int>& ecol,
+                                 const std::vector<double>& eval, const Rows& rows) {
+    const long off = (long)buf.size();
+    uint16_t end[dev::kSlice];
+    std::vector<int> cols;
+    std::vector<R> vals;
+    for (int r = 0; r < dev::kSlice; ++r) {
+        int row, b, e;
+        rows(r, row, b, e);
+        for (int k = b; k < e; ++k) { cols.push_back(ecol[k]); vals.push_back((R)eval[k]); }
+        while (cols.size() % 4) { cols.push_back(row); vals.push_back((R)0); }
+        if (cols.size() > 65535) throw std::runtime_error("slice segment too large");
+        end[r] = (uint16_t)cols.size();
+    }
+    const size_t n = cols.size();
+    const size_t bytes = dev::kSegHeader + (4 + sizeof(R)) * n;
+    buf.resize(off + bytes, 0);
+    std::memcpy(buf.data() + off, end, sizeof(end));
+    std::memcpy(buf.data() + off + dev::kSegHeader, cols.data(), 4 * n);
+    std::memcpy(buf.data() + off + dev::kSegHeader + 4 * n, vals.data(), sizeof(R) * n);
+    if ((long)(bytes / 16) > 65535) throw std::runtime_error("slice segment too large");
+    if (off / 16 > 2000000000L) throw std::runtime_error("mesh too large for segments");
+    return {off / 16, (int)(bytes / 16)};
+}
+
+}  // namespace
+
+// Row segments of both precisions (the FP32 ones for the free rows, which are
+// all the inner solve's products read, and the rest for FGMRES).
+void GpuSolver::build_row_segments(const std::vector<int>& op_rp, const std::vector<int>& ecol,
+                                   const std::vector<double>& eval) {
     d_seg_err = dalloc<unsigned>(1);
     cuda_ok(cudaMemsetAsync(d_seg_err, 0, sizeof(unsigned), stream), "memset");
-    seg64 = dev::SegView<double>{d_seg64, d_work64, d_work64 + ns, s64, l64, u64, d_seg_err};
-    seg32 = dev::SegView<float>{d_seg32, d_work32, d_work32 + ns, s32, l32, u32, d_seg_err};
     dc.seg_err = d_seg_err;
+    auto build = [&](auto& view, unsigned char*& d_seg, int*& d_off) {
+        using R = typename std::decay_t<decltype(view)>::Real;
+        std::vector<unsigned char> buf;
+        std::vector<int> off(n_slices + 1, 0);
+        buf.reserve(((size_t)op_rp[n_pad] + 2 * (size_t)n_pad) * (4 + sizeof(R)));
+        for (int s = 0; s < n_slices; ++s) {
+            off[s] = (int)put_segment<R>(buf, ecol, eval, [&](int r, int& row, int& b, int& e) {
+                row = s * dev::kSlice + r;
+                b = op_rp[row];
+                e = op_rp[row + 1];
+            }).first;
+            off[s + 1] = (int)(buf.size() / 16);
+        }
+        view = std::decay_t<decltype(view)>{};
+        for (int j = 0; j < 5; ++j)
+            for (int s = 0; s < n_slices; s += 1 << j)
+                view.stage_row[j] = std::max(view.stage_row[j], (off[std::min(s + (1 << j), n_slices)] - off[s]) * 16);
+        d_seg = dupload(buf, stream);
+        d_off = dupload(off, stream);
+        sync();
+        view.row_seg = d_seg;
+        view.row_off = d_off;
+        view.rows = d_sweep_rows;
+        view.err = d_seg_err;
+    };
+    build(seg64, d_row_seg64, d_row_off64);
+    build(seg32, d_row_seg32, d_row_off32);
 }
+
+// Sweep segments of one precision, built when the first SSOR solve of that
+// precision asks for them (at setup where that is the preconditioner).
+template <class R>
+void GpuSolver::ensure_sweeps(dev::SegView<R>& view) {
+    if (view.seg) return;
+    std::vector<int> rp, rs, ecol;
+    std::vector<double> eval;
+    split_csr(rp, rs, ecol, eval);
+    const int ns = (int)(sweep_rows.size() / dev::kSlice);
+    std::vector<unsigned char> buf;
+    buf.reserve(((size_t)rp[n_pad] + 4 * (size_t)n_pad) * (4 + sizeof(R)));
+    std::vector<int4> work(ns);
+    for (int s = 0; s < ns; ++s) {
+        auto part = [&](bool upper) {
+            return put_segment<R>(buf, ecol, eval, [&](int r, int& row, int& b, int& e) {
+                row = sweep_rows[(size_t)s * dev::kSlice + r];
+                b = upper ? rs[row] : rp[row];
+                e = upper ? rp[row + 1] : rs[row];
+            });
+        };
+        const auto lo = part(false), up = part(true);
+        work[s] = make_int4(s, (int)lo.first, (int)up.first, (lo.second << 16) | up.second);
+        view.stage_lo = std::max(view.stage_lo, lo.second * 16);
+        view.stage_up = std::max(view.stage_up, up.second * 16);
+    }
+    unsigned char* seg = dupload(buf, stream);
+    sweep_mem.push_back((void*)seg);
+    int4* wk = dupload(work, stream);
+    sweep_mem.push_back((void*)wk);
+    sync();
+    view.work_col = wk;
+    view.seg = seg;
+}
+template void GpuSolver::ensure_sweeps<float>(dev::SegView<float>&);
+template void GpuSolver::ensure_sweeps<double>(dev::SegView<double>&);
 
 // Mixed precision: each step computes r = b - A x in FP64, solves A d = r
 // with the complex-FP32 batched BiCGStab (scaled to unit norm, relative
@@ -1469,6 +1580,14 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
     const int max_steps = 2 + std::max(0, P.max_refinements) * 4;
     auto pow2_at_least = [](int n) { int k = 2; while (k < n) k *= 2; return k; };
     auto launch_grid = [](long n) { return (int)((n + 255) / 256); };
+    // identity rows: x = b, exactly; the FP32 solve runs over the free rows
+    {
+        LaneMask on{};
+        for (int k = 0; k < K; ++k) on.v[k] = active[k] != 0;
+        const long n = (long)(n_pad - n_free) * K;
+        k_identity_rows<<<launch_grid(n), 256, 0, stream>>>(x + (size_t)n_free * K, b + (size_t)n_free * K, K, n, on);
+        ++launches;
+    }
     for (int step = 0; step <= max_steps; ++step) {
         // FP64 true residual y = b - A x
         for (int k = 0; k < K; ++k) {
@@ -1546,8 +1665,8 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
                 d = v.sh;
             }
             cuda_ok(cudaMemcpyAsync(d_lane_add, add.data(), sizeof(int) * dev::kMaxRhs, cudaMemcpyHostToDevice, stream), "add");
-            k_add_f32_lanes<<<launch_grid((long)n_pad * Kn), 256, 0, stream>>>(x, K, d, Kn, d_lane_map, d_lane_add,
-                                                                           d_scale, (long)n_pad);
+            k_add_f32_lanes<<<launch_grid((long)n_free * Kn), 256, 0, stream>>>(x, K, d, Kn, d_lane_map, d_lane_add,
+                                                                           d_scale, (long)n_free);
             ++launches;
         };
         auto replace_lanes = [&](int Kn, const KrylovVecs<float>& v) {
@@ -1556,7 +1675,7 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
     {                                                                                                          \
         auto kf = k_replace_lanes<KC>;                                                                         \
         kf<<<wave_grid(kf, red.max_blocks, 256), 256, 0, stream>>>(kv.y, K, v.r, v.x, v.r0, d_lane_map,        \
-                                                                   d_lane_add, d_scale, (long)n_pad, d_states, \
+                                                                   d_lane_add, d_scale, (long)n_free, d_states, \
                                                                    red);                                       \
     }
             switch (Kn) {
@@ -1570,9 +1689,9 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
             ++launches;
         };
         upload_lanes(Kc);
-        k_to_f32_lanes<<<launch_grid((long)n_pad * Kc), 256, 0, stream>>>(kv.y, K, cur.b, Kc, d_lane_map, d_scale,
-                                                                      (long)n_pad);
-        cuda_ok(cudaMemsetAsync(cur.x, 0, sizeof(float2) * (size_t)n_pad * Kc, stream), "memset");
+        k_to_f32_lanes<<<launch_grid((long)n_free * Kc), 256, 0, stream>>>(kv.y, K, cur.b, Kc, d_lane_map, d_scale,
+                                                                      (long)n_free);
+        cuda_ok(cudaMemsetAsync(cur.x, 0, sizeof(float2) * (size_t)n_free * Kc, stream), "memset");
         launches += 2;
         std::vector<BicgState> ls(Kc);
         for (int j = 0; j < Kc; ++j) {
@@ -1587,6 +1706,7 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
             ls[j].status = kRunning;
         }
         cuda_ok(cudaMemcpyAsync(d_states, ls.data(), sizeof(BicgState) * Kc, cudaMemcpyHostToDevice, stream), "states");
+        if (!(use_gc && multigrid)) ensure_sweeps(seg32);
         KrylovCtx<float> c32 = kctx32(Kc, fm.data());
         if (use_gc) attach_gc(c32, multigrid);
         if (eis) eis_init(c32, cur, d_states);
@@ -1661,7 +1781,7 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
                 const float2* srcs[5] = {cur.x, cur.r, cur.r0, cur.p, cur.v};
                 float2* dsts[5] = {other.x, other.r, other.r0, other.p, other.v};
                 for (int v = 0; v < 5; ++v) { mv.src[v] = srcs[v]; mv.dst[v] = dsts[v]; }
-                k_gather_lanes<<<launch_grid((long)n_pad * Kn), 256, 0, stream>>>(mv, Kc, Kn, d_lane_sel, (long)n_pad);
+                k_gather_lanes<<<launch_grid((long)n_free * Kn), 256, 0, stream>>>(mv, Kc, Kn, d_lane_sel, (long)n_free);
                 ++launches;
                 lanes = nl;
                 ls = ns;
@@ -2472,6 +2592,7 @@ std::vector<TuneEntry> GpuSolver::autotune(double freq, int max_K, int reps) {
     max_K = std::max(2, std::min(dev::kMaxRhs, max_K));
     factorize(std::vector<double>{freq});
     ensure_vecs32(max_K);
+    ensure_sweeps(seg32);
     const double om = 2.0 * kPi * freq;
     const bool use_gc = gc_ok && P.gradcorr == 1 && gc.omega_max > 0.0 && om <= gc.omega_max;
     const int rk_saved = P.row_kernels;

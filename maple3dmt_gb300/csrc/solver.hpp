@@ -152,12 +152,14 @@ private:
     long long launches = 0;
 
     // host-side structure
-    std::vector<int> perm, iperm, colour_ptr, colour_list;
-    int* d_colour_list = nullptr;
+    std::vector<int> perm, iperm, colour_ptr, sweep_rows;
+    std::vector<int> edge_group;        // SSOR sweep group of every edge
+    int* d_sweep_rows = nullptr;        // 32 rows of every sweep slice
     int* d_colour_ptr = nullptr;        // device copy of colour_ptr (cooperative sweeps)
     unsigned* d_gridbar = nullptr;      // grid barrier of the cooperative sweeps
     std::vector<unsigned char> flags_ref;  // reference order
     int n_pad = 0, n_slices = 0;
+    int n_free = 0;                     // the free rows are the first n_free (padding included)
     bool hp_sequential = false;
 
     // device mesh
@@ -166,8 +168,9 @@ private:
     double* d_val = nullptr;
     float* d_val32 = nullptr;
     // slice-staged segments of the same operator (staged.cuh), per precision
-    unsigned char *d_seg64 = nullptr, *d_seg32 = nullptr;
-    int4 *d_work64 = nullptr, *d_work32 = nullptr;   // [n_slices] natural order, then colour order
+    unsigned char *d_row_seg64 = nullptr, *d_row_seg32 = nullptr;
+    int *d_row_off64 = nullptr, *d_row_off32 = nullptr;
+    std::vector<void*> sweep_mem;
     dev::SegView<double> seg64{};
     dev::SegView<float> seg32{};
     unsigned* d_seg_err = nullptr;
@@ -191,6 +194,10 @@ private:
     bool gc_ok = false;
     std::vector<void*> gc_mem;
     void build_gc();
+    void build_gc0();
+    void gc_common();
+    bool amg_stale = false;   // emg_ok: the aggregation hierarchy is not that of the current conductivity
+    void need_amg();
     // geometric multigrid preconditioner of the FP32 inner solve
     EmgDev emg{};
     bool emg_ok = false;
@@ -215,8 +222,10 @@ private:
                                                                                                      : nullptr;
     }
     int* d_lap_qpos = nullptr;    // incidence -> value slot in dc.lap_seg
-    void build_segments(const std::vector<int>& op_rp, const std::vector<int>& op_rs, const std::vector<int>& ecol,
-                        const std::vector<double>& eval);
+    void split_csr(std::vector<int>& rp, std::vector<int>& rs, std::vector<int>& col, std::vector<double>& val) const;
+    void build_row_segments(const std::vector<int>& op_rp, const std::vector<int>& ecol,
+                            const std::vector<double>& eval);
+    template <class R> void ensure_sweeps(dev::SegView<R>& view);
     void check_seg_err();
 
     // sigma
@@ -289,7 +298,7 @@ private:
     void ensure_dc(int K);
     void ensure_hc(int nf);
     KrylovCtx<double> kctx(int K, const int* fmap) const;
-    KrylovCtx<float> kctx32(int K, const int* fmap) const;
+    KrylovCtx<float> kctx32(int K, const int* fmap, bool free_rows = true) const;
     void ensure_vecs32(int K);
     // FP32 BiCGStab on the residual equation inside FP64 refinement
     BatchResult solve_batch_mixed(int K, const int* fmap, double2* b, double2* x, const std::vector<int>& active,
