@@ -64,6 +64,42 @@ __device__ __forceinline__ double2 shfl_xor(double2 v, int m) {
     return v;
 }
 
+// A complex sum in the making, 16 bytes: FP64 for FP64 terms; for FP32 terms
+// two floats per part (Knuth's error-free sum of the high parts, 48 bits
+// kept).  An FP64 add holds a warp's pipe for 16 cycles on this GPU and a chain
+// of them is slow: summing lanes, warps and blocks in FP64 was 10 to 25 us of
+// every reducing FP32 kernel.
+template <class R> struct Sum;
+template <> struct Sum<double> {
+    double2 v;
+    __device__ __forceinline__ void set(double2 a) { v = a; }
+    __device__ __forceinline__ void add(const Sum& o) { v = cadd(v, o.v); }
+    __device__ __forceinline__ Sum xor_lane(int m) const { return {shfl_xor(v, m)}; }
+    __device__ __forceinline__ double2 get() const { return v; }
+};
+template <> struct Sum<float> {
+    float4 v;   // x high, x low, y high, y low
+    __device__ __forceinline__ void set(float2 a) { v = make_float4(a.x, 0.0f, a.y, 0.0f); }
+    static __device__ __forceinline__ void add1(float& h, float& l, float h2, float l2) {
+        const float s = __fadd_rn(h, h2), b = __fsub_rn(s, h);
+        float e = __fadd_rn(__fsub_rn(h, __fsub_rn(s, b)), __fsub_rn(h2, b));
+        e = __fadd_rn(e, __fadd_rn(l, l2));
+        h = __fadd_rn(s, e);
+        l = __fsub_rn(e, __fsub_rn(h, s));
+    }
+    __device__ __forceinline__ void add(const Sum& o) {
+        add1(v.x, v.y, o.v.x, o.v.y);
+        add1(v.z, v.w, o.v.z, o.v.w);
+    }
+    __device__ __forceinline__ Sum xor_lane(int m) const {
+        return {make_float4(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m),
+                            __shfl_xor_sync(0xffffffffu, v.z, m), __shfl_xor_sync(0xffffffffu, v.w, m))};
+    }
+    __device__ __forceinline__ double2 get() const {
+        return make_double2((double)v.x + (double)v.y, (double)v.z + (double)v.w);
+    }
+};
+
 // Blocks of `threads` threads with `smem` bytes of dynamic shared memory of
 // `kernel` that are resident on the current device at once (occupancy API x
 // SM count); cached per (device, kernel, threads, smem).
@@ -149,43 +185,48 @@ __device__ bool grid_reduce(const double2 (&acc)[KT][NQ], int rhs0, RedScratch r
     return true;
 }
 
-// Grid reduction for kernels whose lane l always works on right-hand side
-// l % K (K a power of two <= 32, blockDim a multiple of 32): a shuffle tree
-// over the lanes that share a right-hand side, warps combined in warp order,
-// blocks in block order by the last block to arrive (each of the NQ*K totals
-// summed by a fixed set of threads, then in a fixed order).  Deterministic
-// for a fixed launch shape.  Returns true in the last block, where
-// out[q * K + k] (shared, NQ*K entries) holds the totals.
-//
-// LPT: neighbouring right-hand sides per thread (lane l works on LPT (l % (K /
-// LPT)) and the next ones), acc[j] for the j-th of them.
-template <int NQ, int K, int NT, int LPT>
-__device__ bool grid_reduce_multi(double2 (&acc)[LPT][NQ], RedScratch rs, double2* out) {
+// Grid reduction for kernels whose lane l always works on the same right-hand
+// sides: LPT neighbouring ones per thread, LPT (l % (K / LPT)) and the next
+// (K and LPT powers of two, whole warps); acc[j][q] is quantity q of the j-th
+// of them in the kernel's working precision.  Shuffle trees over the lanes that
+// share a right-hand side, then over the block's warps (one warp per total),
+// then, in the last block to arrive, over the blocks: every step in a fixed
+// order, so the result is deterministic for a fixed launch shape.  Returns true
+// in the last block, where out[q * K + k] (shared, NQ*K entries) holds the
+// totals.
+template <int NQ, int K, int NT, int LPT, class C>
+__device__ bool grid_reduce_multi(const C (&acc)[LPT][NQ], RedScratch rs, double2* out) {
     static_assert(K >= LPT && K <= 32 && (K & (K - 1)) == 0, "K must be a power of two <= 32");
-    static_assert(NT % 32 == 0 && NT >= 32, "block size must be whole warps");
+    static_assert(NT % 32 == 0 && NT >= 32 && NT <= 1024, "block size must be whole warps");
+    using S = Sum<decltype(C{}.x)>;
+    static_assert(sizeof(S) == sizeof(double2), "partials are 16 bytes");
     constexpr int PK = NQ * K;
     constexpr int NW = NT / 32;
-    __shared__ double2 sm[NW][PK];
-    __shared__ double2 chunk[NT];
+    __shared__ S sm[NW][PK];
     __shared__ bool am_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int off = 16; off >= K / LPT; off >>= 1)
+    for (int j = 0; j < LPT; ++j)
 #pragma unroll
-        for (int j = 0; j < LPT; ++j)
+        for (int q = 0; q < NQ; ++q) {
+            S s;
+            s.set(acc[j][q]);
 #pragma unroll
-            for (int q = 0; q < NQ; ++q) acc[j][q] = cadd(acc[j][q], shfl_xor(acc[j][q], off));
-    if (lane < K / LPT)
-#pragma unroll
-        for (int j = 0; j < LPT; ++j)
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) sm[warp][q * K + lane * LPT + j] = acc[j][q];
+            for (int off = 16; off >= K / LPT; off >>= 1) s.add(s.xor_lane(off));
+            if (lane < K / LPT) sm[warp][q * K + lane * LPT + j] = s;
+        }
     __syncthreads();
-    if (threadIdx.x < PK) {
-        double2 s = make_double2(0.0, 0.0);
-        for (int w = 0; w < NW; ++w) s = cadd(s, sm[w][threadIdx.x]);
-        __stcg(&rs.partial[(size_t)blockIdx.x * PK + threadIdx.x], s);
-        __threadfence();
+    S zero;
+    zero.set(C{});
+    S* partial = reinterpret_cast<S*>(rs.partial);
+    for (int p = warp; p < PK; p += NW) {
+        S s = lane < NW ? sm[lane][p] : zero;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) s.add(s.xor_lane(off));
+        if (lane == 0) {
+            __stcg(reinterpret_cast<double2*>(&partial[(size_t)blockIdx.x * PK + p]), *reinterpret_cast<double2*>(&s));
+            __threadfence();
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -195,29 +236,25 @@ __device__ bool grid_reduce_multi(double2 (&acc)[LPT][NQ], RedScratch rs, double
     __syncthreads();
     if (!am_last) return false;
     __threadfence();
-    constexpr int CH = NT / PK > 0 ? NT / PK : 1;   // threads per total
-    const int p = threadIdx.x % PK, j = threadIdx.x / PK;
-    // eight loads in flight: one at a time, the last block's walk over the
-    // partials was 10 us of every reducing kernel
-    double2 s = make_double2(0.0, 0.0);
-    if (j < CH)
-        for (int b = j; b < (int)gridDim.x; b += 8 * CH) {
-            double2 v[8];
+    for (int p = warp; p < PK; p += NW) {
+        S s = zero;
+        for (int b = lane; b < (int)gridDim.x; b += 4 * 32) {   // four loads in flight
+            double2 v[4];
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-                v[u] = b + u * CH < (int)gridDim.x ? __ldcg(&rs.partial[(size_t)(b + u * CH) * PK + p])
-                                                   : make_double2(0.0, 0.0);
+            for (int u = 0; u < 4; ++u)
+                v[u] = b + 32 * u < (int)gridDim.x
+                           ? __ldcg(reinterpret_cast<const double2*>(&partial[(size_t)(b + 32 * u) * PK + p]))
+                           : make_double2(0.0, 0.0);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) s = cadd(s, v[u]);
+            for (int u = 0; u < 4; ++u) s.add(*reinterpret_cast<const S*>(&v[u]));
         }
-    chunk[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x < PK) {
-        double2 t = make_double2(0.0, 0.0);
-#pragma unroll 8
-        for (int jj = 0; jj < CH; ++jj) t = cadd(t, chunk[jj * PK + threadIdx.x]);
-        out[threadIdx.x] = t;
-        rs.final_[threadIdx.x] = t;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) s.add(s.xor_lane(off));
+        if (lane == 0) {
+            const double2 t = s.get();
+            out[p] = t;
+            rs.final_[p] = t;
+        }
     }
     if (threadIdx.x == 0) *rs.counter = 0u;
     __syncthreads();
@@ -225,18 +262,21 @@ __device__ bool grid_reduce_multi(double2 (&acc)[LPT][NQ], RedScratch rs, double
 }
 
 // Blocks of a reducing vector kernel over n elements: one resident wave at
-// most, and at least four elements a thread -- on small vectors the walk over
-// more partials costs more than the extra blocks save.
+// most and four elements a thread at least, and beyond two blocks per SM (152
+// of them) 16 elements a thread: the last block's FP64 walk over the blocks'
+// partials (a cycle per pair of adds) costs small vectors more than the extra
+// blocks save.
 template <class F>
-inline int reduce_grid(F* kernel, int cap, long n) {
-    const long b = (n + 4 * kBlock - 1) / (4 * kBlock);
-    const int w = wave_grid(kernel, cap);
+inline int reduce_grid(F* kernel, int cap, long n, int threads = kBlock) {
+    const long lo = (n + 4L * threads - 1) / (4L * threads), hi = (n + 16L * threads - 1) / (16L * threads);
+    const long b = lo < 304 ? lo : hi < 304 ? 304 : hi;
+    const int w = wave_grid(kernel, cap, threads);
     return (int)(b < 1 ? 1 : b < w ? b : w);
 }
 
 template <int NQ, int K, int NT = kBlock>
 __device__ __forceinline__ bool grid_reduce_lanes(double2 (&acc)[NQ], RedScratch rs, double2* out) {
-    return grid_reduce_multi<NQ, K, NT, 1>(*reinterpret_cast<double2(*)[1][NQ]>(&acc), rs, out);
+    return grid_reduce_multi<NQ, K, NT, 1>(*reinterpret_cast<const double2(*)[1][NQ]>(&acc), rs, out);
 }
 
 }  // namespace dev

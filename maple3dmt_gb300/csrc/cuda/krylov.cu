@@ -179,7 +179,11 @@ template <class C> __device__ __forceinline__ C smooth_scale(C d) {
 // run by thread k < K of the last block of each reduction.
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ double cabs_(double2 z) { return hypot(z.x, z.y); }
+// |z| < 1e-30, the reference's breakdown tests; the modulus only where a part
+// does not settle it
+__device__ __forceinline__ bool vanishes(double2 z) {
+    return fabs(z.x) < 1e-30 && fabs(z.y) < 1e-30 && hypot(z.x, z.y) < 1e-30;
+}
 
 // r = b - A x0; r0 = r: |b|^2, |r|^2, (r0, r)   (bicgstab.cpp:24-41, :51)
 __device__ void ep_init(BicgState& S, const double2* out, int k, int K) {
@@ -198,14 +202,14 @@ __device__ void ep_init(BicgState& S, const double2* out, int k, int K) {
     S.rho_old = make_double2(1.0, 0.0);
     S.alpha = make_double2(1.0, 0.0);
     S.omega = make_double2(1.0, 0.0);
-    if (cabs_(S.rho) < 1e-30) { S.status = kBreakdown; S.breakdown = 1; S.iter = 1; }
+    if (vanishes(S.rho)) { S.status = kBreakdown; S.breakdown = 1; S.iter = 1; }
 }
 
 // (r0, v) -> alpha   (bicgstab.cpp:79-87)
 __device__ void ep_r0v(BicgState& S, const double2* out, int k, int K) {
     if (S.status != kRunning) return;
     const double2 r0v = out[k];
-    if (cabs_(r0v) < 1e-30) {
+    if (vanishes(r0v)) {
         S.status = kBreakdown; S.breakdown = 2; S.iter += 1; S.res = S.rnorm / S.bnorm;
         return;
     }
@@ -225,7 +229,7 @@ __device__ void ep_s(BicgState& S, const double2* out, int k, int K) {
 __device__ void ep_omega(BicgState& S, const double2* out, int k, int K) {
     if (S.status != kRunning) return;
     const double2 tt = out[0 * K + k], ts = out[1 * K + k];
-    if (cabs_(tt) < 1e-30) {
+    if (vanishes(tt)) {
         S.status = kBreakdown; S.breakdown = 3; S.pend_x = 1; S.iter += 1; S.res = S.snorm / S.bnorm;
         return;
     }
@@ -241,11 +245,11 @@ __device__ void ep_xr(BicgState& S, const double2* out, int k, int K) {
     const double rel = S.rnorm / S.bnorm;
     S.res = rel;
     if (rel < S.tol) { S.status = kConverged; return; }
-    if (cabs_(S.omega) < 1e-30) { S.status = kBreakdown; S.breakdown = 4; return; }
+    if (vanishes(S.omega)) { S.status = kBreakdown; S.breakdown = 4; return; }
     S.rho_old = S.rho;
     S.rho = out[1 * K + k];
     if (S.iter >= S.maxiter) { S.status = kMaxIter; return; }
-    if (cabs_(S.rho) < 1e-30) { S.status = kBreakdown; S.breakdown = 1; return; }
+    if (vanishes(S.rho)) { S.status = kBreakdown; S.breakdown = 1; return; }
     S.beta = cmul(cdiv(S.rho, S.rho_old), cdiv(S.alpha, S.omega));
 }
 
@@ -417,19 +421,16 @@ __global__ void __launch_bounds__(kBlock) k_ssor_bwd(OpView<R> A, DiagView<R> D,
 
 // Launch shape of the row-staged SpMV: a thread works on one row and, in
 // complex FP32, on two neighbouring right-hand sides (16-byte gathers: half
-// the load instructions of one right-hand side per thread); 256 threads cover
-// ROWS rows a pass, a stage holds T slices = PASSES passes.
+// the load instructions of one right-hand side per thread).  One block per SM
+// of CW consumer warps (24 at 80 registers in complex FP32, 16 in FP64) and a
+// producer warp; a stage is T <= T_MAX slices, one row per thread group.
 template <class R, int K> struct SpmvShape {
-    static constexpr int NT = 256;
+    static constexpr int CW = sizeof(R) == 4 ? 24 : 16;
+    static constexpr int NT = (CW + 1) * 32;
     static constexpr int LPT = sizeof(R) == 4 ? 2 : 1;
     static constexpr int TPR = K / LPT;              // threads per row
-    static constexpr int ROWS = NT / TPR;
-    static constexpr int T = ROWS >= 128 ? ROWS / 32 : ROWS >= 64 ? 4 : ROWS >= 32 ? 2 : 1;
-    static constexpr int PASSES = T * kSlice / ROWS;
-    static constexpr int LOG_T = T == 1 ? 0 : T == 2 ? 1 : T == 4 ? 2 : T == 8 ? 3 : 4;
-    // 24 resident warps of complex FP32 (85 registers, twelve gathers in
-    // flight per thread), 16 of FP64
-    static constexpr int MIN_BLOCKS = sizeof(R) == 4 ? 3 : 2;
+    static constexpr int T_MAX = CW / TPR;           // slices of 32 rows per pass
+    static constexpr int RING = K == 16 ? 6 : K == 8 ? 4 : K == 4 ? 3 : 2;
 };
 
 // The LPT right-hand sides of one thread.
@@ -439,12 +440,12 @@ template <class R, int LPT> struct alignas(LPT * 2 * sizeof(R)) CVec {
 
 // SpMV over row segments, same modes and reductions as k_spmv.  The rows are
 // in the octree's cell order and every block owns a contiguous range of them,
-// so most gathers hit the SM's L1 (see tile_pipeline): at K = 8 on the
-// 1.7 M-edge mesh the pass over colour-sorted slices dealt out to the blocks
-// in turn took 200 us, bound by L2 gathers (13 rows of 64 bytes per row).
+// so most gathers hit the SM's L1 (see tile_ring): at K = 8 on the 1.7 M-edge
+// mesh the pass over colour-sorted slices dealt out to the blocks in turn took
+// 200 us, bound by L2 gathers (13 rows of 64 bytes per row).
 template <class R, int K, int MODE>
-__global__ void __launch_bounds__(SpmvShape<R, K>::NT, SpmvShape<R, K>::MIN_BLOCKS)
-    k_spmv_st(SegView<R> S, int n_slices, DiagView<R> D, BatchView B, const cplx<R>* __restrict__ x,
+__global__ void __launch_bounds__(SpmvShape<R, K>::NT, 1)
+    k_spmv_st(SegView<R> S, int n_slices, int T, DiagView<R> D, BatchView B, const cplx<R>* __restrict__ x,
               cplx<R>* __restrict__ y, const cplx<R>* __restrict__ aux, cplx<R>* __restrict__ aux_out, BicgState* st,
               RedScratch rs) {
     using C = cplx<R>;
@@ -462,21 +463,35 @@ __global__ void __launch_bounds__(SpmvShape<R, K>::NT, SpmvShape<R, K>::MIN_BLOC
     for (int j = 0; j < Sh::LPT; ++j)
 #pragma unroll
         for (int q = 0; q < NQ; ++q) accR[j][q] = cm<R>(0, 0);
-    tile_pipeline<Sh::T>(S.row_seg, S.row_off, n_slices, S.stage_row[Sh::LOG_T], S.err,
-                         [&](int tile, const unsigned char* base) {
-        const int s0 = tile * Sh::T, a0 = __ldg(&S.row_off[s0]);
-#pragma unroll
-        for (int ps = 0; ps < Sh::PASSES; ++ps) {
-            const int lr = ps * Sh::ROWS + r0, sl = s0 + lr / kSlice;
-            if (sl >= n_slices) continue;
+    // this thread's own values of a tile, loaded before its matrix is waited for
+    struct Own {
+        V x, a;
+        C dm;
+        int at;   // 16-byte offset of the slice's segment in the stage, -1: no row
+    };
+    auto own = [&](int tile) {
+        Own o{};
+        const int s0 = tile * T, sl = s0 + r0 / kSlice;
+        o.at = -1;
+        if (r0 < T * kSlice && sl < n_slices) {
+            const size_t i = (size_t)(s0 * kSlice + r0) * Sh::TPR + h;
+            o.x = xv[i];
+            if (MODE != kSpmvPlain) o.a = reinterpret_cast<const V*>(aux)[i];
+            o.dm = D.sm[s0 * kSlice + r0];
+            o.at = __ldg(&S.row_off[sl]) - __ldg(&S.row_off[s0]);
+        }
+        return o;
+    };
+    tile_ring<Sh::CW, Sh::RING>(S.row_seg, S.row_off, n_slices, T, S.stage_row[T], S.err, own,
+                                [&](int tile, const Own& o, const unsigned char* base) {
+        if (o.at < 0) return;
+        {
             SegRows<R> A;
-            A.bind(base + (size_t)(__ldg(&S.row_off[sl]) - a0) * 16);
-            const int row = s0 * kSlice + lr;
-            const size_t i = (size_t)row * Sh::TPR + h;
-            const V xi = xv[i];
-            V av{};
-            if (MODE != kSpmvPlain) av = reinterpret_cast<const V*>(aux)[i];
-            const cplx<R> dm = D.sm[row];
+            A.bind(base + (size_t)o.at * 16);
+            const int lr = r0;
+            const size_t i = (size_t)(tile * T * kSlice + r0) * Sh::TPR + h;
+            const V xi = o.x, av = o.a;
+            const C dm = o.dm;
             V s{};
             int k = A.begin_of(lr % kSlice);
             const int e = A.end[lr % kSlice];
@@ -556,14 +571,8 @@ __global__ void __launch_bounds__(SpmvShape<R, K>::NT, SpmvShape<R, K>::MIN_BLOC
         }
     });
     if (!REDUCE) return;
-    double2 acc[Sh::LPT][NQ];
-#pragma unroll
-    for (int j = 0; j < Sh::LPT; ++j)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) acc[j][q] = to_d(accR[j][q]);
     __shared__ double2 out[NQ * K];
-    __syncthreads();
-    if (grid_reduce_multi<NQ, K, Sh::NT, Sh::LPT>(acc, rs, out)) {
+    if (grid_reduce_multi<NQ, K, Sh::NT, Sh::LPT>(accR, rs, out)) {
         if (threadIdx.x < K) {
             BicgState T = st[threadIdx.x];
             if (MODE == kSpmvAp) ep_r0v(T, out, threadIdx.x, K);
@@ -745,52 +754,84 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
 }
 
 // ---------------------------------------------------------------------------
-// Vector updates (thread per element (row, rhs); rhs = element % K is fixed
-// per thread because the grid stride is a multiple of K).
+// Vector updates: a thread takes LPT neighbouring right-hand sides of a row
+// (two in complex FP32, 16-byte accesses), the same ones throughout because
+// the grid stride is a multiple of K.
 // ---------------------------------------------------------------------------
+constexpr int kVecNT = 512;
+template <class R> constexpr int kVecLpt = sizeof(R) == 4 ? 2 : 1;
 
 // p = r (first iteration) or r + beta (p - omega v)   (bicgstab.cpp:60-67)
 template <class R, int K>
-__global__ void __launch_bounds__(kBlock) k_update_p(long n, const cplx<R>* __restrict__ r,
-                                                     cplx<R>* __restrict__ p, const cplx<R>* __restrict__ v,
+__global__ void __launch_bounds__(kVecNT) k_update_p(long n, const cplx<R>* __restrict__ r_,
+                                                     cplx<R>* __restrict__ p_, const cplx<R>* __restrict__ v_,
                                                      const BicgState* __restrict__ st) {
     using C = cplx<R>;
+    constexpr int LPT = kVecLpt<R>;
+    using V = CVec<R, LPT>;
+    const V *r = reinterpret_cast<const V*>(r_), *v = reinterpret_cast<const V*>(v_);
+    V* p = reinterpret_cast<V*>(p_);
     const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long stride = (long)gridDim.x * blockDim.x;
-    if (i0 >= n) return;
-    const BicgState S = st[i0 % K];
-    const bool run = S.status == kRunning;
-    const bool first = S.iter == 0;
-    const C beta = from_d<C>(S.beta), om = from_d<C>(S.omega);
-    for (long i = i0; i < n; i += stride) {
-        if (!run) { p[i] = cm<R>(0, 0); continue; }
-        if (first) { p[i] = r[i]; continue; }
-        p[i] = cadd(r[i], cmul(beta, csub(p[i], cmul(om, v[i]))));
+    const long stride = (long)gridDim.x * blockDim.x, m = n / LPT;
+    if (i0 >= m) return;
+    C beta[LPT], om[LPT];
+    bool run[LPT], first[LPT];
+#pragma unroll
+    for (int j = 0; j < LPT; ++j) {
+        const BicgState& S = st[(i0 * LPT + j) % K];
+        run[j] = S.status == kRunning;
+        first[j] = S.iter == 0;
+        beta[j] = from_d<C>(S.beta);
+        om[j] = from_d<C>(S.omega);
+    }
+    for (long i = i0; i < m; i += stride) {
+        const V rv = r[i], vv = v[i];
+        V pv = p[i];
+#pragma unroll
+        for (int j = 0; j < LPT; ++j) {
+            if (!run[j]) pv.v[j] = cm<R>(0, 0);
+            else if (first[j]) pv.v[j] = rv.v[j];
+            else pv.v[j] = cadd(rv.v[j], cmul(beta[j], csub(pv.v[j], cmul(om[j], vv.v[j]))));
+        }
+        p[i] = pv;
     }
 }
 
 // s = r - alpha v, |s|^2   (bicgstab.cpp:89-94)
 template <class R, int K>
-__global__ void __launch_bounds__(kBlock) k_update_s(long n, const cplx<R>* __restrict__ r,
-                                                     const cplx<R>* __restrict__ v, cplx<R>* __restrict__ s,
+__global__ void __launch_bounds__(kVecNT) k_update_s(long n, const cplx<R>* __restrict__ r_,
+                                                     const cplx<R>* __restrict__ v_, cplx<R>* __restrict__ s_,
                                                      BicgState* st, RedScratch rs) {
     using C = cplx<R>;
+    constexpr int LPT = kVecLpt<R>;
+    using V = CVec<R, LPT>;
+    const V *r = reinterpret_cast<const V*>(r_), *v = reinterpret_cast<const V*>(v_);
+    V* s = reinterpret_cast<V*>(s_);
     const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long stride = (long)gridDim.x * blockDim.x;
-    const int rhs = (int)(i0 % K);
-    const BicgState S = st[rhs];
-    const bool run = S.status == kRunning;
-    const C al = from_d<C>(S.alpha);
-    R ss = 0;
-    for (long i = i0; i < n; i += stride) {
-        if (!run) { s[i] = cm<R>(0, 0); continue; }
-        const C sv = csub(r[i], cmul(al, v[i]));
-        s[i] = sv;
-        ss += sv.x * sv.x + sv.y * sv.y;
+    const long stride = (long)gridDim.x * blockDim.x, m = n / LPT;
+    C al[LPT], acc[LPT][1];
+    bool run[LPT];
+#pragma unroll
+    for (int j = 0; j < LPT; ++j) {
+        const BicgState& S = st[(i0 * LPT + j) % K];
+        run[j] = S.status == kRunning;
+        al[j] = from_d<C>(S.alpha);
+        acc[j][0] = cm<R>(0, 0);
     }
-    double2 acc[1] = {make_double2((double)ss, 0.0)};
+    for (long i = i0; i < m; i += stride) {
+        const V rv = r[i], vv = v[i];
+        V sv{};
+#pragma unroll
+        for (int j = 0; j < LPT; ++j)
+            if (run[j]) {
+                const C q = csub(rv.v[j], cmul(al[j], vv.v[j]));
+                sv.v[j] = q;
+                acc[j][0].x += q.x * q.x + q.y * q.y;
+            }
+        s[i] = sv;
+    }
     __shared__ double2 out[K];
-    if (grid_reduce_lanes<1, K>(acc, rs, out)) {
+    if (grid_reduce_multi<1, K, kVecNT, LPT>(acc, rs, out)) {
         if (threadIdx.x < K) {
             BicgState T = st[threadIdx.x];
             ep_s(T, out, threadIdx.x, K);
@@ -803,35 +844,52 @@ __global__ void __launch_bounds__(kBlock) k_update_s(long n, const cplx<R>* __re
 // (bicgstab.cpp:127-133); right-hand sides that stopped at the s test or at
 // a (t, t) breakdown take x += alpha p_hat only (:96, :123).
 template <class R, int K>
-__global__ void __launch_bounds__(kBlock) k_update_xr(long n, cplx<R>* __restrict__ x, cplx<R>* __restrict__ r,
-                                                      const cplx<R>* __restrict__ r0,
-                                                      const cplx<R>* __restrict__ ph,
-                                                      const cplx<R>* __restrict__ sh,
-                                                      const cplx<R>* __restrict__ s,
-                                                      const cplx<R>* __restrict__ t, BicgState* st,
+__global__ void __launch_bounds__(kVecNT) k_update_xr(long n, cplx<R>* __restrict__ x_, cplx<R>* __restrict__ r_,
+                                                      const cplx<R>* __restrict__ r0_,
+                                                      const cplx<R>* __restrict__ ph_,
+                                                      const cplx<R>* __restrict__ sh_,
+                                                      const cplx<R>* __restrict__ s_,
+                                                      const cplx<R>* __restrict__ t_, BicgState* st,
                                                       RedScratch rs) {
     using C = cplx<R>;
+    constexpr int LPT = kVecLpt<R>;
+    using V = CVec<R, LPT>;
+    V *x = reinterpret_cast<V*>(x_), *r = reinterpret_cast<V*>(r_);
+    const V *r0 = reinterpret_cast<const V*>(r0_), *ph = reinterpret_cast<const V*>(ph_),
+            *sh = reinterpret_cast<const V*>(sh_), *s = reinterpret_cast<const V*>(s_),
+            *t = reinterpret_cast<const V*>(t_);
     const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long stride = (long)gridDim.x * blockDim.x;
-    const int rhs = (int)(i0 % K);
-    const BicgState S = st[rhs];
-    const bool run = S.status == kRunning;
-    const bool pend = S.pend_x != 0;
-    const C al = from_d<C>(S.alpha), om = from_d<C>(S.omega);
-    R rr = 0;
-    C r0r = cm<R>(0, 0);
-    for (long i = i0; i < n; i += stride) {
-        if (pend) { x[i] = cadd(x[i], cmul(al, ph[i])); continue; }
-        if (!run) continue;
-        x[i] = cadd(x[i], cadd(cmul(al, ph[i]), cmul(om, sh[i])));
-        const C rv = csub(s[i], cmul(om, t[i]));
-        r[i] = rv;
-        rr += rv.x * rv.x + rv.y * rv.y;
-        r0r = cadd(r0r, cjmul(r0[i], rv));
+    const long stride = (long)gridDim.x * blockDim.x, m = n / LPT;
+    C al[LPT], om[LPT], acc[LPT][2];
+    bool run[LPT], pend[LPT], any = false;
+#pragma unroll
+    for (int j = 0; j < LPT; ++j) {
+        const BicgState& S = st[(i0 * LPT + j) % K];
+        pend[j] = S.pend_x != 0;
+        run[j] = S.status == kRunning && !pend[j];
+        al[j] = from_d<C>(S.alpha);
+        om[j] = from_d<C>(S.omega);
+        acc[j][0] = acc[j][1] = cm<R>(0, 0);
+        any |= run[j] || pend[j];
     }
-    double2 acc[2] = {make_double2((double)rr, 0.0), to_d(r0r)};
+    for (long i = i0; i < m && any; i += stride) {
+        const V pv = ph[i], qv = sh[i], sv = s[i], tv = t[i], zv = r0[i];
+        V xv = x[i], rv = r[i];
+#pragma unroll
+        for (int j = 0; j < LPT; ++j) {
+            if (pend[j]) xv.v[j] = cadd(xv.v[j], cmul(al[j], pv.v[j]));
+            if (!run[j]) continue;
+            xv.v[j] = cadd(xv.v[j], cadd(cmul(al[j], pv.v[j]), cmul(om[j], qv.v[j])));
+            const C q = csub(sv.v[j], cmul(om[j], tv.v[j]));
+            rv.v[j] = q;
+            acc[j][0].x += q.x * q.x + q.y * q.y;
+            acc[j][1] = cadd(acc[j][1], cjmul(zv.v[j], q));
+        }
+        x[i] = xv;
+        r[i] = rv;
+    }
     __shared__ double2 out[2 * K];
-    if (grid_reduce_lanes<2, K>(acc, rs, out)) {
+    if (grid_reduce_multi<2, K, kVecNT, LPT>(acc, rs, out)) {
         if (threadIdx.x < K) {
             BicgState T = st[threadIdx.x];
             ep_xr(T, out, threadIdx.x, K);
@@ -872,8 +930,15 @@ void spmv_staged_mode(const KrylovCtx<R>& c, const cplx<R>* x, cplx<R>* y, const
     // reducing modes: every block must reach the reduction, so the grid stays
     // within the partial-sum scratch
     const int cap = (MODE == kSpmvPlain || MODE == kSpmvSmooth) ? (1 << 20) : c.red.max_blocks;
-    launch_staged(k_spmv_st<R, K, MODE>, Sh::NT, c.seg.stage_row[Sh::LOG_T], (ns + Sh::T - 1) / Sh::T, cap, c.stream,
-                  c.seg, ns, c.D, c.B, x, y, aux, aux_out, st, c.red);
+    // whole passes where there are tiles for every SM, fewer slices per tile on
+    // small meshes (152 SMs)
+    const int T = std::max(1, std::min(Sh::T_MAX, ns / 152));
+    auto kf = k_spmv_st<R, K, MODE>;
+    const int smem = Sh::RING * c.seg.stage_row[T];
+    if (smem > 16 * 1024)   // with the reduction's static arrays beyond 48 KB
+        cudaFuncSetAttribute(reinterpret_cast<const void*>(kf), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const int g = std::min(wave_grid(kf, cap, Sh::NT, smem), std::max(1, (ns + T - 1) / T));
+    kf<<<g, Sh::NT, smem, c.stream>>>(c.seg, ns, T, c.D, c.B, x, y, aux, aux_out, st, c.red);
 }
 
 template <class R, int K>
@@ -1129,19 +1194,19 @@ void iteration_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* st) {
     const int gv = c.grid_vec;
     const double vb = (double)c.n_rows * K * sizeof(cplx<R>);
     int th = c.timer ? c.timer->begin(kClsVec, 4 * vb, K) : -1;
-    k_update_p<R, K><<<blocks_for(n, 2 * kBlock, gv), kBlock, 0, c.stream>>>(n, v.r, v.p, v.v, st);
+    k_update_p<R, K><<<blocks_for(n / kVecLpt<R>, 2 * kVecNT, gv), kVecNT, 0, c.stream>>>(n, v.r, v.p, v.v, st);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);
     precond_k<R, K>(c, v.p, v.y, v.ph);
     spmv_k<R, K>(c, kSpmvAp, v.ph, v.v, v.r0, nullptr, st);
     th = c.timer ? c.timer->begin(kClsVec, 3 * vb, K) : -1;
-    k_update_s<R, K><<<reduce_grid(k_update_s<R, K>, gv, n), kBlock, 0, c.stream>>>(n, v.r, v.v, v.s, st, c.red);
+    k_update_s<R, K><<<reduce_grid(k_update_s<R, K>, gv, n / kVecLpt<R>, kVecNT), kVecNT, 0, c.stream>>>(n, v.r, v.v, v.s, st, c.red);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);
     precond_k<R, K>(c, v.s, v.y, v.sh);
     spmv_k<R, K>(c, kSpmvAs, v.sh, v.t, v.s, nullptr, st);
     th = c.timer ? c.timer->begin(kClsVec, 8 * vb, K) : -1;
-    k_update_xr<R, K><<<reduce_grid(k_update_xr<R, K>, gv, n), kBlock, 0, c.stream>>>(n, v.x, v.r, v.r0, v.ph, v.sh, v.s, v.t, st, c.red);
+    k_update_xr<R, K><<<reduce_grid(k_update_xr<R, K>, gv, n / kVecLpt<R>, kVecNT), kVecNT, 0, c.stream>>>(n, v.x, v.r, v.r0, v.ph, v.sh, v.s, v.t, st, c.red);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);
 }
@@ -1467,7 +1532,7 @@ void eis_iteration_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* s
     eis_apply_k<R, K, 2, kEisAsS>(c, nullptr, v.s, v.r, v.v, st, v.ph, v.y, v.t, v.s);
     if (c.timer) c.timer->end(th);
     th = c.timer ? c.timer->begin(kClsVec, 8 * vb, K) : -1;
-    k_update_xr<R, K><<<reduce_grid(k_update_xr<R, K>, gv, n), kBlock, 0, c.stream>>>(n, v.x, v.r, v.r0, v.p, v.s, v.s,
+    k_update_xr<R, K><<<reduce_grid(k_update_xr<R, K>, gv, n / kVecLpt<R>, kVecNT), kVecNT, 0, c.stream>>>(n, v.x, v.r, v.r0, v.p, v.s, v.s,
                                                                               v.t, st, c.red);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);

@@ -47,7 +47,7 @@ struct SegView {
     using Real = R;
     const unsigned char* row_seg = nullptr;   // row segments
     const int* row_off = nullptr;             // [n_slices + 1] their offsets, 16-byte units
-    int stage_row[5] = {};      // bytes of the largest run of 1, 2, 4, 8, 16 neighbouring row segments
+    int stage_row[25] = {};     // [T]: bytes of the largest run of T neighbouring row segments (T > 0)
     const unsigned char* seg = nullptr;       // sweep segments (null until a sweep is asked for)
     const int4* work_col = nullptr;           // sweep order (sweep slices of group g at colour_ptr[g])
     const int* rows = nullptr;                // [sweep slices][32] row numbers (-1: none)
@@ -256,57 +256,77 @@ __device__ __forceinline__ void slice_pipeline(const unsigned char* __restrict__
     }
 }
 
-// The same for row segments: block b owns the tiles (T slices, one copy each)
-// [n b / grid, n (b + 1) / grid) and runs them in order.  A contiguous range
-// keeps a block on neighbouring rows, whose gathers hit its SM's L1: on the
-// benchmark mesh half of a row's columns lie within 13 rows of it and three
-// quarters within 86.
-template <int T, class Body>
-__device__ __forceinline__ void tile_pipeline(const unsigned char* __restrict__ seg, const int* __restrict__ off,
-                                              int n_slices, int stage_bytes, unsigned* err, Body body) {
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// Row segments: block b owns the tiles (T slices, one copy each) [n b / grid,
+// n (b + 1) / grid) and runs them in order.  A contiguous range keeps a block
+// on neighbouring rows, whose gathers hit its SM's L1: on the benchmark mesh
+// half of a row's columns lie within 13 rows of it and three quarters within
+// 86.  The last warp copies tiles into a ring of RING stages; the CW other
+// warps each wait for a stage, run body() and give the stage back on their
+// own, so a warp whose gathers miss does not hold up the others (with a block
+// barrier per tile the SpMV ran at 2.9 TB/s, all warps in step).
+// Every wait is bounded: a consumer whose stage does not arrive sets
+// kErrCopyTimeout, skips this and all later tiles but still gives the stages
+// back; the producer reuses a stage only when its copy has landed, and waits
+// for the copies in flight before it leaves.
+template <int CW, int RING, class Prefetch, class Body>
+__device__ __forceinline__ void tile_ring(const unsigned char* __restrict__ seg, const int* __restrict__ off,
+                                          int n_slices, int T, int stage_bytes, unsigned* err, Prefetch prefetch,
+                                          Body body) {
     extern __shared__ __align__(128) unsigned char dsm[];
-    __shared__ __align__(8) uint64_t bar[2];
-    __shared__ int no_wait;
+    __shared__ __align__(8) uint64_t full[RING], empty[RING];
     if (threadIdx.x == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        for (int s = 0; s < RING; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], CW);
+        }
         fence_mbar_init();
-        no_wait = (*reinterpret_cast<volatile unsigned*>(err) & kTestConsumeNoWait) != 0;
     }
     __syncthreads();
     const long n_tiles = (n_slices + T - 1) / T;
     const int t0 = (int)(n_tiles * blockIdx.x / gridDim.x), t1 = (int)(n_tiles * (blockIdx.x + 1) / gridDim.x);
-    auto issue = [&](int t, int stg) {   // thread 0 only
-        const int s0 = t * T, s1 = min(s0 + T, n_slices);
-        const int a = __ldg(&off[s0]);
-        const unsigned bytes = (unsigned)(__ldg(&off[s1]) - a) * 16u;
-        mbar_expect_tx(&bar[stg], bytes);
-        bulk_g2s(dsm + (size_t)stg * stage_bytes, seg + (size_t)a * 16, bytes, &bar[stg]);
-    };
-    auto wait_stage = [&](int stg, unsigned parity) {
-        return no_wait ? mbar_test_wait(&bar[stg], parity) : mbar_wait_bounded(&bar[stg], parity);
-    };
-    if (t0 >= t1) return;   // uniform: the whole block has no tile
-    if (threadIdx.x == 0) issue(t0, 0);
-    bool fail = __syncthreads_or(!wait_stage(0, 0u)) != 0;
-    for (int t = t0, k = 0;; ++t, ++k) {
-        const int stg = k & 1;
-        if (fail) {   // as in slice_pipeline
-            if (threadIdx.x == 0) {
-                atomicOr(err, kErrCopyTimeout);
-                mbar_wait_bounded(&bar[stg], (unsigned)(k >> 1) & 1u);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == CW) {
+        if (lane == 0) {
+            int issued = 0;
+            for (int t = t0; t < t1; ++t, ++issued) {
+                const int s = issued % RING, use = issued / RING;
+                if (use > 0 && (!mbar_wait_bounded(&empty[s], (unsigned)(use - 1) & 1u) ||
+                                !mbar_wait_bounded(&full[s], (unsigned)(use - 1) & 1u))) {
+                    atomicOr(err, kErrCopyTimeout);
+                    break;
+                }
+                const int a = __ldg(&off[t * T]);
+                const unsigned bytes = (unsigned)(__ldg(&off[min(t * T + T, n_slices)]) - a) * 16u;
+                mbar_expect_tx(&full[s], bytes);
+                bulk_g2s(dsm + (size_t)s * stage_bytes, seg + (size_t)a * 16, bytes, &full[s]);
             }
-            __syncthreads();
-            return;
+            for (int k = issued > RING ? issued - RING : 0; k < issued; ++k)
+                mbar_wait_bounded(&full[k % RING], (unsigned)(k / RING) & 1u);
         }
-        if (threadIdx.x == 0 && t + 1 < t1) {
-            fence_proxy_async_smem();
-            issue(t + 1, stg ^ 1);
+    } else {
+        const bool no_wait = (*reinterpret_cast<volatile unsigned*>(err) & kTestConsumeNoWait) != 0;
+        bool dead = false;
+        for (int t = t0, k = 0; t < t1; ++t, ++k) {
+            const int s = k % RING;
+            const unsigned parity = (unsigned)(k / RING) & 1u;
+            auto pre = prefetch(t);
+            if (!dead) {
+                const bool ok = no_wait ? mbar_test_wait(&full[s], parity) : mbar_wait_bounded(&full[s], parity);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    dead = true;
+                    if (lane == 0) atomicOr(err, kErrCopyTimeout);
+                }
+            }
+            if (!dead) body(t, pre, dsm + (size_t)s * stage_bytes);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[s]);
         }
-        body(t, dsm + (size_t)stg * stage_bytes);
-        if (t + 1 >= t1) return;
-        fail = __syncthreads_or(!wait_stage(stg ^ 1, (unsigned)((k + 1) >> 1) & 1u)) != 0;
     }
+    __syncthreads();
 }
 
 // Barrier over all blocks of a cooperative launch (every block resident):

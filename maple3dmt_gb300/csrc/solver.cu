@@ -1433,9 +1433,9 @@ void GpuSolver::build_row_segments(const std::vector<int>& op_rp, const std::vec
             off[s + 1] = (int)(buf.size() / 16);
         }
         view = std::decay_t<decltype(view)>{};
-        for (int j = 0; j < 5; ++j)
-            for (int s = 0; s < n_slices; s += 1 << j)
-                view.stage_row[j] = std::max(view.stage_row[j], (off[std::min(s + (1 << j), n_slices)] - off[s]) * 16);
+        for (int T = 1; T < 25; ++T)
+            for (int s = 0; s < n_slices; s += T)
+                view.stage_row[T] = std::max(view.stage_row[T], (off[std::min(s + T, n_slices)] - off[s]) * 16);
         d_seg = dupload(buf, stream);
         d_off = dupload(off, stream);
         sync();
