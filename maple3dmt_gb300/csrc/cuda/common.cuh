@@ -112,6 +112,19 @@ inline int wave_grid(F* kernel, int cap, int threads = kBlock, int smem = 0) {
     return g < cap ? g : cap;
 }
 
+// This block's contiguous range of n work items, and the blocks of such a
+// launch: eight per SM at 256 threads (152 SMs).  Gathers of rows numbered
+// along the octree's cell order hit L1 when a block keeps to neighbouring rows;
+// items dealt out block by block spread neighbours over the SMs.
+struct Range { long b, e; };
+__device__ __forceinline__ Range block_range(long n) {
+    return {n * blockIdx.x / gridDim.x, n * (blockIdx.x + 1) / gridDim.x};
+}
+inline int range_grid(long n, int threads = kBlock) {
+    const long b = (n + threads - 1) / threads;
+    return (int)(b < 1 ? 1 : b < 1216 ? b : 1216);
+}
+
 // Scratch for grid reductions: partial[block][kMaxQ * kMaxRhs] and a counter
 // that the last block resets.
 struct RedScratch {

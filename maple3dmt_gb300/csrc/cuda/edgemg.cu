@@ -3,7 +3,6 @@
 
 #include <algorithm>
 #include <stdexcept>
-#include <type_traits>
 
 namespace m3d {
 
@@ -12,10 +11,8 @@ using namespace dev;
 namespace {
 
 constexpr int kNT = 256;
-constexpr int kLongRow = 24;    // transfer rows longer than this (two levels of refinement) are summed by a block
+constexpr int kLongRow = 32;    // transfer rows longer than this (two levels of refinement) are summed by a block
 constexpr int kLongNT = 128;
-
-template <int D> using Dir = std::integral_constant<int, D>;   // direction tag
 
 void ck(long long* launches) {
     if (launches) ++*launches;
@@ -69,102 +66,112 @@ struct Omegas { float v[kMaxRhs]; };
 __device__ __forceinline__ Om<float4> om_of(const Omegas& o, int h, float4*) { return {o.v[2 * h], o.v[2 * h + 1]}; }
 
 // index helpers of an n^3 grid (host/edgemg.hpp)
-template <int D> __device__ __forceinline__ int ex(int n) { return D == 0 ? n : n + 1; }
-template <int D> __device__ __forceinline__ int ey(int n) { return D == 1 ? n : n + 1; }
-template <int D> __device__ __forceinline__ int eid(int n, int i, int j, int k) {
-    return D * n * (n + 1) * (n + 1) + (k * ey<D>(n) + j) * ex<D>(n) + i;
-}
-template <int D> __device__ __forceinline__ int fid(int n, int i, int j, int k) {
-    return D * n * n * (n + 1) + (k * (D == 1 ? n + 1 : n) + j) * (D == 0 ? n + 1 : n) + i;
-}
-__device__ __forceinline__ int nid(int n, int i, int j, int k) { return (k * (n + 1) + j) * (n + 1) + i; }
+__device__ __forceinline__ int pid(int n, int i, int j, int k) { return (k * (n + 1) + j) * (n + 1) + i; }
 
-// Curl-curl row of edge (D; i, j, k) and its diagonal: four faces, thirteen
-// points; at(e) reads the vector at edge e.
-template <int D, class V, class At>
-__device__ __forceinline__ V curl_row(const EmgLevel& L, int i, int j, int k, V xc, const At& at, float& S) {
+// Which of the three edges starting at a point are free: inside the grid
+// across their direction and not above the surface.
+struct Free { bool e[3]; };
+__device__ __forceinline__ Free edges_free(const EmgLevel& L, int i, int j, int k) {
     const int n = L.n;
-    V acc = vz<V>();
-    S = 0.0f;
-    auto dir = [&](auto tag) {
-        constexpr int A = decltype(tag)::value;      // transverse direction
-        constexpr int B = 3 - D - A;             // normal of the two faces
-        constexpr int ai = A == 0, aj = A == 1, ak = A == 2, di = D == 0, dj = D == 1, dk = D == 2;
-        const float wp = __ldg(&L.w[fid<B>(n, i, j, k)]), wm = __ldg(&L.w[fid<B>(n, i - ai, j - aj, k - ak)]);
-        const float hd = L.h[D], ha = L.h[A];
-        const V xp = at(eid<D>(n, i + ai, j + aj, k + ak)), xm = at(eid<D>(n, i - ai, j - aj, k - ak));
-        const V a0 = at(eid<A>(n, i, j, k)), a1 = at(eid<A>(n, i + di, j + dj, k + dk));
-        const V b0 = at(eid<A>(n, i - ai, j - aj, k - ak)), b1 = at(eid<A>(n, i - ai + di, j - aj + dj, k - ak + dk));
-        const V cp = hd * (xc - xp) + ha * (a1 - a0);
-        const V cm = hd * (xm - xc) + ha * (b1 - b0);
-        acc = acc + hd * (wp * cp - wm * cm);
-        S += hd * hd * (wp + wm);
-    };
-    dir(Dir<D == 0 ? 1 : 0>{});
-    dir(Dir<D == 2 ? 1 : 2>{});
-    return acc;
-}
-
-template <int D> __device__ __forceinline__ float edge_diag(const EmgLevel& L, int i, int j, int k) {
-    const int n = L.n;
-    constexpr int A = D == 0 ? 1 : 0, B = D == 2 ? 1 : 2;
-    // faces of normal A are spanned by D and B, and the other way round
-    const float sa = __ldg(&L.w[fid<A>(n, i, j, k)]) + __ldg(&L.w[fid<A>(n, i - (B == 0), j - (B == 1), k - (B == 2))]);
-    const float sb = __ldg(&L.w[fid<B>(n, i, j, k)]) + __ldg(&L.w[fid<B>(n, i - (A == 0), j - (A == 1), k - (A == 2))]);
-    return L.h[D] * L.h[D] * (sa + sb);
-}
-
-// interior of the grid across direction D and not above the surface
-template <int D> __device__ __forceinline__ bool edge_free(const EmgLevel& L, int i, int j, int k) {
-    const int n = L.n;
-    if (D != 0 && (i <= 0 || i >= n)) return false;
-    if (D != 1 && (j <= 0 || j >= n)) return false;
-    if (D != 2) return k > 0 && k < L.ph;
-    return k < L.pv;
+    const bool in = i < n && j < n && k < n;
+    return {{in && j > 0 && k > 0 && k < L.ph, in && i > 0 && k > 0 && k < L.ph, in && i > 0 && j > 0 && k < L.pv}};
 }
 __device__ __forceinline__ bool node_free(const EmgLevel& L, int i, int j, int k) {
     return i > 0 && i < L.n && j > 0 && j < L.n && k > 0 && k < L.pn;
 }
 
-// Work split of an edge kernel: blockIdx.y is a plane of one direction (the
-// planes that may be free and the one above them, which is written as zeros
-// because the stencils read it), threads run over (row of the plane, lanes).
-__host__ __device__ inline int edge_planes(const EmgLevel& L, int D) {
-    const int p = (D == 2 ? L.pv : L.ph) + 1, most = D == 2 ? L.n : L.n + 1;
-    return p < most ? p : most;
+// Weights of the nine faces that the three edges of a point touch, by normal:
+// at the point and one step down in each of the two other directions (those
+// clamp at the grid's side, where no free edge uses them).
+struct Faces { float x, xj, xk, y, yi, yk, z, zi, zj; };
+__device__ __forceinline__ Faces face_weights(const EmgLevel& L, int i, int j, int k) {
+    const int n1 = L.n + 1, p = pid(L.n, i, j, k);
+    const int pi = p - (i > 0), pj = p - (j > 0 ? n1 : 0), pk = p - (k > 0 ? n1 * n1 : 0);
+    const float* w = L.w;
+    return {__ldg(&w[3 * p]),     __ldg(&w[3 * pj]),     __ldg(&w[3 * pk]),
+            __ldg(&w[3 * p + 1]), __ldg(&w[3 * pi + 1]), __ldg(&w[3 * pk + 1]),
+            __ldg(&w[3 * p + 2]), __ldg(&w[3 * pi + 2]), __ldg(&w[3 * pj + 2])};
 }
-inline int edge_planes_all(const EmgLevel& L) { return 2 * edge_planes(L, 0) + edge_planes(L, 2); }
+// diagonals of the curl-curl rows
+__device__ __forceinline__ void edge_diags(const EmgLevel& L, const Faces& f, float (&S)[3]) {
+    S[0] = L.h[0] * L.h[0] * (f.y + f.yk + f.z + f.zj);
+    S[1] = L.h[1] * L.h[1] * (f.z + f.zi + f.x + f.xk);
+    S[2] = L.h[2] * L.h[2] * (f.y + f.yi + f.x + f.xj);
+}
+
+// Curl-curl rows of the three edges of a point (i, j, k < n): nine face
+// circulations from 24 edge values, where three 13-point rows would read 39;
+// at(e) reads the vector at edge entry e.
+template <class V, class At>
+__device__ __forceinline__ void curl_rows(const EmgLevel& L, const Faces& f, int i, int j, int k, const At& at,
+                                          V (&xc)[3], V (&ax)[3]) {
+    const int n1 = L.n + 1, p = pid(L.n, i, j, k);
+    const int di = 3, dj = 3 * n1, dk = 3 * n1 * n1, mi = i > 0 ? di : 0, mj = j > 0 ? dj : 0, mk = k > 0 ? dk : 0;
+    const int x = 3 * p, y = 3 * p + 1, z = 3 * p + 2;
+    const float hx = L.h[0], hy = L.h[1], hz = L.h[2];
+    const V X = at(x), Y = at(y), Z = at(z);
+    const V Xj = at(x + dj), Xk = at(x + dk), Yi = at(y + di), Yk = at(y + dk), Zi = at(z + di), Zj = at(z + dj);
+    xc[0] = X;
+    xc[1] = Y;
+    xc[2] = Z;
+    // circulations times weights: normal x, y, z at the point
+    const V cx = f.x * (hy * (Y - Yk) + hz * (Zj - Z));
+    const V cy = f.y * (hx * (X - Xk) + hz * (Zi - Z));
+    const V cz = f.z * (hx * (X - Xj) + hy * (Yi - Y));
+    // one step down
+    const V Xmj = at(x - mj), Xmk = at(x - mk), Ymi = at(y - mi), Ymk = at(y - mk), Zmi = at(z - mi), Zmj = at(z - mj);
+    const V cxk = f.xk * (hy * (Ymk - Y) + hz * (at(z - mk + dj) - at(z - mk)));
+    const V cxj = f.xj * (hy * (at(y - mj) - at(y - mj + dk)) + hz * (Z - Zmj));
+    const V cyk = f.yk * (hx * (Xmk - X) + hz * (at(z - mk + di) - at(z - mk)));
+    const V cyi = f.yi * (hx * (at(x - mi) - at(x - mi + dk)) + hz * (Z - Zmi));
+    const V czj = f.zj * (hx * (Xmj - X) + hy * (at(y - mj + di) - at(y - mj)));
+    const V czi = f.zi * (hx * (at(x - mi) - at(x - mi + dj)) + hy * (Y - Ymi));
+    ax[0] = hx * ((cy - cyk) + (cz - czj));
+    ax[1] = hy * ((czi - cz) + (cx - cxk));
+    ax[2] = hz * ((cyi - cy) + (cxj - cx));
+}
+
+// Work split of a grid kernel: threads over (point of a plane, pairs of
+// right-hand sides), blockIdx.y the plane.  The planes are those that may hold
+// free edges or nodes and the ones above them, which are written as zeros
+// because the stencils read them.
+__host__ __device__ inline int edge_planes(const EmgLevel& L) {
+    const int p = (L.ph > L.pv ? L.ph : L.pv) + 1;
+    return p < L.n + 1 ? p : L.n + 1;
+}
 __host__ __device__ inline int node_planes(const EmgLevel& L) { return L.pn + 2 < L.n + 1 ? L.pn + 2 : L.n + 1; }
 
-template <int H, class F> __device__ __forceinline__ void each_edge(const EmgLevel& L, const F& f) {
-    const int p0 = edge_planes(L, 0);
-    const int t = blockIdx.x * kNT + threadIdx.x;
-    const int q = t / H, h = t % H;
-    const int y = blockIdx.y, n = L.n;
-    if (y < p0) {
-        if (q < n * (n + 1)) f(Dir<0>{}, q % n, q / n, y, h);
-    } else if (y < 2 * p0) {
-        if (q < (n + 1) * n) f(Dir<1>{}, q % (n + 1), q / (n + 1), y - p0, h);
-    } else {
-        if (q < (n + 1) * (n + 1)) f(Dir<2>{}, q % (n + 1), q / (n + 1), y - 2 * p0, h);
-    }
-}
-template <int H, class F> __device__ __forceinline__ void each_node(const EmgLevel& L, const F& f) {
+template <int H, class F> __device__ __forceinline__ void each_point(const EmgLevel& L, const F& f) {
     const int t = blockIdx.x * kNT + threadIdx.x;
     const int q = t / H, h = t % H, n1 = L.n + 1;
     if (q < n1 * n1) f(q % n1, q / n1, (int)blockIdx.y, h);
 }
-template <int K> dim3 edge_grid(const EmgLevel& L) {
+template <int K> dim3 point_grid(const EmgLevel& L, int planes) {
     const long rows = (long)(L.n + 1) * (L.n + 1) * (K / 2);
-    return dim3((unsigned)((rows + kNT - 1) / kNT), (unsigned)edge_planes_all(L));
-}
-template <int K> dim3 node_grid(const EmgLevel& L) {
-    const long rows = (long)(L.n + 1) * (L.n + 1) * (K / 2);
-    return dim3((unsigned)((rows + kNT - 1) / kNT), (unsigned)node_planes(L));
+    return dim3((unsigned)((rows + kNT - 1) / kNT), (unsigned)planes);
 }
 
 __host__ __device__ __forceinline__ float4* f4(float2* p) { return reinterpret_cast<float4*>(p); }
 __host__ __device__ __forceinline__ const float4* f4(const float2* p) { return reinterpret_cast<const float4*>(p); }
+
+// Two right-hand sides of an entry: [entry][K], or [K][entry] on a grid of the
+// bottom kernels (n entries).
+__host__ __device__ inline bool lane_major(const EmgLevel& L) { return L.n <= kEmgBottom; }
+template <int K> __device__ __forceinline__ float4 load2(const float2* v, bool lm, int n, int e, int h) {
+    if (!lm) return f4(v)[(size_t)e * (K / 2) + h];
+    const float2 a = v[(size_t)(2 * h) * n + e], b = v[(size_t)(2 * h + 1) * n + e];
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+template <int K> __device__ __forceinline__ void store2(float2* v, bool lm, int n, int e, int h, float4 q) {
+    if (!lm) {
+        f4(v)[(size_t)e * (K / 2) + h] = q;
+        return;
+    }
+    v[(size_t)(2 * h) * n + e] = make_float2(q.x, q.y);
+    v[(size_t)(2 * h + 1) * n + e] = make_float2(q.z, q.w);
+}
+__device__ __forceinline__ int entries(const EmgLevel& L) { return 3 * (L.n + 1) * (L.n + 1) * (L.n + 1); }
+__device__ __forceinline__ int points(const EmgLevel& L) { return (L.n + 1) * (L.n + 1) * (L.n + 1); }
 
 // ---------------------------------------------------------------------------
 // coarse edge masses
@@ -177,7 +184,8 @@ __global__ void k_mass0(EmgDev g, const double* __restrict__ Me, int n) {
     g.lv[0].me[c] = (float)s;
 }
 
-// sum over the fine edges of a coarse edge: 2 along it, (1/2, 1, 1/2) across
+// sum over the fine edges of the coarse edge of direction D at (I, J, Kk): 2
+// along it, (1/2, 1, 1/2) across
 template <int D, class V, class At>
 __device__ __forceinline__ V gather_edge(int n, int I, int J, int Kk, const At& at) {
     V s = vz<V>();
@@ -188,65 +196,38 @@ __device__ __forceinline__ V gather_edge(int n, int I, int J, int Kk, const At& 
             const float w = (a ? 0.5f : 1.0f) * (b ? 0.5f : 1.0f);
             const int i = 2 * I + (D == 0 ? 0 : a), j = 2 * J + (D == 1 ? 0 : (D == 0 ? a : b)),
                       k = 2 * Kk + (D == 2 ? 0 : b);
-            const int e = eid<D>(n, i, j, k), f = eid<D>(n, i + (D == 0), j + (D == 1), k + (D == 2));
-            s = s + w * (at(e) + at(f));
+            s = s + w * (at(3 * pid(n, i, j, k) + D) + at(3 * pid(n, i + (D == 0), j + (D == 1), k + (D == 2)) + D));
         }
     return s;
+}
+// the same for the free edges of a point
+template <class V, class At>
+__device__ __forceinline__ void gather_edges(const Free& f, int n, int I, int J, int Kk, const At& at, V (&s)[3]) {
+    s[0] = f.e[0] ? gather_edge<0, V>(n, I, J, Kk, at) : vz<V>();
+    s[1] = f.e[1] ? gather_edge<1, V>(n, I, J, Kk, at) : vz<V>();
+    s[2] = f.e[2] ? gather_edge<2, V>(n, I, J, Kk, at) : vz<V>();
 }
 
 struct F1 { float v; };
 __device__ __forceinline__ F1 vzero(F1*) { return {0.f}; }
 __device__ __forceinline__ F1 operator+(F1 a, F1 b) { return {a.v + b.v}; }
+__device__ __forceinline__ F1 operator-(F1 a, F1 b) { return {a.v - b.v}; }
 __device__ __forceinline__ F1 operator*(float s, F1 b) { return {s * b.v}; }
 
 __global__ void k_mass(EmgLevel F, EmgLevel C) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, n = C.n;
-    auto put = [&](auto tag, int q) {
-        constexpr int D = decltype(tag)::value;
-        const int i = q % ex<D>(n), j = q / ex<D>(n) % ey<D>(n), k = q / (ex<D>(n) * ey<D>(n));
-        if (!edge_free<D>(C, i, j, k)) return;
-        C.me[eid<D>(n, i, j, k)] = gather_edge<D, F1>(F.n, i, j, k, [&](int e) { return F1{F.me[e]}; }).v;
-    };
-    const int per = n * (n + 1) * (n + 1);
-    if (t < per) put(Dir<0>{}, t);
-    else if (t < 2 * per) put(Dir<1>{}, t - per);
-    else if (t < 3 * per) put(Dir<2>{}, t - 2 * per);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, n1 = C.n + 1;
+    if (t >= n1 * n1 * n1) return;
+    const int i = t % n1, j = t / n1 % n1, k = t / (n1 * n1);
+    const Free f = edges_free(C, i, j, k);
+    F1 s[3];
+    gather_edges<F1>(f, F.n, i, j, k, [&](int e) { return F1{F.me[e]}; }, s);
+    for (int D = 0; D < 3; ++D)
+        if (f.e[D]) C.me[3 * t + D] = s[D].v;
 }
 
 // ---------------------------------------------------------------------------
 // edge cycle
 // ---------------------------------------------------------------------------
-
-// b0 = P^T r from the octree rows, x0 = w b0 / d
-template <int K>
-__global__ void __launch_bounds__(kNT) k_restrict0(EmgDev g, Omegas om, const float4* __restrict__ r) {
-    constexpr int H = K / 2;
-    const EmgLevel& L = g.lv[0];
-    each_edge<H>(L, [&](auto tag, int i, int j, int k, int h) {
-        constexpr int D = decltype(tag)::value;
-        const int c = eid<D>(L.n, i, j, k);
-        float4 s = vz<float4>(), x = vz<float4>();
-        if (edge_free<D>(L, i, j, k)) {
-            const int q0 = __ldg(&g.r_ptr[c]), q1 = __ldg(&g.r_ptr[c + 1]);
-            if (q1 - q0 > kLongRow) return;   // k_restrict0_long
-            for (int q = q0; q < q1; q += 4) {
-                float w[4];
-                float4 v[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const bool ok = q + u < q1;
-                    w[u] = ok ? __ldg(&g.r_w[q + u]) : 0.0f;
-                    v[u] = ok ? r[(size_t)__ldg(&g.r_row[q + u]) * H + h] : vz<float4>();
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) s = s + w[u] * v[u];
-            }
-            x = idiag(om_of(om, h, (float4*)nullptr), kEmgEdge, edge_diag<D>(L, i, j, k), __ldg(&L.me[c]), s);
-        }
-        f4(L.b)[(size_t)c * H + h] = s;
-        f4(L.x)[(size_t)c * H + h] = x;
-    });
-}
 
 // Sum of w_q v[idx_q] over one long transfer row by a block of kLongNT threads
 // (lanes H, the entries dealt out to the rest); the total on the first H.
@@ -267,6 +248,38 @@ __device__ __forceinline__ float4 long_row(const int* __restrict__ idx, const fl
     return part[threadIdx.x];
 }
 
+// b0 = P^T r from the octree rows, x0 = w b0 / d; a thread per edge entry
+template <int K>
+__global__ void __launch_bounds__(kNT) k_restrict0(EmgDev g, Omegas om, const float4* __restrict__ r, int n) {
+    constexpr int H = K / 2;
+    const EmgLevel& L = g.lv[0];
+    const int t = blockIdx.x * kNT + threadIdx.x, c = t / H, h = t % H;
+    if (c >= n) return;
+    const int n1 = L.n + 1, p = c / 3, i = p % n1, j = p / n1 % n1, k = p / (n1 * n1), D = c % 3;
+    const int q0 = __ldg(&g.r_ptr[c]), q1 = __ldg(&g.r_ptr[c + 1]);
+    if (q1 - q0 > kLongRow) return;   // k_restrict0_long
+    float4 s = vz<float4>(), x = vz<float4>();
+    for (int q = q0; q < q1; q += 6) {   // 18 entries under one level of refinement
+        float w[6];
+        float4 v[6];
+#pragma unroll
+        for (int u = 0; u < 6; ++u) {
+            const bool ok = q + u < q1;
+            w[u] = ok ? __ldg(&g.r_w[q + u]) : 0.0f;
+            v[u] = ok ? r[(size_t)__ldg(&g.r_row[q + u]) * H + h] : vz<float4>();
+        }
+#pragma unroll
+        for (int u = 0; u < 6; ++u) s = s + w[u] * v[u];
+    }
+    if (q1 > q0) {
+        float S[3];
+        edge_diags(L, face_weights(L, i, j, k), S);
+        x = idiag(om_of(om, h, (float4*)nullptr), kEmgEdge, S[D], __ldg(&L.me[c]), s);
+    }
+    store2<K>(L.b, lane_major(L), entries(L), c, h, s);
+    store2<K>(L.x, lane_major(L), entries(L), c, h, x);
+}
+
 // The rows of P^T with more than kLongRow entries: coarse edges inside a
 // refinement of two or three levels collect up to 196 or 1800 octree edges,
 // which one thread after another made 50 us on the 157 k-edge mesh.
@@ -274,32 +287,44 @@ template <int K>
 __global__ void __launch_bounds__(kLongNT) k_restrict0_long(EmgDev g, Omegas om, const float4* __restrict__ r) {
     constexpr int H = K / 2;
     const EmgLevel& L = g.lv[0];
-    const int c = g.r_long[blockIdx.x], n = L.n, h = threadIdx.x % H;
+    const int c = g.r_long[blockIdx.x], h = threadIdx.x % H;
     const float4 s = long_row<H>(g.r_row, g.r_w, g.r_ptr[c], g.r_ptr[c + 1], r);
     if (threadIdx.x >= H) return;
-    const int per = n * (n + 1) * (n + 1), D = c / per, q = c % per;
-    const int nx = D == 0 ? n : n + 1, ny = D == 1 ? n : n + 1, i = q % nx, j = q / nx % ny, k = q / (nx * ny);
-    const float S = D == 0 ? edge_diag<0>(L, i, j, k) : D == 1 ? edge_diag<1>(L, i, j, k) : edge_diag<2>(L, i, j, k);
-    f4(L.b)[(size_t)c * H + h] = s;
-    f4(L.x)[(size_t)c * H + h] = idiag(om_of(om, h, (float4*)nullptr), kEmgEdge, S, __ldg(&L.me[c]), s);
+    const int n1 = L.n + 1, p = c / 3;
+    float S[3];
+    edge_diags(L, face_weights(L, p % n1, p / n1 % n1, p / (n1 * n1)), S);
+    store2<K>(L.b, lane_major(L), entries(L), c, h, s);
+    store2<K>(L.x, lane_major(L), entries(L), c, h,
+              idiag(om_of(om, h, (float4*)nullptr), kEmgEdge, S[c % 3], __ldg(&L.me[c]), s));
 }
 
-// y = b - A x
-template <int K>
-__global__ void __launch_bounds__(kNT) k_resid(EmgLevel L, Omegas om) {
+// y = b - A x, or (SMOOTH) y = x + w (b - A x) / d
+template <int K, bool SMOOTH>
+__global__ void __launch_bounds__(kNT, 3) k_edge_step(EmgLevel L, Omegas oms) {
     constexpr int H = K / 2;
-    each_edge<H>(L, [&](auto tag, int i, int j, int k, int h) {
-        constexpr int D = decltype(tag)::value;
-        const int c = eid<D>(L.n, i, j, k);
-        float4 res = vz<float4>();
-        if (edge_free<D>(L, i, j, k)) {
-            const float4* x = f4(L.x);
-            const float4 xc = x[(size_t)c * H + h];
-            float S;
-            const float4 ax = curl_row<D, float4>(L, i, j, k, xc, [&](int e) { return x[(size_t)e * H + h]; }, S);
-            res = f4(L.b)[(size_t)c * H + h] - ax - imass(om_of(om, h, (float4*)nullptr), __ldg(&L.me[c]), xc);
+    each_point<H>(L, [&](int i, int j, int k, int h) {
+        const Free f = edges_free(L, i, j, k);
+        const int p = pid(L.n, i, j, k);
+        const float4 *xv = f4(L.x), *b = f4(L.b);
+        float4* y = f4(L.y);
+        float4 out[3] = {vz<float4>(), vz<float4>(), vz<float4>()};
+        if (f.e[0] || f.e[1] || f.e[2]) {
+            const Faces w = face_weights(L, i, j, k);
+            const Om<float4> om = om_of(oms, h, (float4*)nullptr);
+            float4 x[3], ax[3];
+            curl_rows<float4>(L, w, i, j, k, [&](int e) { return xv[(size_t)e * H + h]; }, x, ax);
+            float S[3];
+            edge_diags(L, w, S);
+#pragma unroll
+            for (int D = 0; D < 3; ++D)
+                if (f.e[D]) {
+                    const float m = __ldg(&L.me[3 * p + D]);
+                    const float4 r = b[(size_t)(3 * p + D) * H + h] - ax[D] - imass(om, m, x[D]);
+                    out[D] = SMOOTH ? x[D] + idiag(om, kEmgEdge, S[D], m, r) : r;
+                }
         }
-        f4(L.y)[(size_t)c * H + h] = res;
+#pragma unroll
+        for (int D = 0; D < 3; ++D) y[(size_t)(3 * p + D) * H + h] = out[D];
     });
 }
 
@@ -307,198 +332,282 @@ __global__ void __launch_bounds__(kNT) k_resid(EmgLevel L, Omegas om) {
 template <int K>
 __global__ void __launch_bounds__(kNT) k_restrict(EmgLevel F, EmgLevel L, Omegas om) {
     constexpr int H = K / 2;
-    each_edge<H>(L, [&](auto tag, int i, int j, int k, int h) {
-        constexpr int D = decltype(tag)::value;
-        const int c = eid<D>(L.n, i, j, k);
-        float4 s = vz<float4>(), x = vz<float4>();
-        if (edge_free<D>(L, i, j, k)) {
-            const float4* y = f4(F.y);
-            s = gather_edge<D, float4>(F.n, i, j, k, [&](int e) { return y[(size_t)e * H + h]; });
-            x = idiag(om_of(om, h, (float4*)nullptr), kEmgEdge, edge_diag<D>(L, i, j, k), __ldg(&L.me[c]), s);
+    each_point<H>(L, [&](int i, int j, int k, int h) {
+        const Free f = edges_free(L, i, j, k);
+        const int p = pid(L.n, i, j, k), ne = entries(L);
+        const bool lm = lane_major(L);
+        float4 s[3], x[3] = {vz<float4>(), vz<float4>(), vz<float4>()};
+        const float4* y = f4(F.y);
+        gather_edges<float4>(f, F.n, i, j, k, [&](int e) { return y[(size_t)e * H + h]; }, s);
+        if (f.e[0] || f.e[1] || f.e[2]) {
+            float S[3];
+            edge_diags(L, face_weights(L, i, j, k), S);
+#pragma unroll
+            for (int D = 0; D < 3; ++D)
+                x[D] = idiag(om_of(om, h, (float4*)nullptr), kEmgEdge, S[D], __ldg(&L.me[3 * p + D]), s[D]);
         }
-        f4(L.b)[(size_t)c * H + h] = s;
-        f4(L.x)[(size_t)c * H + h] = x;
+#pragma unroll
+        for (int D = 0; D < 3; ++D) {
+            store2<K>(L.b, lm, ne, 3 * p + D, h, s[D]);
+            store2<K>(L.x, lm, ne, 3 * p + D, h, x[D]);
+        }
     });
 }
 
-// value of the coarse vector interpolated to fine edge (D; i, j, k)
+// value of the coarse vector interpolated to the fine edge of direction D at (i, j, k)
 template <int D, class V, class At>
 __device__ __forceinline__ V interp_edge(int n, int i, int j, int k, const At& at) {
-    const int I = i >> 1, J = j >> 1, Kk = k >> 1;
+    const int n1 = n + 1, e = 3 * pid(n, i >> 1, j >> 1, k >> 1) + D;
     constexpr int A = D == 0 ? 1 : 0, B = D == 2 ? 1 : 2;
-    const int p[3] = {i, j, k};
-    const bool oa = p[A] & 1, ob = p[B] & 1;
-    auto e = [&](int sa, int sb) {
-        return eid<D>(n, I + (A == 0 ? sa : 0), J + (A == 1 ? sa : 0) + (B == 1 ? sb : 0), Kk + (B == 2 ? sb : 0));
-    };
-    V s = at(e(0, 0));
-    if (oa) s = s + at(e(1, 0));
-    if (ob) s = s + at(e(0, 1));
-    if (oa && ob) s = s + at(e(1, 1));
-    return ((oa ? 0.5f : 1.0f) * (ob ? 0.5f : 1.0f)) * s;
+    const int q[3] = {i, j, k}, st[3] = {3, 3 * n1, 3 * n1 * n1};
+    const int sa = q[A] & 1 ? st[A] : 0, sb = q[B] & 1 ? st[B] : 0;
+    V s = at(e);
+    if (sa) s = s + at(e + sa);
+    if (sb) s = s + at(e + sb);
+    if (sa && sb) s = s + at(e + sa + sb);
+    return ((sa ? 0.5f : 1.0f) * (sb ? 0.5f : 1.0f)) * s;
+}
+template <class V, class At>
+__device__ __forceinline__ void interp_edges(const Free& f, int n, int i, int j, int k, const At& at, V (&s)[3]) {
+    s[0] = f.e[0] ? interp_edge<0, V>(n, i, j, k, at) : vz<V>();
+    s[1] = f.e[1] ? interp_edge<1, V>(n, i, j, k, at) : vz<V>();
+    s[2] = f.e[2] ? interp_edge<2, V>(n, i, j, k, at) : vz<V>();
 }
 
 // x += P y_coarse
 template <int K>
 __global__ void __launch_bounds__(kNT) k_prolong(EmgLevel L, EmgLevel C) {
     constexpr int H = K / 2;
-    each_edge<H>(L, [&](auto tag, int i, int j, int k, int h) {
-        constexpr int D = decltype(tag)::value;
-        if (!edge_free<D>(L, i, j, k)) return;
-        const size_t c = (size_t)eid<D>(L.n, i, j, k) * H + h;
-        const float4* y = f4(C.y);
-        f4(L.x)[c] = f4(L.x)[c] + interp_edge<D, float4>(C.n, i, j, k, [&](int e) { return y[(size_t)e * H + h]; });
+    each_point<H>(L, [&](int i, int j, int k, int h) {
+        const Free f = edges_free(L, i, j, k);
+        const int p = pid(L.n, i, j, k), ne = entries(C);
+        const bool lm = lane_major(C);
+        float4 s[3];
+        interp_edges<float4>(f, C.n, i, j, k, [&](int e) { return load2<K>(C.y, lm, ne, e, h); }, s);
+#pragma unroll
+        for (int D = 0; D < 3; ++D)
+            if (f.e[D]) {
+                const size_t c = (size_t)(3 * p + D) * H + h;
+                f4(L.x)[c] = f4(L.x)[c] + s[D];
+            }
     });
 }
 
-// y = x + w (b - A x) / d
-template <int K>
-__global__ void __launch_bounds__(kNT) k_smooth(EmgLevel L, Omegas om) {
-    constexpr int H = K / 2;
-    each_edge<H>(L, [&](auto tag, int i, int j, int k, int h) {
-        constexpr int D = decltype(tag)::value;
-        const int c = eid<D>(L.n, i, j, k);
-        float4 v = vz<float4>();
-        if (edge_free<D>(L, i, j, k)) {
-            const float4* x = f4(L.x);
-            const float4 xc = x[(size_t)c * H + h];
-            const Om<float4> o = om_of(om, h, (float4*)nullptr);
-            const float m = __ldg(&L.me[c]);
-            float S;
-            const float4 ax = curl_row<D, float4>(L, i, j, k, xc, [&](int e) { return x[(size_t)e * H + h]; }, S);
-            v = xc + idiag(o, kEmgEdge, S, m, f4(L.b)[(size_t)c * H + h] - ax - imass(o, m, xc));
-        }
-        f4(L.y)[(size_t)c * H + h] = v;
-    });
+// ---------------------------------------------------------------------------
+// The small grids.  Launched step by step, the grids of 16 cells per side and
+// less (15 k edges) took five launches of 4 to 16 us; one block for all of
+// them was slower still (50 us, one SM's issue rate).  Here a cluster of
+// four or eight blocks runs them for one right-hand side: the 16-cell grid is split
+// over the cluster's blocks with its vectors in global memory (a right-hand
+// side's values together, read past L1), cluster barriers between the steps;
+// the grids of 8 and 4 cells run in the shared memory of the first block.
+// ---------------------------------------------------------------------------
+constexpr int kBottomNT = 768;
+constexpr int kCoarsestSteps = 8;
+static_assert(kBottomNT >= 9 * 9 * 9 && 8 * kBottomNT >= 17 * 17 * 17, "a point per thread of eight blocks");
+// Blocks per cluster: eight up to K = 8, one point of the 16-cell grid per
+// thread; four at K = 16, where sixteen clusters of eight took two waves (46
+// against 28 us at K = 8).
+constexpr int cluster_blocks(int K) { return K > 8 ? 4 : 8; }
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ int cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return (int)r;
 }
 
-// The grids of at most kEmgBottom cells per side: one block per right-hand
-// side runs their whole cycle, vectors in shared memory (a launch per step
-// would cost more than the steps: 2 k edges).  Reads b and x of the first such
-// level, writes its y.  The coarsest grid's Jacobi steps keep each edge's
-// stencil in registers: twelve weights and positions, one edge per thread.
-constexpr int kBottomNT = 1024;
-constexpr int kCoarsestSteps = 12;
-
-template <class F> __device__ __forceinline__ void with_edge(const EmgLevel& L, int t, const F& f) {
-    const int n = L.n, per = n * (n + 1) * (n + 1);
-    if (t < per) {
-        const int i = t % n, j = t / n % (n + 1), k = t / (n * (n + 1));
-        if (edge_free<0>(L, i, j, k)) f(Dir<0>{}, i, j, k);
-    } else if (t < 2 * per) {
-        const int q = t - per, i = q % (n + 1), j = q / (n + 1) % n, k = q / (n * (n + 1));
-        if (edge_free<1>(L, i, j, k)) f(Dir<1>{}, i, j, k);
-    } else if (t < 3 * per) {
-        const int q = t - 2 * per, i = q % (n + 1), j = q / (n + 1) % (n + 1), k = q / ((n + 1) * (n + 1));
-        if (edge_free<2>(L, i, j, k)) f(Dir<2>{}, i, j, k);
+// A grid point's three edges: which are free, their face weights and masses,
+// loaded ahead of the phases that use them.
+struct Point {
+    int i, j, k, p;
+    Free f;
+    bool any;
+    Faces w;
+    float m[3];
+    __device__ __forceinline__ void load(const EmgLevel& L, int point, bool on) {
+        const int n1 = L.n + 1;
+        p = point;
+        i = p % n1;
+        j = p / n1 % n1;
+        k = p / (n1 * n1);
+        f = Free{};
+        if (on) f = edges_free(L, i, j, k);
+        any = f.e[0] || f.e[1] || f.e[2];
+        w = Faces{};
+        if (any) w = face_weights(L, i, j, k);
+#pragma unroll
+        for (int D = 0; D < 3; ++D) m[D] = any ? __ldg(&L.me[3 * p + D]) : 0.0f;
     }
+};
+
+// Jacobi step or residual at one point, any memory
+template <class In, class Rhs>
+__device__ __forceinline__ void point_step(const EmgLevel& L, Om<float2> om, const Point& q, bool resid, const In& in,
+                                           const Rhs& rhs, float2 (&v)[3]) {
+    v[0] = v[1] = v[2] = vz<float2>();
+    if (!q.any) return;
+    float2 xc[3], ax[3];
+    float S[3];
+    curl_rows<float2>(L, q.w, q.i, q.j, q.k, in, xc, ax);
+    edge_diags(L, q.w, S);
+#pragma unroll
+    for (int D = 0; D < 3; ++D)
+        if (q.f.e[D]) {
+            const float2 r = rhs(3 * q.p + D) - ax[D] - imass(om, q.m[D], xc[D]);
+            v[D] = resid ? r : xc[D] + idiag(om, kEmgEdge, S[D], q.m[D], r);
+        }
 }
 
-// positions and weights of the twelve neighbours of an edge, as curl_row sums them
-template <int D>
-__device__ __forceinline__ void curl_stencil(const EmgLevel& L, int i, int j, int k, int (&at)[12], float (&w)[12],
-                                             float& S) {
-    const int n = L.n;
-    S = 0.0f;
-    auto dir = [&](auto tag, int o) {
-        constexpr int A = decltype(tag)::value, B = 3 - D - A;
-        constexpr int ai = A == 0, aj = A == 1, ak = A == 2, di = D == 0, dj = D == 1, dk = D == 2;
-        const float hd = L.h[D], ha = L.h[A];
-        const float wp = __ldg(&L.w[fid<B>(n, i, j, k)]), wm = __ldg(&L.w[fid<B>(n, i - ai, j - aj, k - ak)]);
-        at[o] = eid<D>(n, i + ai, j + aj, k + ak);
-        at[o + 1] = eid<D>(n, i - ai, j - aj, k - ak);
-        at[o + 2] = eid<A>(n, i + di, j + dj, k + dk);
-        at[o + 3] = eid<A>(n, i, j, k);
-        at[o + 4] = eid<A>(n, i - ai + di, j - aj + dj, k - ak + dk);
-        at[o + 5] = eid<A>(n, i - ai, j - aj, k - ak);
-        w[o] = -hd * hd * wp;
-        w[o + 1] = -hd * hd * wm;
-        w[o + 2] = hd * ha * wp;
-        w[o + 3] = -hd * ha * wp;
-        w[o + 4] = -hd * ha * wm;
-        w[o + 5] = hd * ha * wm;
-        S += hd * hd * (wp + wm);
-    };
-    dir(Dir<D == 0 ? 1 : 0>{}, 0);
-    dir(Dir<D == 2 ? 1 : 2>{}, 6);
-}
-
-__global__ void __launch_bounds__(kBottomNT) k_bottom(EmgDev g, int l0, int K, Omegas oms) {
-    extern __shared__ float2 sm[];
-    const int lane = blockIdx.x, tid = threadIdx.x;
-    const Om<float2> om{oms.v[lane]};
-    const int nl = g.n_levels;
-    const bool two = l0 + 1 < nl;
-    const EmgLevel& L = g.lv[l0];
+// Cycle of the levels from l1 (8 or 4 cells) on, by one block: three vectors
+// per level in sm; b and x of the first level are filled in by load(b, x).
+// Returns the first level's result (shared memory).
+template <class Load>
+__device__ __forceinline__ const float2* small_cycle(const EmgDev& g, int l1, Om<float2> om, float2* sm,
+                                                     const Load& load) {
+    const int tid = threadIdx.x, nl = g.n_levels;
+    const EmgLevel& L = g.lv[l1];
     const EmgLevel& C = g.lv[nl - 1];
-    const int nL = 3 * L.n * (L.n + 1) * (L.n + 1), nC = 3 * C.n * (C.n + 1) * (C.n + 1);
-    // b, x and a third vector per level (the levels' own b, x: zero on edges that are not free)
+    const bool two = l1 + 1 < nl;
+    const int nL = entries(L), nC = entries(C);
     float2 *b = sm, *x = sm + nL, *y = sm + 2 * nL;
     float2 *cb = two ? sm + 3 * nL : b, *cx = two ? cb + nC : x, *cy = two ? cx + nC : y;
-    for (int e = tid; e < nL; e += kBottomNT) {
-        b[e] = L.b[(size_t)e * K + lane];
-        x[e] = L.x[(size_t)e * K + lane];
-        y[e] = make_float2(0.f, 0.f);
-    }
-    if (two)
-        for (int e = tid; e < nC; e += kBottomNT) cx[e] = cy[e] = make_float2(0.f, 0.f);
-    // the coarsest grid's stencil (at most 300 edges, one per thread)
-    int at[12];
-    float w[12], S = 0.0f, m = 0.0f;
-    bool mine = false;
-    with_edge(C, tid, [&](auto tag, int i, int j, int k) {
-        curl_stencil<decltype(tag)::value>(C, i, j, k, at, w, S);
-        m = __ldg(&C.me[tid]);
-        mine = true;
-    });
+    for (float2* z = sm + tid; z < cy + nC; z += kBottomNT) *z = vz<float2>();
+    const bool in = tid < points(L);
+    Point pl, pc;
+    pl.load(L, tid, in && two);
+    pc.load(C, tid, tid < points(C));
+    float S[3];
+    edge_diags(C, pc.w, S);
+    float2 rhs[3] = {};
     __syncthreads();
-    auto step = [&](const float2* in, float2* out, bool resid) {
-        for (int e = tid; e < nL; e += kBottomNT)
-            with_edge(L, e, [&](auto tag, int i, int j, int k) {
-                const float me = __ldg(&L.me[e]);
-                float d;
-                const float2 ax = curl_row<decltype(tag)::value, float2>(L, i, j, k, in[e],
-                                                                         [&](int q) { return in[q]; }, d);
-                const float2 r = b[e] - ax - imass(om, me, in[e]);
-                out[e] = resid ? r : in[e] + idiag(om, kEmgEdge, d, me, r);
-            });
-        __syncthreads();
-    };
+    load(b, x);
+    __syncthreads();
     if (two) {
-        step(x, y, true);
-        if (mine)
-            with_edge(C, tid, [&](auto tag, int i, int j, int k) {
-                const float2 s = gather_edge<decltype(tag)::value, float2>(L.n, i, j, k, [&](int q) { return y[q]; });
-                cb[tid] = s;
-                cx[tid] = idiag(om, kEmgEdge, S, m, s);
-            });
-        __syncthreads();
-    }
-    const float2 bb = mine ? cb[tid] : make_float2(0.f, 0.f);
-    for (int q = 0; q < kCoarsestSteps; ++q) {
-        const float2* in = q & 1 ? cy : cx;
-        if (mine) {
-            const float2 xc = in[tid];
-            float2 ax = S * xc;
+        if (in) {
+            float2 v[3];
+            point_step(L, om, pl, true, [&](int e) { return x[e]; }, [&](int e) { return b[e]; }, v);
 #pragma unroll
-            for (int u = 0; u < 12; ++u) ax = ax + w[u] * in[at[u]];
-            (q & 1 ? cx : cy)[tid] = xc + idiag(om, kEmgEdge, S, m, bb - ax - imass(om, m, xc));
+            for (int D = 0; D < 3; ++D) y[3 * tid + D] = v[D];
+        }
+        __syncthreads();
+        if (pc.any) {
+            gather_edges<float2>(pc.f, L.n, pc.i, pc.j, pc.k, [&](int e) { return y[e]; }, rhs);
+#pragma unroll
+            for (int D = 0; D < 3; ++D) cx[3 * tid + D] = idiag(om, kEmgEdge, S[D], pc.m[D], rhs[D]);
+        }
+        __syncthreads();
+    } else if (pc.any) {
+#pragma unroll
+        for (int D = 0; D < 3; ++D) rhs[D] = b[3 * tid + D];
+    }
+    for (int q = 0; q < kCoarsestSteps; ++q) {
+        const float2* u = q & 1 ? cy : cx;
+        float2* v = q & 1 ? cx : cy;
+        if (pc.any) {
+            float2 xc[3], ax[3];
+            curl_rows<float2>(C, pc.w, pc.i, pc.j, pc.k, [&](int e) { return u[e]; }, xc, ax);
+#pragma unroll
+            for (int D = 0; D < 3; ++D)
+                if (pc.f.e[D])
+                    v[3 * tid + D] =
+                        xc[D] + idiag(om, kEmgEdge, S[D], pc.m[D], rhs[D] - ax[D] - imass(om, pc.m[D], xc[D]));
         }
         __syncthreads();
     }
-    const float2* out = cx;
-    if (two) {
-        for (int e = tid; e < nL; e += kBottomNT)
-            with_edge(L, e, [&](auto tag, int i, int j, int k) {
-                x[e] = x[e] + interp_edge<decltype(tag)::value, float2>(C.n, i, j, k, [&](int q) { return cx[q]; });
-            });
-        __syncthreads();
-        // y holds the residual on free edges only, which the step overwrites
-        step(x, y, false);
-        out = y;
+    if (!two) return cx;
+    if (in) {
+        float2 s[3];
+        interp_edges<float2>(pl.f, C.n, pl.i, pl.j, pl.k, [&](int e) { return cx[e]; }, s);
+#pragma unroll
+        for (int D = 0; D < 3; ++D) x[3 * tid + D] = x[3 * tid + D] + s[D];
     }
-    // every edge: the finer level's interpolation reads the zeros too
-    for (int e = tid; e < nL; e += kBottomNT) L.y[(size_t)e * K + lane] = out[e];
+    __syncthreads();
+    if (in) {
+        float2 v[3];
+        point_step(L, om, pl, false, [&](int e) { return x[e]; }, [&](int e) { return b[e]; }, v);
+#pragma unroll
+        for (int D = 0; D < 3; ++D) y[3 * tid + D] = v[D];
+    }
+    __syncthreads();
+    return y;
+}
+
+// From level l0 of 8 or 4 cells: one block per right-hand side.
+__global__ void __launch_bounds__(kBottomNT) k_bottom(EmgDev g, int l0, Omegas oms) {
+    extern __shared__ float2 sm[];
+    const EmgLevel& L = g.lv[l0];
+    const int lane = blockIdx.x, ne = entries(L);
+    const float2* v = small_cycle(g, l0, Om<float2>{oms.v[lane]}, sm, [&](float2* b, float2* x) {
+        for (int e = threadIdx.x; e < ne; e += kBottomNT) {
+            b[e] = L.b[(size_t)lane * ne + e];
+            x[e] = L.x[(size_t)lane * ne + e];
+        }
+    });
+    for (int e = threadIdx.x; e < ne; e += kBottomNT) L.y[(size_t)lane * ne + e] = v[e];
+}
+
+// From level l0 of 16 cells: a cluster of NC blocks per right-hand side.
+template <int NC>
+__global__ void __launch_bounds__(kBottomNT) k_bottom16(EmgDev g, int l0, Omegas oms) {
+    extern __shared__ float2 sm[];
+    constexpr int PT = 8 / NC;   // points per thread
+    const EmgLevel& L = g.lv[l0];
+    const EmgLevel& C = g.lv[l0 + 1];
+    const int lane = blockIdx.x / NC, rank = cluster_rank(), tid = threadIdx.x, ne = entries(L), nc = entries(C);
+    const Om<float2> om{oms.v[lane]};
+    const float2* b = L.b + (size_t)lane * ne;
+    float2 *x = L.x + (size_t)lane * ne, *y = L.y + (size_t)lane * ne, *cy = C.y + (size_t)lane * nc;
+    const int m = (L.n + 1) * (L.n + 1) * edge_planes(L);
+    Point q[PT];
+    float2 v[3];
+#pragma unroll
+    for (int u = 0; u < PT; ++u) {
+        const int p = (u * NC + rank) * kBottomNT + tid;
+        q[u].load(L, p, p < m);
+        if (p < m) {
+            point_step(L, om, q[u], true, [&](int e) { return x[e]; }, [&](int e) { return b[e]; }, v);
+#pragma unroll
+            for (int D = 0; D < 3; ++D) y[3 * p + D] = v[D];
+        }
+    }
+    cluster_sync();
+    if (rank == 0) {
+        const float2* r = small_cycle(g, l0 + 1, om, sm, [&](float2* cb, float2* cx) {
+            Point c;
+            c.load(C, tid, tid < points(C));
+            if (!c.any) return;
+            float2 s[3];
+            float S[3];
+            gather_edges<float2>(c.f, L.n, c.i, c.j, c.k, [&](int e) { return __ldcg(&y[e]); }, s);
+            edge_diags(C, c.w, S);
+#pragma unroll
+            for (int D = 0; D < 3; ++D) {
+                cb[3 * tid + D] = s[D];
+                cx[3 * tid + D] = idiag(om, kEmgEdge, S[D], c.m[D], s[D]);
+            }
+        });
+        for (int e = tid; e < nc; e += kBottomNT) cy[e] = r[e];
+    }
+    cluster_sync();
+#pragma unroll
+    for (int u = 0; u < PT; ++u)
+        if (q[u].any) {
+            interp_edges<float2>(q[u].f, C.n, q[u].i, q[u].j, q[u].k, [&](int e) { return __ldcg(&cy[e]); }, v);
+#pragma unroll
+            for (int D = 0; D < 3; ++D)
+                if (q[u].f.e[D]) x[3 * q[u].p + D] = x[3 * q[u].p + D] + v[D];
+        }
+    cluster_sync();
+#pragma unroll
+    for (int u = 0; u < PT; ++u)
+        if (q[u].p < m) {
+            point_step(L, om, q[u], false, [&](int e) { return __ldcg(&x[e]); }, [&](int e) { return b[e]; }, v);
+#pragma unroll
+            for (int D = 0; D < 3; ++D) y[3 * q[u].p + D] = v[D];
+        }
 }
 
 // ---------------------------------------------------------------------------
@@ -509,7 +618,7 @@ __global__ void __launch_bounds__(kBottomNT) k_bottom(EmgDev g, int l0, int K, O
 // Laplacian row on a uniform grid: six edges, coarse edge masses over h^2
 template <class V, class At>
 __device__ __forceinline__ V lap_row(const EmgLevel& L, int i, int j, int k, V xc, const At& at, float& d) {
-    const int n = L.n;
+    const int n1 = L.n + 1, p = pid(L.n, i, j, k);
     V s = vz<V>();
     d = 0.0f;
     auto put = [&](int e, int v, float ih2) {
@@ -518,26 +627,20 @@ __device__ __forceinline__ V lap_row(const EmgLevel& L, int i, int j, int k, V x
         d += m;
     };
     const float a = 1.0f / (L.h[0] * L.h[0]), b = 1.0f / (L.h[1] * L.h[1]), c = 1.0f / (L.h[2] * L.h[2]);
-    put(eid<0>(n, i - 1, j, k), nid(n, i - 1, j, k), a);
-    put(eid<0>(n, i, j, k), nid(n, i + 1, j, k), a);
-    put(eid<1>(n, i, j - 1, k), nid(n, i, j - 1, k), b);
-    put(eid<1>(n, i, j, k), nid(n, i, j + 1, k), b);
-    put(eid<2>(n, i, j, k - 1), nid(n, i, j, k - 1), c);
-    put(eid<2>(n, i, j, k), nid(n, i, j, k + 1), c);
+    put(3 * (p - 1), p - 1, a);
+    put(3 * p, p + 1, a);
+    put(3 * (p - n1) + 1, p - n1, b);
+    put(3 * p + 1, p + n1, b);
+    put(3 * (p - n1 * n1) + 2, p - n1 * n1, c);
+    put(3 * p + 2, p + n1 * n1, c);
     return s;
-}
-
-// diagonal of the node Laplacian on a uniform grid
-__device__ __forceinline__ float lap_diag(const EmgLevel& L, int i, int j, int k) {
-    const int n = L.n;
-    return (__ldg(&L.me[eid<0>(n, i - 1, j, k)]) + __ldg(&L.me[eid<0>(n, i, j, k)])) / (L.h[0] * L.h[0]) +
-           (__ldg(&L.me[eid<1>(n, i, j - 1, k)]) + __ldg(&L.me[eid<1>(n, i, j, k)])) / (L.h[1] * L.h[1]) +
-           (__ldg(&L.me[eid<2>(n, i, j, k - 1)]) + __ldg(&L.me[eid<2>(n, i, j, k)])) / (L.h[2] * L.h[2]);
 }
 
 // w b / diag, the pre-smoothed iterate of the V(1,1) cycle
 template <class V> __device__ __forceinline__ V node_pre(const EmgLevel& L, int i, int j, int k, V b) {
-    const float d = node_free(L, i, j, k) ? lap_diag(L, i, j, k) : 0.0f;
+    if (!node_free(L, i, j, k)) return vz<V>();
+    float d;
+    lap_row<F1>(L, i, j, k, F1{0.0f}, [&](int) { return F1{0.0f}; }, d);
     return d > 0.0f ? (kEmgNode / d) * b : vz<V>();
 }
 
@@ -546,25 +649,25 @@ template <int K, bool PRE>
 __global__ void __launch_bounds__(kNT) k_node_restrict0(EmgDev g, const float4* __restrict__ b) {
     constexpr int H = K / 2;
     const EmgLevel& L = g.lv[0];
-    each_node<H>(L, [&](int i, int j, int k, int h) {
-        const int c = nid(L.n, i, j, k);
+    each_point<H>(L, [&](int i, int j, int k, int h) {
+        const int c = pid(L.n, i, j, k);
         float4 s = vz<float4>();
         const int q0 = __ldg(&g.nr_ptr[c]), q1 = __ldg(&g.nr_ptr[c + 1]);
         if (q1 - q0 > kLongRow) return;   // k_node_restrict0_long
-        for (int q = q0; q < q1; q += 4) {
-            float w[4];
-            float4 v[4];
+        for (int q = q0; q < q1; q += 9) {   // 27 entries under one level of refinement
+            float w[9];
+            float4 v[9];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < 9; ++u) {
                 const bool ok = q + u < q1;
                 w[u] = ok ? __ldg(&g.nr_w[q + u]) : 0.0f;
                 v[u] = ok ? b[(size_t)__ldg(&g.nr_node[q + u]) * H + h] : vz<float4>();
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) s = s + w[u] * v[u];
+            for (int u = 0; u < 9; ++u) s = s + w[u] * v[u];
         }
-        f4(L.nb)[(size_t)c * H + h] = s;
-        if (PRE) f4(L.nt)[(size_t)c * H + h] = node_pre(L, i, j, k, s);
+        store2<K>(L.nb, lane_major(L), points(L), c, h, s);
+        if (PRE && !lane_major(L)) f4(L.nt)[(size_t)c * H + h] = node_pre(L, i, j, k, s);
     });
 }
 
@@ -575,26 +678,28 @@ __global__ void __launch_bounds__(kLongNT) k_node_restrict0_long(EmgDev g, const
     const int c = g.nr_long[blockIdx.x], n1 = L.n + 1, h = threadIdx.x % H;
     const float4 s = long_row<H>(g.nr_node, g.nr_w, g.nr_ptr[c], g.nr_ptr[c + 1], b);
     if (threadIdx.x >= H) return;
-    f4(L.nb)[(size_t)c * H + h] = s;
-    if (PRE) f4(L.nt)[(size_t)c * H + h] = node_pre(L, c % n1, c / n1 % n1, c / (n1 * n1), s);
+    store2<K>(L.nb, lane_major(L), points(L), c, h, s);
+    if (PRE && !lane_major(L))
+        f4(L.nt)[(size_t)c * H + h] = node_pre(L, c % n1, c / n1 % n1, c / (n1 * n1), s);
 }
 
-// ny = nb - L nt
-template <int K>
-__global__ void __launch_bounds__(kNT) k_node_resid(EmgLevel L) {
+// ny = nb - L nt, or (SMOOTH) ny = nt + w (nb - L nt) / diag
+template <int K, bool SMOOTH>
+__global__ void __launch_bounds__(kNT) k_node_step(EmgLevel L) {
     constexpr int H = K / 2;
-    each_node<H>(L, [&](int i, int j, int k, int h) {
-        const size_t c = (size_t)nid(L.n, i, j, k) * H + h;
+    each_point<H>(L, [&](int i, int j, int k, int h) {
+        const size_t c = (size_t)pid(L.n, i, j, k) * H + h;
         float4 v = vz<float4>();
         if (node_free(L, i, j, k)) {
             const float4* t = f4(L.nt);
+            const float4 tc = t[c];
             float d;
-            v = f4(L.nb)[c] - lap_row<float4>(L, i, j, k, t[c], [&](int q) { return t[(size_t)q * H + h]; }, d);
+            v = f4(L.nb)[c] - lap_row<float4>(L, i, j, k, tc, [&](int q) { return t[(size_t)q * H + h]; }, d);
+            if (SMOOTH) v = d > 0.0f ? tc + (kEmgNode / d) * v : tc;
         }
         f4(L.ny)[c] = v;
     });
 }
-
 
 template <class V, class At>
 __device__ __forceinline__ V gather_node(int n, int I, int J, int Kk, const At& at) {
@@ -606,7 +711,7 @@ __device__ __forceinline__ V gather_node(int n, int I, int J, int Kk, const At& 
 #pragma unroll
             for (int a = -1; a <= 1; ++a)
                 s = s + ((a ? 0.5f : 1.0f) * (b ? 0.5f : 1.0f) * (c ? 0.5f : 1.0f)) *
-                            at(nid(n, 2 * I + a, 2 * J + b, 2 * Kk + c));
+                            at(pid(n, 2 * I + a, 2 * J + b, 2 * Kk + c));
     return s;
 }
 template <class V, class At>
@@ -615,7 +720,7 @@ __device__ __forceinline__ V interp_node(int n, int i, int j, int k, const At& a
     V s = vz<V>();
     for (int c = 0; c <= ok; ++c)
         for (int b = 0; b <= oj; ++b)
-            for (int a = 0; a <= oi; ++a) s = s + at(nid(n, (i >> 1) + a, (j >> 1) + b, (k >> 1) + c));
+            for (int a = 0; a <= oi; ++a) s = s + at(pid(n, (i >> 1) + a, (j >> 1) + b, (k >> 1) + c));
     return ((oi ? 0.5f : 1.0f) * (oj ? 0.5f : 1.0f) * (ok ? 0.5f : 1.0f)) * s;
 }
 
@@ -624,14 +729,14 @@ __device__ __forceinline__ V interp_node(int n, int i, int j, int k, const At& a
 template <int K, bool PRE>
 __global__ void __launch_bounds__(kNT) k_node_restrict(EmgLevel F, EmgLevel L) {
     constexpr int H = K / 2;
-    each_node<H>(L, [&](int i, int j, int k, int h) {
+    each_point<H>(L, [&](int i, int j, int k, int h) {
         float4 s = vz<float4>();
         const float4* b = f4(PRE ? F.ny : F.nb);
         if (node_free(L, i, j, k))
             s = gather_node<float4>(F.n, i, j, k, [&](int v) { return b[(size_t)v * H + h]; });
-        const size_t c = (size_t)nid(L.n, i, j, k) * H + h;
-        f4(L.nb)[c] = s;
-        if (PRE) f4(L.nt)[c] = node_pre(L, i, j, k, s);
+        const int c = pid(L.n, i, j, k);
+        store2<K>(L.nb, lane_major(L), points(L), c, h, s);
+        if (PRE && !lane_major(L)) f4(L.nt)[(size_t)c * H + h] = node_pre(L, i, j, k, s);
     });
 }
 
@@ -639,91 +744,133 @@ __global__ void __launch_bounds__(kNT) k_node_restrict(EmgLevel F, EmgLevel L) {
 template <int K, bool PRE>
 __global__ void __launch_bounds__(kNT) k_node_prolong(EmgLevel L, EmgLevel C) {
     constexpr int H = K / 2;
-    each_node<H>(L, [&](int i, int j, int k, int h) {
+    each_point<H>(L, [&](int i, int j, int k, int h) {
         float4 s = vz<float4>();
-        const float4* y = f4(C.ny);
+        const bool lm = lane_major(C);
+        const int np = points(C);
         if (node_free(L, i, j, k))
-            s = interp_node<float4>(C.n, i, j, k, [&](int v) { return y[(size_t)v * H + h]; });
-        const size_t c = (size_t)nid(L.n, i, j, k) * H + h;
+            s = interp_node<float4>(C.n, i, j, k, [&](int v) { return load2<K>(C.ny, lm, np, v, h); });
+        const size_t c = (size_t)pid(L.n, i, j, k) * H + h;
         f4(L.nt)[c] = PRE ? f4(L.nt)[c] + s : s;
     });
 }
 
-// ny = t + w (nb - L t) / diag
-template <int K>
-__global__ void __launch_bounds__(kNT) k_node_smooth(EmgLevel L) {
-    constexpr int H = K / 2;
-    each_node<H>(L, [&](int i, int j, int k, int h) {
-        const size_t c = (size_t)nid(L.n, i, j, k) * H + h;
-        float4 v = vz<float4>();
-        if (node_free(L, i, j, k)) {
-            const float4* t = f4(L.nt);
-            const float4 tc = t[c];
-            float d;
-            const float4 lt = lap_row<float4>(L, i, j, k, tc, [&](int q) { return t[(size_t)q * H + h]; }, d);
-            v = d > 0.0f ? tc + (kEmgNode / d) * (f4(L.nb)[c] - lt) : tc;
-        }
-        f4(L.ny)[c] = v;
-    });
-}
-
-template <bool PRE>
-__global__ void __launch_bounds__(kBottomNT) k_node_bottom(EmgDev g, int l0, int K) {
-    constexpr int kN = (kEmgBottom + 1) * (kEmgBottom + 1) * (kEmgBottom + 1);
-    constexpr int kNc = 5 * 5 * 5;
-    static_assert(kN <= kBottomNT, "one node per thread");
-    __shared__ float2 b[kN], x[kN], y[kN], cb[kNc], cx[kNc], cy[kNc];
-    const int lane = blockIdx.x, tid = threadIdx.x, nl = g.n_levels;
-    const bool two = l0 + 1 < nl;
-    const EmgLevel& L = g.lv[l0];
+// The small node grids, as the small edge grids above.
+template <bool PRE, class Load>
+__device__ __forceinline__ const float2* small_node_cycle(const EmgDev& g, int l1, float2* sm, const Load& load) {
+    const int tid = threadIdx.x, nl = g.n_levels;
+    const EmgLevel& L = g.lv[l1];
     const EmgLevel& C = g.lv[nl - 1];
-    const int nL = (L.n + 1) * (L.n + 1) * (L.n + 1);
-    const int i = tid % (L.n + 1), j = tid / (L.n + 1) % (L.n + 1), k = tid / ((L.n + 1) * (L.n + 1));
-    const int ci = tid % 5, cj = tid / 5 % 5, ck = tid / 25;   // two: the coarsest grid has 4 cells per side
-    const bool in = tid < nL && node_free(L, i, j, k);
-    const bool cin = two && tid < kNc && node_free(C, ci, cj, ck);
-    if (tid < nL) {
-        b[tid] = in ? L.nb[(size_t)tid * K + lane] : make_float2(0.f, 0.f);
-        x[tid] = y[tid] = make_float2(0.f, 0.f);
-    }
-    if (tid < kNc) cb[tid] = cx[tid] = cy[tid] = make_float2(0.f, 0.f);
+    const bool two = l1 + 1 < nl;
+    const int nL = points(L), nC = points(C);
+    float2 *b = sm, *x = sm + nL, *y = sm + 2 * nL;
+    float2 *cb = two ? sm + 3 * nL : b, *cx = two ? cb + nC : x, *cy = two ? cx + nC : y;
+    for (float2* z = sm + tid; z < cy + nC; z += kBottomNT) *z = vz<float2>();
+    const int n1 = L.n + 1, i = tid % n1, j = tid / n1 % n1, k = tid / (n1 * n1);
+    const int c1 = C.n + 1, ci = tid % c1, cj = tid / c1 % c1, ck = tid / (c1 * c1);
+    const bool in = tid < nL && node_free(L, i, j, k), cin = tid < nC && node_free(C, ci, cj, ck);
     __syncthreads();
-    auto jacobi = [&](const EmgLevel& M, bool on, int a, int c, int d, const float2* rhs, const float2* v, float2* out) {
+    load(b);
+    __syncthreads();
+    auto step = [&](const EmgLevel& M, bool on, int a, int c, int d, const float2* rhs, const float2* v, float2* out) {
         if (on) {
             float dg;
-            const float2 lv = lap_row<float2>(M, a, c, d, v[tid], [&](int q) { return v[q]; }, dg);
-            out[tid] = dg > 0.0f ? v[tid] + (kEmgNode / dg) * (rhs[tid] - lv) : v[tid];
+            const float2 r = rhs[tid] - lap_row<float2>(M, a, c, d, v[tid], [&](int q) { return v[q]; }, dg);
+            out[tid] = dg > 0.0f ? v[tid] + (kEmgNode / dg) * r : v[tid];
         }
         __syncthreads();
     };
-    const float2* rc = b;   // what the coarsest grid gets
-    if (two && PRE) {
-        if (in) x[tid] = node_pre(L, i, j, k, b[tid]);
-        __syncthreads();
-        if (in) {
-            float dg;
-            y[tid] = b[tid] - lap_row<float2>(L, i, j, k, x[tid], [&](int q) { return x[q]; }, dg);
-        }
-        __syncthreads();
-        rc = y;
-    }
     if (two) {
-        if (cin) cb[tid] = gather_node<float2>(L.n, ci, cj, ck, [&](int q) { return rc[q]; });
-        __syncthreads();
-        for (int q = 0; q < kCoarsestSteps; q += 2) {   // from zero
-            jacobi(C, cin, ci, cj, ck, cb, cx, cy);
-            jacobi(C, cin, ci, cj, ck, cb, cy, cx);
+        const float2* src = b;
+        if (PRE) {
+            if (in) x[tid] = node_pre(L, i, j, k, b[tid]);
+            __syncthreads();
+            if (in) {
+                float dg;
+                y[tid] = b[tid] - lap_row<float2>(L, i, j, k, x[tid], [&](int q) { return x[q]; }, dg);
+            }
+            __syncthreads();
+            src = y;
         }
-        if (in) x[tid] = x[tid] + interp_node<float2>(C.n, i, j, k, [&](int q) { return cx[q]; });
+        if (cin) cb[tid] = gather_node<float2>(L.n, ci, cj, ck, [&](int q) { return src[q]; });
         __syncthreads();
-        jacobi(L, in, i, j, k, b, x, y);
-    } else {
-        for (int q = 0; q < kCoarsestSteps; q += 2) {
-            jacobi(L, in, i, j, k, b, x, y);
-            jacobi(L, in, i, j, k, b, y, x);
-        }
     }
-    if (tid < nL) L.ny[(size_t)tid * K + lane] = two ? y[tid] : x[tid];
+    for (int q = 0; q < kCoarsestSteps; q += 2) {   // from zero
+        step(C, cin, ci, cj, ck, cb, cx, cy);
+        step(C, cin, ci, cj, ck, cb, cy, cx);
+    }
+    if (!two) return cx;
+    if (in) x[tid] = x[tid] + interp_node<float2>(C.n, i, j, k, [&](int q) { return cx[q]; });
+    __syncthreads();
+    step(L, in, i, j, k, b, x, y);
+    return y;
+}
+
+template <bool PRE> __global__ void __launch_bounds__(kBottomNT) k_node_bottom(EmgDev g, int l0) {
+    extern __shared__ float2 sm[];
+    const EmgLevel& L = g.lv[l0];
+    const int lane = blockIdx.x, np = points(L);
+    const float2* v = small_node_cycle<PRE>(g, l0, sm, [&](float2* b) {
+        for (int t = threadIdx.x; t < np; t += kBottomNT) b[t] = L.nb[(size_t)lane * np + t];
+    });
+    for (int t = threadIdx.x; t < np; t += kBottomNT) L.ny[(size_t)lane * np + t] = v[t];
+}
+
+template <int NC, bool PRE> __global__ void __launch_bounds__(kBottomNT) k_node_bottom16(EmgDev g, int l0) {
+    extern __shared__ float2 sm[];
+    constexpr int PT = 8 / NC;
+    const EmgLevel& L = g.lv[l0];
+    const EmgLevel& C = g.lv[l0 + 1];
+    const int lane = blockIdx.x / NC, rank = cluster_rank(), tid = threadIdx.x, np = points(L), nc = points(C);
+    const float2* b = L.nb + (size_t)lane * np;
+    float2 *x = L.nt + (size_t)lane * np, *y = L.ny + (size_t)lane * np, *cy = C.ny + (size_t)lane * nc;
+    float2 xv[PT];
+    auto each = [&](const auto& f) {   // f(u, i, j, k, p, free)
+#pragma unroll
+        for (int u = 0; u < PT; ++u) {
+            const int p = (u * NC + rank) * kBottomNT + tid, n1 = L.n + 1;
+            const int i = p % n1, j = p / n1 % n1, k = p / (n1 * n1);
+            if (p < np) f(u, i, j, k, p, node_free(L, i, j, k));
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < PT; ++u) xv[u] = vz<float2>();
+    if (PRE) {
+        each([&](int u, int i, int j, int k, int p, bool in) {
+            if (in) xv[u] = node_pre(L, i, j, k, b[p]);
+            x[p] = xv[u];
+        });
+        cluster_sync();
+        each([&](int u, int i, int j, int k, int p, bool in) {
+            float d;
+            y[p] = in ? b[p] - lap_row<float2>(L, i, j, k, xv[u], [&](int q) { return __ldcg(&x[q]); }, d) : vz<float2>();
+        });
+        cluster_sync();
+    }
+    if (rank == 0) {
+        const float2* src = PRE ? y : b;
+        const float2* r = small_node_cycle<PRE>(g, l0 + 1, sm, [&](float2* cb) {
+            const int m1 = C.n + 1, ci = tid % m1, cj = tid / m1 % m1, ck = tid / (m1 * m1);
+            if (tid < nc && node_free(C, ci, cj, ck))
+                cb[tid] = gather_node<float2>(L.n, ci, cj, ck, [&](int q) { return __ldcg(&src[q]); });
+        });
+        for (int t = tid; t < nc; t += kBottomNT) cy[t] = r[t];
+    }
+    cluster_sync();
+    each([&](int u, int i, int j, int k, int p, bool in) {
+        if (in) xv[u] = xv[u] + interp_node<float2>(C.n, i, j, k, [&](int q) { return __ldcg(&cy[q]); });
+        x[p] = xv[u];
+    });
+    cluster_sync();
+    each([&](int u, int i, int j, int k, int p, bool in) {
+        float2 v = vz<float2>();
+        if (in) {
+            float d;
+            v = b[p] - lap_row<float2>(L, i, j, k, xv[u], [&](int q) { return __ldcg(&x[q]); }, d);
+            v = d > 0.0f ? xv[u] + (kEmgNode / d) * v : xv[u];
+        }
+        y[p] = v;
+    });
 }
 
 // t = Pn ny0 on the octree nodes (0 on Dirichlet nodes), plus x if given
@@ -740,13 +887,14 @@ __global__ void __launch_bounds__(kNT) k_node_prolong0(EmgDev g, int nn, const f
         const unsigned code = __ldg(&g.n_code[v]);
         const float u = 1.0f / (float)(1 << g.gap);
         const float fx = (float)(code & 15u) * u, fy = (float)(code >> 4 & 15u) * u, fz = (float)(code >> 8 & 15u) * u;
-        const int n1 = g.lv[0].n + 1;
-        const float4* y = f4(g.lv[0].ny);
+        const EmgLevel& L = g.lv[0];
+        const int n1 = L.n + 1, np = points(L);
+        const bool lm = lane_major(L);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const float w = (q & 1 ? fx : 1.0f - fx) * (q & 2 ? fy : 1.0f - fy) * (q & 4 ? fz : 1.0f - fz);
             if (w > 0.0f)
-                s = s + w * y[(size_t)(base + (q & 1) + (q >> 1 & 1) * n1 + (q >> 2) * n1 * n1) * H + h];
+                s = s + w * load2<K>(L.ny, lm, np, base + (q & 1) + (q >> 1 & 1) * n1 + (q >> 2) * n1 * n1, h);
         }
     }
     out[i] = s;
@@ -767,9 +915,10 @@ __global__ void __launch_bounds__(kNT) k_combine(EmgDev g, GcRowTerm gt, DiagVie
         const unsigned code = __ldg(&g.p_code[row]);
         const float u = 1.0f / (float)(1 << g.gap);
         const float fa = (float)(code >> 2 & 15u) * u, fb = (float)(code >> 6 & 15u) * u;
-        const int d = code & 3u, m = g.lv[0].n, nx = d == 0 ? m : m + 1, ny = d == 1 ? m : m + 1;
-        const int sa = d == 0 ? nx : 1, sb = d == 2 ? nx : nx * ny;
-        const float4* y = f4(g.lv[0].y);
+        const EmgLevel& L = g.lv[0];
+        const int d = code & 3u, n1 = L.n + 1, ne = entries(L);
+        const int sa = d == 0 ? 3 * n1 : 3, sb = d == 2 ? 3 * n1 : 3 * n1 * n1;
+        const bool lm = lane_major(L);
         const int2 nd = __ldg(reinterpret_cast<const int2*>(gt.e_node) + row);
         const float2 ge = __ldg(reinterpret_cast<const float2*>(gt.e_g) + row);
         const float4* yn = f4(gt.ya);
@@ -780,7 +929,7 @@ __global__ void __launch_bounds__(kNT) k_combine(EmgDev g, GcRowTerm gt, DiagVie
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const float w = wa[q & 1] * wb[q >> 1];
-            if (w > 0.0f) z = z + w * y[(size_t)(base + (q & 1) * sa + (q >> 1) * sb) * H + h];
+            if (w > 0.0f) z = z + w * load2<K>(L.y, lm, ne, base + (q & 1) * sa + (q >> 1) * sb, h);
         }
         const float s0 = gt.s[2 * h], s1 = gt.s[2 * h + 1];
         z = z + make_float4(s0 * c.y, -s0 * c.x, s1 * c.w, -s1 * c.z);
@@ -796,36 +945,58 @@ int bottom_level(const EmgDev& g) {
     return l;
 }
 
-// shared memory of the bottom edge kernel: three vectors of each of its levels
-int bottom_smem(const EmgDev& g, int l0) {
-    size_t b = 0;
-    for (int l = l0; l < g.n_levels; ++l) b += 3 * sizeof(float2) * (size_t)emg_edges(g.lv[l].n);
-    return (int)b;
+// Launches the kernel of the small grids from level l0 on: 16 cells as a
+// cluster per right-hand side (its own grid in global memory), less as a block.
+// per: vectors' entries per level in shared memory, three of them.
+template <class F16, class F8, class... Args>
+void launch_bottom(F16* k16, F8* k8, const EmgDev& g, int l0, int K, long (*per)(int), cudaStream_t s, Args... args) {
+    const int nc = cluster_blocks(K);
+    const bool big = g.lv[l0].n > 8;
+    int smem = 0;
+    for (int l = l0 + (big ? 1 : 0); l < g.n_levels; ++l) smem += 3 * (int)(per(g.lv[l].n) * sizeof(float2));
+    const void* f = big ? reinterpret_cast<const void*>(k16) : reinterpret_cast<const void*>(k8);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (!big) {
+        k8<<<K, kBottomNT, smem, s>>>(g, l0, args...);
+        return;
+    }
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = nc;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(K * nc));
+    cfg.blockDim = dim3(kBottomNT);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k16, g, l0, args...);
+    if (e != cudaSuccess) throw std::runtime_error(cudaGetErrorString(e));
 }
 
 template <int K>
 void edge_cycle(const EmgDev& g, const Omegas& om, const float2* r, cudaStream_t s, long long* launches) {
-    const int l0 = bottom_level(g);
-    k_restrict0<K><<<edge_grid<K>(g.lv[0]), kNT, 0, s>>>(g, om, f4(r));
+    const int l0 = bottom_level(g), n = (int)(3L * (g.lv[0].n + 1) * (g.lv[0].n + 1) * edge_planes(g.lv[0]));
+    k_restrict0<K><<<grid1((long)n * (K / 2)), kNT, 0, s>>>(g, om, f4(r), n);
     ck(launches);
     if (g.n_r_long) {
         k_restrict0_long<K><<<g.n_r_long, kLongNT, 0, s>>>(g, om, f4(r));
         ck(launches);
     }
+    auto grid = [&](int l) { return point_grid<K>(g.lv[l], edge_planes(g.lv[l])); };
     for (int l = 0; l < l0; ++l) {
-        k_resid<K><<<edge_grid<K>(g.lv[l]), kNT, 0, s>>>(g.lv[l], om);
+        k_edge_step<K, false><<<grid(l), kNT, 0, s>>>(g.lv[l], om);
         ck(launches);
-        k_restrict<K><<<edge_grid<K>(g.lv[l + 1]), kNT, 0, s>>>(g.lv[l], g.lv[l + 1], om);
+        k_restrict<K><<<grid(l + 1), kNT, 0, s>>>(g.lv[l], g.lv[l + 1], om);
         ck(launches);
     }
-    const int smem = bottom_smem(g, l0);
-    cudaFuncSetAttribute(reinterpret_cast<const void*>(k_bottom), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k_bottom<<<K, kBottomNT, smem, s>>>(g, l0, K, om);
+    launch_bottom(k_bottom16<cluster_blocks(K)>, k_bottom, g, l0, K, emg_entries, s, om);
     ck(launches);
     for (int l = l0 - 1; l >= 0; --l) {
-        k_prolong<K><<<edge_grid<K>(g.lv[l]), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
+        k_prolong<K><<<grid(l), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
         ck(launches);
-        k_smooth<K><<<edge_grid<K>(g.lv[l]), kNT, 0, s>>>(g.lv[l], om);
+        k_edge_step<K, true><<<grid(l), kNT, 0, s>>>(g.lv[l], om);
         ck(launches);
     }
 }
@@ -834,7 +1005,8 @@ void edge_cycle(const EmgDev& g, const Omegas& om, const float2* r, cudaStream_t
 template <int K, bool PRE>
 void node_grids(const EmgDev& g, const float2* b, cudaStream_t s, long long* launches) {
     const int l0 = bottom_level(g);
-    k_node_restrict0<K, PRE><<<node_grid<K>(g.lv[0]), kNT, 0, s>>>(g, f4(b));
+    auto grid = [&](int l) { return point_grid<K>(g.lv[l], node_planes(g.lv[l])); };
+    k_node_restrict0<K, PRE><<<grid(0), kNT, 0, s>>>(g, f4(b));
     ck(launches);
     if (g.n_nr_long) {
         k_node_restrict0_long<K, PRE><<<g.n_nr_long, kLongNT, 0, s>>>(g, f4(b));
@@ -842,18 +1014,18 @@ void node_grids(const EmgDev& g, const float2* b, cudaStream_t s, long long* lau
     }
     for (int l = 0; l < l0; ++l) {
         if (PRE) {
-            k_node_resid<K><<<node_grid<K>(g.lv[l]), kNT, 0, s>>>(g.lv[l]);
+            k_node_step<K, false><<<grid(l), kNT, 0, s>>>(g.lv[l]);
             ck(launches);
         }
-        k_node_restrict<K, PRE><<<node_grid<K>(g.lv[l + 1]), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
+        k_node_restrict<K, PRE><<<grid(l + 1), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
         ck(launches);
     }
-    k_node_bottom<PRE><<<K, kBottomNT, 0, s>>>(g, l0, K);
+    launch_bottom(k_node_bottom16<cluster_blocks(K), PRE>, k_node_bottom<PRE>, g, l0, K, emg_points, s);
     ck(launches);
     for (int l = l0 - 1; l >= 0; --l) {
-        k_node_prolong<K, PRE><<<node_grid<K>(g.lv[l]), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
+        k_node_prolong<K, PRE><<<grid(l), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
         ck(launches);
-        k_node_smooth<K><<<node_grid<K>(g.lv[l]), kNT, 0, s>>>(g.lv[l]);
+        k_node_step<K, true><<<grid(l), kNT, 0, s>>>(g.lv[l]);
         ck(launches);
     }
 }
@@ -877,11 +1049,11 @@ std::vector<int> emg_long_rows(const std::vector<int>& ptr) {
 }
 
 void emg_set_mass(const EmgDev& g, const double* Me, cudaStream_t s, long long* launches) {
-    const int n = (int)emg_edges(g.lv[0].n);
+    const int n = (int)emg_entries(g.lv[0].n);
     k_mass0<<<(n + 255) / 256, 256, 0, s>>>(g, Me, n);
     ck(launches);
     for (int l = 1; l < g.n_levels; ++l) {
-        k_mass<<<(int)((emg_edges(g.lv[l].n) + 255) / 256), 256, 0, s>>>(g.lv[l - 1], g.lv[l]);
+        k_mass<<<(int)((emg_points(g.lv[l].n) + 255) / 256), 256, 0, s>>>(g.lv[l - 1], g.lv[l]);
         ck(launches);
     }
 }
@@ -892,7 +1064,7 @@ void emg_coarse_k(const KrylovCtx<float>& c, const float2* r, float2* z0) {
     const GcDev& gc = *c.gc;
     Omegas om;
     for (int k = 0; k < kMaxRhs; ++k) om.v[k] = k < K ? (float)c.B.omega[k] : 0.0f;
-    const double nb = (double)c.n_rows * K * sizeof(float2), e0 = (double)emg_edges(g.lv[0].n) * K * sizeof(float2),
+    const double nb = (double)c.n_rows * K * sizeof(float2), e0 = (double)emg_entries(g.lv[0].n) * K * sizeof(float2),
                  nn = (double)gc.nn * K * sizeof(float2);
     // r gathered by both restrictions and read by the last kernel, z0 written;
     // level-0 edge vectors b, x written and read, residual, x updated, y;

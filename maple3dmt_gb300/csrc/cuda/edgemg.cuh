@@ -31,7 +31,7 @@
 
 namespace m3d {
 
-constexpr int kEmgBottom = 8;      // grids of at most this many cells per side run in one block per right-hand side
+constexpr int kEmgBottom = 16;     // grids of at most this many cells per side run in one block per right-hand side
 constexpr float kEmgFine = kSmoothDamping;   // damping of the fine level's two Jacobi steps
 constexpr float kEmgEdge = 0.5f;   // ... of the uniform edge grids
 constexpr float kEmgNode = 0.6f;   // ... of the uniform node grids
@@ -42,8 +42,10 @@ struct EmgLevel {
     int ph = 0, pv = 0, pn = 0;    // planes that may hold free horizontal edges, vertical edges, nodes
     const float* w = nullptr;      // face weights
     float* me = nullptr;           // edge masses P^T Me, zero on edges that are not free
-    float2 *b = nullptr, *x = nullptr, *y = nullptr;     // edge vectors [edges][K]
-    float2 *nb = nullptr, *ny = nullptr, *nt = nullptr;  // node vectors [nodes][K]
+    // edge and node vectors, [entry][K]; on grids of the bottom kernels
+    // [K][entry], a right-hand side's values together
+    float2 *b = nullptr, *x = nullptr, *y = nullptr;
+    float2 *nb = nullptr, *ny = nullptr, *nt = nullptr;
 };
 
 struct EmgDev {

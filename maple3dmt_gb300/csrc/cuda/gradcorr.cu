@@ -359,15 +359,87 @@ GcRowTerm gc_row_term(const GcDev& g, const BatchView& B) {
     return t;
 }
 
+// b0 = G~^T in, two right-hand sides per thread and all six edges of a node in
+// flight.
+template <int K>
+__global__ void __launch_bounds__(kGcBlock) k_gc_restrict_edges2(GcDev g, const float4* __restrict__ in,
+                                                                 float4* __restrict__ out) {
+    constexpr int H = K / 2;
+    const long n = (long)g.nn * H;
+    for (long i = (long)blockIdx.x * kGcBlock + threadIdx.x; i < n; i += (long)gridDim.x * kGcBlock) {
+        const int v = (int)(i / H), h = (int)(i % H);
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int q0 = __ldg(&g.inc_ptr[v]), q1 = __ldg(&g.inc_ptr[v + 1]);
+        for (int q = q0; q < q1; q += 6) {
+            float w[6];
+            float4 e[6];
+#pragma unroll
+            for (int u = 0; u < 6; ++u) {
+                w[u] = q + u < q1 ? __ldg(&g.inc_g[q + u]) : 0.0f;
+                e[u] = w[u] != 0.0f ? in[(size_t)__ldg(&g.inc_edge[q + u]) * H + h] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < 6; ++u) {
+                s.x += w[u] * e[u].x;
+                s.y += w[u] * e[u].y;
+                s.z += w[u] * e[u].z;
+                s.w += w[u] * e[u].w;
+            }
+        }
+        out[i] = s;
+    }
+}
+
+// out = t + omega D^-1 (b - L t) on the octree's nodes, or (RESID) b - L t: two
+// right-hand sides per thread, a contiguous range of nodes per block (84 -> 76
+// us at K = 16 on 565 k nodes against a thread per right-hand side with the
+// nodes dealt out).
+template <int K, bool RESID>
+__global__ void __launch_bounds__(kGcBlock) k_gc_step0(GcDev g, const float4* __restrict__ b,
+                                                       const float4* __restrict__ t, float4* __restrict__ out) {
+    constexpr int H = K / 2;
+    const Range range = block_range(g.nn);
+    for (long i = range.b * H + threadIdx.x; i < range.e * H; i += kGcBlock) {
+        const int v = (int)(i / H), h = (int)(i % H);
+        const float4 tc = t[i], bv = b[i];
+        const float dg = __ldg(&g.lap_diag32[v]);
+        float4 s = make_float4(dg * tc.x, dg * tc.y, dg * tc.z, dg * tc.w);
+        const int q0 = __ldg(&g.inc_ptr[v]), q1 = __ldg(&g.inc_ptr[v + 1]);
+        for (int q = q0; q < q1; q += 6) {
+            float a[6];
+            float4 x[6];
+#pragma unroll
+            for (int u = 0; u < 6; ++u) {
+                const int2 e = q + u < q1 ? __ldg(&g.lap_pk[q + u]) : make_int2(0, 0);
+                a[u] = __int_as_float(e.y);
+                x[u] = a[u] != 0.0f ? t[(size_t)e.x * H + h] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < 6; ++u) {
+                s.x += a[u] * x[u].x;
+                s.y += a[u] * x[u].y;
+                s.z += a[u] * x[u].z;
+                s.w += a[u] * x[u].w;
+            }
+        }
+        const float4 r = make_float4(bv.x - s.x, bv.y - s.y, bv.z - s.z, bv.w - s.w);
+        const float c = RESID ? 1.0f : g.omega * __ldg(&g.lv[0].dinv32[v]);
+        out[i] = RESID ? r : make_float4(tc.x + c * r.x, tc.y + c * r.y, tc.z + c * r.z, tc.w + c * r.w);
+    }
+}
+
+const float4* as4(const float2* p) { return reinterpret_cast<const float4*>(p); }
+float4* as4(float2* p) { return reinterpret_cast<float4*>(p); }
+
 template <int K>
 void gc_restrict_edges_k(const GcDev& g, const float2* in, cudaStream_t s, long long* launches) {
-    k_gc_restrict_edges<K><<<gc_grid((long)g.nn * K), kGcBlock, 0, s>>>(g, in, 0);
+    k_gc_restrict_edges2<K><<<gc_grid((long)g.nn * (K / 2)), kGcBlock, 0, s>>>(g, as4(in), as4(g.lv[0].b));
     gc_check(launches);
 }
 
 template <int K>
 void gc_smooth0_k(const GcDev& g, const float2* t, float2* out, cudaStream_t s, long long* launches) {
-    k_gc_smooth0<K><<<gc_grid((long)g.nn * K), kGcBlock, 0, s>>>(g, t, out);
+    k_gc_step0<K, false><<<range_grid((long)g.nn * (K / 2)), kGcBlock, 0, s>>>(g, as4(g.lv[0].b), as4(t), as4(out));
     gc_check(launches);
 }
 
@@ -376,7 +448,8 @@ void gc_presmooth0_k(const GcDev& g, cudaStream_t s, long long* launches) {
     const int grid = gc_grid((long)g.nn * K);
     k_gc_pre0<K><<<grid, kGcBlock, 0, s>>>(g);
     gc_check(launches);
-    k_gc_resid<K, true><<<grid, kGcBlock, 0, s>>>(g, g.lv[0]);
+    k_gc_step0<K, true><<<range_grid((long)g.nn * (K / 2)), kGcBlock, 0, s>>>(g, as4(g.lv[0].b), as4(g.lv[0].x),
+                                                                            as4(g.lv[0].y));
     gc_check(launches);
 }
 

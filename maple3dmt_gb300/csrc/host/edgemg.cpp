@@ -101,7 +101,7 @@ void emg_build(const HostLayout& L, const std::vector<char>& free, const std::ve
                 }
             }
             const int a = D == 0 ? 1 : 0, b = D == 2 ? 1 : 2;
-            H.p_base[r] = (int)emg_edge_id(n0, D, base[0], base[1], base[2]);
+            H.p_base[r] = (int)emg_entry(n0, D, base[0], base[1], base[2]);
             H.p_code[r] = (uint32_t)D | (uint32_t)fr[a] << 2 | (uint32_t)fr[b] << 6;
             for (int s = 0; s < 4; ++s) {
                 int q[3] = {base[0], base[1], base[2]};
@@ -109,10 +109,10 @@ void emg_build(const HostLayout& L, const std::vector<char>& free, const std::ve
                 q[b] += s >> 1;
                 const float w = (float)((s & 1 ? fr[a] : S - fr[a]) * (s >> 1 ? fr[b] : S - fr[b])) / (float)(S * S);
                 if (w > 0.0f && free_edge(G0, D, q))
-                    ent.push_back({(int)emg_edge_id(n0, D, q[0], q[1], q[2]), r, w});
+                    ent.push_back({(int)emg_entry(n0, D, q[0], q[1], q[2]), r, w});
             }
         }
-        transpose(ent, emg_edges(n0), H.r_ptr, H.r_row, H.r_w);
+        transpose(ent, emg_entries(n0), H.r_ptr, H.r_row, H.r_w);
     }
 
     // ---- nodes ----
@@ -140,7 +140,7 @@ void emg_build(const HostLayout& L, const std::vector<char>& free, const std::ve
                 fr[a] = m - (base[a] << H.gap);
                 if (fr[a] < 0 || fr[a] > S) return;
             }
-            H.n_base[v] = (int)emg_node_id(n0, base[0], base[1], base[2]);
+            H.n_base[v] = (int)emg_point(n0, base[0], base[1], base[2]);
             H.n_code[v] = (uint32_t)fr[0] | (uint32_t)fr[1] << 4 | (uint32_t)fr[2] << 8;
             for (int s = 0; s < 8; ++s) {
                 int q[3];
@@ -150,16 +150,15 @@ void emg_build(const HostLayout& L, const std::vector<char>& free, const std::ve
                     q[a] = base[a] + t;
                     w *= (float)(t ? fr[a] : S - fr[a]) / (float)S;
                 }
-                if (w > 0.0f && free_node(G0, q)) ent.push_back({(int)emg_node_id(n0, q[0], q[1], q[2]), v, w});
+                if (w > 0.0f && free_node(G0, q)) ent.push_back({(int)emg_point(n0, q[0], q[1], q[2]), v, w});
             }
         }
-        const long nn0 = (long)(n0 + 1) * (n0 + 1) * (n0 + 1);
-        transpose(ent, nn0, H.nr_ptr, H.nr_node, H.nr_w);
+        transpose(ent, emg_points(n0), H.nr_ptr, H.nr_node, H.nr_w);
     }
 
     // ---- face weights: level 0 from the octree's faces ----
     {
-        std::vector<double> w(emg_faces(n0), 0.0);
+        std::vector<double> w(emg_entries(n0), 0.0);
         for (int f = 0; f < L.nf; ++f) {
             if (L.dead_f[f]) continue;
             const int D = L.fnorm[f];
@@ -182,9 +181,9 @@ void emg_build(const HostLayout& L, const std::vector<char>& free, const std::ve
                 if (a == D) fr = std::min(std::max(u - q[a], 0.0), 1.0);
             }
             const double m = L.fdual[f] / (kMu0 * L.farea[f]) * ratio * ratio;
-            w[emg_face_id(n0, D, q[0], q[1], q[2])] += m * (1.0 - fr);
+            w[emg_entry(n0, D, q[0], q[1], q[2])] += m * (1.0 - fr);
             ++q[D];
-            w[emg_face_id(n0, D, q[0], q[1], q[2])] += m * fr;
+            w[emg_entry(n0, D, q[0], q[1], q[2])] += m * fr;
         }
         // coarser grids from the next finer one
         std::vector<std::vector<double>> wl;
@@ -192,23 +191,24 @@ void emg_build(const HostLayout& L, const std::vector<char>& free, const std::ve
         for (size_t l = 1; l < H.lv.size(); ++l) {
             const EmgHostLevel &C = H.lv[l], &F = H.lv[l - 1];
             const std::vector<double>& wf = wl.back();
-            std::vector<double> wc(emg_faces(C.n), 0.0);
+            std::vector<double> wc(emg_entries(C.n), 0.0);
+            auto dim = [](int n, int D, int a) { return n + (a == D ? 1 : 0); };   // faces of normal D along a
             for (int D = 0; D < 3; ++D)
-                for (int k = 0; k < emg_face_dim(F.n, D, 2); ++k)
-                    for (int j = 0; j < emg_face_dim(F.n, D, 1); ++j)
-                        for (int i = 0; i < emg_face_dim(F.n, D, 0); ++i) {
-                            double v = wf[emg_face_id(F.n, D, i, j, k)];
+                for (int k = 0; k < dim(F.n, D, 2); ++k)
+                    for (int j = 0; j < dim(F.n, D, 1); ++j)
+                        for (int i = 0; i < dim(F.n, D, 0); ++i) {
+                            double v = wf[emg_entry(F.n, D, i, j, k)];
                             if (v == 0.0) continue;
                             // vertical faces just above the surface (k = planes_v): ratio of lengths
                             const bool top = D != 2 && k >= F.planes_v;
                             v *= top ? 0.25 : 0.0625;
                             int q[3] = {i, j, k};
                             const int o = q[D] & 1;
-                            for (int a = 0; a < 3; ++a) q[a] = std::min(q[a] >> 1, emg_face_dim(C.n, D, a) - 1);
-                            wc[emg_face_id(C.n, D, q[0], q[1], q[2])] += o ? 0.5 * v : v;
+                            for (int a = 0; a < 3; ++a) q[a] = std::min(q[a] >> 1, dim(C.n, D, a) - 1);
+                            wc[emg_entry(C.n, D, q[0], q[1], q[2])] += o ? 0.5 * v : v;
                             if (o) {
                                 ++q[D];
-                                wc[emg_face_id(C.n, D, q[0], q[1], q[2])] += 0.5 * v;
+                                wc[emg_entry(C.n, D, q[0], q[1], q[2])] += 0.5 * v;
                             }
                         }
             wl.push_back(std::move(wc));

@@ -34,7 +34,7 @@ struct EmgHostLevel {
     int planes_h = 0;        // horizontal-edge planes k < planes_h may be free (z_k <= air)
     int planes_v = 0;        // vertical-edge layers k < planes_v may be free
     int planes_n = 0;        // node planes k < planes_n may be free
-    std::vector<float> w;    // face weights, by normal direction, x fastest
+    std::vector<float> w;    // face weights
 };
 
 struct EmgHost {
@@ -55,20 +55,13 @@ struct EmgHost {
     std::vector<float> nr_w;
 };
 
-// Index helpers of an n^3 grid: direction / normal D arrays one after another.
-inline int emg_edge_dim(int n, int D, int a) { return n + (a == D ? 0 : 1); }
-inline long emg_edge_off(int n, int D) { return (long)D * n * (n + 1) * (n + 1); }
-inline long emg_edges(int n) { return emg_edge_off(n, 3); }
-inline long emg_edge_id(int n, int D, int i, int j, int k) {
-    return emg_edge_off(n, D) + ((long)k * emg_edge_dim(n, D, 1) + j) * emg_edge_dim(n, D, 0) + i;
-}
-inline int emg_face_dim(int n, int D, int a) { return n + (a == D ? 1 : 0); }
-inline long emg_face_off(int n, int D) { return (long)D * n * n * (n + 1); }
-inline long emg_faces(int n) { return emg_face_off(n, 3); }
-inline long emg_face_id(int n, int D, int i, int j, int k) {
-    return emg_face_off(n, D) + ((long)k * emg_face_dim(n, D, 1) + j) * emg_face_dim(n, D, 0) + i;
-}
-inline long emg_node_id(int n, int i, int j, int k) { return ((long)k * (n + 1) + j) * (n + 1) + i; }
+// Index helpers of an n^3 grid: the points (i, j, k), x fastest; the edge of
+// direction D that starts at a point, and the face of normal D whose lowest
+// corner it is, are entry 3 point + D (entries beyond the grid stay zero).
+inline long emg_point(int n, int i, int j, int k) { return ((long)k * (n + 1) + j) * (n + 1) + i; }
+inline long emg_points(int n) { return (long)(n + 1) * (n + 1) * (n + 1); }
+inline long emg_entries(int n) { return 3 * emg_points(n); }
+inline long emg_entry(int n, int D, int i, int j, int k) { return 3 * emg_point(n, i, j, k) + D; }
 
 // free[e]: edge e (reference numbering) is a row of the eliminated system;
 // node_free[v]: node v is not a Dirichlet node; iperm: edge -> permuted row;

@@ -650,9 +650,12 @@ void GpuSolver::build_emg() {
         g.pv = h.planes_v;
         g.pn = h.planes_n;
         g.w = up(h.w);
-        const size_t ne = (size_t)emg_edges(h.n), nn = (size_t)(h.n + 1) * (h.n + 1) * (h.n + 1);
+        const size_t ne = (size_t)emg_entries(h.n), nn = (size_t)emg_points(h.n);
         g.me = dalloc_zero<float>(ne, stream);
         emg_mem.push_back((void*)g.me);
+        // the grids of 8 and 4 cells live in shared memory under one of 16
+        // cells, which reads their result
+        if (l > 1 && emg.lv[l - 2].n <= kEmgBottom) continue;
         for (float2** q : {&g.b, &g.x, &g.y}) *q = zeros(ne * dev::kMaxRhs);
         for (float2** q : {&g.nb, &g.ny, &g.nt}) *q = zeros(nn * dev::kMaxRhs);
     }
