@@ -95,6 +95,7 @@ template <> struct Sum<float> {
         return {make_float4(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m),
                             __shfl_xor_sync(0xffffffffu, v.z, m), __shfl_xor_sync(0xffffffffu, v.w, m))};
     }
+    __device__ __forceinline__ void add_real(float a) { add1(v.x, v.y, a, 0.0f); }
     __device__ __forceinline__ double2 get() const {
         return make_double2((double)v.x + (double)v.y, (double)v.z + (double)v.w);
     }
@@ -207,11 +208,10 @@ __device__ bool grid_reduce(const double2 (&acc)[KT][NQ], int rhs0, RedScratch r
 // order, so the result is deterministic for a fixed launch shape.  Returns true
 // in the last block, where out[q * K + k] (shared, NQ*K entries) holds the
 // totals.
-template <int NQ, int K, int NT, int LPT, class C>
-__device__ bool grid_reduce_multi(const C (&acc)[LPT][NQ], RedScratch rs, double2* out) {
+template <int NQ, int K, int NT, int LPT, class S>
+__device__ bool grid_reduce_sums(const S (&acc)[LPT][NQ], RedScratch rs, double2* out) {
     static_assert(K >= LPT && K <= 32 && (K & (K - 1)) == 0, "K must be a power of two <= 32");
     static_assert(NT % 32 == 0 && NT >= 32 && NT <= 1024, "block size must be whole warps");
-    using S = Sum<decltype(C{}.x)>;
     static_assert(sizeof(S) == sizeof(double2), "partials are 16 bytes");
     constexpr int PK = NQ * K;
     constexpr int NW = NT / 32;
@@ -222,15 +222,13 @@ __device__ bool grid_reduce_multi(const C (&acc)[LPT][NQ], RedScratch rs, double
     for (int j = 0; j < LPT; ++j)
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
-            S s;
-            s.set(acc[j][q]);
+            S s = acc[j][q];
 #pragma unroll
             for (int off = 16; off >= K / LPT; off >>= 1) s.add(s.xor_lane(off));
             if (lane < K / LPT) sm[warp][q * K + lane * LPT + j] = s;
         }
     __syncthreads();
-    S zero;
-    zero.set(C{});
+    S zero{};
     S* partial = reinterpret_cast<S*>(rs.partial);
     for (int p = warp; p < PK; p += NW) {
         S s = lane < NW ? sm[lane][p] : zero;
@@ -272,6 +270,16 @@ __device__ bool grid_reduce_multi(const C (&acc)[LPT][NQ], RedScratch rs, double
     if (threadIdx.x == 0) *rs.counter = 0u;
     __syncthreads();
     return true;
+}
+
+template <int NQ, int K, int NT, int LPT, class C>
+__device__ __forceinline__ bool grid_reduce_multi(const C (&acc)[LPT][NQ], RedScratch rs, double2* out) {
+    Sum<decltype(C{}.x)> s[LPT][NQ];
+#pragma unroll
+    for (int j = 0; j < LPT; ++j)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) s[j][q].set(acc[j][q]);
+    return grid_reduce_sums<NQ, K, NT, LPT>(s, rs, out);
 }
 
 // Blocks of a reducing vector kernel over n elements: one resident wave at

@@ -11,7 +11,8 @@ using namespace dev;
 namespace {
 
 constexpr int kNT = 256;
-constexpr int kLongRow = 32;    // transfer rows longer than this (two levels of refinement) are summed by a block
+// transfer rows longer than these (one level of refinement gives them) are summed by a block
+constexpr int kLongEdge = 18, kLongNode = 27;
 constexpr int kLongNT = 128;
 
 void ck(long long* launches) {
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(kNT) k_restrict0(EmgDev g, Omegas om, const fl
     if (c >= n) return;
     const int n1 = L.n + 1, p = c / 3, i = p % n1, j = p / n1 % n1, k = p / (n1 * n1), D = c % 3;
     const int q0 = __ldg(&g.r_ptr[c]), q1 = __ldg(&g.r_ptr[c + 1]);
-    if (q1 - q0 > kLongRow) return;   // k_restrict0_long
+    if (q1 - q0 > kLongEdge) return;   // k_restrict0_long
     float4 s = vz<float4>(), x = vz<float4>();
     for (int q = q0; q < q1; q += 6) {   // 18 entries under one level of refinement
         float w[6];
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(kNT) k_restrict0(EmgDev g, Omegas om, const fl
     store2<K>(L.x, lane_major(L), entries(L), c, h, x);
 }
 
-// The rows of P^T with more than kLongRow entries: coarse edges inside a
+// The rows of P^T with more than kLongEdge entries: coarse edges inside a
 // refinement of two or three levels collect up to 196 or 1800 octree edges,
 // which one thread after another made 50 us on the 157 k-edge mesh.
 template <int K>
@@ -653,7 +654,7 @@ __global__ void __launch_bounds__(kNT) k_node_restrict0(EmgDev g, const float4* 
         const int c = pid(L.n, i, j, k);
         float4 s = vz<float4>();
         const int q0 = __ldg(&g.nr_ptr[c]), q1 = __ldg(&g.nr_ptr[c + 1]);
-        if (q1 - q0 > kLongRow) return;   // k_node_restrict0_long
+        if (q1 - q0 > kLongNode) return;   // k_node_restrict0_long
         for (int q = q0; q < q1; q += 9) {   // 27 entries under one level of refinement
             float w[9];
             float4 v[9];
@@ -1041,10 +1042,10 @@ void node_cycle(const EmgDev& g, const GcDev& gc, const float2* r, cudaStream_t 
 
 }  // namespace
 
-std::vector<int> emg_long_rows(const std::vector<int>& ptr) {
+std::vector<int> emg_long_rows(const std::vector<int>& ptr, bool nodes) {
     std::vector<int> rows;
     for (size_t c = 0; c + 1 < ptr.size(); ++c)
-        if (ptr[c + 1] - ptr[c] > kLongRow) rows.push_back((int)c);
+        if (ptr[c + 1] - ptr[c] > (nodes ? kLongNode : kLongEdge)) rows.push_back((int)c);
     return rows;
 }
 

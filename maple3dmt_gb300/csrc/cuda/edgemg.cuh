@@ -66,7 +66,7 @@ struct EmgDev {
 };
 
 // The rows of a transfer (CSR row pointers) that take a block each.
-std::vector<int> emg_long_rows(const std::vector<int>& ptr);
+std::vector<int> emg_long_rows(const std::vector<int>& ptr, bool nodes);
 
 // Coarse edge masses for the current conductivity (Me per permuted row).
 void emg_set_mass(const EmgDev& g, const double* Me, cudaStream_t s, long long* launches);

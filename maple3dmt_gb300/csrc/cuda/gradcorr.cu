@@ -552,21 +552,29 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_start(int nn, DcWork w, GcDev 
     }
 }
 
+// The FP32 PCG's kernels: two right-hand sides per thread; the inner products'
+// FP32 terms are summed as two floats (dev::Sum), 48 bits -- FP64 adds per
+// element made each of them 13 to 20 us on the 157 k-edge mesh.
+__device__ __forceinline__ const float4* c4(const float2* p) { return reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4* m4(float2* p) { return reinterpret_cast<float4*>(p); }
+
 // p = z, rz = (r, z) (real: L and the V-cycle are real symmetric)
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_dcm_first(int nn, GcDev g, RedScratch rs) {
-    const long n = (long)nn * K;
+    const long n = (long)nn * (K / 2);
     const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long stride = (long)gridDim.x * blockDim.x;
-    const bool run = g.dc_st[i0 % K].run;
-    double2 acc[1] = {make_double2(0.0, 0.0)};
-    for (long i = i0; i < n && run; i += stride) {
-        const float2 r = g.dc_r[i], z = g.dc_z[i];
-        g.dc_p[i] = z;
-        acc[0].x += (double)(r.x * z.x + r.y * z.y);
+    const int k = (int)(2 * i0 % K);
+    const bool ra = g.dc_st[k].run, rb = g.dc_st[k + 1].run;
+    Sum<float> acc[2][1] = {};
+    for (long i = i0; i < n && (ra || rb); i += stride) {
+        const float4 r = c4(g.dc_r)[i], z = c4(g.dc_z)[i];
+        m4(g.dc_p)[i] = z;
+        acc[0][0].add_real(r.x * z.x + r.y * z.y);
+        acc[1][0].add_real(r.z * z.z + r.w * z.w);
     }
     __shared__ double2 out[K];
-    if (grid_reduce_lanes<1, K, kGcBlock>(acc, rs, out)) {
+    if (grid_reduce_sums<1, K, kGcBlock, 2>(acc, rs, out)) {
         if (threadIdx.x < K && g.dc_st[threadIdx.x].run) g.dc_st[threadIdx.x].rz = out[threadIdx.x].x;
     }
 }
@@ -574,21 +582,43 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_first(int nn, GcDev g, RedScra
 // Ap = L p (FP32, incidence form), (p, Ap) -> alpha
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_dcm_ap(int nn, GcDev g, RedScratch rs) {
-    const long n = (long)nn * K;
+    constexpr int H = K / 2;
+    const long n = (long)nn * H;
     const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long stride = (long)gridDim.x * blockDim.x;
-    const bool run = g.dc_st[i0 % K].run;
-    const XPlain xf{g.dc_p};
-    double2 acc[1] = {make_double2(0.0, 0.0)};
-    for (long i = i0; i < n && run; i += stride) {
-        const int v = (int)(i / K), k = (int)(i % K);
-        const float2 ap = level_row<K, true>(g, g.lv[0], v, xf, k);
-        const float2 p = g.dc_p[i];
-        g.dc_ap[i] = ap;
-        acc[0].x += (double)(p.x * ap.x + p.y * ap.y);
+    const int k = (int)(2 * i0 % K);
+    const bool ra = g.dc_st[k].run, rb = g.dc_st[k + 1].run;
+    const float4* p = c4(g.dc_p);
+    Sum<float> acc[2][1] = {};
+    for (long i = i0; i < n && (ra || rb); i += stride) {
+        const int v = (int)(i / H), h = (int)(i % H);
+        const float4 pv = p[i];
+        const float dg = __ldg(&g.lap_diag32[v]);
+        float4 s = make_float4(dg * pv.x, dg * pv.y, dg * pv.z, dg * pv.w);
+        const int q0 = __ldg(&g.inc_ptr[v]), q1 = __ldg(&g.inc_ptr[v + 1]);
+        for (int q = q0; q < q1; q += 6) {
+            float a[6];
+            float4 x[6];
+#pragma unroll
+            for (int u = 0; u < 6; ++u) {
+                const int2 e = q + u < q1 ? __ldg(&g.lap_pk[q + u]) : make_int2(0, 0);
+                a[u] = __int_as_float(e.y);
+                x[u] = a[u] != 0.0f ? p[(size_t)e.x * H + h] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < 6; ++u) {
+                s.x += a[u] * x[u].x;
+                s.y += a[u] * x[u].y;
+                s.z += a[u] * x[u].z;
+                s.w += a[u] * x[u].w;
+            }
+        }
+        m4(g.dc_ap)[i] = s;
+        acc[0][0].add_real(pv.x * s.x + pv.y * s.y);
+        acc[1][0].add_real(pv.z * s.z + pv.w * s.w);
     }
     __shared__ double2 out[K];
-    if (grid_reduce_lanes<1, K, kGcBlock>(acc, rs, out)) {
+    if (grid_reduce_sums<1, K, kGcBlock, 2>(acc, rs, out)) {
         if (threadIdx.x < K) {
             GcPcgState T = g.dc_st[threadIdx.x];
             if (T.run) {
@@ -604,25 +634,35 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_ap(int nn, GcDev g, RedScratch
 // x += alpha p, r -= alpha Ap, |r| <= tol (|b| = 1) or the iteration cap stops
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_dcm_update(int nn, GcDev g, int cap, RedScratch rs) {
-    const long n = (long)nn * K;
+    const long n = (long)nn * (K / 2);
     const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long stride = (long)gridDim.x * blockDim.x;
-    const GcPcgState T0 = g.dc_st[i0 % K];
-    const float al = (float)T0.alpha;
-    double2 acc[1] = {make_double2(0.0, 0.0)};
-    for (long i = i0; i < n && T0.run; i += stride) {
-        const float2 p = g.dc_p[i], ap = g.dc_ap[i];
-        float2 x = g.dc_x[i], r = g.dc_r[i];
-        x.x += al * p.x;
-        x.y += al * p.y;
-        r.x -= al * ap.x;
-        r.y -= al * ap.y;
-        g.dc_x[i] = x;
-        g.dc_r[i] = r;
-        acc[0].x += (double)(r.x * r.x + r.y * r.y);
+    const int k = (int)(2 * i0 % K);
+    const bool ra = g.dc_st[k].run, rb = g.dc_st[k + 1].run;
+    const float la = ra ? (float)g.dc_st[k].alpha : 0.0f, lb = rb ? (float)g.dc_st[k + 1].alpha : 0.0f;
+    Sum<float> acc[2][1] = {};
+    for (long i = i0; i < n && (ra || rb); i += stride) {
+        const float4 p = c4(g.dc_p)[i], ap = c4(g.dc_ap)[i];
+        float4 x = c4(g.dc_x)[i], r = c4(g.dc_r)[i];
+        if (ra) {
+            x.x += la * p.x;
+            x.y += la * p.y;
+            r.x -= la * ap.x;
+            r.y -= la * ap.y;
+        }
+        if (rb) {
+            x.z += lb * p.z;
+            x.w += lb * p.w;
+            r.z -= lb * ap.z;
+            r.w -= lb * ap.w;
+        }
+        m4(g.dc_x)[i] = x;
+        m4(g.dc_r)[i] = r;
+        acc[0][0].add_real(r.x * r.x + r.y * r.y);
+        acc[1][0].add_real(r.z * r.z + r.w * r.w);
     }
     __shared__ double2 out[K];
-    if (grid_reduce_lanes<1, K, kGcBlock>(acc, rs, out)) {
+    if (grid_reduce_sums<1, K, kGcBlock, 2>(acc, rs, out)) {
         if (threadIdx.x < K) {
             GcPcgState T = g.dc_st[threadIdx.x];
             if (T.run) {
@@ -637,17 +677,19 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_update(int nn, GcDev g, int ca
 // (r, z) -> beta
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_dcm_rz(int nn, GcDev g, RedScratch rs) {
-    const long n = (long)nn * K;
+    const long n = (long)nn * (K / 2);
     const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long stride = (long)gridDim.x * blockDim.x;
-    const bool run = g.dc_st[i0 % K].run;
-    double2 acc[1] = {make_double2(0.0, 0.0)};
+    const int k = (int)(2 * i0 % K);
+    const bool run = g.dc_st[k].run || g.dc_st[k + 1].run;
+    Sum<float> acc[2][1] = {};
     for (long i = i0; i < n && run; i += stride) {
-        const float2 r = g.dc_r[i], z = g.dc_z[i];
-        acc[0].x += (double)(r.x * z.x + r.y * z.y);
+        const float4 r = c4(g.dc_r)[i], z = c4(g.dc_z)[i];
+        acc[0][0].add_real(r.x * z.x + r.y * z.y);
+        acc[1][0].add_real(r.z * z.z + r.w * z.w);
     }
     __shared__ double2 out[K];
-    if (grid_reduce_lanes<1, K, kGcBlock>(acc, rs, out)) {
+    if (grid_reduce_sums<1, K, kGcBlock, 2>(acc, rs, out)) {
         if (threadIdx.x < K) {
             GcPcgState T = g.dc_st[threadIdx.x];
             if (T.run) {
@@ -748,9 +790,9 @@ long long dc_poisson_mixed_k(const GcDev& g, int nn, DcWork w, RedScratch red, c
     const int cap = red.max_blocks;
     const int g_n = gc_grid((long)nn * K);
     const long n = (long)nn * K;
-    const int g_norm = reduce_grid(k_dcm_norm<K>, cap, n), g_first = reduce_grid(k_dcm_first<K>, cap, n);
-    const int g_ap = reduce_grid(k_dcm_ap<K>, cap, n), g_up = reduce_grid(k_dcm_update<K>, cap, n);
-    const int g_rz = reduce_grid(k_dcm_rz<K>, cap, n);
+    const int g_norm = reduce_grid(k_dcm_norm<K>, cap, n), g_first = reduce_grid(k_dcm_first<K>, cap, n / 2);
+    const int g_ap = reduce_grid(k_dcm_ap<K>, cap, n / 2), g_up = reduce_grid(k_dcm_update<K>, cap, n / 2);
+    const int g_rz = reduce_grid(k_dcm_rz<K>, cap, n / 2);
     constexpr int kMaxRef = 8, kCap = 400;
     // iterations between polls: the geometric cycle needs about ten in all
     const int kPoll = g.emg ? 4 : 8;

@@ -128,26 +128,17 @@ __global__ void k_vsub(long n, const double2* __restrict__ a, const double2* __r
     if (i < n) out[i] = csub(a[i], b[i]);
 }
 
-__global__ void k_hanging(MeshDev m, VecK x) {
+// pairs [h0, h1): of one dependency level, so that a pair whose child is itself
+// a coarse edge runs in the list's order (a serial pass over the list was 1.7 ms
+// on the 157 k-edge mesh)
+__global__ void k_hanging(MeshDev m, VecK x, int h0, int h1) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int K = x.K;
-    if (i >= (long)m.nhp * K) return;
-    const int h = (int)(i / K), k = (int)(i % K);
+    if (i >= (long)(h1 - h0) * K) return;
+    const int h = h0 + (int)(i / K), k = (int)(i % K);
     const int c = m.hp[3 * h], c1 = m.hp[3 * h + 1], c2 = m.hp[3 * h + 2];
     const double2 a = x.p[(size_t)c1 * K + k], b = x.p[(size_t)c2 * K + k];
     x.p[(size_t)c * K + k] = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y + b.y));
-}
-
-// list order matters when a child is itself a coarse edge: one thread per rhs
-__global__ void k_hanging_seq(MeshDev m, VecK x) {
-    const int k = threadIdx.x;
-    if (k >= x.K) return;
-    const int K = x.K;
-    for (int h = 0; h < m.nhp; ++h) {
-        const int c = m.hp[3 * h], c1 = m.hp[3 * h + 1], c2 = m.hp[3 * h + 2];
-        const double2 a = x.p[(size_t)c1 * K + k], b = x.p[(size_t)c2 * K + k];
-        x.p[(size_t)c * K + k] = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y + b.y));
-    }
 }
 
 __global__ void k_combine(MeshDev m, VecK epri, VecK esec, VecK ebc, VecK e) {
@@ -873,20 +864,25 @@ __global__ void k_wr(int ns, int nf, int nf_total, int f0, const double2* __rest
 }
 
 // forward_solver_fv.cpp:1837-2010, one thread per frequency (stations may share edges)
-// Thread f builds source f: wr[f] [ns][4], the station cache hcs[f * hc_stride]
+// A thread per (source, station): source f: wr[f] [ns][4], the station cache hcs[f * hc_stride]
 // and omegas[f * om_stride] (strides ns and 1 over frequencies, 0 and 0 for
-// many sources at one frequency), into lanes 2f and 2f + 1.
+// many sources at one frequency), to lanes 2f and 2f + 1.
+// Stations share edges, so each writes the terms it adds to its edges (two per
+// edge and polarisation) to st.term, and k_adjoint_sum adds them up per edge in
+// station order: one thread per source walking over all stations took 3 ms for
+// 81 stations.
 __global__ void k_adjoint_rhs(StationDev st, const double2* __restrict__ wr, const HCache* __restrict__ hcs,
-                              const double* __restrict__ omegas, int nf, int hc_stride, int om_stride, VecK out) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+                              const double* __restrict__ omegas, int nf, int hc_stride, int om_stride) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, f = t / st.ns, s = t % st.ns;
     if (f >= nf) return;
-    const int K = out.K;
+    double2* term = st.term + (size_t)f * st.n_terms * 4;
+    for (int q = 4 * st.e_ptr[s]; q < 4 * st.e_ptr[s + 1]; ++q) term[q] = zero2();
     const double2 iwmu = make_double2(0.0, omegas[(size_t)f * om_stride] * kMu0);
-    for (int s = 0; s < st.ns; ++s) {
-        if (st.cell[s] < 0) continue;
+    {
+        if (st.cell[s] < 0) return;
         const double2* w = wr + ((size_t)f * st.ns + s) * 4;
         const HCache hc = hcs[(size_t)f * hc_stride + s];
-        if (hypot(hc.det.x, hc.det.y) < 1e-30) continue;
+        if (hypot(hc.det.x, hc.det.y) < 1e-30) return;
         const double2 sx1 = cdiv(csub(cmul(w[0], hc.Hy2), cmul(w[1], hc.Hx2)), hc.det);
         const double2 sy1 = cdiv(csub(cmul(w[2], hc.Hy2), cmul(w[3], hc.Hx2)), hc.det);
         const double2 sx2 = cdiv(cadd(cmul(cneg(w[0]), hc.Hy1), cmul(w[1], hc.Hx1)), hc.det);
@@ -913,55 +909,69 @@ __global__ void k_adjoint_rhs(StationDev st, const double2* __restrict__ wr, con
         const double2 icdx = cdiv(make_double2(1.0, 0.0), make_double2(iwmu.x * hc.cdx, iwmu.y * hc.cdx));
         const double2 icdy = cdiv(make_double2(1.0, 0.0), make_double2(iwmu.x * hc.cdy, iwmu.y * hc.cdy));
         for (int q = st.e_ptr[s]; q < st.e_ptr[s + 1]; ++q) {
-            const int row = st.e_row[q];
             const unsigned char code = st.e_code[q];
             const int d = code & 3;
-            double2* a1 = out.p + (size_t)row * K + 2 * f;
-            double2* a2 = a1 + 1;
+            // first and second term of polarisation 1, then of polarisation 2
+            double2 *t1 = term + 4 * (size_t)q, *t2 = t1 + 2;
             if (d == 0) {
                 const bool top = code & 4;
                 const double we = top ? wxt : wxb;
-                *a1 = cadd(*a1, cscale(sx1, we));
-                *a2 = cadd(*a2, cscale(sx2, we));
+                t1[0] = cscale(sx1, we);
+                t2[0] = cscale(sx2, we);
                 if (top && nxt > 0) {
                     const double2 wh = make_double2(icdz.x / nxt, icdz.y / nxt);
-                    *a1 = cadd(*a1, cmul(aHy1, wh)); *a2 = cadd(*a2, cmul(aHy2, wh));
+                    t1[1] = cmul(aHy1, wh); t2[1] = cmul(aHy2, wh);
                 } else if (!top && nxb > 0) {
                     const double2 wh = make_double2(-icdz.x / nxb, -icdz.y / nxb);
-                    *a1 = cadd(*a1, cmul(aHy1, wh)); *a2 = cadd(*a2, cmul(aHy2, wh));
+                    t1[1] = cmul(aHy1, wh); t2[1] = cmul(aHy2, wh);
                 }
             } else if (d == 1) {
                 const bool top = code & 4;
                 const double we = top ? wyt : wyb;
-                *a1 = cadd(*a1, cscale(sy1, we));
-                *a2 = cadd(*a2, cscale(sy2, we));
+                t1[0] = cscale(sy1, we);
+                t2[0] = cscale(sy2, we);
                 if (top && nyt > 0) {
                     const double2 wh = make_double2(-icdz.x / nyt, -icdz.y / nyt);
-                    *a1 = cadd(*a1, cmul(aHx1, wh)); *a2 = cadd(*a2, cmul(aHx2, wh));
+                    t1[1] = cmul(aHx1, wh); t2[1] = cmul(aHx2, wh);
                 } else if (!top && nyb > 0) {
                     const double2 wh = make_double2(icdz.x / nyb, icdz.y / nyb);
-                    *a1 = cadd(*a1, cmul(aHx1, wh)); *a2 = cadd(*a2, cmul(aHx2, wh));
+                    t1[1] = cmul(aHx1, wh); t2[1] = cmul(aHx2, wh);
                 }
             } else {
                 const bool py = code & 16;
                 if (py && npy > 0) {
                     const double2 wh = make_double2(icdy.x / npy, icdy.y / npy);
-                    *a1 = cadd(*a1, cmul(aHx1, wh)); *a2 = cadd(*a2, cmul(aHx2, wh));
+                    t1[0] = cmul(aHx1, wh); t2[0] = cmul(aHx2, wh);
                 } else if (!py && nmy > 0) {
                     const double2 wh = make_double2(-icdy.x / nmy, -icdy.y / nmy);
-                    *a1 = cadd(*a1, cmul(aHx1, wh)); *a2 = cadd(*a2, cmul(aHx2, wh));
+                    t1[0] = cmul(aHx1, wh); t2[0] = cmul(aHx2, wh);
                 }
                 const bool px = code & 8;
                 if (px && npx > 0) {
                     const double2 wh = make_double2(-icdx.x / npx, -icdx.y / npx);
-                    *a1 = cadd(*a1, cmul(aHy1, wh)); *a2 = cadd(*a2, cmul(aHy2, wh));
+                    t1[1] = cmul(aHy1, wh); t2[1] = cmul(aHy2, wh);
                 } else if (!px && nmx > 0) {
                     const double2 wh = make_double2(icdx.x / nmx, icdx.y / nmx);
-                    *a1 = cadd(*a1, cmul(aHy1, wh)); *a2 = cadd(*a2, cmul(aHy2, wh));
+                    t1[1] = cmul(aHy1, wh); t2[1] = cmul(aHy2, wh);
                 }
             }
         }
     }
+}
+
+// out[row][2f], [2f + 1] += the terms of the row's edges, in station order.
+__global__ void k_adjoint_sum(StationDev st, int nf, VecK out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, r = t / nf, f = t % nf;
+    if (r >= st.n_rows) return;
+    double2* a = out.p + (size_t)st.sum_row[r] * out.K + 2 * f;
+    double2 a1 = a[0], a2 = a[1];
+    for (int p = st.sum_ptr[r]; p < st.sum_ptr[r + 1]; ++p) {
+        const double2* term = st.term + ((size_t)f * st.n_terms + st.sum_q[p]) * 4;
+        a1 = cadd(cadd(a1, term[0]), term[1]);
+        a2 = cadd(cadd(a2, term[2]), term[3]);
+    }
+    a[0] = a1;
+    a[1] = a2;
 }
 
 // sum over cell c's edges of Im(lambda_e E_e) * w_e (w_e = A_dual L / n_adj,
@@ -1132,15 +1142,16 @@ void vsub(long n, const double2* a, const double2* b, double2* out, cudaStream_t
     ck();
 }
 
-void interpolate_hanging(const MeshDev& m, VecK x, bool sequential, cudaStream_t s) {
-    if (m.nhp == 0) return;
-    if (sequential) {
-        k_hanging_seq<<<1, 32, 0, s>>>(m, x);
-    } else {
-        const long n = (long)m.nhp * x.K;
-        k_hanging<<<(int)((n + kBlock - 1) / kBlock), kBlock, 0, s>>>(m, x);
+int interpolate_hanging(const MeshDev& m, VecK x, const std::vector<int>& levels, cudaStream_t s) {
+    int n = 0;
+    for (size_t l = 0; l + 1 < levels.size(); ++l) {
+        const long w = (long)(levels[l + 1] - levels[l]) * x.K;
+        if (w == 0) continue;
+        k_hanging<<<(int)((w + kBlock - 1) / kBlock), kBlock, 0, s>>>(m, x, levels[l], levels[l + 1]);
+        ck();
+        ++n;
     }
-    ck();
+    return n;
 }
 
 void combine_total(const MeshDev& m, VecK epri, VecK esec, VecK ebc, VecK e, cudaStream_t s) {
@@ -1336,18 +1347,29 @@ void pick_pol_lanes(long n_pad, int K, const double2* a, const double2* b, doubl
     ck();
 }
 
+namespace {
+void adjoint_terms(const StationDev& st, const double2* wr, const HCache* hc, const double* omegas, int nf,
+                   int hc_stride, int om_stride, VecK out, cudaStream_t s) {
+    if (st.ns == 0 || nf == 0) return;
+    if (nf > dev::kMaxRhs / 2) throw std::invalid_argument("adjoint sources: at most 8");
+    k_adjoint_rhs<<<(nf * st.ns + 31) / 32, 32, 0, s>>>(st, wr, hc, omegas, nf, hc_stride, om_stride);
+    ck();
+    if (st.n_rows == 0) return;
+    k_adjoint_sum<<<(nf * st.n_rows + 127) / 128, 128, 0, s>>>(st, nf, out);
+    ck();
+}
+}  // namespace
+
 void adjoint_rhs(const StationDev& st, const MeshDev& m, const double2* wr, const HCache* hc,
                  const double* omegas, int nf, VecK out, cudaStream_t s) {
     (void)m;
-    k_adjoint_rhs<<<1, 32, 0, s>>>(st, wr, hc, omegas, nf, st.ns, 1, out);
-    ck();
+    adjoint_terms(st, wr, hc, omegas, nf, st.ns, 1, out, s);
 }
 
 void adjoint_rhs_sources(const StationDev& st, const double2* wr, const HCache* hc, const double* omega, int n_src,
                          VecK out, cudaStream_t s) {
     if (n_src < 1 || 2 * n_src > out.K) throw std::invalid_argument("adjoint sources: 1 .. K/2");
-    k_adjoint_rhs<<<1, 32, 0, s>>>(st, wr, hc, omega, n_src, 0, 0, out);
-    ck();
+    adjoint_terms(st, wr, hc, omega, n_src, 0, 0, out, s);
 }
 
 void sensitivity(const MeshDev& m, const double* sigma, VecK E, VecK lam, const double* omegas, int nf,

@@ -42,7 +42,7 @@ struct MeshDev {
     int* lift_col;
     double* lift_val;
     int nhp;
-    int* hp;            // [nhp][3] coarse, child1, child2 (permuted rows)
+    int* hp;            // [nhp][3] coarse, child1, child2 (permuted rows), by dependency level
     // nodes
     int* inc_ptr;       // [nn + 1] node -> incident edges, reference edge order
     int* inc_edge;      // permuted edge row
@@ -67,6 +67,14 @@ struct StationDev {
     int* e_row;         // permuted rows of the cell's edges, cell_edges order
     unsigned char* e_code;  // bit0-1 direction, bit2 top (z > cz), bit3 +x (x > cx), bit4 +y (y > cy)
     double* sigma_cell; // [ns] sigma of the station cell (1-D fallback)
+    // adjoint sources: the distinct rows among e_row, the entries of each in
+    // station order, and the terms of up to 8 sources
+    int n_terms;        // entries of e_row
+    int n_rows;
+    int* sum_row;       // [n_rows]
+    int* sum_ptr;       // [n_rows + 1]
+    int* sum_q;         // [n_terms]
+    double2* term;      // [8][n_terms][4]
 };
 
 // Cached H / Z of a station at one frequency (StationHCache, forward_solver_fv.h:216-223).
@@ -107,7 +115,8 @@ void lift_rhs(const MeshDev& m, VecK ebc, VecK rhs, cudaStream_t s);
 // out = a - b (elementwise, all rhs).
 void vsub(long n, const double2* a, const double2* b, double2* out, cudaStream_t s);
 // interpolate_hanging (:258-261) on every rhs of x.
-void interpolate_hanging(const MeshDev& m, VecK x, bool sequential, cudaStream_t s);
+// levels: ranges of m.hp, one dependency level each; returns the launches.
+int interpolate_hanging(const MeshDev& m, VecK x, const std::vector<int>& levels, cudaStream_t s);
 // E = E_pri + E_sec; E_bc on BC rows (:357-361).
 void combine_total(const MeshDev& m, VecK epri, VecK esec, VecK ebc, VecK e, cudaStream_t s);
 // gather / scatter between reference order (host layout [K][ne]) and permuted [n_pad][K]

@@ -249,6 +249,7 @@ void GpuSolver::free_all() {
     reg_free();
     dc.lap_work = nullptr; dc.lap_qpos = nullptr;
     dfree(sd.cell); dfree(sd.geom); dfree(sd.e_ptr); dfree(sd.e_row); dfree(sd.e_code); dfree(sd.sigma_cell);
+    dfree(sd.sum_row); dfree(sd.sum_ptr); dfree(sd.sum_q); dfree(sd.term);
     dfree(d_hc); dfree(d_Z); dfree(d_wr); dfree(d_obs); dfree(d_err); dfree(d_grad);
     dfree(d_jtj_rhs); dfree(d_jtj_dE); dfree(d_jtj_a); dfree(d_jtj_b); dfree(d_jtj_dz); dfree(d_jtj_wr0);
     dfree(d_jtj_wr1); dfree(d_jtj_ds); dfree(d_jtj_err);
@@ -440,14 +441,28 @@ void GpuSolver::setup(const m3d_leaves* lv, const m3d_params* params) {
         adj_ptr[r + 1] = (int)adj_cell.size();
         lift_ptr[r + 1] = (int)lift_col.size();
     }
-    std::vector<int> hp(3 * L.hp.size());
+    // Hanging pairs by dependency level: the reference runs the list in order,
+    // and a pair comes after the earlier pairs that write its children, and
+    // after those that read or write its coarse edge.
+    std::vector<int> hp;
     {
-        std::vector<char> coarse(ne, 0);
-        for (const auto& h : L.hp) coarse[h[0]] = 1;
-        hp_sequential = false;
+        std::vector<int> wrote(ne, -1), read(ne, -1), level(L.hp.size(), 0);
+        int n_lv = 0;
         for (size_t i = 0; i < L.hp.size(); ++i) {
-            for (int k = 0; k < 3; ++k) hp[3 * i + k] = iperm[L.hp[i][k]];
-            if (coarse[L.hp[i][1]] || coarse[L.hp[i][2]]) hp_sequential = true;
+            const auto& h = L.hp[i];
+            const int l = std::max({wrote[h[1]], wrote[h[2]], wrote[h[0]], read[h[0]]}) + 1;
+            level[i] = l;
+            wrote[h[0]] = l;
+            read[h[1]] = std::max(read[h[1]], l);
+            read[h[2]] = std::max(read[h[2]], l);
+            n_lv = std::max(n_lv, l + 1);
+        }
+        hp_levels.assign(1, 0);
+        for (int l = 0; l < n_lv; ++l) {
+            for (size_t i = 0; i < L.hp.size(); ++i)
+                if (level[i] == l)
+                    for (int k = 0; k < 3; ++k) hp.push_back(iperm[L.hp[i][k]]);
+            hp_levels.push_back((int)(hp.size() / 3));
         }
     }
     // node incidence in reference edge order; G[e, n1] = -1/L, G[e, n2] = +1/L
@@ -669,7 +684,7 @@ void GpuSolver::build_emg() {
     emg.nr_ptr = up(H.nr_ptr);
     emg.nr_node = up(H.nr_node);
     emg.nr_w = up(H.nr_w);
-    const std::vector<int> rl = emg_long_rows(H.r_ptr), nl = emg_long_rows(H.nr_ptr);
+    const std::vector<int> rl = emg_long_rows(H.r_ptr, false), nl = emg_long_rows(H.nr_ptr, true);
     emg.n_r_long = (int)rl.size();
     emg.n_nr_long = (int)nl.size();
     emg.r_long = up(rl);
@@ -751,12 +766,32 @@ void GpuSolver::set_stations(const double* xyz, int n) {
         eptr[s + 1] = (int)erow.size();
     }
     dfree(sd.cell); dfree(sd.geom); dfree(sd.e_ptr); dfree(sd.e_row); dfree(sd.e_code); dfree(sd.sigma_cell);
+    dfree(sd.sum_row); dfree(sd.sum_ptr); dfree(sd.sum_q); dfree(sd.term);
     sd.ns = n;
     sd.cell = dupload(st_cell, stream);
     sd.geom = dupload(geom, stream);
     sd.e_ptr = dupload(eptr, stream);
     sd.e_row = dupload(erow, stream);
     sd.e_code = dupload(ecode, stream);
+    {
+        std::vector<int> order(erow.size()), rows, ptr(1, 0);
+        for (size_t q = 0; q < order.size(); ++q) order[q] = (int)q;
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return erow[a] < erow[b]; });
+        for (size_t q = 0; q < order.size(); ++q) {
+            if (q == 0 || erow[order[q]] != erow[order[q - 1]]) {
+                rows.push_back(erow[order[q]]);
+                ptr.push_back((int)q);
+            }
+            ptr.back() = (int)q + 1;
+        }
+        sd.n_terms = (int)erow.size();
+        sd.n_rows = (int)rows.size();
+        sd.sum_row = dupload(rows, stream);
+        sd.sum_ptr = dupload(ptr, stream);
+        sd.sum_q = dupload(order, stream);
+        sd.term = dalloc<double2>(erow.size() * 4 * (dev::kMaxRhs / 2));
+        sync();
+    }
     sd.sigma_cell = dupload(sc, stream);
     stations_set = true;
     hc_cap = 0;
@@ -1924,7 +1959,7 @@ void GpuSolver::run_forward(const std::vector<double>& freqs, double* Z_out) {
     } else {
         R = solve_any(K, fmap.data(), kv.b, kv.x, active, P.bicgstab_tol, P.bicgstab_maxiter);
     }
-    phys::interpolate_hanging(md, X, hp_sequential, stream);
+    launches += phys::interpolate_hanging(md, X, hp_levels, stream) - 1;
     phys::combine_total(md, Epri, X, Ebc, E, stream);
     launches += 2;
     if (P.div_correction) {

@@ -160,7 +160,7 @@ private:
     std::vector<unsigned char> flags_ref;  // reference order
     int n_pad = 0, n_slices = 0;
     int n_free = 0;                     // the free rows are the first n_free (padding included)
-    bool hp_sequential = false;
+    std::vector<int> hp_levels;         // dependency levels of the hanging pairs (ranges of md.hp)
 
     // device mesh
     MeshDev md{};
