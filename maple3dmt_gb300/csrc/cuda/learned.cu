@@ -16,11 +16,11 @@
 // and its border arrive once per x shift and the taps are line offsets into
 // those boxes (see the kernel's comment).
 // GEMM view: M = voxels, N = output channels, K = 27 taps x 32 channels.
-// Weight gradient: dW[t] = sum_v dY[v]^T X[v + off_t] as one GEMM with
-// M = 27 x 32 (tap, input channel) rows padded to 896, N = 32 output channels,
-// K = every voxel of the batch, both operands K-major (the shifted inputs
-// gathered once per layer, the output gradient transposed), split over K
-// across CTAs and summed in a fixed order.
+// Weight gradient: dW[t] = sum_v X[v + off_t]^T dY[v], M = (tap, input
+// channel), N = 32 output channels, K = every voxel of the batch: both
+// operands as they lie in memory, read M- and N-major, the taps line offsets
+// into the same halo boxes; split over K across CTAs and summed in a fixed
+// order (k_wgrad_tc).
 //
 // Every barrier wait is bounded; a timeout sets an error flag that the host
 // turns into an error, the CTA waits (bounded) for its copies and MMAs in
@@ -44,10 +44,8 @@ namespace {
 constexpr int kStages = 4;
 constexpr int kTileA = 128 * 64;      // bytes of a 128-row, 64-byte-row operand tile
 constexpr int kTapB = 32 * 64;        // bytes of one tap's 32 x 32 weights
+constexpr int kMseBlocks = 1024;      // partial sums of the loss
 constexpr int kConvSmem = kTaps * kTapB + kStages * kTileA + 1024;
-constexpr int kGemmStage = kTileA + kTapB;
-constexpr int kGemmSmem = kStages * kGemmStage + 1024;
-constexpr int kMPad = 896;            // 27 x 32 weight-gradient rows padded to 7 x 128
 
 void ck(cudaError_t e, const char* what) {
     if (e != cudaSuccess) {
@@ -214,7 +212,8 @@ __global__ void __launch_bounds__(128, 1) k_conv3d_tc(const __grid_constant__ CU
 //   warps 0-3        epilogue: tcgen05.ld of their 32 lanes, release of the
 //                    accumulator, bias / ReLU / mask, BF16 store.
 // Every wait is bounded; a timeout flags an error and every role stops.
-constexpr int kHaloMaxW = 64;
+constexpr int kHaloMaxW = 64;      // three boxes and the weights in shared memory
+constexpr int kWgradMaxW = 128;     // two boxes of one x shift
 __host__ __device__ constexpr int halo_box_bytes(int W) { return (128 + 2 * W) * 3 * 64; }
 constexpr int halo_smem(int W) { return kTaps * kTapB + 3 * halo_box_bytes(W) + 1024; }
 
@@ -392,176 +391,217 @@ __global__ void __launch_bounds__(192, 1) k_conv3d_halo(const __grid_constant__ 
     if (warp == 5) tc::tmem_dealloc(tmem, 64);
 }
 
-struct GemmArgs {
-    int k_steps;        // 32-element K steps per split
-    float* ws;          // [splits][kMPad][32]
+struct WgradArgs {
+    int D, bw, bh, tiles_h;
+    int n_tiles;        // 128-voxel tiles of the batch
+    float* ws;          // [splits][27][32 c_in][32 c_out]
+    double* bias_ws;    // [splits][32]
     unsigned* err;
 };
 
-// D[896 x 32] partial = A[896 x K] B[32 x K]^T over this CTA's K range;
-// blockIdx.x = 128-row M tile, blockIdx.y = K split.
-__global__ void __launch_bounds__(128, 1) k_gemm_tn_tc(const __grid_constant__ CUtensorMap amap,
-                                                       const __grid_constant__ CUtensorMap bmap, GemmArgs a) {
+constexpr int kWgradStages = 2;
+__host__ __device__ constexpr int wgrad_stage(int W) { return halo_box_bytes(W) + kTileA; }
+constexpr int wgrad_smem(int W) { return kWgradStages * wgrad_stage(W) + 1024; }
+
+// Weight and bias gradients of a layer.  blockIdx.y is the taps' x shift dx,
+// blockIdx.x a split of the 128-voxel tiles.  A tile's input comes in as the
+// halo box of the forward convolution ((bh + 2) x 3 lines of W voxels, 64
+// bytes a voxel), its output gradient as 128 rows of 64 bytes, and neither is
+// transposed or gathered: M runs along the 32 channels of a voxel and goes on
+// one line further down (descriptor group stride = one line), so one MMA of
+// M = 128 covers the taps dy = -1, 0, 1 of a dz (96 rows; the last 32 belong
+// to no tap and are not read back -- for the last dz they lie past the box, in
+// the gradient rows behind it), and K = 16 voxels are 16 rows of the tile's
+// contiguous lines.  24 MMAs a tile into three accumulators of 32 columns.
+//   warp 4 / lane 0  TMA producer, two stages;
+//   warp 5           allocates 128 TMEM columns; lane 0 issues the MMAs;
+//   warps 0-3        sum the gradient rows per channel in two-float arithmetic
+//                    (blockIdx.y = 1 only), at the end store the accumulators.
+// Bound by the copies from L2 (45 KB a tile and shift at W = 32).  The former
+// path gathered 27 shifted, transposed copies of the input (226 MB a layer for
+// 131 k voxels, 72 us), transposed the gradient (5 us), multiplied (52 us) and
+// summed the biases with one warp in FP64 (21 + 338 us).
+// Every wait is bounded; a timeout flags an error and every role stops.
+__global__ void __launch_bounds__(192) k_wgrad_tc(const __grid_constant__ CUtensorMap hmap,
+                                                  const __grid_constant__ CUtensorMap dmap, WgradArgs a) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                            ~static_cast<uintptr_t>(1023));
-    __shared__ __align__(8) uint64_t full[kStages], empty[kStages], done;
+    __shared__ __align__(8) uint64_t full[kWgradStages], empty[kWgradStages], done;
     __shared__ uint32_t tmem_base;
-    __shared__ int fail;
+    __shared__ volatile int fail;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int mt = blockIdx.x, split = blockIdx.y;
-    const int k0 = split * a.k_steps;
+    const int box_bytes = halo_box_bytes(a.bw), stage_bytes = wgrad_stage(a.bw);
+    const int per_n = a.D * a.tiles_h;
+    const int dx = blockIdx.y, split = blockIdx.x;
+    const bool bias = dx == 1;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) {
+        for (int s = 0; s < kWgradStages; ++s) {
             tc::mbar_init(&full[s], 1);
-            tc::mbar_init(&empty[s], 1);
+            tc::mbar_init(&empty[s], bias ? 129 : 1);   // the MMAs' commit and the bias readers
         }
         tc::mbar_init(&done, 1);
         tc::fence_barrier_init();
         fail = 0;
     }
-    if (warp == 1) {
-        tc::tmem_alloc(&tmem_base, 32);
+    if (warp == 5) {
+        tc::tmem_alloc(&tmem_base, 128);
         tc::tmem_relinquish();
     }
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = tmem_base;
-    if (warp == 0 && lane == 0) {
-        int issued = 0;
-        for (int j = 0; j < a.k_steps; ++j) {
-            const int s = j % kStages;
-            if (j >= kStages && !tc::mbar_wait(&empty[s], (unsigned)((j / kStages) - 1) & 1u)) {
+    float hi[8], lo[8];   // warps 0-3: column sums of 8 channels
+#pragma unroll
+    for (int j = 0; j < 8; ++j) hi[j] = lo[j] = 0.0f;
+    if (warp == 4) {
+        if (lane == 0) {
+            int it = 0;
+            for (int tile = split; tile < a.n_tiles && !fail; tile += gridDim.x, ++it) {
+                const int s = it % kWgradStages;
+                if (it >= kWgradStages && !tc::mbar_wait(&empty[s], (unsigned)(it / kWgradStages - 1) & 1u)) {
+                    atomicOr(a.err, tc::kErrWait);
+                    fail = 1;
+                    break;
+                }
+                const int n = tile / per_n, rem = tile % per_n;
+                const int z = rem / a.tiles_h, y0 = (rem % a.tiles_h) * a.bh;
+                unsigned char* box = base + s * stage_bytes;
+                tc::mbar_expect_tx(&full[s], stage_bytes);
+                tc::tma_load_5d(box, &hmap, &full[s], 0, dx - 1, y0 - 1, z - 1, n);
+                tc::tma_load_5d(box + box_bytes, &dmap, &full[s], 0, 0, y0, z, n);
+            }
+            // every issued copy lands before the CTA leaves
+            for (int j = it - 1; j >= 0 && j >= it - kWgradStages; --j)
+                tc::mbar_wait(&full[j % kWgradStages], (unsigned)(j / kWgradStages) & 1u);
+        }
+    } else if (warp == 5) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = tc::idesc_bf16_mn(128, 32);
+            bool ok = true;
+            int it = 0;
+            for (int tile = split; tile < a.n_tiles && !fail; tile += gridDim.x, ++it) {
+                const int s = it % kWgradStages;
+                if (!tc::mbar_wait(&full[s], (unsigned)(it / kWgradStages) & 1u)) {
+                    ok = false;
+                    break;
+                }
+                tc::tc_fence_after();
+                const int line = a.bw * 64;
+                const unsigned char* box = base + s * stage_bytes;
+                const uint64_t bd = tc::sdesc_sw64_mn(box + box_bytes, 512);
+                for (int dz = 0; dz < 3; ++dz) {
+                    const uint64_t ad = tc::sdesc_sw64_mn(box + dz * (a.bh + 2) * line, (uint32_t)line);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)   // 16 voxels = 1 KB of either operand
+                        tc::mma_bf16(tmem + 32u * (uint32_t)dz, ad + 64 * k, bd + 64 * k, idesc,
+                                     it > 0 || k > 0 ? 1u : 0u);
+                }
+                tc::mma_commit(&empty[s]);
+            }
+            if (!ok) {
                 atomicOr(a.err, tc::kErrWait);
                 fail = 1;
-                break;
             }
-            unsigned char* st = base + s * kGemmStage;
-            tc::mbar_expect_tx(&full[s], kGemmStage);
-            tc::tma_load_2d(st, &amap, &full[s], (k0 + j) * 32, mt * 128);
-            tc::tma_load_2d(st + kTileA, &bmap, &full[s], (k0 + j) * 32, 0);
-            ++issued;
+            tc::mma_commit(&done);
+            tc::mbar_wait(&done, 0);   // every issued MMA completes before the accumulators are freed
         }
-        for (int j = issued - 1; j >= 0 && j >= issued - kStages; --j)
-            tc::mbar_wait(&full[j % kStages], (unsigned)(j / kStages) & 1u);
-    } else if (warp == 1 && lane == 0) {
-        constexpr uint32_t idesc = tc::idesc_bf16(128, 32);
-        bool ok = true;
-        for (int j = 0; j < a.k_steps; ++j) {
-            const int s = j % kStages;
-            if (!tc::mbar_wait(&full[s], (unsigned)(j / kStages) & 1u)) {
-                ok = false;
-                break;
+    } else {
+        if (bias) {
+            int it = 0;
+            for (int tile = split; tile < a.n_tiles && !fail; tile += gridDim.x, ++it) {
+                const int s = it % kWgradStages;
+                if (!tc::mbar_wait(&full[s], (unsigned)(it / kWgradStages) & 1u)) {
+                    atomicOr(a.err, tc::kErrWait);
+                    fail = 1;
+                    break;
+                }
+                const unsigned char* dy = base + s * stage_bytes + box_bytes;
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int row = (threadIdx.x >> 2) + 32 * r;
+                    const int q = (threadIdx.x & 3) ^ ((row >> 1) & 3);   // 64-byte swizzle
+                    const uint4 u = *reinterpret_cast<const uint4*>(dy + row * 64 + q * 16);
+                    const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&u);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float x = __bfloat162float(h[j]);
+                        const float t = hi[j] + x, v = t - hi[j];
+                        lo[j] += (hi[j] - (t - v)) + (x - v);
+                        hi[j] = t;
+                    }
+                }
+                tc::mbar_arrive(&empty[s]);
             }
-            tc::tc_fence_after();
-            unsigned char* st = base + s * kGemmStage;
-            const uint64_t ad = tc::sdesc_sw64(st), bd = tc::sdesc_sw64(st + kTileA);
-            tc::mma_bf16(tmem, ad, bd, idesc, j > 0 ? 1u : 0u);
-            tc::mma_bf16(tmem, ad + 2, bd + 2, idesc, 1u);
-            tc::mma_commit(&empty[s]);
         }
-        if (!ok) {
+        if (!tc::mbar_wait(&done, 0)) {
             atomicOr(a.err, tc::kErrWait);
             fail = 1;
         }
-        tc::mma_commit(&done);
     }
-    __syncwarp();
-    const bool got = tc::mbar_wait(&done, 0);
+    __syncthreads();   // copies landed, MMAs done, `fail` final
     tc::tc_fence_after();
-    if (!got) atomicOr(a.err, tc::kErrWait);
-    float acc[32];
-    tc::tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16), acc);
-    __syncthreads();
-    const int m = mt * 128 + warp * 32 + lane;
-    float* o = a.ws + ((size_t)split * kMPad + m) * 32;
+    const bool good = !fail;
+    if (warp < 3) {
+        // accumulator rows 32 dy + c_in, one TMEM lane each
+        for (int dz = 0; dz < 3; ++dz) {
+            float acc[32];
+            tc::tmem_ld32(tmem + 32u * (uint32_t)dz + ((uint32_t)(warp * 32) << 16), acc);
+            const int t = dz * 9 + warp * 3 + dx;
+            float4* o = reinterpret_cast<float4*>(a.ws + (((size_t)split * kTaps + t) * kCh + lane) * kCh);
 #pragma unroll
-    for (int c = 0; c < 32; ++c) o[c] = (got && !fail && a.k_steps > 0) ? acc[c] : 0.0f;
-    if (!got) tc::mbar_wait(&done, 0);
+            for (int q = 0; q < 8; ++q)
+                o[q] = good ? make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3])
+                            : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    }
+    // the stages' memory is free: nothing reads or writes it any more
+    double* sb = reinterpret_cast<double*>(base);   // [32 row groups][32 channels]
+    if (bias && warp < 4) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            sb[(threadIdx.x >> 2) * kCh + (threadIdx.x & 3) * 8 + j] =
+                isfinite(hi[j]) ? (double)hi[j] + (double)lo[j] : (double)hi[j];
+    }
     tc::tc_fence_before();
     __syncthreads();
-    if (warp == 1) tc::tmem_dealloc(tmem, 32);
+    if (bias && warp == 0) {
+        double s = 0.0;
+        for (int r = 0; r < 32; ++r) s += sb[r * kCh + lane];
+        a.bias_ws[(size_t)split * kCh + lane] = good ? s : 0.0;
+    }
+    if (warp == 5) tc::tmem_dealloc(tmem, 128);
 }
 
-// xcol[t * 32 + c][g] = x[n][z + dz][y + dy][x + dx][c] (zero outside),
-// g = n V + voxel < G, rows `ld` long; one thread per (voxel, tap).
-__global__ void k_im2col_t(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ xcol, int D, int H,
-                           int W, long long G, long long ld) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= G * kTaps) return;
-    const int t = (int)(i / G);
-    const long long g = i % G;
-    const int V = D * H * W;
-    const int s = (int)(g / V), v = (int)(g % V);
-    const int xx = v % W, yy = (v / W) % H, zz = v / (W * H);
-    const int dz = t / 9 - 1, dy = (t / 3) % 3 - 1, dx = t % 3 - 1;
-    const int z2 = zz + dz, y2 = yy + dy, x2 = xx + dx;
-    __nv_bfloat16 vals[32];
-    if (z2 >= 0 && z2 < D && y2 >= 0 && y2 < H && x2 >= 0 && x2 < W) {
-        const uint4* p = reinterpret_cast<const uint4*>(x + (((size_t)s * D + z2) * H * W + (size_t)y2 * W + x2) * kCh);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint4 u = p[q];
-            const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&u);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) vals[8 * q + j] = h[j];
-        }
+// dW[t][co][ci] = sum over splits of ws[s][t][ci][co] and, in the last block,
+// db[co] = sum of bias_ws[s][co]: eight interleaved partial sums, then those
+// in order.
+__global__ void __launch_bounds__(256) k_wgrad_reduce(const float* __restrict__ ws,
+                                                      const double* __restrict__ bias_ws, int splits,
+                                                      float* __restrict__ gw, float* __restrict__ gb) {
+    __shared__ double sh[8][kCh];
+    const int co = threadIdx.x & 31, r = threadIdx.x >> 5;
+    const int m = blockIdx.x;   // t * 32 + ci
+    if (m < kTaps * kCh) {
+        float s = 0.0f;
+#pragma unroll 4
+        for (int p = r; p < splits; p += 8) s += ws[(size_t)p * kWElems + m * kCh + co];
+        sh[r][co] = (double)s;
     } else {
-#pragma unroll
-        for (int c = 0; c < 32; ++c) vals[c] = __float2bfloat16_rn(0.0f);
+        double s = 0.0;
+        for (int p = r; p < splits; p += 8) s += bias_ws[(size_t)p * kCh + co];
+        sh[r][co] = s;
     }
-#pragma unroll
-    for (int c = 0; c < 32; ++c) xcol[(size_t)(t * kCh + c) * ld + g] = vals[c];
-}
-
-// dyt[c][g] = d[g][c], g < G, rows `ld` long
-__global__ void k_transpose_ch(const __nv_bfloat16* __restrict__ d, __nv_bfloat16* __restrict__ dyt, long long G,
-                               long long ld) {
-    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= G) return;
-    const uint4* p = reinterpret_cast<const uint4*>(d + g * kCh);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const uint4 u = p[q];
-        const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&u);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) dyt[(size_t)(8 * q + j) * ld + g] = h[j];
-    }
-}
-
-// dW[t][co][ci] = sum over splits of ws[s][t * 32 + ci][co] (fixed order)
-__global__ void k_wgrad_reduce(const float* __restrict__ ws, int splits, float* __restrict__ gw) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kWElems) return;
-    const int t = i / (kCh * kCh), co = (i / kCh) % kCh, ci = i % kCh;
-    float s = 0.0f;
-    for (int p = 0; p < splits; ++p) s += ws[((size_t)p * kMPad + t * kCh + ci) * kCh + co];
-    gw[i] = s;
-}
-
-// db[c] = sum_g d[g][c]: per-block partials (double) then one block sums them
-__global__ void k_bias_partial(const __nv_bfloat16* __restrict__ d, long long G, double* __restrict__ part) {
-    __shared__ double sh[256];
-    const int c = threadIdx.x & 31, r = threadIdx.x >> 5;   // 8 rows of 32 channels per pass
-    double acc = 0.0;
-    for (long long g = (long long)blockIdx.x * 8 + r; g < G; g += (long long)gridDim.x * 8)
-        acc += (double)__bfloat162float(d[g * kCh + c]);
-    sh[threadIdx.x] = acc;
     __syncthreads();
     if (r == 0) {
         double s = 0.0;
-        for (int k = 0; k < 8; ++k) s += sh[k * 32 + c];
-        part[(size_t)blockIdx.x * kCh + c] = s;
+        for (int k = 0; k < 8; ++k) s += sh[k][co];
+        if (m < kTaps * kCh)
+            gw[((m >> 5) * kCh + co) * kCh + (m & 31)] = (float)s;
+        else
+            gb[co] = (float)s;
     }
-}
-
-__global__ void k_bias_final(const double* __restrict__ part, int nb, float* __restrict__ gb) {
-    const int c = threadIdx.x;
-    if (c >= kCh) return;
-    double s = 0.0;
-    for (int b = 0; b < nb; ++b) s += part[(size_t)b * kCh + c];
-    gb[c] = (float)s;
 }
 
 // delta = dout (FP32 [G][c_out]) as BF16 [G][32]
@@ -755,8 +795,6 @@ void Cnn::free_grid() {
     dfree(delta[1]);
     dfree(out32);
     dfree(dout32);
-    dfree(xcol);
-    dfree(dyt);
     dfree(ws);
     dfree(red);
     n_cap = 0;
@@ -827,25 +865,22 @@ void Cnn::ensure(int n, int D_, int H_, int W_) {
     for (auto*& p : delta) p = dmalloc<__nv_bfloat16>(G * kCh);
     out32 = dmalloc<float>(G * cout);
     dout32 = dmalloc<float>(G * cout);
-    xcol = dmalloc<__nv_bfloat16>((size_t)kMPad * G);
-    ck(cudaMemsetAsync(xcol, 0, (size_t)kMPad * G * 2, st), "memset");   // rows 864.. stay zero
-    dyt = dmalloc<__nv_bfloat16>((size_t)kCh * G);
-    const long long ksteps = (long long)G / 32;
-    splits = (int)std::max<long long>(1, std::min<long long>(64, ksteps / 8));
-    ws = dmalloc<float>((size_t)splits * kMPad * kCh);
-    red = dmalloc<double>(4096 * kCh);
+    // weight gradients: two CTAs on each SM, three x shifts; at least one
+    // 128-voxel tile per split
+    int sms = 0;
+    ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
+    splits = (int)std::max<long long>(1, std::min<long long>((long long)G / 128, 2 * sms / 3));
+    ws = dmalloc<float>((size_t)splits * kWElems);
+    red = dmalloc<double>((size_t)std::max(splits * kCh, kMseBlocks));
     act_map.resize(L + 1);
     for (int l = 0; l <= L; ++l) encode_act_map(&act_map[l], act[l], n, D, H, W, bw, bh);
     delta_map.resize(2);
     for (int k = 0; k < 2; ++k) encode_act_map(&delta_map[k], delta[k], n, D, H, W, bw, bh);
     act_hmap.assign(L + 1, CUtensorMap{});
     delta_hmap.assign(2, CUtensorMap{});
-    if (W <= kHaloMaxW) {
-        for (int l = 0; l <= L; ++l) encode_act_map(&act_hmap[l], act[l], n, D, H, W, bw, bh, 1);
+    for (int l = 0; l <= L; ++l) encode_act_map(&act_hmap[l], act[l], n, D, H, W, bw, bh, 1);
+    if (W <= kHaloMaxW)
         for (int k = 0; k < 2; ++k) encode_act_map(&delta_hmap[k], delta[k], n, D, H, W, bw, bh, 1);
-    }
-    encode_2d_map(&xcol_map, xcol, (long long)G, kMPad, 128);
-    encode_2d_map(&dyt_map, dyt, (long long)G, kCh, kCh);
     ck(cudaStreamSynchronize(st), "sync");
 }
 
@@ -888,31 +923,23 @@ const float* Cnn::forward(int n) {
     return out32;
 }
 
-void Cnn::wgrad(int l, const __nv_bfloat16* x, const __nv_bfloat16* d, int n) {
+void Cnn::wgrad(int l, const CUtensorMap& x_hmap, const CUtensorMap& d_map, int n) {
     static bool attr = false;
     if (!attr) {
-        ck(cudaFuncSetAttribute(k_gemm_tn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem), "attr");
+        ck(cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem(kWgradMaxW)),
+           "attr");
         attr = true;
     }
-    const long long G = (long long)n * V;
-    const long long Gcap = (long long)n_cap * V;
-    // the operand rows are n_cap samples long (the tensor maps' extent);
-    // only this call's first G columns are written and read
-    k_im2col_t<<<(unsigned)((G * kTaps + 255) / 256), 256, 0, st>>>(x, xcol, D, H, W, G, Gcap);
-    k_transpose_ch<<<(unsigned)((G + 255) / 256), 256, 0, st>>>(d, dyt, G, Gcap);
-    ck(cudaGetLastError(), "im2col");
-    // K split over CTAs: the largest divisor of the 32-voxel step count
-    // not above `splits`
-    const long long ksteps = G / 32;
-    int sp = (int)std::max<long long>(1, std::min<long long>(splits, ksteps));
-    while (ksteps % sp) --sp;
-    GemmArgs a{(int)(ksteps / sp), ws, err};
-    k_gemm_tn_tc<<<dim3(kMPad / 128, sp), 128, kGemmSmem, st>>>(xcol_map, dyt_map, a);
-    ck(cudaGetLastError(), "gemm launch");
-    k_wgrad_reduce<<<(kWElems + 255) / 256, 256, 0, st>>>(ws, sp, gw + (size_t)l * kWElems);
-    const int nb = (int)std::min<long long>(4096, (G + 7) / 8);
-    k_bias_partial<<<nb, 256, 0, st>>>(d, G, red);
-    k_bias_final<<<1, 32, 0, st>>>(red, nb, gb + (size_t)l * kCh);
+    WgradArgs a{};
+    a.D = D; a.bw = bw; a.bh = bh; a.tiles_h = H / bh;
+    a.n_tiles = n * D * (H / bh);
+    a.ws = ws;
+    a.bias_ws = red;
+    a.err = err;
+    const int sp = std::min(a.n_tiles, splits);
+    k_wgrad_tc<<<dim3(sp, 3), 192, wgrad_smem(W), st>>>(x_hmap, d_map, a);
+    ck(cudaGetLastError(), "wgrad launch");
+    k_wgrad_reduce<<<kTaps * kCh + 1, 256, 0, st>>>(ws, red, sp, gw + (size_t)l * kWElems, gb + (size_t)l * kCh);
     ck(cudaGetLastError(), "wgrad");
 }
 
@@ -923,7 +950,7 @@ void Cnn::backward(int n, const float* dout, float* dx) {
     ck(cudaGetLastError(), "delta");
     int cur = 0;
     for (int l = L - 1; l >= 0; --l) {
-        wgrad(l, act[l], delta[cur], n);
+        wgrad(l, act_hmap[l], delta_map[cur], n);
         if (l > 0 || dx) {
             // input gradient; for l > 0 masked by ReLU'(act[l]) into the next delta
             conv(l, true, delta_map[cur], delta_hmap[cur], l > 0 ? act[l] : nullptr, delta[cur ^ 1],
@@ -936,7 +963,7 @@ void Cnn::backward(int n, const float* dout, float* dx) {
 double Cnn::loss_backward(int n, const float* target) {
     const long long G = (long long)n * V;
     const long long n_el = G * cout;
-    const int nb = 1024;
+    const int nb = kMseBlocks;
     k_mse<<<nb, 256, 0, st>>>(out32, target, n_el, 1.0 / (double)G, dout32, red);
     ck(cudaGetLastError(), "mse");
     std::vector<double> h(nb);

@@ -76,7 +76,6 @@ private:
     __nv_bfloat16* delta[2] = {nullptr, nullptr};
     float* out32 = nullptr;
     float* dout32 = nullptr;
-    __nv_bfloat16 *xcol = nullptr, *dyt = nullptr;
     float* ws = nullptr;
     double* red = nullptr;
     unsigned* err = nullptr;
@@ -84,15 +83,14 @@ private:
     int splits = 0;
     long long adam_t = 0;
     std::vector<CUtensorMap> act_map, delta_map, w_map, wt_map;
-    // the same buffers with a halo box (W <= 64): a tile's input and its
-    // one-voxel border in y and z, loaded once per x shift
+    // the same buffers with a halo box (delta: W <= 64): a tile's input and
+    // its one-voxel border in y and z, loaded once per x shift
     std::vector<CUtensorMap> act_hmap, delta_hmap;
-    CUtensorMap xcol_map{}, dyt_map{};
     void free_grid();
     void upload_bf16();
     void conv(int l, bool transposed, const CUtensorMap& in_map, const CUtensorMap& in_hmap,
               const __nv_bfloat16* mask, __nv_bfloat16* out, float* o32, int n32, int n);
-    void wgrad(int l, const __nv_bfloat16* x, const __nv_bfloat16* d, int n);
+    void wgrad(int l, const CUtensorMap& x_hmap, const CUtensorMap& d_map, int n);
 };
 
 // ---------------------------------------------------------------------------

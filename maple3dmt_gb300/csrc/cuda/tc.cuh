@@ -7,7 +7,8 @@
 // TMA with 64-byte swizzling; the matching tcgen05 shared-memory descriptor
 // uses layout SWIZZLE_64B with 8-row groups 512 bytes apart.  One MMA reads
 // K = 16 (32 bytes), the second half of a row is reached by advancing the
-// descriptor's start address by 32 bytes.
+// descriptor's start address by 32 bytes.  The weight gradient reads the same
+// tiles M- and N-major (sdesc_sw64_mn).
 #pragma once
 
 #include <cuda.h>
@@ -116,10 +117,29 @@ __device__ __forceinline__ uint64_t sdesc_sw64(const void* tile) {
     return d;
 }
 
+// The same 64-byte rows read the other way round: M (or N) runs along a row's
+// 32 elements and continues in the row `group` bytes further on, K runs down
+// the rows, eight of them 512 bytes.  A tensor stored [voxel][channel] is so
+// the transposed operand of a contraction over voxels, without a transposition
+// in memory.  Tiles start on 512-byte boundaries.
+__device__ __forceinline__ uint64_t sdesc_sw64_mn(const void* tile, uint32_t group) {
+    const uint32_t a = smem_u32(tile);
+    uint64_t d = (uint64_t)((a >> 4) & 0x3FFFu);
+    d |= (uint64_t)((group >> 4) & 0x3FFFu) << 16;   // to the next 32 elements of M or N
+    d |= (uint64_t)(512 >> 4) << 32;                 // to the next eight of K
+    d |= (uint64_t)1 << 46;                          // version
+    d |= (uint64_t)4 << 61;                          // SWIZZLE_64B
+    return d;
+}
+
 // Instruction descriptor of kind::f16: BF16 A and B, FP32 accumulator,
-// both K-major, M x N.
+// both K-major, M x N; idesc_bf16_mn: both M- and N-major.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+__host__ __device__ constexpr uint32_t idesc_bf16_mn(int M, int N) {
+    return idesc_bf16(M, N) | (1u << 15) | (1u << 16);
 }
 
 // D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.

@@ -106,6 +106,36 @@ def test_backward_matches_cpu_gradients(lib, layers, tol):
     assert ex < tol
 
 
+@pytest.mark.parametrize("n_cap,grid", [(1, (1, 1, 8, 16)), (1, (1, 3, 16, 16)), (3, (2, 5, 8, 32)), (1, (2, 3, 6, 64)),
+                                        (1, (1, 3, 5, 128)), (3, (3, 13, 32, 16))])
+def test_weight_gradients_over_grids(lib, n_cap, grid):
+    """dW and db of a two-layer network at each tile width, at grids of one
+    tile and of more tiles than splits, and for fewer samples than the buffers
+    hold, within the two-layer bound of the gradient check above (2.5e-2: BF16
+    activations); a tap or a line out of place is an error of order one."""
+    from oracle import cnn
+    net = _net(lib, 2, 8, 32, 6, seed=7)
+    rng = np.random.default_rng(8)
+    x = rng.normal(size=grid + (8,)).astype(np.float32)
+    dy = rng.normal(size=grid + (6,)).astype(np.float32)
+    if n_cap > grid[0]:
+        big = (n_cap,) + grid[1:]
+        net.backward(rng.normal(size=big + (8,)).astype(np.float32), rng.normal(size=big + (6,)).astype(np.float32))
+    dw, db, _ = net.backward(x, dy)
+    ws, bs = _cpu_params(net, 2, 8, 32, 6)
+    xb = bf16(x)
+    cdw, cdb = [np.zeros_like(w) for w in ws], [np.zeros_like(b) for b in bs]
+    for i in range(grid[0]):
+        gw, gb, _ = cnn.backward(cnn.forward(xb[i], ws, bs), ws, dy[i].astype(np.float64))
+        for l in range(2):
+            cdw[l] += gw[l]
+            cdb[l] += gb[l]
+    for l, (ci, co) in enumerate([(8, 32), (32, 6)]):
+        ew, eb = nrel(dw[l][:, :co, :ci], cdw[l]), nrel(db[l][:co], cdb[l])
+        print(f"grid {grid}, layer {l}: dW {ew:.2e} db {eb:.2e}")
+        assert ew < 2.5e-2 and eb < 2.5e-2
+
+
 def test_training_reduces_loss(lib):
     """Adam on the tensor-core forward and backward passes fits a fixed
     teacher network's outputs on random inputs."""
