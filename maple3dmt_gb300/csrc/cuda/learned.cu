@@ -604,13 +604,18 @@ __global__ void __launch_bounds__(256) k_wgrad_reduce(const float* __restrict__ 
     }
 }
 
-// delta = dout (FP32 [G][c_out]) as BF16 [G][32]
-__global__ void k_dout_to_delta(const float* __restrict__ dout, int c_out, long long G, __nv_bfloat16* __restrict__ d) {
+// FP32 [G][c] -> BF16 [G][32], channels c.. zero; one thread per eight
+// channels (one 16-byte store)
+__global__ void k_pack(const float* __restrict__ x, int c, long long G, __nv_bfloat16* __restrict__ d) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= G * kCh) return;
-    const long long g = i / kCh;
-    const int c = (int)(i % kCh);
-    d[i] = __float2bfloat16_rn(c < c_out ? dout[g * c_out + c] : 0.0f);
+    if (i >= G * 4) return;
+    const int q = (int)(i & 3) * 8;
+    const float* p = x + (i >> 2) * c;
+    uint4 u;
+    __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(&u);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) h[j] = __float2bfloat16_rn(q + j < c ? p[q + j] : 0.0f);
+    reinterpret_cast<uint4*>(d)[i] = u;
 }
 
 // MSE loss: dout = (out - target) / (G), partial sums of (out - target)^2
@@ -828,10 +833,11 @@ void Cnn::get_weights(float* w, float* b) const {
     ck(cudaMemcpy(b, b32, (size_t)L * kCh * sizeof(float), cudaMemcpyDeviceToHost), "b");
 }
 
-void Cnn::get_grads(float* dw, float* db) const {
-    ck(cudaStreamSynchronize(st), "sync");
-    ck(cudaMemcpy(dw, gw, (size_t)L * kWElems * sizeof(float), cudaMemcpyDeviceToHost), "dw");
-    ck(cudaMemcpy(db, gb, (size_t)L * kCh * sizeof(float), cudaMemcpyDeviceToHost), "db");
+void Cnn::pack_input(const float* x, int n) {
+    ck(cudaSetDevice(dev), "cudaSetDevice");
+    const long long G = (long long)n * V;
+    k_pack<<<(unsigned)((G * 4 + 255) / 256), 256, 0, st>>>(x, cin, G, act[0]);
+    ck(cudaGetLastError(), "input");
 }
 
 unsigned Cnn::error_flag() {
@@ -851,8 +857,8 @@ void Cnn::ensure(int n, int D_, int H_, int W_) {
         throw std::invalid_argument("cnn: grid W must be 16, 32, 64 or 128");
     const int bw_ = W_, bh_ = 128 / W_;
     if (H_ % bh_ != 0 || D_ < 1 || n < 1) throw std::invalid_argument("cnn: grid H must be a multiple of 128 / W");
-    if (n <= n_cap && D_ == D && H_ == H && W_ == W) return;
     ck(cudaSetDevice(dev), "cudaSetDevice");
+    if (n <= n_cap && D_ == D && H_ == H && W_ == W) return;
     free_grid();
     D = D_; H = H_; W = W_; V = D * H * W; bw = bw_; bh = bh_;
     n_cap = n;
@@ -946,7 +952,7 @@ void Cnn::wgrad(int l, const CUtensorMap& x_hmap, const CUtensorMap& d_map, int 
 void Cnn::backward(int n, const float* dout, float* dx) {
     ck(cudaSetDevice(dev), "cudaSetDevice");
     const long long G = (long long)n * V;
-    k_dout_to_delta<<<(unsigned)((G * kCh + 255) / 256), 256, 0, st>>>(dout, cout, G, delta[0]);
+    k_pack<<<(unsigned)((G * 4 + 255) / 256), 256, 0, st>>>(dout, cout, G, delta[0]);
     ck(cudaGetLastError(), "delta");
     int cur = 0;
     for (int l = L - 1; l >= 0; --l) {
@@ -954,7 +960,7 @@ void Cnn::backward(int n, const float* dout, float* dx) {
         if (l > 0 || dx) {
             // input gradient; for l > 0 masked by ReLU'(act[l]) into the next delta
             conv(l, true, delta_map[cur], delta_hmap[cur], l > 0 ? act[l] : nullptr, delta[cur ^ 1],
-                 (l == 0 && dx) ? dx : nullptr, kCh, n);
+                 (l == 0 && dx) ? dx : nullptr, cin, n);
             cur ^= 1;
         }
     }

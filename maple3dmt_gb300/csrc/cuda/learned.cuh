@@ -45,16 +45,19 @@ public:
     void ensure(int n, int D, int H, int W);
     // input activations: [n][D][H][W][32] BF16, channels >= c_in zero
     __nv_bfloat16* input() { return act[0]; }
+    // its first n samples from device FP32 [n V][c_in]
+    void pack_input(const float* x, int n);
     // the network on the first n samples of input(); output FP32 [n V][c_out]
     const float* forward(int n);
     // gradients of sum(dout * out) for dout FP32 [n V][c_out] (after forward(n));
-    // into the FP32 gradient buffers; d/dinput to dx ([n V][32] FP32) if given
+    // into the FP32 gradient buffers; d/dinput to dx ([n V][c_in] FP32) if given
     void backward(int n, const float* dout, float* dx);
     // 0.5 * mean over samples and voxels of |out - target|^2 and its backward
     double loss_backward(int n, const float* target);
     void adam_step(float lr, float beta1 = 0.9f, float beta2 = 0.999f, float eps = 1e-8f);
-    // host FP32 gradients: dw [L][27][32][32], db [L][32]
-    void get_grads(float* dw, float* db) const;
+    // device FP32 gradients: dw [L][27][32][32], db [L][32]
+    const float* grad_w() const { return gw; }
+    const float* grad_b() const { return gb; }
     unsigned error_flag();
     cudaStream_t stream() const { return st; }
     // run on the caller's stream (the caller keeps ownership; null: the
