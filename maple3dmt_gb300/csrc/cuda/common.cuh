@@ -101,6 +101,52 @@ template <> struct Sum<float> {
     }
 };
 
+// Dependent launches.  A kernel launched by launch_dep may start while its
+// predecessor in the stream still runs: its blocks are scheduled and whatever
+// no kernel writes (matrix copies, index arrays, barriers) is under way when
+// the predecessor ends, and dep_wait() returns then, with all of the
+// predecessor's writes visible.  The small grids' and the small meshes'
+// kernels run for 5-30 us, of which the way from one launch to the next was 1
+// to 2: the all-frequency solve of 58 k edges and eight right-hand sides 40.5
+// -> 35.8 ms, one frequency of 20 k edges 11.2 -> 9.4 ms.  Rules:
+//  * a kernel launched so calls dep_wait() before its first access to anything
+//    that a kernel of the chain writes, and every block calls it;
+//  * such data is not read through `const __restrict__` pointers or __ldg (the
+//    read-only path is not ordered behind the wait);
+//  * what is read before the wait was complete when the chain's first, plain
+//    launch started: a plain launch waits for all work before it.
+// dep_begin() is dep_trigger() (let the successor start) and dep_wait(); both
+// do nothing under a plain launch.
+__device__ __forceinline__ void dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dep_begin() {
+    dep_trigger();
+    dep_wait();
+}
+
+// Adds the attribute of a dependent launch, if the stream is not being captured.
+inline void dep_attr(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(cfg.stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return;
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+}
+
+// Launch errors stay with the runtime, for the caller's cudaGetLastError().
+template <class... P, class... A>
+inline void launch_dep(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    dep_attr(cfg, at);
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Blocks of `threads` threads with `smem` bytes of dynamic shared memory of
 // `kernel` that are resident on the current device at once (occupancy API x
 // SM count); cached per (device, kernel, threads, smem).

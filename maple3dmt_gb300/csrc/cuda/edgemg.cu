@@ -234,7 +234,7 @@ __global__ void k_mass(EmgLevel F, EmgLevel C) {
 // (lanes H, the entries dealt out to the rest); the total on the first H.
 template <int H>
 __device__ __forceinline__ float4 long_row(const int* __restrict__ idx, const float* __restrict__ w, int q0, int q1,
-                                           const float4* __restrict__ v) {
+                                           const float4* v) {
     constexpr int G = kLongNT / H;
     __shared__ float4 part[kLongNT];
     const int h = threadIdx.x % H, g = threadIdx.x / H;
@@ -251,7 +251,8 @@ __device__ __forceinline__ float4 long_row(const int* __restrict__ idx, const fl
 
 // b0 = P^T r from the octree rows, x0 = w b0 / d; a thread per edge entry
 template <int K>
-__global__ void __launch_bounds__(kNT) k_restrict0(EmgDev g, Omegas om, const float4* __restrict__ r, int n) {
+__global__ void __launch_bounds__(kNT) k_restrict0(EmgDev g, Omegas om, const float4* r, int n) {
+    dep_begin();
     constexpr int H = K / 2;
     const EmgLevel& L = g.lv[0];
     const int t = blockIdx.x * kNT + threadIdx.x, c = t / H, h = t % H;
@@ -285,7 +286,8 @@ __global__ void __launch_bounds__(kNT) k_restrict0(EmgDev g, Omegas om, const fl
 // refinement of two or three levels collect up to 196 or 1800 octree edges,
 // which one thread after another made 50 us on the 157 k-edge mesh.
 template <int K>
-__global__ void __launch_bounds__(kLongNT) k_restrict0_long(EmgDev g, Omegas om, const float4* __restrict__ r) {
+__global__ void __launch_bounds__(kLongNT) k_restrict0_long(EmgDev g, Omegas om, const float4* r) {
+    dep_begin();
     constexpr int H = K / 2;
     const EmgLevel& L = g.lv[0];
     const int c = g.r_long[blockIdx.x], h = threadIdx.x % H;
@@ -302,6 +304,7 @@ __global__ void __launch_bounds__(kLongNT) k_restrict0_long(EmgDev g, Omegas om,
 // y = b - A x, or (SMOOTH) y = x + w (b - A x) / d
 template <int K, bool SMOOTH>
 __global__ void __launch_bounds__(kNT, 3) k_edge_step(EmgLevel L, Omegas oms) {
+    dep_begin();
     constexpr int H = K / 2;
     each_point<H>(L, [&](int i, int j, int k, int h) {
         const Free f = edges_free(L, i, j, k);
@@ -332,6 +335,7 @@ __global__ void __launch_bounds__(kNT, 3) k_edge_step(EmgLevel L, Omegas oms) {
 // b = P^T y_fine, x = w b / d
 template <int K>
 __global__ void __launch_bounds__(kNT) k_restrict(EmgLevel F, EmgLevel L, Omegas om) {
+    dep_begin();
     constexpr int H = K / 2;
     each_point<H>(L, [&](int i, int j, int k, int h) {
         const Free f = edges_free(L, i, j, k);
@@ -378,6 +382,7 @@ __device__ __forceinline__ void interp_edges(const Free& f, int n, int i, int j,
 // x += P y_coarse
 template <int K>
 __global__ void __launch_bounds__(kNT) k_prolong(EmgLevel L, EmgLevel C) {
+    dep_begin();
     constexpr int H = K / 2;
     each_point<H>(L, [&](int i, int j, int k, int h) {
         const Free f = edges_free(L, i, j, k);
@@ -538,6 +543,7 @@ __device__ __forceinline__ const float2* small_cycle(const EmgDev& g, int l1, Om
 
 // From level l0 of 8 or 4 cells: one block per right-hand side.
 __global__ void __launch_bounds__(kBottomNT) k_bottom(EmgDev g, int l0, Omegas oms) {
+    dep_begin();
     extern __shared__ float2 sm[];
     const EmgLevel& L = g.lv[l0];
     const int lane = blockIdx.x, ne = entries(L);
@@ -553,6 +559,7 @@ __global__ void __launch_bounds__(kBottomNT) k_bottom(EmgDev g, int l0, Omegas o
 // From level l0 of 16 cells: a cluster of NC blocks per right-hand side.
 template <int NC>
 __global__ void __launch_bounds__(kBottomNT) k_bottom16(EmgDev g, int l0, Omegas oms) {
+    dep_begin();
     extern __shared__ float2 sm[];
     constexpr int PT = 8 / NC;   // points per thread
     const EmgLevel& L = g.lv[l0];
@@ -647,7 +654,8 @@ template <class V> __device__ __forceinline__ V node_pre(const EmgLevel& L, int 
 
 // nb0 = Pn^T b from the octree nodes; PRE: nt0 = w nb0 / diag
 template <int K, bool PRE>
-__global__ void __launch_bounds__(kNT) k_node_restrict0(EmgDev g, const float4* __restrict__ b) {
+__global__ void __launch_bounds__(kNT) k_node_restrict0(EmgDev g, const float4* b) {
+    dep_begin();
     constexpr int H = K / 2;
     const EmgLevel& L = g.lv[0];
     each_point<H>(L, [&](int i, int j, int k, int h) {
@@ -673,7 +681,8 @@ __global__ void __launch_bounds__(kNT) k_node_restrict0(EmgDev g, const float4* 
 }
 
 template <int K, bool PRE>
-__global__ void __launch_bounds__(kLongNT) k_node_restrict0_long(EmgDev g, const float4* __restrict__ b) {
+__global__ void __launch_bounds__(kLongNT) k_node_restrict0_long(EmgDev g, const float4* b) {
+    dep_begin();
     constexpr int H = K / 2;
     const EmgLevel& L = g.lv[0];
     const int c = g.nr_long[blockIdx.x], n1 = L.n + 1, h = threadIdx.x % H;
@@ -687,6 +696,7 @@ __global__ void __launch_bounds__(kLongNT) k_node_restrict0_long(EmgDev g, const
 // ny = nb - L nt, or (SMOOTH) ny = nt + w (nb - L nt) / diag
 template <int K, bool SMOOTH>
 __global__ void __launch_bounds__(kNT) k_node_step(EmgLevel L) {
+    dep_begin();
     constexpr int H = K / 2;
     each_point<H>(L, [&](int i, int j, int k, int h) {
         const size_t c = (size_t)pid(L.n, i, j, k) * H + h;
@@ -729,6 +739,7 @@ __device__ __forceinline__ V interp_node(int n, int i, int j, int k, const At& a
 // ny, with nt = w nb / diag
 template <int K, bool PRE>
 __global__ void __launch_bounds__(kNT) k_node_restrict(EmgLevel F, EmgLevel L) {
+    dep_begin();
     constexpr int H = K / 2;
     each_point<H>(L, [&](int i, int j, int k, int h) {
         float4 s = vz<float4>();
@@ -744,6 +755,7 @@ __global__ void __launch_bounds__(kNT) k_node_restrict(EmgLevel F, EmgLevel L) {
 // nt = Pn y_coarse, or (PRE) nt += Pn y_coarse
 template <int K, bool PRE>
 __global__ void __launch_bounds__(kNT) k_node_prolong(EmgLevel L, EmgLevel C) {
+    dep_begin();
     constexpr int H = K / 2;
     each_point<H>(L, [&](int i, int j, int k, int h) {
         float4 s = vz<float4>();
@@ -808,6 +820,7 @@ __device__ __forceinline__ const float2* small_node_cycle(const EmgDev& g, int l
 }
 
 template <bool PRE> __global__ void __launch_bounds__(kBottomNT) k_node_bottom(EmgDev g, int l0) {
+    dep_begin();
     extern __shared__ float2 sm[];
     const EmgLevel& L = g.lv[l0];
     const int lane = blockIdx.x, np = points(L);
@@ -818,6 +831,7 @@ template <bool PRE> __global__ void __launch_bounds__(kBottomNT) k_node_bottom(E
 }
 
 template <int NC, bool PRE> __global__ void __launch_bounds__(kBottomNT) k_node_bottom16(EmgDev g, int l0) {
+    dep_begin();
     extern __shared__ float2 sm[];
     constexpr int PT = 8 / NC;
     const EmgLevel& L = g.lv[l0];
@@ -876,8 +890,9 @@ template <int NC, bool PRE> __global__ void __launch_bounds__(kBottomNT) k_node_
 
 // t = Pn ny0 on the octree nodes (0 on Dirichlet nodes), plus x if given
 template <int K>
-__global__ void __launch_bounds__(kNT) k_node_prolong0(EmgDev g, int nn, const float4* __restrict__ x,
+__global__ void __launch_bounds__(kNT) k_node_prolong0(EmgDev g, int nn, const float4* x,
                                                        float4* __restrict__ out) {
+    dep_begin();
     constexpr int H = K / 2;
     const long i = (long)blockIdx.x * kNT + threadIdx.x;
     if (i >= (long)nn * H) return;
@@ -904,7 +919,8 @@ __global__ void __launch_bounds__(kNT) k_node_prolong0(EmgDev g, int nn, const f
 // z0 = P y0 + G~ yn / (i omega) + w r / d on free rows, r on identity rows
 template <int K>
 __global__ void __launch_bounds__(kNT) k_combine(EmgDev g, GcRowTerm gt, DiagView<float> D, Omegas om, long n,
-                                                 const float4* __restrict__ r, float4* __restrict__ z0) {
+                                                 const float4* r, float4* __restrict__ z0) {
+    dep_begin();
     constexpr int H = K / 2;
     const long i = (long)blockIdx.x * kNT + threadIdx.x;
     if (i >= n) return;
@@ -958,20 +974,21 @@ void launch_bottom(F16* k16, F8* k8, const EmgDev& g, int l0, int K, long (*per)
     const void* f = big ? reinterpret_cast<const void*>(k16) : reinterpret_cast<const void*>(k8);
     if (smem > 48 * 1024) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (!big) {
-        k8<<<K, kBottomNT, smem, s>>>(g, l0, args...);
+        launch_dep(k8, K, kBottomNT, (size_t)smem, s, g, l0, args...);
         return;
     }
     cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = nc;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = nc;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)(K * nc));
     cfg.blockDim = dim3(kBottomNT);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = s;
-    cfg.attrs = &at;
+    cfg.attrs = at;
     cfg.numAttrs = 1;
+    dep_attr(cfg, at);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, k16, g, l0, args...);
     if (e != cudaSuccess) throw std::runtime_error(cudaGetErrorString(e));
 }
@@ -982,22 +999,22 @@ void edge_cycle(const EmgDev& g, const Omegas& om, const float2* r, cudaStream_t
     k_restrict0<K><<<grid1((long)n * (K / 2)), kNT, 0, s>>>(g, om, f4(r), n);
     ck(launches);
     if (g.n_r_long) {
-        k_restrict0_long<K><<<g.n_r_long, kLongNT, 0, s>>>(g, om, f4(r));
+        launch_dep(k_restrict0_long<K>, g.n_r_long, kLongNT, 0, s, g, om, f4(r));
         ck(launches);
     }
     auto grid = [&](int l) { return point_grid<K>(g.lv[l], edge_planes(g.lv[l])); };
     for (int l = 0; l < l0; ++l) {
-        k_edge_step<K, false><<<grid(l), kNT, 0, s>>>(g.lv[l], om);
+        launch_dep(k_edge_step<K, false>, grid(l), kNT, 0, s, g.lv[l], om);
         ck(launches);
-        k_restrict<K><<<grid(l + 1), kNT, 0, s>>>(g.lv[l], g.lv[l + 1], om);
+        launch_dep(k_restrict<K>, grid(l + 1), kNT, 0, s, g.lv[l], g.lv[l + 1], om);
         ck(launches);
     }
     launch_bottom(k_bottom16<cluster_blocks(K)>, k_bottom, g, l0, K, emg_entries, s, om);
     ck(launches);
     for (int l = l0 - 1; l >= 0; --l) {
-        k_prolong<K><<<grid(l), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
+        launch_dep(k_prolong<K>, grid(l), kNT, 0, s, g.lv[l], g.lv[l + 1]);
         ck(launches);
-        k_edge_step<K, true><<<grid(l), kNT, 0, s>>>(g.lv[l], om);
+        launch_dep(k_edge_step<K, true>, grid(l), kNT, 0, s, g.lv[l], om);
         ck(launches);
     }
 }
@@ -1007,26 +1024,26 @@ template <int K, bool PRE>
 void node_grids(const EmgDev& g, const float2* b, cudaStream_t s, long long* launches) {
     const int l0 = bottom_level(g);
     auto grid = [&](int l) { return point_grid<K>(g.lv[l], node_planes(g.lv[l])); };
-    k_node_restrict0<K, PRE><<<grid(0), kNT, 0, s>>>(g, f4(b));
+    launch_dep(k_node_restrict0<K, PRE>, grid(0), kNT, 0, s, g, f4(b));
     ck(launches);
     if (g.n_nr_long) {
-        k_node_restrict0_long<K, PRE><<<g.n_nr_long, kLongNT, 0, s>>>(g, f4(b));
+        launch_dep(k_node_restrict0_long<K, PRE>, g.n_nr_long, kLongNT, 0, s, g, f4(b));
         ck(launches);
     }
     for (int l = 0; l < l0; ++l) {
         if (PRE) {
-            k_node_step<K, false><<<grid(l), kNT, 0, s>>>(g.lv[l]);
+            launch_dep(k_node_step<K, false>, grid(l), kNT, 0, s, g.lv[l]);
             ck(launches);
         }
-        k_node_restrict<K, PRE><<<grid(l + 1), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
+        launch_dep(k_node_restrict<K, PRE>, grid(l + 1), kNT, 0, s, g.lv[l], g.lv[l + 1]);
         ck(launches);
     }
     launch_bottom(k_node_bottom16<cluster_blocks(K), PRE>, k_node_bottom<PRE>, g, l0, K, emg_points, s);
     ck(launches);
     for (int l = l0 - 1; l >= 0; --l) {
-        k_node_prolong<K, PRE><<<grid(l), kNT, 0, s>>>(g.lv[l], g.lv[l + 1]);
+        launch_dep(k_node_prolong<K, PRE>, grid(l), kNT, 0, s, g.lv[l], g.lv[l + 1]);
         ck(launches);
-        k_node_step<K, true><<<grid(l), kNT, 0, s>>>(g.lv[l]);
+        launch_dep(k_node_step<K, true>, grid(l), kNT, 0, s, g.lv[l]);
         ck(launches);
     }
 }
@@ -1035,7 +1052,7 @@ template <int K>
 void node_cycle(const EmgDev& g, const GcDev& gc, const float2* r, cudaStream_t s, long long* launches) {
     gc_restrict_edges_k<K>(gc, r, s, launches);
     node_grids<K, false>(g, gc.lv[0].b, s, launches);
-    k_node_prolong0<K><<<grid1((long)gc.nn * (K / 2)), kNT, 0, s>>>(g, gc.nn, nullptr, f4(gc.lv[0].y));
+    launch_dep(k_node_prolong0<K>, grid1((long)gc.nn * (K / 2)), kNT, 0, s, g, gc.nn, nullptr, f4(gc.lv[0].y));
     ck(launches);
     gc_smooth0_k<K>(gc, gc.lv[0].y, gc.out0, s, launches);
 }
@@ -1082,7 +1099,10 @@ void emg_coarse_k(const KrylovCtx<float>& c, const float2* r, float2* z0) {
     edge_cycle<K>(g, om, r, c.stream, c.launches);
     if (c.gc_stream) cudaStreamWaitEvent(c.stream, c.gc_join, 0);
     const long n = (long)c.n_rows_pad * (K / 2);
-    k_combine<K><<<grid1(n), kNT, 0, c.stream>>>(g, gc_row_term(gc, c.B), c.D, om, n, f4(r), f4(z0));
+    if (c.gc_stream)   // behind another stream's kernels: a plain launch
+        k_combine<K><<<grid1(n), kNT, 0, c.stream>>>(g, gc_row_term(gc, c.B), c.D, om, n, f4(r), f4(z0));
+    else
+        launch_dep(k_combine<K>, grid1(n), kNT, 0, c.stream, g, gc_row_term(gc, c.B), c.D, om, n, f4(r), f4(z0));
     ck(c.launches);
     if (c.timer) c.timer->end(th);
 }
@@ -1091,7 +1111,7 @@ template <int K>
 void emg_node_precond_k(const EmgDev& g, const GcDev& gc, float2* z, cudaStream_t s, long long* launches) {
     gc_presmooth0_k<K>(gc, s, launches);   // x = omega D^-1 b, y = b - L x
     node_grids<K, true>(g, gc.lv[0].y, s, launches);
-    k_node_prolong0<K><<<grid1((long)gc.nn * (K / 2)), kNT, 0, s>>>(g, gc.nn, f4(gc.lv[0].x), f4(gc.lv[0].y));
+    launch_dep(k_node_prolong0<K>, grid1((long)gc.nn * (K / 2)), kNT, 0, s, g, gc.nn, f4(gc.lv[0].x), f4(gc.lv[0].y));
     ck(launches);
     gc_smooth0_k<K>(gc, gc.lv[0].y, z, s, launches);
 }

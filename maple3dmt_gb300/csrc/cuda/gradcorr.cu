@@ -281,6 +281,7 @@ __global__ void __launch_bounds__(kGcBlock) k_gc_smooth0(GcDev g, const float2* 
 // x0 = omega D^-1 b0 (pre-smoothing from zero, node-vector input)
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_gc_pre0(GcDev g) {
+    dep_begin();
     const GcLevel& L = g.lv[0];
     const long n = (long)g.nn * K;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
@@ -364,6 +365,7 @@ GcRowTerm gc_row_term(const GcDev& g, const BatchView& B) {
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_gc_restrict_edges2(GcDev g, const float4* __restrict__ in,
                                                                  float4* __restrict__ out) {
+    dep_begin();
     constexpr int H = K / 2;
     const long n = (long)g.nn * H;
     for (long i = (long)blockIdx.x * kGcBlock + threadIdx.x; i < n; i += (long)gridDim.x * kGcBlock) {
@@ -395,8 +397,9 @@ __global__ void __launch_bounds__(kGcBlock) k_gc_restrict_edges2(GcDev g, const 
 // us at K = 16 on 565 k nodes against a thread per right-hand side with the
 // nodes dealt out).
 template <int K, bool RESID>
-__global__ void __launch_bounds__(kGcBlock) k_gc_step0(GcDev g, const float4* __restrict__ b,
-                                                       const float4* __restrict__ t, float4* __restrict__ out) {
+__global__ void __launch_bounds__(kGcBlock) k_gc_step0(GcDev g, const float4* b,
+                                                       const float4* t, float4* __restrict__ out) {
+    dep_begin();
     constexpr int H = K / 2;
     const Range range = block_range(g.nn);
     for (long i = range.b * H + threadIdx.x; i < range.e * H; i += kGcBlock) {
@@ -439,17 +442,17 @@ void gc_restrict_edges_k(const GcDev& g, const float2* in, cudaStream_t s, long 
 
 template <int K>
 void gc_smooth0_k(const GcDev& g, const float2* t, float2* out, cudaStream_t s, long long* launches) {
-    k_gc_step0<K, false><<<range_grid((long)g.nn * (K / 2)), kGcBlock, 0, s>>>(g, as4(g.lv[0].b), as4(t), as4(out));
+    launch_dep(k_gc_step0<K, false>, range_grid((long)g.nn * (K / 2)), kGcBlock, 0, s, g, as4(g.lv[0].b), as4(t), as4(out));
     gc_check(launches);
 }
 
 template <int K>
 void gc_presmooth0_k(const GcDev& g, cudaStream_t s, long long* launches) {
     const int grid = gc_grid((long)g.nn * K);
-    k_gc_pre0<K><<<grid, kGcBlock, 0, s>>>(g);
+    launch_dep(k_gc_pre0<K>, grid, kGcBlock, 0, s, g);
     gc_check(launches);
-    k_gc_step0<K, true><<<range_grid((long)g.nn * (K / 2)), kGcBlock, 0, s>>>(g, as4(g.lv[0].b), as4(g.lv[0].x),
-                                                                            as4(g.lv[0].y));
+    launch_dep(k_gc_step0<K, true>, range_grid((long)g.nn * (K / 2)), kGcBlock, 0, s, g, as4(g.lv[0].b), as4(g.lv[0].x),
+               as4(g.lv[0].y));
     gc_check(launches);
 }
 
@@ -538,6 +541,7 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_norm(int nn, DcWork w, GcDev g
 // r32 = r / rho, x32 = 0
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_dcm_start(int nn, DcWork w, GcDev g) {
+    dep_begin();
     const long n = (long)nn * K;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
         const GcPcgState& T = g.dc_st[i % K];
@@ -561,6 +565,7 @@ __device__ __forceinline__ float4* m4(float2* p) { return reinterpret_cast<float
 // p = z, rz = (r, z) (real: L and the V-cycle are real symmetric)
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_dcm_first(int nn, GcDev g, RedScratch rs) {
+    dep_begin();
     const long n = (long)nn * (K / 2);
     const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long stride = (long)gridDim.x * blockDim.x;
@@ -582,6 +587,7 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_first(int nn, GcDev g, RedScra
 // Ap = L p (FP32, incidence form), (p, Ap) -> alpha
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_dcm_ap(int nn, GcDev g, RedScratch rs) {
+    dep_begin();
     constexpr int H = K / 2;
     const long n = (long)nn * H;
     const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -634,6 +640,7 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_ap(int nn, GcDev g, RedScratch
 // x += alpha p, r -= alpha Ap, |r| <= tol (|b| = 1) or the iteration cap stops
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_dcm_update(int nn, GcDev g, int cap, RedScratch rs) {
+    dep_begin();
     const long n = (long)nn * (K / 2);
     const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long stride = (long)gridDim.x * blockDim.x;
@@ -677,6 +684,7 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_update(int nn, GcDev g, int ca
 // (r, z) -> beta
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_dcm_rz(int nn, GcDev g, RedScratch rs) {
+    dep_begin();
     const long n = (long)nn * (K / 2);
     const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long stride = (long)gridDim.x * blockDim.x;
@@ -705,6 +713,7 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_rz(int nn, GcDev g, RedScratch
 // p = z + beta p
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_dcm_p(int nn, GcDev g) {
+    dep_begin();
     const long n = (long)nn * K;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
         const GcPcgState& T = g.dc_st[i % K];
@@ -824,18 +833,18 @@ long long dc_poisson_mixed_k(const GcDev& g, int nn, DcWork w, RedScratch red, c
         k_dcm_start<K><<<g_n, kGcBlock, 0, s>>>(nn, w, g);
         gc_check(&launches);
         precondition();
-        k_dcm_first<K><<<g_first, kGcBlock, 0, s>>>(nn, g, red);
+        launch_dep(k_dcm_first<K>, g_first, kGcBlock, 0, s, nn, g, red);
         gc_check(&launches);
         for (int it = 0; it < kCap; it += kPoll) {
             for (int j = 0; j < kPoll; ++j) {
-                k_dcm_ap<K><<<g_ap, kGcBlock, 0, s>>>(nn, g, red);
+                launch_dep(k_dcm_ap<K>, g_ap, kGcBlock, 0, s, nn, g, red);
                 gc_check(&launches);
-                k_dcm_update<K><<<g_up, kGcBlock, 0, s>>>(nn, g, kCap, red);
+                launch_dep(k_dcm_update<K>, g_up, kGcBlock, 0, s, nn, g, kCap, red);
                 gc_check(&launches);
                 precondition();
-                k_dcm_rz<K><<<g_rz, kGcBlock, 0, s>>>(nn, g, red);
+                launch_dep(k_dcm_rz<K>, g_rz, kGcBlock, 0, s, nn, g, red);
                 gc_check(&launches);
-                k_dcm_p<K><<<g_n, kGcBlock, 0, s>>>(nn, g);
+                launch_dep(k_dcm_p<K>, g_n, kGcBlock, 0, s, nn, g);
                 gc_check(&launches);
             }
             if (sweeps) *sweeps += kPoll;

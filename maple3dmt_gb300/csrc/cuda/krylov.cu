@@ -445,8 +445,8 @@ template <class R, int LPT> struct alignas(LPT * 2 * sizeof(R)) CVec {
 // 200 us, bound by L2 gathers (13 rows of 64 bytes per row).
 template <class R, int K, int MODE>
 __global__ void __launch_bounds__(SpmvShape<R, K>::NT, 1)
-    k_spmv_st(SegView<R> S, int n_slices, int T, DiagView<R> D, BatchView B, const cplx<R>* __restrict__ x,
-              cplx<R>* __restrict__ y, const cplx<R>* __restrict__ aux, cplx<R>* __restrict__ aux_out, BicgState* st,
+    k_spmv_st(SegView<R> S, int n_slices, int T, DiagView<R> D, BatchView B, const cplx<R>* x,
+              cplx<R>* __restrict__ y, const cplx<R>* aux, cplx<R>* __restrict__ aux_out, BicgState* st,
               RedScratch rs) {
     using C = cplx<R>;
     using Sh = SpmvShape<R, K>;
@@ -763,9 +763,10 @@ template <class R> constexpr int kVecLpt = sizeof(R) == 4 ? 2 : 1;
 
 // p = r (first iteration) or r + beta (p - omega v)   (bicgstab.cpp:60-67)
 template <class R, int K>
-__global__ void __launch_bounds__(kVecNT) k_update_p(long n, const cplx<R>* __restrict__ r_,
-                                                     cplx<R>* __restrict__ p_, const cplx<R>* __restrict__ v_,
-                                                     const BicgState* __restrict__ st) {
+__global__ void __launch_bounds__(kVecNT) k_update_p(long n, const cplx<R>* r_,
+                                                     cplx<R>* __restrict__ p_, const cplx<R>* v_,
+                                                     const BicgState* st) {
+    dep_begin();
     using C = cplx<R>;
     constexpr int LPT = kVecLpt<R>;
     using V = CVec<R, LPT>;
@@ -799,9 +800,10 @@ __global__ void __launch_bounds__(kVecNT) k_update_p(long n, const cplx<R>* __re
 
 // s = r - alpha v, |s|^2   (bicgstab.cpp:89-94)
 template <class R, int K>
-__global__ void __launch_bounds__(kVecNT) k_update_s(long n, const cplx<R>* __restrict__ r_,
-                                                     const cplx<R>* __restrict__ v_, cplx<R>* __restrict__ s_,
+__global__ void __launch_bounds__(kVecNT) k_update_s(long n, const cplx<R>* r_,
+                                                     const cplx<R>* v_, cplx<R>* __restrict__ s_,
                                                      BicgState* st, RedScratch rs) {
+    dep_begin();
     using C = cplx<R>;
     constexpr int LPT = kVecLpt<R>;
     using V = CVec<R, LPT>;
@@ -845,12 +847,13 @@ __global__ void __launch_bounds__(kVecNT) k_update_s(long n, const cplx<R>* __re
 // a (t, t) breakdown take x += alpha p_hat only (:96, :123).
 template <class R, int K>
 __global__ void __launch_bounds__(kVecNT) k_update_xr(long n, cplx<R>* __restrict__ x_, cplx<R>* __restrict__ r_,
-                                                      const cplx<R>* __restrict__ r0_,
-                                                      const cplx<R>* __restrict__ ph_,
-                                                      const cplx<R>* __restrict__ sh_,
-                                                      const cplx<R>* __restrict__ s_,
-                                                      const cplx<R>* __restrict__ t_, BicgState* st,
+                                                      const cplx<R>* r0_,
+                                                      const cplx<R>* ph_,
+                                                      const cplx<R>* sh_,
+                                                      const cplx<R>* s_,
+                                                      const cplx<R>* t_, BicgState* st,
                                                       RedScratch rs) {
+    dep_begin();
     using C = cplx<R>;
     constexpr int LPT = kVecLpt<R>;
     using V = CVec<R, LPT>;
@@ -938,7 +941,13 @@ void spmv_staged_mode(const KrylovCtx<R>& c, const cplx<R>* x, cplx<R>* y, const
     if (smem > 16 * 1024)   // with the reduction's static arrays beyond 48 KB
         cudaFuncSetAttribute(reinterpret_cast<const void*>(kf), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     const int g = std::min(wave_grid(kf, cap, Sh::NT, smem), std::max(1, (ns + T - 1) / T));
-    kf<<<g, Sh::NT, smem, c.stream>>>(c.seg, ns, T, c.D, c.B, x, y, aux, aux_out, st, c.red);
+    // the modes of an iteration: a plain launch (the initial residual's, the
+    // preconditioner's first) lies between them and whatever wrote the matrix
+    if constexpr (MODE == kSpmvAp || MODE == kSpmvAs || MODE == kSpmvSmooth)
+        launch_dep(kf, dim3((unsigned)g), Sh::NT, (size_t)smem, c.stream, c.seg, ns, T, c.D, c.B, x, y, aux, aux_out, st,
+                   c.red);
+    else
+        kf<<<g, Sh::NT, smem, c.stream>>>(c.seg, ns, T, c.D, c.B, x, y, aux, aux_out, st, c.red);
 }
 
 template <class R, int K>
@@ -1108,23 +1117,31 @@ void ssor_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out, 
     }
     if (c.row_kernels == kRowsStaged) {
         constexpr int NT = StagedShape<K>::NT;
+        // one colour's few thousand rows take less time than the way from one
+        // launch to the next: the first launch is a plain one, the others
+        // start early and fetch their matrix slices meanwhile (FP64, 20 k
+        // edges, two right-hand sides, 18 launches: 132 -> 97 us an apply)
+        bool dep = false;
         for (int col = 0; col < nc; ++col) {
             const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
             if (s1 <= s0) continue;
-            launch_staged(k_ssor_fwd_st<R, K>, NT, c.seg.stage_lo, s1 - s0, 1 << 20, c.stream, c.seg,
+            launch_staged(k_ssor_fwd_st<R, K>, NT, c.seg.stage_lo, s1 - s0, 1 << 20, dep, c.stream, c.seg,
                           c.seg.work_col + s0, s1 - s0, c.D, c.B, in, y);
+            dep = true;
             check_launch(c.launches);
         }
         wait_join();
+        dep = dep && !join;   // behind another stream's kernels: a plain launch
         for (int col = nc - 1; col >= 0; --col) {
             const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
             if (s1 <= s0) continue;
             if (gt.ya)
-                launch_staged(k_ssor_bwd_st<R, K, true>, NT, c.seg.stage_up, s1 - s0, 1 << 20, c.stream, c.seg,
+                launch_staged(k_ssor_bwd_st<R, K, true>, NT, c.seg.stage_up, s1 - s0, 1 << 20, dep, c.stream, c.seg,
                               c.seg.work_col + s0, s1 - s0, c.D, c.B, y, out, gt);
             else
-                launch_staged(k_ssor_bwd_st<R, K, false>, NT, c.seg.stage_up, s1 - s0, 1 << 20, c.stream, c.seg,
+                launch_staged(k_ssor_bwd_st<R, K, false>, NT, c.seg.stage_up, s1 - s0, 1 << 20, dep, c.stream, c.seg,
                               c.seg.work_col + s0, s1 - s0, c.D, c.B, y, out, gt);
+            dep = true;
             check_launch(c.launches);
         }
         if (c.timer) c.timer->end(th);
@@ -1194,19 +1211,19 @@ void iteration_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* st) {
     const int gv = c.grid_vec;
     const double vb = (double)c.n_rows * K * sizeof(cplx<R>);
     int th = c.timer ? c.timer->begin(kClsVec, 4 * vb, K) : -1;
-    k_update_p<R, K><<<blocks_for(n / kVecLpt<R>, 2 * kVecNT, gv), kVecNT, 0, c.stream>>>(n, v.r, v.p, v.v, st);
+    launch_dep(k_update_p<R, K>, dim3((unsigned)blocks_for(n / kVecLpt<R>, 2 * kVecNT, gv)), kVecNT, 0, c.stream, n, v.r, v.p, v.v, st);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);
     precond_k<R, K>(c, v.p, v.y, v.ph);
     spmv_k<R, K>(c, kSpmvAp, v.ph, v.v, v.r0, nullptr, st);
     th = c.timer ? c.timer->begin(kClsVec, 3 * vb, K) : -1;
-    k_update_s<R, K><<<reduce_grid(k_update_s<R, K>, gv, n / kVecLpt<R>, kVecNT), kVecNT, 0, c.stream>>>(n, v.r, v.v, v.s, st, c.red);
+    launch_dep(k_update_s<R, K>, dim3((unsigned)reduce_grid(k_update_s<R, K>, gv, n / kVecLpt<R>, kVecNT)), kVecNT, 0, c.stream, n, v.r, v.v, v.s, st, c.red);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);
     precond_k<R, K>(c, v.s, v.y, v.sh);
     spmv_k<R, K>(c, kSpmvAs, v.sh, v.t, v.s, nullptr, st);
     th = c.timer ? c.timer->begin(kClsVec, 8 * vb, K) : -1;
-    k_update_xr<R, K><<<reduce_grid(k_update_xr<R, K>, gv, n / kVecLpt<R>, kVecNT), kVecNT, 0, c.stream>>>(n, v.x, v.r, v.r0, v.ph, v.sh, v.s, v.t, st, c.red);
+    launch_dep(k_update_xr<R, K>, dim3((unsigned)reduce_grid(k_update_xr<R, K>, gv, n / kVecLpt<R>, kVecNT)), kVecNT, 0, c.stream, n, v.x, v.r, v.r0, v.ph, v.sh, v.s, v.t, st, c.red);
     check_launch(c.launches);
     if (c.timer) c.timer->end(th);
 }
@@ -1507,7 +1524,7 @@ void eis_init_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* st) {
     for (int col = 0; col < nc; ++col) {
         const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
         if (s1 <= s0) continue;
-        launch_staged(k_ssor_fwd_st<R, K>, NT, c.seg.stage_lo, s1 - s0, 1 << 20, c.stream, c.seg,
+        launch_staged(k_ssor_fwd_st<R, K>, NT, c.seg.stage_lo, s1 - s0, 1 << 20, false, c.stream, c.seg,
                       c.seg.work_col + s0, s1 - s0, c.D, c.B, (const cplx<R>*)v.b, v.y);
         check_launch(c.launches);
     }
@@ -1545,7 +1562,7 @@ void eis_finish_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, cplx<R>* out) {
     for (int col = nc - 1; col >= 0; --col) {
         const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
         if (s1 <= s0) continue;
-        launch_staged(k_eis_bwd_st<R, K, 0>, NT, c.seg.stage_up, s1 - s0, 1 << 20, c.stream, c.seg,
+        launch_staged(k_eis_bwd_st<R, K, 0>, NT, c.seg.stage_up, s1 - s0, 1 << 20, false, c.stream, c.seg,
                       c.seg.work_col + s0, s1 - s0, c.D, c.B, (const cplx<R>*)v.x, (cplx<R>*)nullptr,
                       (const cplx<R>*)nullptr, (const cplx<R>*)nullptr, (const BicgState*)nullptr, out,
                       (double2*)nullptr);

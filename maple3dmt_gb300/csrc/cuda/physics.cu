@@ -686,7 +686,7 @@ long long mg_apply(const MeshDev& m, DcWork w, const AmgDev& A, RedScratch red, 
     k_mg_pre<K><<<grid((long)m.nn * K), kBlock, 0, s>>>(L0, w.r, L0.x, A.omega, w.st);
     ++launches;
     if (nl > 1) {
-        launch_staged(k_mg0_resid_st<K>, StagedShape<K>::NT, w.lap_stage, w.n_node_slices, 1 << 20, s, m.nn, w,
+        launch_staged(k_mg0_resid_st<K>, StagedShape<K>::NT, w.lap_stage, w.n_node_slices, 1 << 20, false, s, m.nn, w,
                       (const double2*)w.r, (const double2*)L0.x, L0.r);
         k_mg_restrict<K><<<grid((long)A.lv[1].n * K), kBlock, 0, s>>>(L0, A.lv[1].n, L0.r, A.lv[1].b, w.st);
         launches += 2;
@@ -715,7 +715,7 @@ long long mg_apply(const MeshDev& m, DcWork w, const AmgDev& A, RedScratch red, 
         k_mg_prolong<K><<<grid((long)m.nn * K), kBlock, 0, s>>>(L0, x1, L0.x, w.st);
         ++launches;
     }
-    launch_staged(k_mg0_post_st<K>, StagedShape<K>::NT, w.lap_stage, w.n_node_slices, cap, s, m.nn, w, L0.dinv,
+    launch_staged(k_mg0_post_st<K>, StagedShape<K>::NT, w.lap_stage, w.n_node_slices, cap, false, s, m.nn, w, L0.dinv,
                   A.omega, (const double2*)L0.x, red);
     ++launches;
     return launches;
@@ -1246,7 +1246,7 @@ long long divcorr_k(const MeshDev& m, const double* me_dc, VecK E, bool use_phi0
         for (; it < cg_max;) {
             const int n_it = (cg_max - it) < chunk ? (cg_max - it) : chunk;
             for (int j = 0; j < n_it; ++j) {
-                launch_staged(k_dc_cg_ap_st<K>, StagedShape<K>::NT, w.lap_stage, w.n_node_slices, cap, s, m.nn,
+                launch_staged(k_dc_cg_ap_st<K>, StagedShape<K>::NT, w.lap_stage, w.n_node_slices, cap, false, s, m.nn,
                               w, red);
                 if (amg) {
                     k_mg_cg_update<K><<<g_up, kBlock, 0, s>>>(m.nn, cg_max, w, red);

@@ -189,6 +189,7 @@ __device__ __forceinline__ void slice_pipeline(const unsigned char* __restrict__
         fence_mbar_init();
         no_wait = (*reinterpret_cast<volatile unsigned*>(err) & kTestConsumeNoWait) != 0;
     }
+    dep_trigger();
     __syncthreads();
     auto issue = [&](long i, int stg) {   // thread 0 only
         const int4 w = __ldg(&work[i]);
@@ -220,10 +221,12 @@ __device__ __forceinline__ void slice_pipeline(const unsigned char* __restrict__
     };
     long i = blockIdx.x;
     if (i >= n_items) {   // uniform: the whole block has no item
+        dep_wait();
         finish();
         return;
     }
-    if (threadIdx.x == 0) issue(i, 0);
+    if (threadIdx.x == 0) issue(i, 0);   // the matrix: nothing of a sweep's chain writes it
+    dep_wait();
     // outcome of the wait for the item about to be consumed, block-uniform
     bool fail = __syncthreads_or(!wait_stage(0, 0u)) != 0;
     int k = 0;
@@ -285,6 +288,7 @@ __device__ __forceinline__ void tile_ring(const unsigned char* __restrict__ seg,
         }
         fence_mbar_init();
     }
+    dep_trigger();
     __syncthreads();
     const long n_tiles = (n_slices + T - 1) / T;
     const int t0 = (int)(n_tiles * blockIdx.x / gridDim.x), t1 = (int)(n_tiles * (blockIdx.x + 1) / gridDim.x);
@@ -307,7 +311,9 @@ __device__ __forceinline__ void tile_ring(const unsigned char* __restrict__ seg,
             for (int k = issued > RING ? issued - RING : 0; k < issued; ++k)
                 mbar_wait_bounded(&full[k % RING], (unsigned)(k / RING) & 1u);
         }
+        dep_wait();
     } else {
+        dep_wait();   // the copies of the first tiles are on their way
         const bool no_wait = (*reinterpret_cast<volatile unsigned*>(err) & kTestConsumeNoWait) != 0;
         bool dead = false;
         for (int t = t0, k = 0; t < t1; ++t, ++k) {
@@ -453,13 +459,16 @@ template <class R, int K> struct StagedMinBlocks {
 // Launches one staged kernel: at most one resident wave of blocks (of
 // StagedShape<K>::NT threads with two stages of dynamic shared memory), no
 // more than there are work items, no more than `cap`.
+// dep: a dependent launch (launch_dep).
 template <class F, class... Args>
-inline void launch_staged(F* kernel, int nt, int stage_bytes, long items, int cap, cudaStream_t st, Args... args) {
+inline void launch_staged(F* kernel, int nt, int stage_bytes, long items, int cap, bool dep, cudaStream_t st,
+                          Args... args) {
     const int smem = 2 * stage_bytes;
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     long g = std::min<long>((long)wave_grid(kernel, cap, nt, smem), std::max<long>(items, 1));
-    kernel<<<(int)g, nt, smem, st>>>(args...);
+    if (dep) launch_dep(kernel, dim3((unsigned)g), nt, (size_t)smem, st, args...);
+    else kernel<<<(int)g, nt, smem, st>>>(args...);
 }
 
 }  // namespace dev

@@ -67,3 +67,22 @@ def test_multigrid_needs_fewer_iterations(lib):
         it[relax] = s.stats()["total_iterations"]
     assert 2 * it[1.0] < it[1.0001], it
     assert rel(Z[1.0], Z[1.0001]) < TOL
+
+
+@pytest.mark.parametrize("precision,lo,hi,nf", [(0, 3, 5, 1), (1, 3, 5, 1), (1, 5, 6, 3), (1, 2, 6, 3)])
+def test_dependent_launches_give_the_same_bits(lib, precision, lo, hi, nf):
+    """Replayed graphs hold plain launches, everything else dependent ones
+    that start while their predecessor runs: a value read before it was
+    written would change the iteration, so all bits agree, run after run.
+    (2, 6) runs SSOR in mixed precision."""
+    from maple3dmt_gb300.solver import solver_for_survey
+    sv = _survey(lo, hi, np.logspace(-1, 2, 3)[:nf])
+    ref = None
+    for graphs in (1, 0, 0, 0):
+        s = solver_for_survey(sv, bicgstab_tol=1e-10, bicgstab_maxiter=5000, precision=precision, cuda_graphs=graphs)
+        got = s.forward_batch(sv.freqs, with_fields=True)
+        s.close()
+        if ref is None:
+            ref = got
+        for a, b in zip(got, ref):
+            assert np.array_equal(a, b)
