@@ -107,8 +107,8 @@ template <> struct Sum<float> {
 // the predecessor ends, and dep_wait() returns then, with all of the
 // predecessor's writes visible.  The small grids' and the small meshes'
 // kernels run for 5-30 us, of which the way from one launch to the next was 1
-// to 2: the all-frequency solve of 58 k edges and eight right-hand sides 40.5
-// -> 35.8 ms, one frequency of 20 k edges 11.2 -> 9.4 ms.  Rules:
+// to 2: three frequencies and gradient on 149 k edges 40.5 -> 35.8 ms, one
+// frequency on 13 k edges 11.2 -> 9.4 ms.  Rules:
 //  * a kernel launched so calls dep_wait() before its first access to anything
 //    that a kernel of the chain writes, and every block calls it;
 //  * such data is not read through `const __restrict__` pointers or __ldg (the

@@ -1119,8 +1119,10 @@ void ssor_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out, 
         constexpr int NT = StagedShape<K>::NT;
         // one colour's few thousand rows take less time than the way from one
         // launch to the next: the first launch is a plain one, the others
-        // start early and fetch their matrix slices meanwhile (FP64, 20 k
-        // edges, two right-hand sides, 18 launches: 132 -> 97 us an apply)
+        // start early and fetch their matrix slices meanwhile (FP64, 2.8 k
+        // edges, two right-hand sides, 18 launches: 132 -> 97 us an apply; one
+        // cluster for a whole apply, a cluster barrier between the colours, took
+        // 110 us: its eight SMs do not have the FP64 lanes)
         bool dep = false;
         for (int col = 0; col < nc; ++col) {
             const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
