@@ -181,76 +181,12 @@ struct RedScratch {
     int max_blocks;
 };
 
-// Sums, over the grid, NQ complex quantities for each of K right-hand sides.
-// `acc[kt][q]` is this thread's contribution for right-hand side rhs0 + kt.
-// Lanes are combined through shared memory in lane order, warps in warp
-// order and blocks in block order by the last block to arrive, so the result
-// is deterministic for a fixed launch shape.  Returns true in the last block;
-// then `out[q * K + k]` (shared memory, NQ*K entries) holds the totals.
-template <int NQ, int K, int KT>
-__device__ bool grid_reduce(const double2 (&acc)[KT][NQ], int rhs0, RedScratch rs, double2* out) {
-    __shared__ double2 sm[kWarpsPerBlock][NQ][K];
-    __shared__ bool am_last;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < kWarpsPerBlock * NQ * K; i += blockDim.x)
-        (&sm[0][0][0])[i] = make_double2(0.0, 0.0);
-    __syncthreads();
-    for (int l = 0; l < 32; ++l) {
-        if (lane == l) {
-#pragma unroll
-            for (int kt = 0; kt < KT; ++kt)
-#pragma unroll
-                for (int q = 0; q < NQ; ++q)
-                    sm[warp][q][rhs0 + kt] = cadd(sm[warp][q][rhs0 + kt], acc[kt][q]);
-        }
-        __syncwarp();
-    }
-    __syncthreads();
-    if (threadIdx.x < NQ * K) {
-        const int q = threadIdx.x / K, k = threadIdx.x % K;
-        double2 s = make_double2(0.0, 0.0);
-        for (int w = 0; w < kWarpsPerBlock; ++w) s = cadd(s, sm[w][q][k]);
-        __stcg(&rs.partial[(size_t)blockIdx.x * (NQ * K) + threadIdx.x], s);
-        __threadfence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned t = atomicAdd(rs.counter, 1u);
-        am_last = (t == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!am_last) return false;
-    __threadfence();
-    // Last block: for each of the NQ*K totals, thread t sums blocks t, t+256, ...
-    // then a fixed-shape tree over the 256 threads; deterministic and short.
-    __shared__ double2 red[kBlock];
-    for (int qk = 0; qk < NQ * K; ++qk) {
-        double2 s = make_double2(0.0, 0.0);
-        for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
-            s = cadd(s, __ldcg(&rs.partial[(size_t)b * (NQ * K) + qk]));
-        red[threadIdx.x] = s;
-        __syncthreads();
-        for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-            if ((int)threadIdx.x < w) red[threadIdx.x] = cadd(red[threadIdx.x], red[threadIdx.x + w]);
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) {
-            out[qk] = red[0];
-            rs.final_[qk] = red[0];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *rs.counter = 0u;
-    __syncthreads();
-    return true;
-}
-
 // Grid reduction for kernels whose lane l always works on the same right-hand
 // sides: LPT neighbouring ones per thread, LPT (l % (K / LPT)) and the next
 // (K and LPT powers of two, whole warps); acc[j][q] is quantity q of the j-th
 // of them in the kernel's working precision.  Shuffle trees over the lanes that
-// share a right-hand side, then over the block's warps (one warp per total),
-// then, in the last block to arrive, over the blocks: every step in a fixed
+// share a right-hand side, then over the block's warps, then, in the last block
+// to arrive, over the blocks, all totals side by side: every step in a fixed
 // order, so the result is deterministic for a fixed launch shape.  Returns true
 // in the last block, where out[q * K + k] (shared, NQ*K entries) holds the
 // totals.
@@ -276,11 +212,16 @@ __device__ bool grid_reduce_sums(const S (&acc)[LPT][NQ], RedScratch rs, double2
     __syncthreads();
     S zero{};
     S* partial = reinterpret_cast<S*>(rs.partial);
-    for (int p = warp; p < PK; p += NW) {
-        S s = lane < NW ? sm[lane][p] : zero;
+    // GW lanes per total, one for each warp of the block
+    constexpr int GW = NW <= 1 ? 1 : NW <= 2 ? 2 : NW <= 4 ? 4 : NW <= 8 ? 8 : NW <= 16 ? 16 : 32;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) s.add(s.xor_lane(off));
-        if (lane == 0) {
+    for (int p0 = 0; p0 < PK; p0 += NT / GW) {
+        const int p = p0 + threadIdx.x / GW, w = threadIdx.x % GW;
+        if (p0 + warp * (32 / GW) >= PK) break;   // idle warps would add zeros, 16 cycles an FP64 add
+        S s = w < NW && p < PK ? sm[w][p] : zero;
+#pragma unroll
+        for (int off = GW / 2; off > 0; off >>= 1) s.add(s.xor_lane(off));
+        if (w == 0 && p < PK) {
             __stcg(reinterpret_cast<double2*>(&partial[(size_t)blockIdx.x * PK + p]), *reinterpret_cast<double2*>(&s));
             __threadfence();
         }
@@ -293,21 +234,26 @@ __device__ bool grid_reduce_sums(const S (&acc)[LPT][NQ], RedScratch rs, double2
     __syncthreads();
     if (!am_last) return false;
     __threadfence();
-    for (int p = warp; p < PK; p += NW) {
+    // TPT lanes per total, every total at once
+    constexpr int Q = NT / PK;
+    constexpr int TPT = Q >= 32 ? 32 : Q >= 16 ? 16 : Q >= 8 ? 8 : Q >= 4 ? 4 : Q >= 2 ? 2 : 1;
+    static_assert(Q >= 1, "a thread per total");
+    const int p = threadIdx.x / TPT, l = threadIdx.x % TPT;
+    if (warp * (32 / TPT) < PK) {
         S s = zero;
-        for (int b = lane; b < (int)gridDim.x; b += 4 * 32) {   // four loads in flight
+        for (int b = l; p < PK && b < (int)gridDim.x; b += 4 * TPT) {   // four loads in flight
             double2 v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                v[u] = b + 32 * u < (int)gridDim.x
-                           ? __ldcg(reinterpret_cast<const double2*>(&partial[(size_t)(b + 32 * u) * PK + p]))
+                v[u] = b + TPT * u < (int)gridDim.x
+                           ? __ldcg(reinterpret_cast<const double2*>(&partial[(size_t)(b + TPT * u) * PK + p]))
                            : make_double2(0.0, 0.0);
 #pragma unroll
             for (int u = 0; u < 4; ++u) s.add(*reinterpret_cast<const S*>(&v[u]));
         }
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) s.add(s.xor_lane(off));
-        if (lane == 0) {
+        for (int off = TPT / 2; off > 0; off >>= 1) s.add(s.xor_lane(off));
+        if (l == 0 && p < PK) {
             const double2 t = s.get();
             out[p] = t;
             rs.final_[p] = t;

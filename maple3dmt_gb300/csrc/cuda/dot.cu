@@ -11,7 +11,7 @@ namespace {
 // right-hand side l % K, which is what grid_reduce_lanes expects.  Bound by the
 // FP64 units (2 per clock and SM: four fused multiply-adds a pair take 187 us
 // for 27 M pairs, the loads 129 us): four FMAs a pair instead of products and
-// adds apart (six instructions), eight loads in flight.
+// adds apart (six instructions), eight loads in flight: 336 -> 201 us.
 __device__ __forceinline__ void dot_add(double2& s, double2 a, double2 b) {
     s.x = fma(a.x, b.x, fma(a.y, b.y, s.x));
     s.y = fma(a.x, b.y, fma(-a.y, b.x, s.y));
@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(kBlock) k_dot_batched(const double2* __restric
                                                         const double2* __restrict__ y, long long n,
                                                         RedScratch rs, double2* __restrict__ out) {
     __shared__ double2 tot[K];
-    double2 acc[1] = {make_double2(0.0, 0.0)};
+    double2 part[4] = {};   // one running sum per load in flight: short chains, small errors
     const long long total = n * K;
     const long long stride = (long long)gridDim.x * blockDim.x;
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -34,9 +34,13 @@ __global__ void __launch_bounds__(kBlock) k_dot_batched(const double2* __restric
             b[u] = __ldg(y + t + u * stride);
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) dot_add(acc[0], a[u], b[u]);
+        for (int u = 0; u < 4; ++u) dot_add(part[u], a[u], b[u]);
     }
-    for (; t < total; t += stride) dot_add(acc[0], __ldg(x + t), __ldg(y + t));
+    for (int u = 0; t < total; t += stride, ++u) {   // three at most
+        const double2 a = __ldg(x + t), b = __ldg(y + t);
+        dot_add(u == 0 ? part[0] : u == 1 ? part[1] : part[2], a, b);
+    }
+    double2 acc[1] = {cadd(cadd(part[0], part[1]), cadd(part[2], part[3]))};
     if (grid_reduce_lanes<1, K>(acc, rs, tot) && threadIdx.x < K) out[threadIdx.x] = tot[threadIdx.x];
 }
 
@@ -44,9 +48,13 @@ __global__ void __launch_bounds__(kBlock) k_dot_batched(const double2* __restric
 
 int dot_blocks(long long n, int K, int cap) {
     const long long work = n * (long long)K;
-    long long b = (work + kBlock - 1) / kBlock;
+    // two pairs a thread at least, two blocks on each of 152 SMs at most: four
+    // chains a thread keep the FP64 units busy, and every further block is one
+    // more partial for the last one to sum (27 M pairs: 289 us with 152 blocks,
+    // 205 with 304, 217 with 456, 227 with 912; 1 M pairs: 30, 32, 35, 50)
+    long long b = (work + 2 * kBlock - 1) / (2 * kBlock);
     if (b < 1) b = 1;
-    if (b > 912) b = 912;   // six blocks on each of 152 SMs, no uneven last one
+    if (b > 304) b = 304;
     if (b > cap) b = cap;
     return (int)b;
 }
