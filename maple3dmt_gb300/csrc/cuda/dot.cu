@@ -48,11 +48,12 @@ __global__ void __launch_bounds__(kBlock) k_dot_batched(const double2* __restric
 
 int dot_blocks(long long n, int K, int cap) {
     const long long work = n * (long long)K;
-    // two pairs a thread at least, two blocks on each of 152 SMs at most: four
-    // chains a thread keep the FP64 units busy, and every further block is one
-    // more partial for the last one to sum (27 M pairs: 289 us with 152 blocks,
-    // 205 with 304, 217 with 456, 227 with 912; 1 M pairs: 30, 32, 35, 50)
-    long long b = (work + 2 * kBlock - 1) / (2 * kBlock);
+    // two pairs a thread beyond 64 blocks, two blocks on each of 152 SMs at most:
+    // four chains a thread keep the FP64 units busy, and every further block is
+    // one more partial for the last one to sum (27 M pairs: 289 us with 152
+    // blocks, 205 with 304, 217 with 456, 227 with 912; 1 M pairs: 30, 32, 35, 50)
+    const long long one = (work + kBlock - 1) / kBlock, two = (work + 2 * kBlock - 1) / (2 * kBlock);
+    long long b = one < 64 ? one : two < 64 ? 64 : two;
     if (b < 1) b = 1;
     if (b > 304) b = 304;
     if (b > cap) b = cap;
