@@ -157,8 +157,9 @@ typedef struct m3d_params {
                                  edges, so a sweep's gathers stay in L2; 0: colour order over the mesh */
     int coop_sweep;           /* 1: each staged SSOR sweep is one cooperative launch over all its groups
                                  (bounded grid barriers between groups); 0: one launch per group */
-    int cuda_graphs;          /* 1: the mixed-precision inner solve captures its 10-iteration chunk (every
-                                 launch of ten BiCGStab iterations, both streams) in a CUDA graph once per
+    int cuda_graphs;          /* 1: the mixed-precision inner solve captures its chunk (every
+                                 launch of ten BiCGStab iterations, two with the multigrid
+                                 preconditioner, both streams) in a CUDA graph once per
                                  batch shape and refinement step, from the shape's third chunk on, and
                                  replays it; 0 (default): launches issued one by one (measured as fast on
                                  C2 and faster with several meshes at once) */

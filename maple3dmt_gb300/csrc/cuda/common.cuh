@@ -108,7 +108,7 @@ template <> struct Sum<float> {
 // predecessor's writes visible.  The small grids' and the small meshes'
 // kernels run for 5-30 us, of which the way from one launch to the next was 1
 // to 2: three frequencies and gradient on 149 k edges 40.5 -> 35.8 ms, one
-// frequency on 13 k edges 11.2 -> 9.4 ms.  Rules:
+// frequency on 17 k edges 11.2 -> 9.4 ms.  Rules:
 //  * a kernel launched so calls dep_wait() before its first access to anything
 //    that a kernel of the chain writes, and every block calls it;
 //  * such data is not read through `const __restrict__` pointers or __ldg (the

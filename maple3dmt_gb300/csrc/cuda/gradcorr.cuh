@@ -23,6 +23,10 @@
 // and the FP64 true-residual test are unchanged; only the iteration count
 // drops (at 0.01 Hz about five-fold on the 1.7 M-edge mesh).
 //
+// Where the mesh allows the geometric preconditioner (edgemg.cuh), its node
+// cycle takes this V-cycle's place, here and in the divergence-correction PCG;
+// what follows describes the aggregation cycle of the other meshes.
+//
 // The V-cycle (V(0,1) by default: post-smoothing only) runs in FP32 on
 // [n][K] complex node vectors.  Level 0 is read from a packed FP32 copy of the
 // divergence-correction Laplacian's incidence lists (gc_pack_level0, redone

@@ -5,6 +5,8 @@
 // dots include/maple3dmt/forward/bicgstab.h:68-73) and
 // SSORPreconditioner::apply (include/maple3dmt/forward/ssor.h:53-78, omega = 1)
 // for K right-hand sides at once.  Differences from the reference, by design:
+//  * The complex-FP32 inner solve is preconditioned by geometric multigrid
+//    (edgemg.cuh) where the mesh allows it; SSOR serves FP64 and the rest.
 //  * Gauss-Seidel order is colour by colour (a graph colouring of A), so each
 //    sweep is one parallel launch per colour instead of a serial loop; within
 //    a colour the original edge order is kept.  This is SSOR on the colour-

@@ -417,10 +417,11 @@ constexpr int wgrad_smem(int W) { return kWgradStages * wgrad_stage(W) + 1024; }
 //   warp 5           allocates 128 TMEM columns; lane 0 issues the MMAs;
 //   warps 0-3        sum the gradient rows per channel in two-float arithmetic
 //                    (blockIdx.y = 1 only), at the end store the accumulators.
-// Bound by the copies from L2 (45 KB a tile and shift at W = 32).  The former
-// path gathered 27 shifted, transposed copies of the input (226 MB a layer for
-// 131 k voxels, 72 us), transposed the gradient (5 us), multiplied (52 us) and
-// summed the biases with one warp in FP64 (21 + 338 us).
+// Bound by the MMAs themselves (some 70 cycles each at N = 32; L2 at 38 % of its
+// rate, DRAM at 9 %): 22 us for 131 k voxels.  The former path gathered 27
+// shifted, transposed copies of the input (226 MB a layer, 72 us), transposed
+// the gradient (5 us), multiplied (52 us) and summed the biases with one warp
+// in FP64 (21 + 338 us).
 // Every wait is bounded; a timeout flags an error and every role stops.
 __global__ void __launch_bounds__(192) k_wgrad_tc(const __grid_constant__ CUtensorMap hmap,
                                                   const __grid_constant__ CUtensorMap dmap, WgradArgs a) {
