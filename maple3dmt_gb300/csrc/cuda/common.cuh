@@ -152,6 +152,12 @@ inline void launch_dep(void (*kernel)(P...), dim3 grid, int block, size_t smem, 
 // SM count); cached per (device, kernel, threads, smem).
 int resident_blocks(const void* kernel, int threads = kBlock, int smem = 0);
 
+// Lets `kernel` be launched with any dynamic shared memory the device has: the
+// limit is set to the most there is, once per (device, kernel).  It belongs to
+// the function, not to the launch: set to each launch's own size, a second
+// solver's thread could lower it between this one's call and its launch.
+void lift_smem_limit(const void* kernel);
+
 // One resident wave of `kernel`, at most `cap` blocks.
 template <class F>
 inline int wave_grid(F* kernel, int cap, int threads = kBlock, int smem = 0) {

@@ -972,7 +972,7 @@ void launch_bottom(F16* k16, F8* k8, const EmgDev& g, int l0, int K, long (*per)
     int smem = 0;
     for (int l = l0 + (big ? 1 : 0); l < g.n_levels; ++l) smem += 3 * (int)(per(g.lv[l].n) * sizeof(float2));
     const void* f = big ? reinterpret_cast<const void*>(k16) : reinterpret_cast<const void*>(k8);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (smem > 16 * 1024) lift_smem_limit(f);   // with the static arrays beyond 48 KB
     if (!big) {
         launch_dep(k8, K, kBottomNT, (size_t)smem, s, g, l0, args...);
         return;

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <set>
 #include <stdexcept>
 #include <string>
 #include <tuple>
@@ -16,6 +17,23 @@
 namespace m3d {
 
 namespace dev {
+
+void lift_smem_limit(const void* kernel) {
+    static std::mutex mu;
+    static std::set<std::pair<int, const void*>> done;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    if (done.count({dev, kernel})) return;
+    cudaFuncAttributes fa{};
+    int most = 0;
+    if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes) !=
+            cudaSuccess)
+        return;   // the launch reports it
+    done.insert({dev, kernel});
+}
 
 int resident_blocks(const void* kernel, int threads, int smem) {
     static std::mutex mu;
@@ -940,7 +958,7 @@ void spmv_staged_mode(const KrylovCtx<R>& c, const cplx<R>* x, cplx<R>* y, const
     auto kf = k_spmv_st<R, K, MODE>;
     const int smem = Sh::RING * c.seg.stage_row[T];
     if (smem > 16 * 1024)   // with the reduction's static arrays beyond 48 KB
-        cudaFuncSetAttribute(reinterpret_cast<const void*>(kf), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        lift_smem_limit(reinterpret_cast<const void*>(kf));
     const int g = std::min(wave_grid(kf, cap, Sh::NT, smem), std::max(1, (ns + T - 1) / T));
     // the modes of an iteration: a plain launch (the initial residual's, the
     // preconditioner's first) lies between them and whatever wrote the matrix
@@ -1041,7 +1059,7 @@ __global__ void __launch_bounds__(kBlock) k_add_gc_term(long n, cplx<R>* __restr
 // occupancy of the kernel at this shared memory on every SM), less a quarter
 // when another stream's kernels should run beside it.
 inline int coop_grid(const void* kernel, int nt, int smem, bool share) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (smem > 48 * 1024) lift_smem_limit(kernel);
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1473,8 +1491,7 @@ __global__ void __launch_bounds__(kBlock) k_eis_init(long n, DiagView<R> D, Batc
 template <class F>
 int staged_grid(F* kernel, int nt, int stage_bytes, long items, int cap) {
     const int smem = 2 * stage_bytes;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (smem > 48 * 1024) lift_smem_limit(reinterpret_cast<const void*>(kernel));
     return (int)std::min<long>((long)wave_grid(kernel, cap, nt, smem), std::max<long>(items, 1));
 }
 

@@ -464,8 +464,7 @@ template <class F, class... Args>
 inline void launch_staged(F* kernel, int nt, int stage_bytes, long items, int cap, bool dep, cudaStream_t st,
                           Args... args) {
     const int smem = 2 * stage_bytes;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (smem > 48 * 1024) lift_smem_limit(reinterpret_cast<const void*>(kernel));
     long g = std::min<long>((long)wave_grid(kernel, cap, nt, smem), std::max<long>(items, 1));
     if (dep) launch_dep(kernel, dim3((unsigned)g), nt, (size_t)smem, st, args...);
     else kernel<<<(int)g, nt, smem, st>>>(args...);

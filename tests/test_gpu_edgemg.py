@@ -86,3 +86,20 @@ def test_dependent_launches_give_the_same_bits(lib, precision, lo, hi, nf):
             ref = got
         for a, b in zip(got, ref):
             assert np.array_equal(a, b)
+
+
+def test_solvers_of_different_meshes_at_once(lib):
+    """Four handles, four threads: each mesh and batch width launches the same
+    kernels with its own amount of shared memory, and each solve gives the
+    bits that it gives alone."""
+    from concurrent.futures import ThreadPoolExecutor
+    from maple3dmt_gb300.solver import solver_for_survey
+    freqs = np.logspace(-1, 2, 5)
+    surveys = [_survey(*l, freqs[:n]) for l, n in (((3, 5), 1), ((4, 5), 5), ((5, 6), 3), ((2, 4), 4))]
+    solvers = [solver_for_survey(sv, bicgstab_tol=1e-8, bicgstab_maxiter=5000, precision=1) for sv in surveys]
+    run = lambda k: solvers[k].forward_batch(surveys[k].freqs)
+    want = [run(k) for k in range(4)]
+    with ThreadPoolExecutor(4) as pool:
+        for got in pool.map(lambda k: [run(k) for _ in range(25)] + [k], range(4)):
+            for z in got[:-1]:
+                assert np.array_equal(z, want[got[-1]])
