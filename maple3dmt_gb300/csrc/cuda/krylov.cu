@@ -732,11 +732,11 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
 
 // Whole sweeps in one cooperative launch: the sweep groups (colours, or
 // (super-block, colour) pairs) one after another, a grid barrier between
-// groups in place of a kernel boundary.  gptr: device copy of the groups'
+// groups in place of a kernel boundary.  grange: device copy of the groups'
 // slice ranges; bar: the barrier's counter and generation.
 template <class R, int K>
 __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) k_ssor_fwd_coop(
-    SegView<R> S, const int4* __restrict__ work, const int* __restrict__ gptr, int n_groups, DiagView<R> D,
+    SegView<R> S, const int4* __restrict__ work, const int2* __restrict__ grange, int n_groups, DiagView<R> D,
     BatchView B, const cplx<R>* __restrict__ in, cplx<R>* y, unsigned* bar) {
     constexpr int RPW = Rpw<K>::v;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -745,7 +745,7 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
     const R om = (R)B.omega[rhs];
     for (int g = 0; g < n_groups; ++g) {
         if (g > 0) grid_barrier(bar, bar + 1, S.err);
-        const int s0 = gptr[g], s1 = gptr[g + 1];
+        const int s0 = grange[g].x, s1 = grange[g].y;
         slice_pipeline<1>(S.seg, work + s0, s1 - s0, S.stage_lo, S.err,
                           [&](const SegItem& it, const unsigned char* base) {
                               ssor_fwd_rows<R, K>(it, base, S.rows, D, om, (R)B.relax, rhs, lr0, in, y);
@@ -755,7 +755,7 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
 
 template <class R, int K, bool GC>
 __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) k_ssor_bwd_coop(
-    SegView<R> S, const int4* __restrict__ work, const int* __restrict__ gptr, int n_groups, DiagView<R> D,
+    SegView<R> S, const int4* __restrict__ work, const int2* __restrict__ grange, int n_groups, DiagView<R> D,
     BatchView B, cplx<R>* y, cplx<R>* out, GcRowTerm gt, unsigned* bar) {
     constexpr int RPW = Rpw<K>::v;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -764,7 +764,7 @@ __global__ void __launch_bounds__(StagedShape<K>::NT, StagedMinBlocks<R, K>::v) 
     const R om = (R)B.omega[rhs];
     for (int g = n_groups - 1; g >= 0; --g) {
         if (g < n_groups - 1) grid_barrier(bar, bar + 1, S.err);
-        const int s0 = gptr[g], s1 = gptr[g + 1];
+        const int s0 = grange[g].x, s1 = grange[g].y;
         slice_pipeline<2>(S.seg, work + s0, s1 - s0, S.stage_up, S.err,
                           [&](const SegItem& it, const unsigned char* base) {
                               ssor_bwd_rows<R, K, GC>(it, base, S.rows, D, om, (R)B.relax, rhs, lr0, y, out, gt);
@@ -1079,7 +1079,7 @@ inline void cuda_check_launch(cudaError_t e, long long* launches) {
 template <class R, int K>
 void ssor_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out, const GcRowTerm& gt = GcRowTerm{}) {
     constexpr int G = kSlice / Rpw<K>::v;   // row-group tasks per slice
-    const int nc = (int)c.colour_ptr.size() - 1;
+    const int nc = (int)c.sweep_range.size();
     // whole apply: matrix once (lower forward, upper backward), vectors in,
     // y (written, read back), out; with the gradient-space term y written
     // back once more and two node indices and weights per row
@@ -1096,7 +1096,7 @@ void ssor_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out, 
         cudaStreamWaitEvent(c.stream, c.gc_join, 0);
         th = c.timer ? c.timer->begin(kClsSsor, 0.0, K) : -1;
     };
-    if (c.row_kernels == kRowsStaged && c.coop && c.colour_ptr_d && c.gridbar && nc > 1) {
+    if (c.row_kernels == kRowsStaged && c.coop && c.sweep_range_d && c.gridbar && nc > 1) {
         constexpr int NT = StagedShape<K>::NT;
         // with the gradient-space V-cycle running beside the forward sweep,
         // a quarter of the resident blocks is left to it
@@ -1106,7 +1106,7 @@ void ssor_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out, 
             const int smem = 2 * c.seg.stage_lo;
             const int grid = coop_grid(reinterpret_cast<const void*>(kf), NT, smem, share);
             cudaMemsetAsync(c.gridbar, 0, sizeof(unsigned), c.stream);
-            void* args[] = {(void*)&c.seg, (void*)&c.seg.work_col, (void*)&c.colour_ptr_d, (void*)&nc,
+            void* args[] = {(void*)&c.seg, (void*)&c.seg.work_col, (void*)&c.sweep_range_d, (void*)&nc,
                             (void*)&c.D, (void*)&c.B, (void*)&in, (void*)&y, (void*)&c.gridbar};
             cuda_check_launch(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kf), grid, NT, args, smem,
                                                           c.stream), c.launches);
@@ -1118,14 +1118,14 @@ void ssor_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out, 
             if (gt.ya) {
                 auto kf = k_ssor_bwd_coop<R, K, true>;
                 const int grid = coop_grid(reinterpret_cast<const void*>(kf), NT, smem, false);
-                void* args[] = {(void*)&c.seg, (void*)&c.seg.work_col, (void*)&c.colour_ptr_d, (void*)&nc,
+                void* args[] = {(void*)&c.seg, (void*)&c.seg.work_col, (void*)&c.sweep_range_d, (void*)&nc,
                                 (void*)&c.D, (void*)&c.B, (void*)&y, (void*)&out, (void*)&gt, (void*)&c.gridbar};
                 cuda_check_launch(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kf), grid, NT, args,
                                                               smem, c.stream), c.launches);
             } else {
                 auto kf = k_ssor_bwd_coop<R, K, false>;
                 const int grid = coop_grid(reinterpret_cast<const void*>(kf), NT, smem, false);
-                void* args[] = {(void*)&c.seg, (void*)&c.seg.work_col, (void*)&c.colour_ptr_d, (void*)&nc,
+                void* args[] = {(void*)&c.seg, (void*)&c.seg.work_col, (void*)&c.sweep_range_d, (void*)&nc,
                                 (void*)&c.D, (void*)&c.B, (void*)&y, (void*)&out, (void*)&gt, (void*)&c.gridbar};
                 cuda_check_launch(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kf), grid, NT, args,
                                                               smem, c.stream), c.launches);
@@ -1144,7 +1144,7 @@ void ssor_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out, 
         // 110 us: its eight SMs do not have the FP64 lanes)
         bool dep = false;
         for (int col = 0; col < nc; ++col) {
-            const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
+            const int s0 = c.sweep_range[col].x, s1 = c.sweep_range[col].y;
             if (s1 <= s0) continue;
             launch_staged(k_ssor_fwd_st<R, K>, NT, c.seg.stage_lo, s1 - s0, 1 << 20, dep, c.stream, c.seg,
                           c.seg.work_col + s0, s1 - s0, c.D, c.B, in, y);
@@ -1154,7 +1154,7 @@ void ssor_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out, 
         wait_join();
         dep = dep && !join;   // behind another stream's kernels: a plain launch
         for (int col = nc - 1; col >= 0; --col) {
-            const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
+            const int s0 = c.sweep_range[col].x, s1 = c.sweep_range[col].y;
             if (s1 <= s0) continue;
             if (gt.ya)
                 launch_staged(k_ssor_bwd_st<R, K, true>, NT, c.seg.stage_up, s1 - s0, 1 << 20, dep, c.stream, c.seg,
@@ -1169,7 +1169,7 @@ void ssor_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out, 
         return;
     }
     for (int col = 0; col < nc; ++col) {
-        const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
+        const int s0 = c.sweep_range[col].x, s1 = c.sweep_range[col].y;
         if (s1 <= s0) continue;
         const int grid = blocks_for((long)(s1 - s0) * G, kWarpsPerBlock, 1 << 20);
         k_ssor_fwd<R, K><<<grid, kBlock, 0, c.stream>>>(c.A, c.D, c.B, c.sweep_rows + (size_t)s0 * kSlice, s1 - s0, in, y);
@@ -1177,7 +1177,7 @@ void ssor_k(const KrylovCtx<R>& c, const cplx<R>* in, cplx<R>* y, cplx<R>* out, 
     }
     wait_join();
     for (int col = nc - 1; col >= 0; --col) {
-        const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
+        const int s0 = c.sweep_range[col].x, s1 = c.sweep_range[col].y;
         if (s1 <= s0) continue;
         const int grid = blocks_for((long)(s1 - s0) * G, kWarpsPerBlock, 1 << 20);
         k_ssor_bwd<R, K><<<grid, kBlock, 0, c.stream>>>(c.A, c.D, c.B, c.sweep_rows + (size_t)s0 * kSlice, s1 - s0, y, out);
@@ -1504,10 +1504,10 @@ void eis_apply_k(const KrylovCtx<R>& c, const cplx<R>* z, cplx<R>* p, const cplx
                  BicgState* st, cplx<R>* w, cplx<R>* y, cplx<R>* out, const cplx<R>* aux) {
     constexpr int NT = StagedShape<K>::NT;
     constexpr int NQW = (MODE == kSpmvAp) ? 1 : (MODE == kEisAsS) ? 3 : 2;
-    const int nc = (int)c.colour_ptr.size() - 1;
+    const int nc = (int)c.sweep_range.size();
     int slot = 0;
     for (int col = nc - 1; col >= 0; --col) {
-        const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
+        const int s0 = c.sweep_range[col].x, s1 = c.sweep_range[col].y;
         if (s1 <= s0) continue;
         auto kb = k_eis_bwd_st<R, K, FUSE>;
         const int g = staged_grid(kb, NT, c.seg.stage_up, s1 - s0, 1 << 20);
@@ -1520,7 +1520,7 @@ void eis_apply_k(const KrylovCtx<R>& c, const cplx<R>* z, cplx<R>* p, const cplx
     }
     const cplx<R>* zz = FUSE != 0 ? (const cplx<R>*)p : z;
     for (int col = 0; col < nc; ++col) {
-        const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
+        const int s0 = c.sweep_range[col].x, s1 = c.sweep_range[col].y;
         if (s1 <= s0) continue;
         auto kf = k_eis_fwd_st<R, K, MODE>;
         const int g = staged_grid(kf, NT, c.seg.stage_lo, s1 - s0, 1 << 20);
@@ -1540,9 +1540,9 @@ void eis_apply_k(const KrylovCtx<R>& c, const cplx<R>* z, cplx<R>* p, const cplx
 template <class R, int K>
 void eis_init_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* st) {
     constexpr int NT = StagedShape<K>::NT;
-    const int nc = (int)c.colour_ptr.size() - 1;
+    const int nc = (int)c.sweep_range.size();
     for (int col = 0; col < nc; ++col) {
-        const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
+        const int s0 = c.sweep_range[col].x, s1 = c.sweep_range[col].y;
         if (s1 <= s0) continue;
         launch_staged(k_ssor_fwd_st<R, K>, NT, c.seg.stage_lo, s1 - s0, 1 << 20, false, c.stream, c.seg,
                       c.seg.work_col + s0, s1 - s0, c.D, c.B, (const cplx<R>*)v.b, v.y);
@@ -1578,9 +1578,9 @@ void eis_iteration_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, BicgState* s
 template <class R, int K>
 void eis_finish_k(const KrylovCtx<R>& c, const KrylovVecs<R>& v, cplx<R>* out) {
     constexpr int NT = StagedShape<K>::NT;
-    const int nc = (int)c.colour_ptr.size() - 1;
+    const int nc = (int)c.sweep_range.size();
     for (int col = nc - 1; col >= 0; --col) {
-        const int s0 = c.colour_ptr[col], s1 = c.colour_ptr[col + 1];
+        const int s0 = c.sweep_range[col].x, s1 = c.sweep_range[col].y;
         if (s1 <= s0) continue;
         launch_staged(k_eis_bwd_st<R, K, 0>, NT, c.seg.stage_up, s1 - s0, 1 << 20, false, c.stream, c.seg,
                       c.seg.work_col + s0, s1 - s0, c.D, c.B, (const cplx<R>*)v.x, (cplx<R>*)nullptr,

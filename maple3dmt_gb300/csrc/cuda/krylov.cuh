@@ -139,7 +139,8 @@ struct KrylovCtx {
     OpView<R> A;
     DiagView<R> D;
     BatchView B;
-    std::vector<int> colour_ptr;     // [n_colours + 1] ranges of sweep slices per colour
+    std::vector<int2> sweep_range;   // [n_colours] sweep slices [x, y) of each colour: those of its free rows in
+                                     // the FP32 inner solve (no vector has other rows there), of all its rows else
     const int* sweep_rows;           // device: 32 row numbers per sweep slice, slices grouped by colour
     int n_rows_pad;                  // rows the products and vector kernels run over: all, or the free rows
                                      // (the first ones) in the FP32 inner solve
@@ -174,7 +175,7 @@ struct KrylovCtx {
     // staged rows: each SSOR sweep as one cooperative launch over all sweep
     // groups (grid barriers between groups) instead of one launch per group
     int coop = 0;
-    const int* colour_ptr_d = nullptr;   // device copy of colour_ptr
+    const int2* sweep_range_d = nullptr;   // device copy of sweep_range
     unsigned* gridbar = nullptr;         // [2] barrier counter and generation
 };
 

@@ -49,8 +49,8 @@ struct SegView {
     const int* row_off = nullptr;             // [n_slices + 1] their offsets, 16-byte units
     int stage_row[25] = {};     // [T]: bytes of the largest run of T neighbouring row segments (T > 0)
     const unsigned char* seg = nullptr;       // sweep segments (null until a sweep is asked for)
-    const int4* work_col = nullptr;           // sweep order (sweep slices of group g at colour_ptr[g])
-    const int* rows = nullptr;                // [sweep slices][32] row numbers (-1: none)
+    const int4* work_col = nullptr;           // sweep order (a group's slices together, those of its free rows first)
+    const int* rows = nullptr;                // [sweep slices][32] row numbers
     int stage_lo = 0;           // bytes of the largest lower segment
     int stage_up = 0;           // bytes of the largest upper segment
     unsigned* err = nullptr;    // device flag, kErrCopyTimeout on a barrier timeout

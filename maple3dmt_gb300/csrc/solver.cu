@@ -221,7 +221,7 @@ void GpuSolver::free_all() {
     for (void* p : sweep_mem) cudaFree(p);
     sweep_mem.clear();
     seg64 = dev::SegView<double>{}; seg32 = dev::SegView<float>{};
-    dfree(d_sweep_rows); dfree(d_colour_ptr); dfree(d_gridbar);
+    dfree(d_sweep_rows); dfree(d_sweep_range); dfree(d_sweep_range_free); dfree(d_gridbar);
     dfree(d_src_wr); dfree(d_src_g); src_ns = -1;
     dfree(d_sigma); dfree(d_Me); dfree(d_me_dc);
     dfree(d_diag); dfree(d_diag32); dfree(d_omegas);
@@ -363,25 +363,6 @@ void GpuSolver::setup(const m3d_leaves* lv, const m3d_params* params) {
     }
     const int n_col = *std::max_element(colour.begin(), colour.end()) + 1;
 
-    // Row order: the free rows in reference order (cell by cell along the
-    // Morton curve), then the identity rows of the eliminated system (boundary
-    // and air edges, dead hanging edges: a sixth to a third of all), each part
-    // padded to whole slices.  A row's neighbours sit a few rows away, so
-    // gathers hit L1, and the FP32 inner solve runs over the free rows alone.
-    perm.clear();
-    for (int part = 0; part < 2; ++part) {
-        for (int e = 0; e < ne; ++e)
-            if (free_row(e) == (part == 0)) perm.push_back(e);
-        // at least one padding row in the end: sweep slices are filled up with it
-        do perm.push_back(-1);
-        while (perm.size() % dev::kSlice);
-        if (part == 0) n_free = (int)perm.size();
-    }
-    n_pad = (int)perm.size();
-    n_slices = n_pad / dev::kSlice;
-    iperm.assign(ne, -1);
-    for (int r = 0; r < n_pad; ++r) if (perm[r] >= 0) iperm[perm[r]] = r;
-
     // SSOR sweep groups: a group's rows are independent (one colour), swept by
     // one launch over its sweep slices, which list 32 rows each.  With
     // sweep_rows > 0 the reference order is also cut into super-blocks of about
@@ -392,20 +373,58 @@ void GpuSolver::setup(const m3d_leaves* lv, const m3d_params* params) {
     constexpr int kRowBlock = 16384;
     const int blocks_per_sb = P.sweep_rows > 0 ? std::max(1, P.sweep_rows / kRowBlock) : (1 << 30);
     const int n_sb = (int)(((long)(ne + kRowBlock - 1) / kRowBlock + blocks_per_sb - 1) / blocks_per_sb);
+    const int n_grp = n_sb * n_col;
     edge_group.resize(ne);
     for (int e = 0; e < ne; ++e) edge_group[e] = (e / kRowBlock / blocks_per_sb) * n_col + colour[e];
-    {
-        std::vector<std::vector<int>> rows_of((size_t)n_sb * n_col);
-        for (int r = 0; r < n_pad; ++r)
-            if (perm[r] >= 0) rows_of[edge_group[perm[r]]].push_back(r);
-        colour_ptr.assign(1, 0);
-        sweep_rows.clear();
-        for (auto& rows : rows_of) {
-            if (rows.empty()) continue;
+
+    // Row order: the free rows in reference order (cell by cell along the
+    // Morton curve), then the identity rows of the eliminated system (boundary
+    // and air edges, dead hanging edges: a sixth to a third of all), each part
+    // padded to whole slices.  A row's neighbours sit a few rows away, so
+    // gathers hit L1, and the FP32 inner solve runs over the free rows alone.
+    // Each part ends with a padding row of its own for every place that its
+    // groups leave open in their last sweep slice: the sweeps reach every row
+    // once, padding included (a row that none reached would keep its residual).
+    perm.clear();
+    std::vector<std::vector<int>> rows_of[2];   // [part][group]
+    for (int part = 0; part < 2; ++part) {
+        rows_of[part].resize(n_grp);
+        for (int e = 0; e < ne; ++e)
+            if (free_row(e) == (part == 0)) {
+                rows_of[part][edge_group[e]].push_back((int)perm.size());
+                perm.push_back(e);
+            }
+        const bool none = std::all_of(rows_of[part].begin(), rows_of[part].end(), [](auto& v) { return v.empty(); });
+        for (auto& rows : rows_of[part])
+            while (rows.size() % dev::kSlice || (none && rows_of[part][0].empty())) {
+                rows.push_back((int)perm.size());
+                perm.push_back(-1);
+            }
+        if (part == 0) n_free = (int)perm.size();
+    }
+    n_pad = (int)perm.size();
+    n_slices = n_pad / dev::kSlice;
+    iperm.assign(ne, -1);
+    for (int r = 0; r < n_pad; ++r) if (perm[r] >= 0) iperm[perm[r]] = r;
+
+    // Sweep slices group by group, a group's free rows first: the FP32 inner
+    // solve, whose vectors hold nothing of its own on the identity rows (the
+    // memory of narrower batches has other batches' free rows there), sweeps
+    // the free rows' slices alone.
+    sweep_rows.clear();
+    sweep_range.clear();
+    sweep_range_free.clear();
+    for (int g = 0; g < n_grp; ++g) {
+        const int s0 = (int)(sweep_rows.size() / dev::kSlice);
+        int2 range[2];
+        for (int part = 0; part < 2; ++part) {
+            const auto& rows = rows_of[part][g];
             sweep_rows.insert(sweep_rows.end(), rows.begin(), rows.end());
-            sweep_rows.resize((sweep_rows.size() + dev::kSlice - 1) / dev::kSlice * dev::kSlice, n_pad - 1);
-            colour_ptr.push_back((int)(sweep_rows.size() / dev::kSlice));
+            range[part] = make_int2(s0, (int)(sweep_rows.size() / dev::kSlice));
         }
+        if (range[1].y == s0) continue;
+        sweep_range.push_back(range[1]);
+        sweep_range_free.push_back(range[0]);
     }
 
     std::vector<int> op_rp, op_rs, ecol;
@@ -564,7 +583,8 @@ void GpuSolver::setup(const m3d_leaves* lv, const m3d_params* params) {
     d_op_rp = dupload(op_rp, stream); d_op_rs = dupload(op_rs, stream);
     d_col = dupload(ecol, stream); d_val = dupload(eval, stream);
     d_sweep_rows = dupload(sweep_rows, stream);
-    d_colour_ptr = dupload(colour_ptr, stream);
+    d_sweep_range = dupload(sweep_range, stream);
+    d_sweep_range_free = dupload(sweep_range_free, stream);
     d_gridbar = dalloc_zero<unsigned>(2, stream);
     build_row_segments(op_rp, ecol, eval);
     {
@@ -1189,7 +1209,7 @@ KrylovCtx<double> GpuSolver::kctx(int K, const int* fmap) const {
         c.B.fmap[k] = (k < K) ? fmap[k] : 0;
         c.B.omega[k] = (k < K && c.B.fmap[k] < (int)fz_freqs.size()) ? 2.0 * kPi * fz_freqs[c.B.fmap[k]] : 0.0;
     }
-    c.colour_ptr = colour_ptr;
+    c.sweep_range = sweep_range;
     c.sweep_rows = d_sweep_rows;
     c.n_rows_pad = n_pad;
     c.grid_vec = red.max_blocks;
@@ -1206,7 +1226,7 @@ KrylovCtx<double> GpuSolver::kctx(int K, const int* fmap) const {
     c.seg = seg64;
     c.row_kernels = P.row_kernels;
     c.coop = P.coop_sweep;
-    c.colour_ptr_d = d_colour_ptr;
+    c.sweep_range_d = d_sweep_range;
     c.gridbar = d_gridbar;
     return c;
 }
@@ -1363,7 +1383,7 @@ KrylovCtx<float> GpuSolver::kctx32(int K, const int* fmap, bool free_rows) const
     f.D = DiagView<float>{d_diag32};
     f.B = c.B;
     f.B.relax = P.ssor_relax;   // the FP64 context keeps the reference's 1
-    f.colour_ptr = c.colour_ptr;
+    f.sweep_range = free_rows ? sweep_range_free : sweep_range;
     f.sweep_rows = c.sweep_rows;
     f.n_rows_pad = free_rows ? n_free : n_pad;
     f.grid_vec = c.grid_vec;
@@ -1380,7 +1400,7 @@ KrylovCtx<float> GpuSolver::kctx32(int K, const int* fmap, bool free_rows) const
     f.eis_partial = d_eis_partial;
     f.eis_slots = eis_slots;
     f.coop = c.coop;
-    f.colour_ptr_d = c.colour_ptr_d;
+    f.sweep_range_d = free_rows ? d_sweep_range_free : d_sweep_range;
     f.gridbar = c.gridbar;
     return f;
 }

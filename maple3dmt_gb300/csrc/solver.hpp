@@ -144,7 +144,7 @@ public:
     int n_stations() const { return sd.ns; }
     long nnz_off = 0;       // off-diagonal stiffness entries
     int n_nodes() const { return L.nn; }
-    int n_colours() const { return (int)colour_ptr.size() - 1; }
+    int n_colours() const { return (int)sweep_range.size(); }
 
 private:
     HostLayout L;
@@ -152,10 +152,11 @@ private:
     long long launches = 0;
 
     // host-side structure
-    std::vector<int> perm, iperm, colour_ptr, sweep_rows;
+    std::vector<int> perm, iperm, sweep_rows;
+    std::vector<int2> sweep_range, sweep_range_free;   // per sweep group: all its slices, those of its free rows
     std::vector<int> edge_group;        // SSOR sweep group of every edge
     int* d_sweep_rows = nullptr;        // 32 rows of every sweep slice
-    int* d_colour_ptr = nullptr;        // device copy of colour_ptr (cooperative sweeps)
+    int2 *d_sweep_range = nullptr, *d_sweep_range_free = nullptr;   // device copies (cooperative sweeps)
     unsigned* d_gridbar = nullptr;      // grid barrier of the cooperative sweeps
     std::vector<unsigned char> flags_ref;  // reference order
     int n_pad = 0, n_slices = 0;

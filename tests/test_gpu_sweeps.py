@@ -1,0 +1,33 @@
+"""Every row that a solve carries is its own: the memory of a narrow batch holds
+what wider batches left on the rows that the batch does not write (identity rows
+in the mixed-precision solve), and rows that pad the sweeps must be swept too."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("opts", [dict(), dict(gradcorr=0), dict(gradcorr=0, ssor_form=0),
+                                  dict(gradcorr=0, row_kernels=0), dict(gradcorr=0, coop_sweep=1, ssor_form=0),
+                                  dict(gradcorr=0, sweep_rows=16384), dict(ssor_relax=1.0001),
+                                  dict(gradcorr=0, residual_replacement=1, ssor_form=0), dict(krylov=1),
+                                  dict(precision=0), dict(precision=0, row_kernels=0)])
+def test_narrow_batch_after_a_wide_one(lib, opts):
+    """Eight frequencies (16 lanes, narrowing as they converge), then one, on one
+    handle: the bits and the iterations of a fresh handle."""
+    from maple3dmt_gb300 import mesh
+    from maple3dmt_gb300.solver import solver_for_survey
+    freqs = np.logspace(-1, 3, 8)
+    sv = mesh.small_survey(min_level=4, max_level=5, freqs=freqs)
+    par = dict(bicgstab_tol=1e-10, bicgstab_maxiter=5000, precision=1) | opts
+    used = solver_for_survey(sv, **par)
+    used.forward_batch(freqs)
+    for f in (freqs[1], freqs[6]):
+        fresh = solver_for_survey(sv, **par)
+        want = fresh.forward_batch([f], with_fields=True)
+        got = used.forward_batch([f], with_fields=True)
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b)
+        a, b = used.stats(), fresh.stats()
+        assert a["iterations"][:2] == b["iterations"][:2] and a["status"][:2] == [1, 1]
+        fresh.close()
