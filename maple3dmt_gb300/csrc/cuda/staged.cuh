@@ -6,8 +6,8 @@
 //             [int32 col[n]]
 //             [R val[n]]
 //
-// with every row padded to a multiple of four entries (padding entries point
-// at the row itself with value 0), so rows start on 16-byte boundaries and
+// with every row padded to a multiple of four entries (padding entries repeat
+// the row's last column with value 0), so rows start on 16-byte boundaries and
 // are read four entries at a time, and every segment starts and ends on a
 // 16-byte boundary.  Two sets exist per precision:
 //

@@ -1440,8 +1440,10 @@ void GpuSolver::set_test_consume_no_wait(bool on) {
 namespace {
 
 // Appends one segment (staged.cuh): entries [begin(r), end(r)) of up to 32
-// rows, padded to whole groups of four with zero entries on the row itself (a
-// finite value times zero).  Returns its offset and length in 16-byte units.
+// rows, padded to whole groups of four with zero entries in the row's last
+// column, whose value the row takes anyway (in its own column a sweep would
+// find what an earlier solve left: a NaN times zero).  Returns its offset and
+// length in 16-byte units.
 template <class R, class Rows>
 std::pair<long, int> put_segment(std::vector<unsigned char>& buf, const std::vector<int>& ecol,
                                  const std::vector<double>& eval, const Rows& rows) {
@@ -1450,10 +1452,10 @@ std::pair<long, int> put_segment(std::vector<unsigned char>& buf, const std::vec
     std::vector<int> cols;
     std::vector<R> vals;
     for (int r = 0; r < dev::kSlice; ++r) {
-        int row, b, e;
-        rows(r, row, b, e);
+        int b, e;
+        rows(r, b, e);
         for (int k = b; k < e; ++k) { cols.push_back(ecol[k]); vals.push_back((R)eval[k]); }
-        while (cols.size() % 4) { cols.push_back(row); vals.push_back((R)0); }
+        while (cols.size() % 4) { cols.push_back(cols.back()); vals.push_back((R)0); }
         if (cols.size() > 65535) throw std::runtime_error("slice segment too large");
         end[r] = (uint16_t)cols.size();
     }
@@ -1483,8 +1485,8 @@ void GpuSolver::build_row_segments(const std::vector<int>& op_rp, const std::vec
         std::vector<int> off(n_slices + 1, 0);
         buf.reserve(((size_t)op_rp[n_pad] + 2 * (size_t)n_pad) * (4 + sizeof(R)));
         for (int s = 0; s < n_slices; ++s) {
-            off[s] = (int)put_segment<R>(buf, ecol, eval, [&](int r, int& row, int& b, int& e) {
-                row = s * dev::kSlice + r;
+            off[s] = (int)put_segment<R>(buf, ecol, eval, [&](int r, int& b, int& e) {
+                const int row = s * dev::kSlice + r;
                 b = op_rp[row];
                 e = op_rp[row + 1];
             }).first;
@@ -1520,8 +1522,8 @@ void GpuSolver::ensure_sweeps(dev::SegView<R>& view) {
     std::vector<int4> work(ns);
     for (int s = 0; s < ns; ++s) {
         auto part = [&](bool upper) {
-            return put_segment<R>(buf, ecol, eval, [&](int r, int& row, int& b, int& e) {
-                row = sweep_rows[(size_t)s * dev::kSlice + r];
+            return put_segment<R>(buf, ecol, eval, [&](int r, int& b, int& e) {
+                const int row = sweep_rows[(size_t)s * dev::kSlice + r];
                 b = upper ? rs[row] : rp[row];
                 e = upper ? rp[row + 1] : rs[row];
             });

@@ -31,3 +31,30 @@ def test_narrow_batch_after_a_wide_one(lib, opts):
         a, b = used.stats(), fresh.stats()
         assert a["iterations"][:2] == b["iterations"][:2] and a["status"][:2] == [1, 1]
         fresh.close()
+
+
+@pytest.mark.parametrize("opts", [dict(), dict(ssor_form=0), dict(row_kernels=0), dict(coop_sweep=1, ssor_form=0),
+                                  dict(ssor_relax=1.0001), dict(krylov=1), dict(precision=0),
+                                  dict(precision=0, row_kernels=0)])
+def test_solve_after_a_failed_one(lib, opts):
+    """A conductivity beyond the FP32 range and a right-hand side whose square
+    overflows in FP64 leave infinities and NaN in the solver's vectors; the next
+    solve (without divergence correction) gives the bits of a fresh handle."""
+    from maple3dmt_gb300 import mesh
+    from maple3dmt_gb300.solver import solver_for_survey
+    freqs = np.logspace(-1, 1, 2)
+    sv = mesh.small_survey(min_level=4, max_level=5, freqs=freqs)
+    par = dict(bicgstab_tol=1e-10, bicgstab_maxiter=2000, precision=1, div_correction=0) | opts
+    fresh = solver_for_survey(sv, **par)
+    want = fresh.forward_batch(freqs, with_fields=True)
+    s = solver_for_survey(sv, **par)
+    s.set_sigma(np.where(sv.leaves.cell_type == 0, 1e40, sv.sigma))
+    s.forward_batch(freqs)
+    s.set_sigma(sv.sigma)
+    s.factorize_frequency(freqs[0])
+    rng = np.random.default_rng(2)
+    s.solve_rhs_batch(1e200 * (rng.normal(size=(4, s.ne)) + 1j * rng.normal(size=(4, s.ne))))
+    got = s.forward_batch(freqs, with_fields=True)
+    assert s.stats()["status"][:4] == fresh.stats()["status"][:4]
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
