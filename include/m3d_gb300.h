@@ -470,7 +470,7 @@ int m3d_learn_train(m3d_solver* s, int epochs, float lr, int batch, unsigned see
                     double* epoch_loss, double* val_loss);
 
 /* ---------------------------------------------------------------------- */
-/* Test hook (no counterpart in the reference).                           */
+/* Test hooks (no counterpart in the reference).                          */
 /* ---------------------------------------------------------------------- */
 
 /* on != 0: every slice-staged kernel of this solver polls its copy barrier
@@ -479,6 +479,12 @@ int m3d_learn_train(m3d_solver* s, int epochs, float lr, int batch, unsigned see
  * flight); the next solve then fails with M3D_ERR_CUDA.  on = 0 restores
  * the bounded waits.  For testing the error path only. */
 int m3d_test_set_consume_no_wait(m3d_solver* s, int on);
+
+/* Multiplies the cell sizes that the multigrid preconditioner's coarse grids
+ * compute with by f, which spoils its corrections: solves fall back to SSOR.
+ * 1 / f restores them.  M3D_ERR_STATE where the mesh has no such
+ * preconditioner. */
+int m3d_test_set_multigrid_scale(m3d_solver* s, float f);
 
 #ifdef __cplusplus
 }

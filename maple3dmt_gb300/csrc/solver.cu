@@ -1437,6 +1437,14 @@ void GpuSolver::set_test_consume_no_wait(bool on) {
     sync();
 }
 
+// Scales the cell sizes that the coarse grids compute with: their corrections
+// no longer fit the fine operator.
+void GpuSolver::set_test_multigrid_scale(float f) {
+    if (!emg_ok) throw std::logic_error("no multigrid preconditioner on this mesh");
+    for (int l = 0; l < emg.n_levels; ++l)
+        for (float& h : emg.lv[l].h) h *= f;
+}
+
 namespace {
 
 // Appends one segment (staged.cuh): entries [begin(r), end(r)) of up to 32
@@ -1548,7 +1556,12 @@ template void GpuSolver::ensure_sweeps<double>(dev::SegView<double>&);
 // with the complex-FP32 batched BiCGStab (scaled to unit norm, relative
 // tolerance max(tol / ||r||_rel, inner_tol_floor)), and adds d to x in FP64.  Steps repeat
 // until the FP64 true residual meets tol, the iteration budget is spent or a
-// step fails to reduce the residual by 10 %.
+// step fails to reduce the residual by 10 %.  Where such a step ran under the
+// multigrid preconditioner, every right-hand side that it failed goes on with
+// SSOR instead, with the steps and iterations that a solve has.  A multigrid
+// step also counts as failed, and ends, when kMgPatience iterations have not
+// reduced the FP32 residual ten-fold, and a correction that leaves the residual
+// larger (or not finite) is not added.
 //
 // The FP32 solve runs only the right-hand sides that still need it, packed
 // into the narrowest power-of-two batch (>= 2 lanes); whenever at most half of
@@ -1634,10 +1647,13 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
     std::vector<int> run = active;
     std::vector<double> prev(K, 1e300), scale(K, 0.0);
     std::vector<BicgState> hs(K);
-    // the multigrid preconditioner; a step that does not reduce the residual
-    // with it is run again with SSOR
-    bool multigrid = emg_ok;
+    bool multigrid = emg_ok;      // the next step's preconditioner
+    bool ran_multigrid = false;   // the last step's
+    constexpr int kMgPatience = 100;
     const int max_steps = 2 + std::max(0, P.max_refinements) * 4;
+    int last_step = max_steps;
+    std::vector<int> uncounted(K, 0);   // iterations of multigrid steps that failed
+    std::vector<char> gave_up(K, 0);    // the last step was a multigrid one that ended for lack of progress
     auto pow2_at_least = [](int n) { int k = 2; while (k < n) k *= 2; return k; };
     auto launch_grid = [](long n) { return (int)((n + 255) / 256); };
     // identity rows: x = b, exactly; the FP32 solve runs over the free rows
@@ -1648,7 +1664,7 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
         k_identity_rows<<<launch_grid(n), 256, 0, stream>>>(x + (size_t)n_free * K, b + (size_t)n_free * K, K, n, on);
         ++launches;
     }
-    for (int step = 0; step <= max_steps; ++step) {
+    for (int step = 0; step <= last_step; ++step) {
         // FP64 true residual y = b - A x
         for (int k = 0; k < K; ++k) {
             std::memset(&hs[k], 0, sizeof(BicgState));
@@ -1659,6 +1675,7 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
         cuda_ok(cudaMemcpyAsync(hs.data(), d_states, sizeof(BicgState) * K, cudaMemcpyDeviceToHost, stream), "states");
         sync();
         std::vector<int> lanes;   // current lane -> right-hand side of the FP64 batch
+        bool failed = false;
         for (int k = 0; k < K; ++k) {
             if (!active[k]) continue;
             const double rel = hs[k].true_res;
@@ -1671,17 +1688,27 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
                 R.status[k] = kBreakdown;
                 continue;
             }
-            if (rel > 0.9 * prev[k] && multigrid) multigrid = false;
-            else if (rel > 0.9 * prev[k] || R.iters[k] >= maxiter || step == max_steps) {
+            const bool stalled = rel > 0.9 * prev[k] || gave_up[k];
+            if ((stalled && !ran_multigrid) || R.iters[k] - uncounted[k] >= maxiter || step == last_step) {
                 run[k] = 0;
                 if (R.status[k] == kInactive || R.status[k] == kConverged) R.status[k] = kMaxIter;
                 continue;
+            }
+            if (stalled) {
+                failed = true;
+                gave_up[k] = 0;
+                uncounted[k] = R.iters[k];
+                R.status[k] = kInactive;
             }
             prev[k] = rel;
             scale[k] = hs[k].rnorm;
             lanes.push_back(k);
         }
         if (lanes.empty()) break;
+        if (failed) {
+            multigrid = false;
+            last_step = step + max_steps;
+        }
         int Kc = pow2_at_least((int)lanes.size());
         lanes.resize(Kc, -1);
         KrylovVecs<float> cur = kv32, other = kv32b;
@@ -1708,9 +1735,10 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
                     const double om = 2.0 * kPi * fz_freqs[fmap[lanes[j]]];
                     use_gc |= om > 0.0 && om <= gc.omega_max;
                 }
+        ran_multigrid = use_gc && multigrid;
         // iterations between polls of the device's status: a multigrid solve
         // converges in 10 to 20 iterations, which ten at a time would overrun
-        const int chunk = use_gc && multigrid ? 2 : 10;
+        const int chunk = ran_multigrid ? 2 : 10;
         const bool eis = !use_gc && P.ssor_form == 1 && P.row_kernels == kRowsStaged && P.ssor_relax == 1.0;
         // residual replacement needs the untransformed residual of the
         // right-preconditioned form
@@ -1762,11 +1790,11 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
             // tolerance; without, to what complex FP32 reaches reliably
             ls[j].tol = std::min(0.5, std::max(tol / R.true_res[k], replace ? 0.25 * tol / R.true_res[k]
                                                                                     : P.inner_tol_floor));
-            ls[j].maxiter = std::max(1, maxiter - R.iters[k]);
+            ls[j].maxiter = std::max(1, maxiter - (R.iters[k] - uncounted[k]));
             ls[j].status = kRunning;
         }
         cuda_ok(cudaMemcpyAsync(d_states, ls.data(), sizeof(BicgState) * Kc, cudaMemcpyHostToDevice, stream), "states");
-        if (!(use_gc && multigrid)) ensure_sweeps(seg32);
+        if (!ran_multigrid) ensure_sweeps(seg32);
         KrylovCtx<float> c32 = kctx32(Kc, fm.data());
         if (use_gc) attach_gc(c32, multigrid);
         if (eis) eis_init(c32, cur, d_states);
@@ -1778,6 +1806,10 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
             R.iters[k] += ls[j].iter;
             if (ls[j].status == kBreakdown) R.status[k] = kBreakdown;
         };
+        // multigrid: the last ten-fold reduction of a right-hand side's residual
+        std::vector<double> mark_res(K, 1.0);
+        std::vector<int> mark_it(K, 0);
+        auto keep = [&](int j) { return !ran_multigrid || ls[j].res < 1.0; };   // the lane's correction
         int pending_graph = -1;   // replayed graph whose timer pairs wait for this poll
         int chunks_of_shape = 0;  // chunks run since the batch shape last changed
         for (;;) {
@@ -1786,6 +1818,23 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
             if (pending_graph >= 0) {
                 if (timer.on) timer.fold(chunk_graphs[pending_graph].pairs);
                 pending_graph = -1;
+            }
+            if (ran_multigrid) {
+                bool given_up = false;
+                for (int j = 0; j < Kc; ++j) {
+                    const int k = lanes[j];
+                    if (k < 0 || ls[j].status != kRunning) continue;
+                    if (ls[j].res <= 0.1 * mark_res[k]) {
+                        mark_res[k] = ls[j].res;
+                        mark_it[k] = ls[j].iter;
+                    } else if (ls[j].iter - mark_it[k] >= kMgPatience || !std::isfinite(ls[j].res)) {
+                        ls[j].status = kMaxIter;
+                        gave_up[k] = given_up = true;
+                    }
+                }
+                if (given_up)
+                    cuda_ok(cudaMemcpyAsync(d_states, ls.data(), sizeof(BicgState) * Kc, cudaMemcpyHostToDevice, stream),
+                            "states");
             }
             int nrun = 0;
             for (int j = 0; j < Kc; ++j) nrun += (lanes[j] >= 0 && ls[j].status == kRunning);
@@ -1824,7 +1873,7 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
             if (Kn < Kc && Kn <= other_cap) {
                 // finished lanes: add their corrections and record them
                 for (int j = 0; j < dev::kMaxRhs; ++j)
-                    add[j] = (j < Kc && lanes[j] >= 0 && ls[j].status != kRunning) ? 1 : 0;
+                    add[j] = (j < Kc && lanes[j] >= 0 && ls[j].status != kRunning && keep(j)) ? 1 : 0;
                 flush(c32, cur, Kc);
                 std::vector<int> sel(dev::kMaxRhs, -1), nl(Kn, -1);
                 std::vector<BicgState> ns(Kn);
@@ -1878,7 +1927,7 @@ BatchResult GpuSolver::solve_batch_mixed(int K, const int* fmap, double2* b, dou
                 }
             }
         }
-        for (int j = 0; j < dev::kMaxRhs; ++j) add[j] = (j < Kc && lanes[j] >= 0) ? 1 : 0;
+        for (int j = 0; j < dev::kMaxRhs; ++j) add[j] = (j < Kc && lanes[j] >= 0 && keep(j)) ? 1 : 0;
         flush(c32, cur, Kc);
         for (int j = 0; j < Kc; ++j) record(j);
         if (step > 0) ++stats.refinements;

@@ -304,6 +304,10 @@ class ForwardSolverFV:
         """Test hook: staged kernels take their copy-wait timeout path."""
         self._ck(self.lib.m3d_test_set_consume_no_wait(self.h, 1 if on else 0))
 
+    def test_set_multigrid_scale(self, f: float):
+        """Test hook of the fallback from multigrid to SSOR (see m3d_gb300.h)."""
+        self._ck(self.lib.m3d_test_set_multigrid_scale(self.h, f))
+
     def set_kernel_timing(self, on: bool):
         self._ck(self.lib.m3d_set_kernel_timing(self.h, 1 if on else 0))
 
