@@ -272,9 +272,12 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // own, so a warp whose gathers miss does not hold up the others (with a block
 // barrier per tile the SpMV ran at 2.9 TB/s, all warps in step).
 // Every wait is bounded: a consumer whose stage does not arrive sets
-// kErrCopyTimeout, skips this and all later tiles but still gives the stages
-// back; the producer reuses a stage only when its copy has landed, and waits
-// for the copies in flight before it leaves.
+// kErrCopyTimeout and skips this and all later tiles, but gives a stage back
+// only when its copy has landed, as the others do (a warp that ran ahead would
+// stand in for a slower one in the stage's barrier, and the next copy would
+// overwrite rows that are being read); where it never lands the warp leaves.
+// The producer reuses a stage only when its copy has landed, and waits for the
+// copies in flight before it leaves.
 template <int CW, int RING, class Prefetch, class Body>
 __device__ __forceinline__ void tile_ring(const unsigned char* __restrict__ seg, const int* __restrict__ off,
                                           int n_slices, int T, int stage_bytes, unsigned* err, Prefetch prefetch,
@@ -327,6 +330,7 @@ __device__ __forceinline__ void tile_ring(const unsigned char* __restrict__ seg,
                     if (lane == 0) atomicOr(err, kErrCopyTimeout);
                 }
             }
+            if (dead && !__all_sync(0xffffffffu, mbar_wait_bounded(&full[s], parity))) break;
             if (!dead) body(t, pre, dsm + (size_t)s * stage_bytes);
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[s]);

@@ -58,3 +58,23 @@ def test_solve_after_a_failed_one(lib, opts):
     assert s.stats()["status"][:4] == fresh.stats()["status"][:4]
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_copy_wait_timeout_with_reused_stages(lib, precision):
+    """On 201 k edges with 16 lanes each block of the product runs its ring of
+    stages through more than once.  With the hook on, warps that find a copy not
+    landed skip it, in step with the others; the call reports the timeout, and with
+    the hook off the handle solves as a fresh one does."""
+    from maple3dmt_gb300 import mesh
+    from maple3dmt_gb300.solver import SolverError, solver_for_survey
+    freqs = np.logspace(0, 2, 8)
+    sv = mesh.layered_block_survey(min_level=5, max_level=6, n_side=5, freqs=freqs)
+    par = dict(bicgstab_tol=1e-6, bicgstab_maxiter=30, precision=precision)
+    s = solver_for_survey(sv, **par)
+    s.test_set_consume_no_wait(True)
+    with pytest.raises(SolverError) as e:
+        s.forward_batch(freqs)
+    assert e.value.code == 3 and "timed out" in str(e.value)
+    s.test_set_consume_no_wait(False)
+    assert np.array_equal(s.forward_batch(freqs), solver_for_survey(sv, **par).forward_batch(freqs))
