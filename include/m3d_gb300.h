@@ -480,6 +480,11 @@ int m3d_learn_train(m3d_solver* s, int epochs, float lr, int batch, unsigned see
  * the bounded waits.  For testing the error path only. */
 int m3d_test_set_consume_no_wait(m3d_solver* s, int on);
 
+/* The shared memory per block that the sparse product plans its ring of
+ * matrix tiles for (at least two tiles of 32 rows are taken); 0: the
+ * device's. */
+int m3d_test_set_smem_limit(m3d_solver* s, int bytes);
+
 /* Multiplies the cell sizes that the multigrid preconditioner's coarse grids
  * compute with by f, which spoils its corrections: solves fall back to SSOR.
  * 1 / f restores them.  M3D_ERR_STATE where the mesh has no such

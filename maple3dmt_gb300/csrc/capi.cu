@@ -540,6 +540,12 @@ extern "C" int m3d_test_set_consume_no_wait(m3d_solver* h, int on) {
     return guarded(h, [&](m3d::GpuSolver& s) { s.set_test_consume_no_wait(on != 0); });
 }
 
+extern "C" int m3d_test_set_smem_limit(m3d_solver* h, int bytes) {
+    if (!ready(h)) return fail(h, M3D_ERR_STATE, "solver not set up");
+    if (bytes < 0) return fail(h, M3D_ERR_ARG, "limit must be >= 0");
+    return guarded(h, [&](m3d::GpuSolver& s) { s.set_test_smem_limit(bytes); });
+}
+
 extern "C" int m3d_test_set_multigrid_scale(m3d_solver* h, float f) {
     if (!ready(h)) return fail(h, M3D_ERR_STATE, "solver not set up");
     if (!(f > 0.0f)) return fail(h, M3D_ERR_ARG, "scale must be > 0");

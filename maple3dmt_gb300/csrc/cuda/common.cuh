@@ -156,7 +156,8 @@ int resident_blocks(const void* kernel, int threads = kBlock, int smem = 0);
 // limit is set to the most there is, once per (device, kernel).  It belongs to
 // the function, not to the launch: set to each launch's own size, a second
 // solver's thread could lower it between this one's call and its launch.
-void lift_smem_limit(const void* kernel);
+// Returns that size (0: an error, which the launch reports).
+int lift_smem_limit(const void* kernel);
 
 // One resident wave of `kernel`, at most `cap` blocks.
 template <class F>

@@ -7,7 +7,6 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
-#include <set>
 #include <stdexcept>
 #include <string>
 #include <tuple>
@@ -18,21 +17,22 @@ namespace m3d {
 
 namespace dev {
 
-void lift_smem_limit(const void* kernel) {
+int lift_smem_limit(const void* kernel) {
     static std::mutex mu;
-    static std::set<std::pair<int, const void*>> done;
+    static std::map<std::pair<int, const void*>, int> done;
     int dev = 0;
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lock(mu);
-    if (done.count({dev, kernel})) return;
+    auto it = done.find({dev, kernel});
+    if (it != done.end()) return it->second;
     cudaFuncAttributes fa{};
     int most = 0;
     if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess ||
         cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes) !=
             cudaSuccess)
-        return;   // the launch reports it
-    done.insert({dev, kernel});
+        return 0;
+    return done[{dev, kernel}] = most - (int)fa.sharedSizeBytes;
 }
 
 int resident_blocks(const void* kernel, int threads, int smem) {
@@ -464,7 +464,7 @@ template <class R, int LPT> struct alignas(LPT * 2 * sizeof(R)) CVec {
 // a damped Jacobi step (data once: 91 us).
 template <class R, int K, int MODE>
 __global__ void __launch_bounds__(SpmvShape<R, K>::NT, 1)
-    k_spmv_st(SegView<R> S, int n_slices, int T, DiagView<R> D, BatchView B, const cplx<R>* x,
+    k_spmv_st(SegView<R> S, int n_slices, int T, int ring, DiagView<R> D, BatchView B, const cplx<R>* x,
               cplx<R>* __restrict__ y, const cplx<R>* aux, cplx<R>* __restrict__ aux_out, BicgState* st,
               RedScratch rs) {
     using C = cplx<R>;
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(SpmvShape<R, K>::NT, 1)
         }
         return o;
     };
-    tile_ring<Sh::CW, Sh::RING>(S.row_seg, S.row_off, n_slices, T, S.stage_row[T], S.err, own,
+    tile_ring<Sh::CW, Sh::RING>(S.row_seg, S.row_off, n_slices, T, ring, S.stage_row[T], S.err, own,
                                 [&](int tile, const Own& o, const unsigned char* base) {
         if (o.at < 0) return;
         {
@@ -954,19 +954,26 @@ void spmv_staged_mode(const KrylovCtx<R>& c, const cplx<R>* x, cplx<R>* y, const
     const int cap = (MODE == kSpmvPlain || MODE == kSpmvSmooth) ? (1 << 20) : c.red.max_blocks;
     // whole passes where there are tiles for every SM, fewer slices per tile on
     // small meshes (152 SMs)
-    const int T = std::max(1, std::min(Sh::T_MAX, ns / 152));
+    int T = std::max(1, std::min(Sh::T_MAX, ns / 152)), ring = Sh::RING;
     auto kf = k_spmv_st<R, K, MODE>;
-    const int smem = Sh::RING * c.seg.stage_row[T];
-    if (smem > 16 * 1024)   // with the reduction's static arrays beyond 48 KB
-        lift_smem_limit(reinterpret_cast<const void*>(kf));
+    // long rows (several levels of refinement meeting all over a tile) take
+    // fewer slices per tile, then fewer stages: with twelve entries a row the ring
+    // is 28 to 150 KB of the 227 that a block can have
+    if (ring * c.seg.stage_row[T] > 16 * 1024) {   // with the reduction's static arrays beyond 48 KB
+        int most = lift_smem_limit(reinterpret_cast<const void*>(kf));
+        if (c.seg.smem_cap > 0) most = std::min(most, c.seg.smem_cap);
+        while (T > 1 && ring * c.seg.stage_row[T] > most) --T;
+        while (ring > 2 && ring * c.seg.stage_row[T] > most) --ring;
+    }
+    const int smem = ring * c.seg.stage_row[T];
     const int g = std::min(wave_grid(kf, cap, Sh::NT, smem), std::max(1, (ns + T - 1) / T));
     // the modes of an iteration: a plain launch (the initial residual's, the
     // preconditioner's first) lies between them and whatever wrote the matrix
     if constexpr (MODE == kSpmvAp || MODE == kSpmvAs || MODE == kSpmvSmooth)
-        launch_dep(kf, dim3((unsigned)g), Sh::NT, (size_t)smem, c.stream, c.seg, ns, T, c.D, c.B, x, y, aux, aux_out, st,
+        launch_dep(kf, dim3((unsigned)g), Sh::NT, (size_t)smem, c.stream, c.seg, ns, T, ring, c.D, c.B, x, y, aux, aux_out, st,
                    c.red);
     else
-        kf<<<g, Sh::NT, smem, c.stream>>>(c.seg, ns, T, c.D, c.B, x, y, aux, aux_out, st, c.red);
+        kf<<<g, Sh::NT, smem, c.stream>>>(c.seg, ns, T, ring, c.D, c.B, x, y, aux, aux_out, st, c.red);
 }
 
 template <class R, int K>

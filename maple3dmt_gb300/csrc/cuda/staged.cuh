@@ -54,6 +54,7 @@ struct SegView {
     int stage_lo = 0;           // bytes of the largest lower segment
     int stage_up = 0;           // bytes of the largest upper segment
     unsigned* err = nullptr;    // device flag, kErrCopyTimeout on a barrier timeout
+    int smem_cap = 0;           // test hook: shared memory that the SpMV may plan for (0: the device's)
 };
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
@@ -267,7 +268,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // n (b + 1) / grid) and runs them in order.  A contiguous range keeps a block
 // on neighbouring rows, whose gathers hit its SM's L1: on the benchmark mesh
 // half of a row's columns lie within 13 rows of it and three quarters within
-// 86.  The last warp copies tiles into a ring of RING stages; the CW other
+// 86.  The last warp copies tiles into a ring of `ring` <= RING stages; the CW other
 // warps each wait for a stage, run body() and give the stage back on their
 // own, so a warp whose gathers miss does not hold up the others (with a block
 // barrier per tile the SpMV ran at 2.9 TB/s, all warps in step).
@@ -280,8 +281,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // copies in flight before it leaves.
 template <int CW, int RING, class Prefetch, class Body>
 __device__ __forceinline__ void tile_ring(const unsigned char* __restrict__ seg, const int* __restrict__ off,
-                                          int n_slices, int T, int stage_bytes, unsigned* err, Prefetch prefetch,
-                                          Body body) {
+                                          int n_slices, int T, int ring, int stage_bytes, unsigned* err,
+                                          Prefetch prefetch, Body body) {
     extern __shared__ __align__(128) unsigned char dsm[];
     __shared__ __align__(8) uint64_t full[RING], empty[RING];
     if (threadIdx.x == 0) {
@@ -298,11 +299,11 @@ __device__ __forceinline__ void tile_ring(const unsigned char* __restrict__ seg,
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == CW) {
         if (lane == 0) {
-            int issued = 0;
+            int issued = 0, s = 0;
+            unsigned phase = 0;   // of stage s: the number of times the ring went round, mod 2
             for (int t = t0; t < t1; ++t, ++issued) {
-                const int s = issued % RING, use = issued / RING;
-                if (use > 0 && (!mbar_wait_bounded(&empty[s], (unsigned)(use - 1) & 1u) ||
-                                !mbar_wait_bounded(&full[s], (unsigned)(use - 1) & 1u))) {
+                if (issued >= ring &&
+                    (!mbar_wait_bounded(&empty[s], phase ^ 1u) || !mbar_wait_bounded(&full[s], phase ^ 1u))) {
                     atomicOr(err, kErrCopyTimeout);
                     break;
                 }
@@ -310,18 +311,22 @@ __device__ __forceinline__ void tile_ring(const unsigned char* __restrict__ seg,
                 const unsigned bytes = (unsigned)(__ldg(&off[min(t * T + T, n_slices)]) - a) * 16u;
                 mbar_expect_tx(&full[s], bytes);
                 bulk_g2s(dsm + (size_t)s * stage_bytes, seg + (size_t)a * 16, bytes, &full[s]);
+                if (++s == ring) {
+                    s = 0;
+                    phase ^= 1u;
+                }
             }
-            for (int k = issued > RING ? issued - RING : 0; k < issued; ++k)
-                mbar_wait_bounded(&full[k % RING], (unsigned)(k / RING) & 1u);
+            for (int k = issued > ring ? issued - ring : 0; k < issued; ++k)
+                mbar_wait_bounded(&full[k % ring], (unsigned)(k / ring) & 1u);
         }
         dep_wait();
     } else {
         dep_wait();   // the copies of the first tiles are on their way
         const bool no_wait = (*reinterpret_cast<volatile unsigned*>(err) & kTestConsumeNoWait) != 0;
         bool dead = false;
-        for (int t = t0, k = 0; t < t1; ++t, ++k) {
-            const int s = k % RING;
-            const unsigned parity = (unsigned)(k / RING) & 1u;
+        int s = 0;
+        unsigned parity = 0;
+        for (int t = t0; t < t1; ++t) {
             auto pre = prefetch(t);
             if (!dead) {
                 const bool ok = no_wait ? mbar_test_wait(&full[s], parity) : mbar_wait_bounded(&full[s], parity);
@@ -334,6 +339,10 @@ __device__ __forceinline__ void tile_ring(const unsigned char* __restrict__ seg,
             if (!dead) body(t, pre, dsm + (size_t)s * stage_bytes);
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[s]);
+            if (++s == ring) {
+                s = 0;
+                parity ^= 1u;
+            }
         }
     }
     __syncthreads();
