@@ -126,11 +126,11 @@ typedef struct m3d_params {
     int gradcorr;             /* 1: the mixed-precision inner solve of right-hand sides with
                                  f <= gradcorr_fmax is preconditioned by geometric multigrid on the
                                  uniform grids under the octree (edge and node cycles, damped Jacobi
-                                 smoothing), where every leaf is at level 2 or finer and the levels
-                                 span at most 4; on other meshes, and with a setting of the SSOR sweeps
-                                 or of the aggregation cycle other than its default (ssor_relax,
-                                 coop_sweep, sweep_rows, gradcorr_presmooth), by SSOR plus a
-                                 gradient-space term G (i omega L)^-1 G^T (one multigrid V-cycle on
+                                 smoothing), where the coarsest leaves are at level 2 to 8 and the
+                                 finest at most three levels finer; on other meshes, and with a
+                                 setting of the SSOR sweeps or of the aggregation cycle other than its
+                                 default (ssor_relax, coop_sweep, sweep_rows, gradcorr_presmooth), by
+                                 SSOR plus a gradient-space term G (i omega L)^-1 G^T (one multigrid V-cycle on
                                  the divergence-correction Laplacian L); needs div_correction.
                                  Batches with such a right-hand side run the right-preconditioned
                                  form.  0: SSOR alone (the reference's preconditioner) */
@@ -479,6 +479,10 @@ int m3d_learn_train(m3d_solver* s, int epochs, float lr, int batch, unsigned see
  * flight); the next solve then fails with M3D_ERR_CUDA.  on = 0 restores
  * the bounded waits.  For testing the error path only. */
 int m3d_test_set_consume_no_wait(m3d_solver* s, int on);
+
+/* 1 if meshes with leaves at levels lmin to lmax take the multigrid
+ * preconditioner (host only). */
+int m3d_test_multigrid_levels(int lmin, int lmax);
 
 /* The shared memory per block that the sparse product plans its ring of
  * matrix tiles for (at least two tiles of 32 rows are taken); 0: the

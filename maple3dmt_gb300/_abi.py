@@ -66,6 +66,7 @@ def declare(lib) -> None:
         [vp, c_double_p, c_double_p, c_int_p, c_double_p, c_int_p, c_int_p, c_int_p])
     _fn(lib, "m3d_layout_stiffness", C.c_int, [vp, c_int_p, c_int_p, c_double_p])
     _fn(lib, "m3d_layout_hanging", C.c_int, [vp, c_int_p])
+    _fn(lib, "m3d_test_multigrid_levels", C.c_int, [C.c_int, C.c_int])
     if hasattr(lib, "m3d_solver_create"):
         from . import _abi_solver
         _abi_solver.declare(lib)

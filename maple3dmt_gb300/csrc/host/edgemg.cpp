@@ -19,16 +19,19 @@ bool grid_coord(double u, int scale, int& m) {
 
 }  // namespace
 
+// A 4^3 grid is the coarsest one; more than three levels of leaves under one
+// coarse grid leave too much to the fine level's Jacobi steps, and the packed
+// fractions hold three levels; up to 256^3 cells the kernels' thread numbers
+// (eight pairs of right-hand sides per edge entry) fit in 32 bits.
+bool emg_levels_ok(int lmin, int lmax) { return lmin >= 2 && lmin <= 8 && lmax - lmin <= 3; }
+
 void emg_build(const HostLayout& L, const std::vector<char>& free, const std::vector<char>& node_free,
                const std::vector<int>& iperm, int n_pad, double air, EmgHost& H) {
     H = EmgHost();
     if (L.nc == 0) return;
     const int lmin = *std::min_element(L.clevel.begin(), L.clevel.end());
     const int lmax = *std::max_element(L.clevel.begin(), L.clevel.end());
-    // a 4^3 grid is the coarsest one; more than three levels of leaves under
-    // one coarse grid leave too much to the fine level's Jacobi steps, and the
-    // packed fractions hold three levels
-    if (lmin < 2 || lmin > 10 || lmax - lmin > 3) return;
+    if (!emg_levels_ok(lmin, lmax)) return;
     H.lmin = lmin;
     H.gap = lmax - lmin;
     const double ext[3] = {L.domain[1] - L.domain[0], L.domain[3] - L.domain[2], L.domain[5] - L.domain[4]};

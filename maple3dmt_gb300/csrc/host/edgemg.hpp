@@ -63,9 +63,12 @@ inline long emg_points(int n) { return (long)(n + 1) * (n + 1) * (n + 1); }
 inline long emg_entries(int n) { return 3 * emg_points(n); }
 inline long emg_entry(int n, int D, int i, int j, int k) { return 3 * emg_point(n, i, j, k) + D; }
 
+// The rule: leaves at levels lmin to lmax.
+bool emg_levels_ok(int lmin, int lmax);
+
 // free[e]: edge e (reference numbering) is a row of the eliminated system;
 // node_free[v]: node v is not a Dirichlet node; iperm: edge -> permuted row;
-// n_pad: permuted rows.  ok stays false for meshes outside the rule at its top.
+// n_pad: permuted rows.  ok stays false for meshes outside the rule.
 void emg_build(const HostLayout& L, const std::vector<char>& free, const std::vector<char>& node_free,
                const std::vector<int>& iperm, int n_pad, double air, EmgHost& H);
 

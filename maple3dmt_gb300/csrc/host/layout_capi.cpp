@@ -1,5 +1,6 @@
 // Layout introspection C ABI (include/m3d_gb300.h, m3d_layout_*): host only.
 #include "m3d_gb300.h"
+#include "edgemg.hpp"
 #include "layout.hpp"
 
 #include <new>
@@ -94,3 +95,5 @@ extern "C" int m3d_layout_hanging(const m3d_layout* h, int* pairs) {
         for (int k = 0; k < 3; ++k) pairs[3 * i + k] = L.hp[i][k];
     return M3D_OK;
 }
+
+extern "C" int m3d_test_multigrid_levels(int lmin, int lmax) { return m3d::emg_levels_ok(lmin, lmax) ? 1 : 0; }
