@@ -489,6 +489,10 @@ int m3d_test_multigrid_levels(int lmin, int lmax);
  * device's. */
 int m3d_test_set_smem_limit(m3d_solver* s, int bytes);
 
+/* on != 0: the next m3d_solver_setup finds no memory for the multigrid
+ * preconditioner's grids, as a mesh near the device's size would. */
+int m3d_test_fail_multigrid_alloc(m3d_solver* s, int on);
+
 /* Multiplies the cell sizes that the multigrid preconditioner's coarse grids
  * compute with by f, which spoils its corrections: solves fall back to SSOR.
  * 1 / f restores them.  M3D_ERR_STATE where the mesh has no such

@@ -546,6 +546,10 @@ extern "C" int m3d_test_set_smem_limit(m3d_solver* h, int bytes) {
     return guarded(h, [&](m3d::GpuSolver& s) { s.set_test_smem_limit(bytes); });
 }
 
+extern "C" int m3d_test_fail_multigrid_alloc(m3d_solver* h, int on) {
+    return guarded(h, [&](m3d::GpuSolver& s) { s.test_fail_emg = on != 0; });
+}
+
 extern "C" int m3d_test_set_multigrid_scale(m3d_solver* h, float f) {
     if (!ready(h)) return fail(h, M3D_ERR_STATE, "solver not set up");
     if (!(f > 0.0f)) return fail(h, M3D_ERR_ARG, "scale must be > 0");

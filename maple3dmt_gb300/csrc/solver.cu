@@ -657,8 +657,18 @@ void GpuSolver::split_csr(std::vector<int>& rp, std::vector<int>& rs, std::vecto
 
 // Uniform grids, transfers and face weights of the geometric multigrid
 // preconditioner (host/edgemg.cpp), once per mesh; work vectors for up to
-// 16 right-hand sides.  Meshes outside its rule keep emg_ok = false.
+// 16 right-hand sides.  Meshes outside its rule keep emg_ok = false, and so do
+// meshes whose grids do not fit the memory left: they take SSOR.
 void GpuSolver::build_emg() {
+    try {
+        alloc_emg();
+    } catch (const std::bad_alloc&) {
+        cudaGetLastError();
+        free_emg();
+    }
+}
+
+void GpuSolver::alloc_emg() {
     std::vector<char> free(L.ne);
     for (int e = 0; e < L.ne; ++e) free[e] = !(flags_ref[e] & kFlagConstrained);
     EmgHost H;
@@ -670,6 +680,7 @@ void GpuSolver::build_emg() {
         return p;
     };
     auto zeros = [&](size_t n) {
+        if (test_fail_emg && emg_mem.size() > 8) throw std::bad_alloc();
         float2* p = dalloc_zero<float2>(n, stream);
         emg_mem.push_back((void*)p);
         return p;

@@ -304,6 +304,10 @@ class ForwardSolverFV:
         """Test hook: staged kernels take their copy-wait timeout path."""
         self._ck(self.lib.m3d_test_set_consume_no_wait(self.h, 1 if on else 0))
 
+    def test_fail_multigrid_alloc(self, on: bool):
+        """Test hook of set-up without memory for the multigrid grids (see m3d_gb300.h)."""
+        self._ck(self.lib.m3d_test_fail_multigrid_alloc(self.h, 1 if on else 0))
+
     def test_set_smem_limit(self, n_bytes: int):
         """Test hook of the sparse product's launch rule (see m3d_gb300.h)."""
         self._ck(self.lib.m3d_test_set_smem_limit(self.h, int(n_bytes)))

@@ -105,3 +105,30 @@ def test_strong_contrasts(lib, model):
         s.close()
     for f in range(3):
         assert rel(Z[1][f], Z[0][f]) < 1e-6
+
+
+def test_setup_without_memory_for_the_grids(lib):
+    """Set-up succeeds, solves run SSOR: more iterations, the same impedances, no
+    multigrid to scale; set up again with memory, the handle has it."""
+    from maple3dmt_gb300 import mesh
+    from maple3dmt_gb300.solver import ForwardSolverFV, SolverError, solver_for_survey
+    sv = mesh.small_survey(min_level=4, max_level=5, freqs=FREQS)
+    par = dict(bicgstab_tol=1e-10, bicgstab_maxiter=5000, precision=1)
+    m = solver_for_survey(sv, **par)
+    want = m.forward_batch(FREQS)
+    s = ForwardSolverFV(0)
+    for fail in (True, False):
+        s.test_fail_multigrid_alloc(fail)
+        s.setup(sv.leaves, sigma_bg=sv.sigma_bg, **par)
+        s.set_sigma(sv.sigma)
+        s.set_stations(sv.stations)
+        got = s.forward_batch(FREQS)
+        st = s.stats()
+        assert st["status"][:6] == [CONVERGED] * 6
+        if fail:
+            assert rel(got, want) < 1e-6
+            assert sum(st["iterations"][:6]) > 1.5 * sum(m.stats()["iterations"][:6])
+            with pytest.raises(SolverError):
+                s.test_set_multigrid_scale(1.0)
+        else:
+            assert np.array_equal(got, want)
