@@ -34,6 +34,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "common.cuh"
 #include "tc.cuh"
 
 namespace m3d {
@@ -213,7 +214,6 @@ __global__ void __launch_bounds__(128, 1) k_conv3d_tc(const __grid_constant__ CU
 //                    accumulator, bias / ReLU / mask, BF16 store.
 // Every wait is bounded; a timeout flags an error and every role stops.
 constexpr int kHaloMaxW = 64;      // three boxes and the weights in shared memory
-constexpr int kWgradMaxW = 128;     // two boxes of one x shift
 __host__ __device__ constexpr int halo_box_bytes(int W) { return (128 + 2 * W) * 3 * 64; }
 constexpr int halo_smem(int W) { return kTaps * kTapB + 3 * halo_box_bytes(W) + 1024; }
 
@@ -893,13 +893,8 @@ void Cnn::ensure(int n, int D_, int H_, int W_) {
 
 void Cnn::conv(int l, bool transposed, const CUtensorMap& in_map, const CUtensorMap& in_hmap,
                const __nv_bfloat16* mask, __nv_bfloat16* out, float* o32, int n32, int n) {
-    static bool attr = false;
-    if (!attr) {
-        ck(cudaFuncSetAttribute(k_conv3d_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem), "attr");
-        ck(cudaFuncSetAttribute(k_conv3d_halo, cudaFuncAttributeMaxDynamicSharedMemorySize, halo_smem(kHaloMaxW)),
-           "attr");
-        attr = true;
-    }
+    dev::lift_smem_limit(reinterpret_cast<const void*>(k_conv3d_tc));
+    dev::lift_smem_limit(reinterpret_cast<const void*>(k_conv3d_halo));
     ConvArgs a{};
     a.D = D; a.H = H; a.W = W; a.bw = bw; a.bh = bh; a.tiles_h = H / bh;
     a.bias = transposed ? nullptr : b32 + (size_t)l * kCh;
@@ -931,12 +926,7 @@ const float* Cnn::forward(int n) {
 }
 
 void Cnn::wgrad(int l, const CUtensorMap& x_hmap, const CUtensorMap& d_map, int n) {
-    static bool attr = false;
-    if (!attr) {
-        ck(cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem(kWgradMaxW)),
-           "attr");
-        attr = true;
-    }
+    dev::lift_smem_limit(reinterpret_cast<const void*>(k_wgrad_tc));
     WgradArgs a{};
     a.D = D; a.bw = bw; a.bh = bh; a.tiles_h = H / bh;
     a.n_tiles = n * D * (H / bh);
