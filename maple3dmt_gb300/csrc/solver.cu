@@ -2712,9 +2712,9 @@ std::vector<TuneEntry> GpuSolver::autotune(double freq, int max_K, int reps) {
     max_K = std::max(2, std::min(dev::kMaxRhs, max_K));
     factorize(std::vector<double>{freq});
     ensure_vecs32(max_K);
-    ensure_sweeps(seg32);
     const double om = 2.0 * kPi * freq;
     const bool use_gc = gc_ok && P.gradcorr == 1 && gc.omega_max > 0.0 && om <= gc.omega_max;
+    if (!(use_gc && emg_ok)) ensure_sweeps(seg32);
     const int rk_saved = P.row_kernels;
     std::vector<TuneEntry> out;
     cudaEvent_t e0, e1;
