@@ -484,6 +484,11 @@ int m3d_test_set_consume_no_wait(m3d_solver* s, int on);
  * preconditioner (host only). */
 int m3d_test_multigrid_levels(int lmin, int lmax);
 
+/* Sums v[n][K] (complex, interleaved, host; K = 2, 4, 8 or 16) over n by the
+ * grid reductions of the FP32 kernels into out[K] (complex): a value a thread
+ * (n K <= 311296), or, with many != 0, many values a thread. */
+int m3d_test_sum_f32(const float* v, long long n, int K, int many, double* out);
+
 /* The shared memory per block that the sparse product plans its ring of
  * matrix tiles for (at least two tiles of 32 rows are taken); 0: the
  * device's. */

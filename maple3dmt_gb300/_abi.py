@@ -67,6 +67,7 @@ def declare(lib) -> None:
     _fn(lib, "m3d_layout_stiffness", C.c_int, [vp, c_int_p, c_int_p, c_double_p])
     _fn(lib, "m3d_layout_hanging", C.c_int, [vp, c_int_p])
     _fn(lib, "m3d_test_multigrid_levels", C.c_int, [C.c_int, C.c_int])
+    _fn(lib, "m3d_test_sum_f32", C.c_int, [C.POINTER(C.c_float), C.c_longlong, C.c_int, C.c_int, c_double_p])
     if hasattr(lib, "m3d_solver_create"):
         from . import _abi_solver
         _abi_solver.declare(lib)

@@ -25,7 +25,8 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 HOST_SRCS = ["host/octree_build.cpp", "host/mesh_capi.cpp", "host/layout.cpp", "host/layout_capi.cpp", "host/amg.cpp",
              "host/regularization.cpp", "host/edgemg.cpp"]
 CUDA_SRCS = ["cuda/krylov.cu", "cuda/physics.cu", "cuda/gradcorr.cu", "cuda/edgemg.cu", "cuda/regularization.cu", "cuda/dot.cu",
-             "cuda/learned.cu", "solver.cu", "learned_solver.cu", "capi.cu", "noalloc.cu", "learned_capi.cu"]
+             "cuda/learned.cu", "solver.cu", "learned_solver.cu", "capi.cu", "noalloc.cu", "learned_capi.cu",
+             "sum_test.cu"]
 
 
 def _nvcc() -> str:

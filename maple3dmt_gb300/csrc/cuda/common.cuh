@@ -64,40 +64,57 @@ __device__ __forceinline__ double2 shfl_xor(double2 v, int m) {
     return v;
 }
 
-// A complex sum in the making, 16 bytes: FP64 for FP64 terms; for FP32 terms
-// two floats per part (Knuth's error-free sum of the high parts, 48 bits
-// kept).  An FP64 add holds a warp's pipe for 16 cycles on this GPU and a chain
-// of them is slow: summing lanes, warps and blocks in FP64 was 10 to 25 us of
-// every reducing FP32 kernel.
-template <class R> struct Sum;
-template <> struct Sum<double> {
-    double2 v;
-    __device__ __forceinline__ void set(double2 a) { v = a; }
-    __device__ __forceinline__ void add(const Sum& o) { v = cadd(v, o.v); }
-    __device__ __forceinline__ Sum xor_lane(int m) const { return {shfl_xor(v, m)}; }
-    __device__ __forceinline__ double2 get() const { return v; }
+// A sum of FP32 terms in the making: three floats, the sum, the sum of its
+// rounding errors and that of theirs (Knuth's error-free two-sum; Ogita, Rump
+// and Oishi's SumK, 2005, K = 3), some 70 bits in all; each waits four cycles
+// for its own last value only.  An FP64 add holds a warp's pipe for 16 cycles
+// on this GPU and a chain of them is slow: summing lanes, warps and blocks in
+// FP64 was 10 to 25 us of every reducing FP32 kernel; two floats would keep 48
+// bits where FP64 keeps 53.  Sums that leave the FP32 range are done over in
+// FP64 (grid_reduce_f32).
+struct Sum3 {
+    float h = 0.0f, m = 0.0f, l = 0.0f;
+    static __device__ __forceinline__ float two_sum(float a, float b, float& e) {
+        const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+        e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+        return s;
+    }
+    __device__ __forceinline__ void add(float a) {
+        float e, f;
+        h = two_sum(h, a, e);
+        m = two_sum(m, e, f);
+        l = __fadd_rn(l, f);
+    }
+    __device__ __forceinline__ void add(const Sum3& o) {
+        float e, f, g;
+        h = two_sum(h, o.h, e);
+        m = two_sum(m, o.m, f);
+        m = two_sum(m, e, g);
+        l = __fadd_rn(l, __fadd_rn(o.l, __fadd_rn(f, g)));
+    }
+    __device__ __forceinline__ Sum3 xor_lane(int q) const {
+        Sum3 o;
+        o.h = __shfl_xor_sync(0xffffffffu, h, q);
+        o.m = __shfl_xor_sync(0xffffffffu, m, q);
+        o.l = __shfl_xor_sync(0xffffffffu, l, q);
+        return o;
+    }
+    __device__ __forceinline__ bool finite() const { return fabsf(h) <= 3.402823466e38f && m == m; }
+    __device__ __forceinline__ double get() const { return (double)h + ((double)m + (double)l); }
 };
-template <> struct Sum<float> {
-    float4 v;   // x high, x low, y high, y low
-    __device__ __forceinline__ void set(float2 a) { v = make_float4(a.x, 0.0f, a.y, 0.0f); }
-    static __device__ __forceinline__ void add1(float& h, float& l, float h2, float l2) {
-        const float s = __fadd_rn(h, h2), b = __fsub_rn(s, h);
-        float e = __fadd_rn(__fsub_rn(h, __fsub_rn(s, b)), __fsub_rn(h2, b));
-        e = __fadd_rn(e, __fadd_rn(l, l2));
-        h = __fadd_rn(s, e);
-        l = __fsub_rn(e, __fsub_rn(h, s));
-    }
-    __device__ __forceinline__ void add(const Sum& o) {
-        add1(v.x, v.y, o.v.x, o.v.y);
-        add1(v.z, v.w, o.v.z, o.v.w);
-    }
-    __device__ __forceinline__ Sum xor_lane(int m) const {
-        return {make_float4(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m),
-                            __shfl_xor_sync(0xffffffffu, v.z, m), __shfl_xor_sync(0xffffffffu, v.w, m))};
-    }
-    __device__ __forceinline__ void add_real(float a) { add1(v.x, v.y, a, 0.0f); }
-    __device__ __forceinline__ double2 get() const {
-        return make_double2((double)v.x + (double)v.y, (double)v.z + (double)v.w);
+
+// One thread's sum over many terms: what would leave the FP32 range goes on in
+// FP64.
+struct ThreadSum {
+    Sum3 s;
+    double over = 0.0;
+    __device__ __forceinline__ void add(float a) {
+        if (fabsf(s.h) + fabsf(a) <= 3e38f) {
+            s.add(a);
+        } else {
+            over += s.get() + (double)a;
+            s = Sum3();
+        }
     }
 };
 
@@ -179,8 +196,8 @@ inline int range_grid(long n, int threads = kBlock) {
     return (int)(b < 1 ? 1 : b < 1216 ? b : 1216);
 }
 
-// Scratch for grid reductions: partial[block][kMaxQ * kMaxRhs] and a counter
-// that the last block resets.
+// Scratch for grid reductions: partial[block][kMaxQ * kMaxRhs] (two double2
+// each) and a counter that the last block resets.
 struct RedScratch {
     double2* partial;
     double2* final_;      // [kMaxQ * kMaxRhs], result of the last reduction
@@ -188,48 +205,43 @@ struct RedScratch {
     int max_blocks;
 };
 
-// Grid reduction for kernels whose lane l always works on the same right-hand
-// sides: LPT neighbouring ones per thread, LPT (l % (K / LPT)) and the next
-// (K and LPT powers of two, whole warps); acc[j][q] is quantity q of the j-th
-// of them in the kernel's working precision.  Shuffle trees over the lanes that
-// share a right-hand side, then over the block's warps, then, in the last block
-// to arrive, over the blocks, all totals side by side: every step in a fixed
-// order, so the result is deterministic for a fixed launch shape.  Returns true
-// in the last block, where out[q * K + k] (shared, NQ*K entries) holds the
-// totals.
-template <int NQ, int K, int NT, int LPT, class S>
-__device__ bool grid_reduce_sums(const S (&acc)[LPT][NQ], RedScratch rs, double2* out) {
-    static_assert(K >= LPT && K <= 32 && (K & (K - 1)) == 0, "K must be a power of two <= 32");
+// Grid reductions for kernels whose thread t always works on the same
+// right-hand sides, LPT neighbouring ones, LPT (t % (K / LPT)) and the next (K
+// and LPT powers of two, whole warps).  Every step in a fixed order, so the
+// result is deterministic for a fixed launch shape.  They return true in the
+// last block to arrive, where out (shared) holds the totals.
+
+// FP64 terms, one right-hand side a thread: acc[q] is quantity q; out[q * K + k].
+// Shuffle trees over the lanes that share a right-hand side, then over the
+// block's warps, then, in the last block, over the blocks, all totals at once.
+template <int NQ, int K, int NT = kBlock>
+__device__ bool grid_reduce_lanes(const double2 (&acc)[NQ], RedScratch rs, double2* out) {
+    static_assert(K >= 1 && K <= 32 && (K & (K - 1)) == 0, "K must be a power of two <= 32");
     static_assert(NT % 32 == 0 && NT >= 32 && NT <= 1024, "block size must be whole warps");
-    static_assert(sizeof(S) == sizeof(double2), "partials are 16 bytes");
     constexpr int PK = NQ * K;
     constexpr int NW = NT / 32;
-    __shared__ S sm[NW][PK];
+    __shared__ double2 sm[NW][PK];
     __shared__ bool am_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int j = 0; j < LPT; ++j)
+    for (int q = 0; q < NQ; ++q) {
+        double2 s = acc[q];
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            S s = acc[j][q];
-#pragma unroll
-            for (int off = 16; off >= K / LPT; off >>= 1) s.add(s.xor_lane(off));
-            if (lane < K / LPT) sm[warp][q * K + lane * LPT + j] = s;
-        }
+        for (int off = 16; off >= K; off >>= 1) s = cadd(s, shfl_xor(s, off));
+        if (lane < K) sm[warp][q * K + lane] = s;
+    }
     __syncthreads();
-    S zero{};
-    S* partial = reinterpret_cast<S*>(rs.partial);
     // GW lanes per total, one for each warp of the block
     constexpr int GW = NW <= 1 ? 1 : NW <= 2 ? 2 : NW <= 4 ? 4 : NW <= 8 ? 8 : NW <= 16 ? 16 : 32;
 #pragma unroll
     for (int p0 = 0; p0 < PK; p0 += NT / GW) {
         const int p = p0 + threadIdx.x / GW, w = threadIdx.x % GW;
         if (p0 + warp * (32 / GW) >= PK) break;   // idle warps would add zeros, 16 cycles an FP64 add
-        S s = w < NW && p < PK ? sm[w][p] : zero;
+        double2 s = w < NW && p < PK ? sm[w][p] : make_double2(0.0, 0.0);
 #pragma unroll
-        for (int off = GW / 2; off > 0; off >>= 1) s.add(s.xor_lane(off));
+        for (int off = GW / 2; off > 0; off >>= 1) s = cadd(s, shfl_xor(s, off));
         if (w == 0 && p < PK) {
-            __stcg(reinterpret_cast<double2*>(&partial[(size_t)blockIdx.x * PK + p]), *reinterpret_cast<double2*>(&s));
+            __stcg(&rs.partial[(size_t)blockIdx.x * PK + p], s);
             __threadfence();
         }
     }
@@ -247,23 +259,21 @@ __device__ bool grid_reduce_sums(const S (&acc)[LPT][NQ], RedScratch rs, double2
     static_assert(Q >= 1, "a thread per total");
     const int p = threadIdx.x / TPT, l = threadIdx.x % TPT;
     if (warp * (32 / TPT) < PK) {
-        S s = zero;
+        double2 s = make_double2(0.0, 0.0);
         for (int b = l; p < PK && b < (int)gridDim.x; b += 4 * TPT) {   // four loads in flight
             double2 v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                v[u] = b + TPT * u < (int)gridDim.x
-                           ? __ldcg(reinterpret_cast<const double2*>(&partial[(size_t)(b + TPT * u) * PK + p]))
-                           : make_double2(0.0, 0.0);
+                v[u] = b + TPT * u < (int)gridDim.x ? __ldcg(&rs.partial[(size_t)(b + TPT * u) * PK + p])
+                                                    : make_double2(0.0, 0.0);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) s.add(*reinterpret_cast<const S*>(&v[u]));
+            for (int u = 0; u < 4; ++u) s = cadd(s, v[u]);
         }
 #pragma unroll
-        for (int off = TPT / 2; off > 0; off >>= 1) s.add(s.xor_lane(off));
+        for (int off = TPT / 2; off > 0; off >>= 1) s = cadd(s, shfl_xor(s, off));
         if (l == 0 && p < PK) {
-            const double2 t = s.get();
-            out[p] = t;
-            rs.final_[p] = t;
+            out[p] = s;
+            rs.final_[p] = s;
         }
     }
     if (threadIdx.x == 0) *rs.counter = 0u;
@@ -271,14 +281,174 @@ __device__ bool grid_reduce_sums(const S (&acc)[LPT][NQ], RedScratch rs, double2
     return true;
 }
 
-template <int NQ, int K, int NT, int LPT, class C>
-__device__ __forceinline__ bool grid_reduce_multi(const C (&acc)[LPT][NQ], RedScratch rs, double2* out) {
-    Sum<decltype(C{}.x)> s[LPT][NQ];
+// FP32 terms: v[j][r] is real quantity r of this thread's j-th right-hand side,
+// a float or a ThreadSum; total r of right-hand side k goes to out[r K + k].x, or
+// (CPLX) out[(r / 2) K + k], x for even r and y for odd.  sh: scratch of
+// red_floats<T>(NT, LPT * NR) floats, free at the call.  The threads' values go
+// through shared memory: GL lanes per total sum those of its row groups, then a
+// tree; the block totals lie in rs.partial as (h, m, l, 1), or, where a sum has
+// left the FP32 range or is not finite, as an FP64 sum of the same values (its
+// two words, 0, 2), and the last block does likewise.
+template <class T> struct RedTerm;
+template <> struct RedTerm<float> {
+    static constexpr int kParts = 1;
+    static __device__ __forceinline__ void put(float* at, int, float v) { *at = v; }
+    static __device__ __forceinline__ bool over(float) { return false; }
+};
+template <> struct RedTerm<ThreadSum> {
+    static constexpr int kParts = 3;
+    static __device__ __forceinline__ void put(float* at, int stride, const ThreadSum& v) {
+        at[0] = v.s.h;
+        at[stride] = v.s.m;
+        at[2 * stride] = v.s.l;
+    }
+    static __device__ __forceinline__ bool over(const ThreadSum& v) { return !(v.over == 0.0); }
+};
+template <class T> constexpr int red_floats(int NT, int values) { return NT * values * RedTerm<T>::kParts; }
+
+template <int NR, bool CPLX, int K, int NT, int LPT, class T>
+__device__ bool grid_reduce_f32(const T (&v)[LPT][NR], RedScratch rs, double2* out, float* sh) {
+    using Term = RedTerm<T>;
+    constexpr int P = Term::kParts, TPR = K / LPT, G = NT / TPR, R = NR * K, Q = NT / R;
+    constexpr int GL = Q >= 32 ? 32 : Q >= 16 ? 16 : Q >= 8 ? 8 : Q >= 4 ? 4 : Q >= 2 ? 2 : 1;
+    static_assert(K >= LPT && K <= 32 && (K & (K - 1)) == 0 && NT % 32 == 0 && NT % TPR == 0, "launch shape");
+    static_assert(Q >= 1 && R <= 2 * kMaxQ * kMaxRhs, "a thread per total, and its place in the scratch");
+    __shared__ bool am_last;
+    const int warp = threadIdx.x >> 5, p = threadIdx.x / GL, l = threadIdx.x % GL;
+    const bool mine = p < R, busy = warp * (32 / GL) < R;
+    const int k = p % K, r = p / K;
+    bool wide = false;   // this block's totals in FP64
 #pragma unroll
     for (int j = 0; j < LPT; ++j)
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) s[j][q].set(acc[j][q]);
-    return grid_reduce_sums<NQ, K, NT, LPT>(s, rs, out);
+        for (int q = 0; q < NR; ++q) {
+            Term::put(sh + (size_t)((j * NR + q) * P) * NT + threadIdx.x, NT, v[j][q]);
+            wide |= Term::over(v[j][q]);
+        }
+    if constexpr (P == 1) __syncthreads();
+    else wide = __syncthreads_or(wide) != 0;
+    const float* at = sh + (size_t)(((k % LPT) * NR + r) * P) * NT + k / LPT;
+    Sum3 s;
+    if (busy && !wide) {
+        // in rounds of eight, their loads and sums side by side
+#pragma unroll
+        for (int g0 = 0; g0 < G; g0 += 8 * GL) {
+            float a[8 * P];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int u = 0; u < P; ++u) {
+                    const int g = g0 + i * GL + l;
+                    a[i * P + u] = mine && g < G ? at[u * NT + g * TPR] : 0.0f;
+                }
+#pragma unroll
+            for (int i = 0; i < 8 * P; ++i)
+                if (g0 + i / P * GL < G) s.add(a[i]);
+        }
+#pragma unroll
+        for (int off = GL / 2; off > 0; off >>= 1) s.add(s.xor_lane(off));
+    }
+    float4* partial = reinterpret_cast<float4*>(rs.partial);
+    auto publish = [&](float4 q) {
+        if (mine && l == 0) {
+            __stcg(&partial[(size_t)blockIdx.x * R + p], q);
+            __threadfence();
+        }
+    };
+    publish(make_float4(s.h, s.m, s.l, 1.0f));
+    wide = __syncthreads_or(wide || (mine && !s.finite())) != 0;
+    if (wide) {
+        double* shd = reinterpret_cast<double*>(sh);
+        if constexpr (P == 3) {   // room for a double in a ThreadSum's three floats
+#pragma unroll
+            for (int j = 0; j < LPT; ++j)
+#pragma unroll
+                for (int q = 0; q < NR; ++q) shd[(size_t)(j * NR + q) * NT + threadIdx.x] = v[j][q].s.get() + v[j][q].over;
+            __syncthreads();
+        }
+        double d = 0.0;
+        if (busy) {
+            for (int g = l; mine && g < G; g += GL)
+                d += P == 3 ? shd[(size_t)((k % LPT) * NR + r) * NT + k / LPT + g * TPR] : (double)at[g * TPR];
+#pragma unroll
+            for (int off = GL / 2; off > 0; off >>= 1) d += shfl_xor(d, off);
+        }
+        publish(make_float4(__int_as_float(__double2hiint(d)), __int_as_float(__double2loint(d)), 0.0f, 2.0f));
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const unsigned t = atomicAdd(rs.counter, 1u);
+        am_last = (t == gridDim.x - 1);
+    }
+    __syncthreads();
+    if (!am_last) return false;
+    __threadfence();
+    s = Sum3();
+    wide = false;
+    if (busy) {
+        for (int b = l; mine && b < (int)gridDim.x; b += 8 * GL) {   // eight loads in flight
+            float4 q[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                q[u] = b + GL * u < (int)gridDim.x ? __ldcg(&partial[(size_t)(b + GL * u) * R + p])
+                                                   : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                Sum3 o;
+                o.h = q[u].x;
+                o.m = q[u].y;
+                o.l = q[u].z;
+                s.add(o);
+                wide |= q[u].w != 1.0f;
+            }
+        }
+#pragma unroll
+        for (int off = GL / 2; off > 0; off >>= 1) s.add(s.xor_lane(off));
+    }
+    double total = s.get();
+    if (__syncthreads_or(wide || (mine && !s.finite()))) {
+        total = 0.0;
+        if (busy) {
+            for (int b = l; mine && b < (int)gridDim.x; b += GL) {
+                const float4 q = __ldcg(&partial[(size_t)b * R + p]);
+                total += q.w == 1.0f ? (double)q.x + ((double)q.y + (double)q.z)
+                                     : __hiloint2double(__float_as_int(q.x), __float_as_int(q.y));
+            }
+#pragma unroll
+            for (int off = GL / 2; off > 0; off >>= 1) total += shfl_xor(total, off);
+        }
+    }
+    if (mine && l == 0) {
+        double2* o = &out[(CPLX ? r / 2 : r) * K + k];
+        if (CPLX && (r & 1)) o->y = total;
+        else o->x = total;
+    }
+    if (threadIdx.x == 0) *rs.counter = 0u;
+    __syncthreads();
+    return true;
+}
+
+// The same for complex terms of either precision, acc[j][q]; out[q * K + k].
+template <int NQ, int K, int NT, int LPT>
+__device__ __forceinline__ bool grid_reduce_multi(const float2 (&acc)[LPT][NQ], RedScratch rs, double2* out, float* sh) {
+    float v[LPT][2 * NQ];
+#pragma unroll
+    for (int j = 0; j < LPT; ++j)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            v[j][2 * q] = acc[j][q].x;
+            v[j][2 * q + 1] = acc[j][q].y;
+        }
+    return grid_reduce_f32<2 * NQ, true, K, NT, LPT>(v, rs, out, sh);
+}
+template <int NQ, int K, int NT, int LPT>
+__device__ __forceinline__ bool grid_reduce_multi(const double2 (&acc)[LPT][NQ], RedScratch rs, double2* out, float*) {
+    static_assert(LPT == 1, "FP64 kernels take one right-hand side a thread");
+    return grid_reduce_lanes<NQ, K, NT>(acc[0], rs, out);
+}
+// floats of scratch that it needs
+template <class R, int NQ> constexpr int multi_floats(int NT, int LPT) {
+    return sizeof(R) == 4 ? red_floats<float>(NT, LPT * 2 * NQ) : 0;
 }
 
 // Blocks of a reducing vector kernel over n elements: one resident wave at
@@ -292,11 +462,6 @@ inline int reduce_grid(F* kernel, int cap, long n, int threads = kBlock) {
     const long b = lo < 304 ? lo : hi < 304 ? 304 : hi;
     const int w = wave_grid(kernel, cap, threads);
     return (int)(b < 1 ? 1 : b < w ? b : w);
-}
-
-template <int NQ, int K, int NT = kBlock>
-__device__ __forceinline__ bool grid_reduce_lanes(double2 (&acc)[NQ], RedScratch rs, double2* out) {
-    return grid_reduce_multi<NQ, K, NT, 1>(*reinterpret_cast<const double2(*)[1][NQ]>(&acc), rs, out);
 }
 
 }  // namespace dev

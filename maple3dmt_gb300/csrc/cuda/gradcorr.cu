@@ -557,8 +557,8 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_start(int nn, DcWork w, GcDev 
 }
 
 // The FP32 PCG's kernels: two right-hand sides per thread; the inner products'
-// FP32 terms are summed as two floats (dev::Sum), 48 bits -- FP64 adds per
-// element made each of them 13 to 20 us on the 157 k-edge mesh.
+// FP32 terms are summed as three floats (dev::ThreadSum), 70 bits -- FP64 adds
+// per element made each of them 13 to 20 us on the 157 k-edge mesh.
 __device__ __forceinline__ const float4* c4(const float2* p) { return reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4* m4(float2* p) { return reinterpret_cast<float4*>(p); }
 
@@ -571,15 +571,16 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_first(int nn, GcDev g, RedScra
     const long stride = (long)gridDim.x * blockDim.x;
     const int k = (int)(2 * i0 % K);
     const bool ra = g.dc_st[k].run, rb = g.dc_st[k + 1].run;
-    Sum<float> acc[2][1] = {};
+    ThreadSum acc[2][1];
     for (long i = i0; i < n && (ra || rb); i += stride) {
         const float4 r = c4(g.dc_r)[i], z = c4(g.dc_z)[i];
         m4(g.dc_p)[i] = z;
-        acc[0][0].add_real(r.x * z.x + r.y * z.y);
-        acc[1][0].add_real(r.z * z.z + r.w * z.w);
+        acc[0][0].add(r.x * z.x + r.y * z.y);
+        acc[1][0].add(r.z * z.z + r.w * z.w);
     }
     __shared__ double2 out[K];
-    if (grid_reduce_sums<1, K, kGcBlock, 2>(acc, rs, out)) {
+    __shared__ __align__(8) float sh[red_floats<ThreadSum>(kGcBlock, 2)];
+    if (grid_reduce_f32<1, false, K, kGcBlock, 2>(acc, rs, out, sh)) {
         if (threadIdx.x < K && g.dc_st[threadIdx.x].run) g.dc_st[threadIdx.x].rz = out[threadIdx.x].x;
     }
 }
@@ -595,7 +596,7 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_ap(int nn, GcDev g, RedScratch
     const int k = (int)(2 * i0 % K);
     const bool ra = g.dc_st[k].run, rb = g.dc_st[k + 1].run;
     const float4* p = c4(g.dc_p);
-    Sum<float> acc[2][1] = {};
+    ThreadSum acc[2][1];
     for (long i = i0; i < n && (ra || rb); i += stride) {
         const int v = (int)(i / H), h = (int)(i % H);
         const float4 pv = p[i];
@@ -620,11 +621,12 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_ap(int nn, GcDev g, RedScratch
             }
         }
         m4(g.dc_ap)[i] = s;
-        acc[0][0].add_real(pv.x * s.x + pv.y * s.y);
-        acc[1][0].add_real(pv.z * s.z + pv.w * s.w);
+        acc[0][0].add(pv.x * s.x + pv.y * s.y);
+        acc[1][0].add(pv.z * s.z + pv.w * s.w);
     }
     __shared__ double2 out[K];
-    if (grid_reduce_sums<1, K, kGcBlock, 2>(acc, rs, out)) {
+    __shared__ __align__(8) float sh[red_floats<ThreadSum>(kGcBlock, 2)];
+    if (grid_reduce_f32<1, false, K, kGcBlock, 2>(acc, rs, out, sh)) {
         if (threadIdx.x < K) {
             GcPcgState T = g.dc_st[threadIdx.x];
             if (T.run) {
@@ -647,7 +649,7 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_update(int nn, GcDev g, int ca
     const int k = (int)(2 * i0 % K);
     const bool ra = g.dc_st[k].run, rb = g.dc_st[k + 1].run;
     const float la = ra ? (float)g.dc_st[k].alpha : 0.0f, lb = rb ? (float)g.dc_st[k + 1].alpha : 0.0f;
-    Sum<float> acc[2][1] = {};
+    ThreadSum acc[2][1];
     for (long i = i0; i < n && (ra || rb); i += stride) {
         const float4 p = c4(g.dc_p)[i], ap = c4(g.dc_ap)[i];
         float4 x = c4(g.dc_x)[i], r = c4(g.dc_r)[i];
@@ -665,11 +667,12 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_update(int nn, GcDev g, int ca
         }
         m4(g.dc_x)[i] = x;
         m4(g.dc_r)[i] = r;
-        acc[0][0].add_real(r.x * r.x + r.y * r.y);
-        acc[1][0].add_real(r.z * r.z + r.w * r.w);
+        acc[0][0].add(r.x * r.x + r.y * r.y);
+        acc[1][0].add(r.z * r.z + r.w * r.w);
     }
     __shared__ double2 out[K];
-    if (grid_reduce_sums<1, K, kGcBlock, 2>(acc, rs, out)) {
+    __shared__ __align__(8) float sh[red_floats<ThreadSum>(kGcBlock, 2)];
+    if (grid_reduce_f32<1, false, K, kGcBlock, 2>(acc, rs, out, sh)) {
         if (threadIdx.x < K) {
             GcPcgState T = g.dc_st[threadIdx.x];
             if (T.run) {
@@ -690,14 +693,15 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_rz(int nn, GcDev g, RedScratch
     const long stride = (long)gridDim.x * blockDim.x;
     const int k = (int)(2 * i0 % K);
     const bool run = g.dc_st[k].run || g.dc_st[k + 1].run;
-    Sum<float> acc[2][1] = {};
+    ThreadSum acc[2][1];
     for (long i = i0; i < n && run; i += stride) {
         const float4 r = c4(g.dc_r)[i], z = c4(g.dc_z)[i];
-        acc[0][0].add_real(r.x * z.x + r.y * z.y);
-        acc[1][0].add_real(r.z * z.z + r.w * z.w);
+        acc[0][0].add(r.x * z.x + r.y * z.y);
+        acc[1][0].add(r.z * z.z + r.w * z.w);
     }
     __shared__ double2 out[K];
-    if (grid_reduce_sums<1, K, kGcBlock, 2>(acc, rs, out)) {
+    __shared__ __align__(8) float sh[red_floats<ThreadSum>(kGcBlock, 2)];
+    if (grid_reduce_f32<1, false, K, kGcBlock, 2>(acc, rs, out, sh)) {
         if (threadIdx.x < K) {
             GcPcgState T = g.dc_st[threadIdx.x];
             if (T.run) {

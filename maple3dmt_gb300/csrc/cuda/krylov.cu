@@ -591,7 +591,9 @@ __global__ void __launch_bounds__(SpmvShape<R, K>::NT, 1)
     });
     if (!REDUCE) return;
     __shared__ double2 out[NQ * K];
-    if (grid_reduce_multi<NQ, K, Sh::NT, Sh::LPT>(accR, rs, out)) {
+    // the ring's memory is free: every copy has landed and been read
+    extern __shared__ __align__(128) unsigned char dsm[];
+    if (grid_reduce_multi<NQ, K, Sh::NT, Sh::LPT>(accR, rs, out, reinterpret_cast<float*>(dsm))) {
         if (threadIdx.x < K) {
             BicgState T = st[threadIdx.x];
             if (MODE == kSpmvAp) ep_r0v(T, out, threadIdx.x, K);
@@ -852,7 +854,8 @@ __global__ void __launch_bounds__(kVecNT) k_update_s(long n, const cplx<R>* r_,
         s[i] = sv;
     }
     __shared__ double2 out[K];
-    if (grid_reduce_multi<1, K, kVecNT, LPT>(acc, rs, out)) {
+    __shared__ float red[multi_floats<R, 1>(kVecNT, LPT) + 1];
+    if (grid_reduce_multi<1, K, kVecNT, LPT>(acc, rs, out, red)) {
         if (threadIdx.x < K) {
             BicgState T = st[threadIdx.x];
             ep_s(T, out, threadIdx.x, K);
@@ -911,7 +914,8 @@ __global__ void __launch_bounds__(kVecNT) k_update_xr(long n, cplx<R>* __restric
         r[i] = rv;
     }
     __shared__ double2 out[2 * K];
-    if (grid_reduce_multi<2, K, kVecNT, LPT>(acc, rs, out)) {
+    __shared__ float red[multi_floats<R, 2>(kVecNT, LPT) + 1];
+    if (grid_reduce_multi<2, K, kVecNT, LPT>(acc, rs, out, red)) {
         if (threadIdx.x < K) {
             BicgState T = st[threadIdx.x];
             ep_xr(T, out, threadIdx.x, K);
@@ -965,7 +969,9 @@ void spmv_staged_mode(const KrylovCtx<R>& c, const cplx<R>* x, cplx<R>* y, const
         while (T > 1 && ring * c.seg.stage_row[T] > most) --T;
         while (ring > 2 && ring * c.seg.stage_row[T] > most) --ring;
     }
-    const int smem = ring * c.seg.stage_row[T];
+    constexpr int NQ = MODE == kSpmvAp ? 1 : MODE == kSpmvAs || MODE == kSpmvTrueRes ? 2 : 3;
+    constexpr int sums = MODE == kSpmvPlain || MODE == kSpmvSmooth ? 0 : 4 * multi_floats<R, NQ>(Sh::NT, Sh::LPT);
+    const int smem = std::max(ring * c.seg.stage_row[T], sums);
     const int g = std::min(wave_grid(kf, cap, Sh::NT, smem), std::max(1, (ns + T - 1) / T));
     // the modes of an iteration: a plain launch (the initial residual's, the
     // preconditioner's first) lies between them and whatever wrote the matrix

@@ -596,7 +596,7 @@ void GpuSolver::setup(const m3d_leaves* lv, const m3d_params* params) {
     cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "sm count");
     red.max_blocks = std::max(2, 8 * sms);
     red.max_blocks += red.max_blocks & 1;
-    red.partial = dalloc<double2>((size_t)red.max_blocks * dev::kMaxQ * dev::kMaxRhs);
+    red.partial = dalloc<double2>((size_t)red.max_blocks * 2 * dev::kMaxQ * dev::kMaxRhs);
     red.final_ = dalloc<double2>(dev::kMaxQ * dev::kMaxRhs);
     red.counter = dalloc<unsigned int>(1);
     cuda_ok(cudaMemsetAsync(red.counter, 0, sizeof(unsigned int), stream), "memset");
