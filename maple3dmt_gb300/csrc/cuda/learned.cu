@@ -415,7 +415,7 @@ constexpr int wgrad_smem(int W) { return kWgradStages * wgrad_stage(W) + 1024; }
 // contiguous lines.  24 MMAs a tile into three accumulators of 32 columns.
 //   warp 4 / lane 0  TMA producer, two stages;
 //   warp 5           allocates 128 TMEM columns; lane 0 issues the MMAs;
-//   warps 0-3        sum the gradient rows per channel in two-float arithmetic
+//   warps 0-3        sum the gradient rows per channel (dev::ThreadSum)
 //                    (blockIdx.y = 1 only), at the end store the accumulators.
 // Bound by the MMAs themselves (some 70 cycles each at N = 32; L2 at 38 % of its
 // rate, DRAM at 9 %): 22 us for 131 k voxels.  The former path gathered 27
@@ -453,9 +453,7 @@ __global__ void __launch_bounds__(192) k_wgrad_tc(const __grid_constant__ CUtens
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = tmem_base;
-    float hi[8], lo[8];   // warps 0-3: column sums of 8 channels
-#pragma unroll
-    for (int j = 0; j < 8; ++j) hi[j] = lo[j] = 0.0f;
+    dev::ThreadSum col[8];   // warps 0-3: column sums of 8 channels
     if (warp == 4) {
         if (lane == 0) {
             int it = 0;
@@ -526,12 +524,7 @@ __global__ void __launch_bounds__(192) k_wgrad_tc(const __grid_constant__ CUtens
                     const uint4 u = *reinterpret_cast<const uint4*>(dy + row * 64 + q * 16);
                     const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&u);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float x = __bfloat162float(h[j]);
-                        const float t = hi[j] + x, v = t - hi[j];
-                        lo[j] += (hi[j] - (t - v)) + (x - v);
-                        hi[j] = t;
-                    }
+                    for (int j = 0; j < 8; ++j) col[j].add(__bfloat162float(h[j]));
                 }
                 tc::mbar_arrive(&empty[s]);
             }
@@ -562,8 +555,7 @@ __global__ void __launch_bounds__(192) k_wgrad_tc(const __grid_constant__ CUtens
     if (bias && warp < 4) {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            sb[(threadIdx.x >> 2) * kCh + (threadIdx.x & 3) * 8 + j] =
-                isfinite(hi[j]) ? (double)hi[j] + (double)lo[j] : (double)hi[j];
+            sb[(threadIdx.x >> 2) * kCh + (threadIdx.x & 3) * 8 + j] = col[j].s.get() + col[j].over;
     }
     tc::tc_fence_before();
     __syncthreads();
