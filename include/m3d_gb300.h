@@ -494,6 +494,10 @@ int m3d_test_sum_f32(const float* v, long long n, int K, int many, double* out);
  * device's. */
 int m3d_test_set_smem_limit(m3d_solver* s, int bytes);
 
+/* on != 0: this solver's calls launch every kernel plainly, none as the
+ * dependent of its predecessor. */
+int m3d_test_set_plain_launches(m3d_solver* s, int on);
+
 /* on != 0: the next m3d_solver_setup finds no memory for the multigrid
  * preconditioner's grids, as a mesh near the device's size would. */
 int m3d_test_fail_multigrid_alloc(m3d_solver* s, int on);

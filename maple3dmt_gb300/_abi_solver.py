@@ -108,7 +108,7 @@ SOLVER_SYMBOLS = [
     "m3d_reg_apply_wtw", "m3d_reg_apply_cmcmt", "m3d_reg_diagonal_wtw", "m3d_reg_evaluate", "m3d_dot_batched", "m3d_dot_batched_noalloc", "m3d_get_stats",
     "m3d_timer_start", "m3d_timer_stop", "m3d_set_kernel_timing", "m3d_get_kernel_times",
     "m3d_test_set_consume_no_wait", "m3d_test_set_smem_limit",
-    "m3d_test_fail_multigrid_alloc", "m3d_test_set_multigrid_scale", "m3d_autotune",
+    "m3d_test_set_plain_launches", "m3d_test_fail_multigrid_alloc", "m3d_test_set_multigrid_scale", "m3d_autotune",
     "m3d_cnn_create", "m3d_cnn_destroy", "m3d_cnn_last_error", "m3d_cnn_get_weights", "m3d_cnn_set_weights",
     "m3d_cnn_forward", "m3d_cnn_backward", "m3d_cnn_train_step",
     "m3d_learn_setup", "m3d_learn_collect", "m3d_learn_train", "m3d_set_krylov",
@@ -163,6 +163,7 @@ def declare(lib) -> None:
     _fn(lib, "m3d_get_kernel_times", C.c_int, [vp, C.POINTER(KernelTimes)])
     _fn(lib, "m3d_test_set_consume_no_wait", C.c_int, [vp, C.c_int])
     _fn(lib, "m3d_test_set_smem_limit", C.c_int, [vp, C.c_int])
+    _fn(lib, "m3d_test_set_plain_launches", C.c_int, [vp, C.c_int])
     _fn(lib, "m3d_test_fail_multigrid_alloc", C.c_int, [vp, C.c_int])
     _fn(lib, "m3d_test_set_multigrid_scale", C.c_int, [vp, C.c_float])
     fp = C.POINTER(C.c_float)

@@ -33,6 +33,10 @@ int fail(m3d_solver* h, int code, const std::string& msg) {
 template <class F>
 int guarded(m3d_solver* h, F&& f) {
     if (!h || !h->s) return M3D_ERR_ARG;
+    struct Plain {
+        explicit Plain(bool on) { m3d::dev::plain_launches = on; }
+        ~Plain() { m3d::dev::plain_launches = false; }
+    } plain(h->s->test_plain_launches);
     try {
         f(*h->s);
         h->err.clear();
@@ -548,6 +552,10 @@ extern "C" int m3d_test_set_smem_limit(m3d_solver* h, int bytes) {
 
 extern "C" int m3d_test_fail_multigrid_alloc(m3d_solver* h, int on) {
     return guarded(h, [&](m3d::GpuSolver& s) { s.test_fail_emg = on != 0; });
+}
+
+extern "C" int m3d_test_set_plain_launches(m3d_solver* h, int on) {
+    return guarded(h, [&](m3d::GpuSolver& s) { s.test_plain_launches = on != 0; });
 }
 
 extern "C" int m3d_test_set_multigrid_scale(m3d_solver* h, float f) {

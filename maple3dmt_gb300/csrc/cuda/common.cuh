@@ -131,9 +131,10 @@ struct ThreadSum {
 //  * such data is not read through `const __restrict__` pointers or __ldg (the
 //    read-only path is not ordered behind the wait);
 //  * what is read before the wait was complete when the chain's first, plain
-//    launch started: a plain launch waits for all work before it.
-// dep_begin() is dep_trigger() (let the successor start) and dep_wait(); both
-// do nothing under a plain launch.
+//    launch started (a plain launch waits for all work before it) and is not
+//    written by that kernel either: it lets its successor start like the others.
+// dep_begin() is dep_trigger() (let the successor start, under any launch) and
+// dep_wait() (which does nothing under a plain launch).
 __device__ __forceinline__ void dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dep_begin() {
@@ -141,8 +142,12 @@ __device__ __forceinline__ void dep_begin() {
     dep_wait();
 }
 
+// Test hook: this thread's launches are plain ones (set for the time of a call).
+inline thread_local bool plain_launches = false;
+
 // Adds the attribute of a dependent launch, if the stream is not being captured.
 inline void dep_attr(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at) {
+    if (plain_launches) return;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(cfg.stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return;
     at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -60,6 +60,7 @@ public:
     void background_E(int pol, double* out);
     void set_test_consume_no_wait(bool on);   // test hook of the staged kernels' error path
     void set_test_smem_limit(int bytes) { seg64.smem_cap = seg32.smem_cap = bytes; }   // ... of the SpMV's launch rule
+    bool test_plain_launches = false;         // ... of dependent launches
     bool test_fail_emg = false;               // ... of set-up without memory for the multigrid preconditioner
     void set_test_multigrid_scale(float f);   // test hook of the fallback from multigrid to SSOR
     // times the FP32 inner solve for each row-kernel layout and batch width

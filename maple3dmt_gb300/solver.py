@@ -304,6 +304,10 @@ class ForwardSolverFV:
         """Test hook: staged kernels take their copy-wait timeout path."""
         self._ck(self.lib.m3d_test_set_consume_no_wait(self.h, 1 if on else 0))
 
+    def test_set_plain_launches(self, on: bool):
+        """Test hook of the dependent launches (see m3d_gb300.h)."""
+        self._ck(self.lib.m3d_test_set_plain_launches(self.h, 1 if on else 0))
+
     def test_fail_multigrid_alloc(self, on: bool):
         """Test hook of set-up without memory for the multigrid grids (see m3d_gb300.h)."""
         self._ck(self.lib.m3d_test_fail_multigrid_alloc(self.h, 1 if on else 0))
