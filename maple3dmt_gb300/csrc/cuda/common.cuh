@@ -70,8 +70,9 @@ __device__ __forceinline__ double2 shfl_xor(double2 v, int m) {
 // for its own last value only.  An FP64 add holds a warp's pipe for 16 cycles
 // on this GPU and a chain of them is slow: summing lanes, warps and blocks in
 // FP64 was 10 to 25 us of every reducing FP32 kernel; two floats would keep 48
-// bits where FP64 keeps 53.  Sums that leave the FP32 range are done over in
-// FP64 (grid_reduce_f32).
+// bits where FP64 keeps 53, and save 0.6 us a kernel (an iteration of two
+// right-hand sides on 20 k edges: 131 us, with two floats 129).  Sums that leave
+// the FP32 range are done over in FP64 (grid_reduce_f32).
 struct Sum3 {
     float h = 0.0f, m = 0.0f, l = 0.0f;
     static __device__ __forceinline__ float two_sum(float a, float b, float& e) {
@@ -103,19 +104,15 @@ struct Sum3 {
     __device__ __forceinline__ double get() const { return (double)h + ((double)m + (double)l); }
 };
 
-// One thread's sum over many terms: what would leave the FP32 range goes on in
-// FP64.
+// One thread's sum over up to 10^5 terms.  The terms of a round go to s if the
+// largest modulus among them is small, so that no such sum leaves the FP32
+// range, and to FP64 else: one test a round (a test a term kept the adds of
+// several sums from overlapping: 22 -> 35 us a layer in k_wgrad_tc).
 struct ThreadSum {
     Sum3 s;
     double over = 0.0;
-    __device__ __forceinline__ void add(float a) {
-        if (fabsf(s.h) + fabsf(a) <= 3e38f) {
-            s.add(a);
-        } else {
-            over += s.get() + (double)a;
-            s = Sum3();
-        }
-    }
+    static __device__ __forceinline__ bool small(float modulus) { return modulus <= 1e33f; }
+    __device__ __forceinline__ void add_large(float a) { over += (double)a; }
 };
 
 // Dependent launches.  A kernel launched by launch_dep may start while its
@@ -316,6 +313,7 @@ __device__ bool grid_reduce_f32(const T (&v)[LPT][NR], RedScratch rs, double2* o
     using Term = RedTerm<T>;
     constexpr int P = Term::kParts, TPR = K / LPT, G = NT / TPR, R = NR * K, Q = NT / R;
     constexpr int GL = Q >= 32 ? 32 : Q >= 16 ? 16 : Q >= 8 ? 8 : Q >= 4 ? 4 : Q >= 2 ? 2 : 1;
+    constexpr int U = (G + GL - 1) / GL < 4 ? (G + GL - 1) / GL : 4;
     static_assert(K >= LPT && K <= 32 && (K & (K - 1)) == 0 && NT % 32 == 0 && NT % TPR == 0, "launch shape");
     static_assert(Q >= 1 && R <= 2 * kMaxQ * kMaxRhs, "a thread per total, and its place in the scratch");
     __shared__ bool am_last;
@@ -335,20 +333,19 @@ __device__ bool grid_reduce_f32(const T (&v)[LPT][NR], RedScratch rs, double2* o
     const float* at = sh + (size_t)(((k % LPT) * NR + r) * P) * NT + k / LPT;
     Sum3 s;
     if (busy && !wide) {
-        // in rounds of eight, their loads and sums side by side
+        // in rounds, their loads and sums side by side
+#pragma unroll 1
+        for (int g0 = 0; g0 < G; g0 += U * GL) {
+            float a[U * P];
 #pragma unroll
-        for (int g0 = 0; g0 < G; g0 += 8 * GL) {
-            float a[8 * P];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < U; ++i)
 #pragma unroll
                 for (int u = 0; u < P; ++u) {
                     const int g = g0 + i * GL + l;
                     a[i * P + u] = mine && g < G ? at[u * NT + g * TPR] : 0.0f;
                 }
 #pragma unroll
-            for (int i = 0; i < 8 * P; ++i)
-                if (g0 + i / P * GL < G) s.add(a[i]);
+            for (int i = 0; i < U * P; ++i) s.add(a[i]);
         }
 #pragma unroll
         for (int off = GL / 2; off > 0; off >>= 1) s.add(s.xor_lane(off));
@@ -391,14 +388,18 @@ __device__ bool grid_reduce_f32(const T (&v)[LPT][NR], RedScratch rs, double2* o
     s = Sum3();
     wide = false;
     if (busy) {
-        for (int b = l; mine && b < (int)gridDim.x; b += 8 * GL) {   // eight loads in flight
-            float4 q[8];
+#pragma unroll 1
+        for (int b0 = 0; b0 < (int)gridDim.x; b0 += 4 * GL) {   // four loads in flight
+            float4 q[4];
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-                q[u] = b + GL * u < (int)gridDim.x ? __ldcg(&partial[(size_t)(b + GL * u) * R + p])
-                                                   : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+            for (int u = 0; u < 4; ++u) {
+                const int b = b0 + GL * u + l;
+                q[u] = mine && b < (int)gridDim.x ? __ldcg(&partial[(size_t)b * R + p])
+                                                  : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+            }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < 4; ++u) {
+                if (b0 + GL * u >= (int)gridDim.x) break;
                 Sum3 o;
                 o.h = q[u].x;
                 o.m = q[u].y;

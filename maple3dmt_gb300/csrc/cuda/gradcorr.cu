@@ -562,6 +562,16 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_start(int nn, DcWork w, GcDev 
 __device__ __forceinline__ const float4* c4(const float2* p) { return reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4* m4(float2* p) { return reinterpret_cast<float4*>(p); }
 
+__device__ __forceinline__ void add_pair(ThreadSum (&acc)[2][1], float a, float b) {
+    if (ThreadSum::small(fmaxf(fabsf(a), fabsf(b)))) {
+        acc[0][0].s.add(a);
+        acc[1][0].s.add(b);
+    } else {
+        acc[0][0].add_large(a);
+        acc[1][0].add_large(b);
+    }
+}
+
 // p = z, rz = (r, z) (real: L and the V-cycle are real symmetric)
 template <int K>
 __global__ void __launch_bounds__(kGcBlock) k_dcm_first(int nn, GcDev g, RedScratch rs) {
@@ -575,8 +585,7 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_first(int nn, GcDev g, RedScra
     for (long i = i0; i < n && (ra || rb); i += stride) {
         const float4 r = c4(g.dc_r)[i], z = c4(g.dc_z)[i];
         m4(g.dc_p)[i] = z;
-        acc[0][0].add(r.x * z.x + r.y * z.y);
-        acc[1][0].add(r.z * z.z + r.w * z.w);
+        add_pair(acc, r.x * z.x + r.y * z.y, r.z * z.z + r.w * z.w);
     }
     __shared__ double2 out[K];
     __shared__ __align__(8) float sh[red_floats<ThreadSum>(kGcBlock, 2)];
@@ -621,8 +630,7 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_ap(int nn, GcDev g, RedScratch
             }
         }
         m4(g.dc_ap)[i] = s;
-        acc[0][0].add(pv.x * s.x + pv.y * s.y);
-        acc[1][0].add(pv.z * s.z + pv.w * s.w);
+        add_pair(acc, pv.x * s.x + pv.y * s.y, pv.z * s.z + pv.w * s.w);
     }
     __shared__ double2 out[K];
     __shared__ __align__(8) float sh[red_floats<ThreadSum>(kGcBlock, 2)];
@@ -667,8 +675,7 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_update(int nn, GcDev g, int ca
         }
         m4(g.dc_x)[i] = x;
         m4(g.dc_r)[i] = r;
-        acc[0][0].add(r.x * r.x + r.y * r.y);
-        acc[1][0].add(r.z * r.z + r.w * r.w);
+        add_pair(acc, r.x * r.x + r.y * r.y, r.z * r.z + r.w * r.w);
     }
     __shared__ double2 out[K];
     __shared__ __align__(8) float sh[red_floats<ThreadSum>(kGcBlock, 2)];
@@ -696,8 +703,7 @@ __global__ void __launch_bounds__(kGcBlock) k_dcm_rz(int nn, GcDev g, RedScratch
     ThreadSum acc[2][1];
     for (long i = i0; i < n && run; i += stride) {
         const float4 r = c4(g.dc_r)[i], z = c4(g.dc_z)[i];
-        acc[0][0].add(r.x * z.x + r.y * z.y);
-        acc[1][0].add(r.z * z.z + r.w * z.w);
+        add_pair(acc, r.x * z.x + r.y * z.y, r.z * z.z + r.w * z.w);
     }
     __shared__ double2 out[K];
     __shared__ __align__(8) float sh[red_floats<ThreadSum>(kGcBlock, 2)];

@@ -517,14 +517,28 @@ __global__ void __launch_bounds__(192) k_wgrad_tc(const __grid_constant__ CUtens
                     break;
                 }
                 const unsigned char* dy = base + s * stage_bytes + box_bytes;
+                uint4 u[4];
+                __nv_bfloat162 most = __float2bfloat162_rn(0.0f);
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
                     const int row = (threadIdx.x >> 2) + 32 * r;
                     const int q = (threadIdx.x & 3) ^ ((row >> 1) & 3);   // 64-byte swizzle
-                    const uint4 u = *reinterpret_cast<const uint4*>(dy + row * 64 + q * 16);
-                    const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&u);
+                    u[r] = *reinterpret_cast<const uint4*>(dy + row * 64 + q * 16);
+                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u[r]);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) col[j].add(__bfloat162float(h[j]));
+                    for (int j = 0; j < 4; ++j) most = __hmax2(most, __habs2(h[j]));
+                }
+                const bool small = dev::ThreadSum::small(fmaxf(__low2float(most), __high2float(most)));
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&u[r]);
+                    if (small) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) col[j].s.add(__bfloat162float(h[j]));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) col[j].add_large(__bfloat162float(h[j]));
+                    }
                 }
                 tc::mbar_arrive(&empty[s]);
             }

@@ -24,10 +24,17 @@ __global__ void __launch_bounds__(kNT) k_sum(const float4* __restrict__ v, long 
         ThreadSum acc[2][2];
         for (long i = i0; i < m; i += stride) {
             const float4 q = v[i];
-            acc[0][0].add(q.x);
-            acc[0][1].add(q.y);
-            acc[1][0].add(q.z);
-            acc[1][1].add(q.w);
+            if (ThreadSum::small(fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))))) {
+                acc[0][0].s.add(q.x);
+                acc[0][1].s.add(q.y);
+                acc[1][0].s.add(q.z);
+                acc[1][1].s.add(q.w);
+            } else {
+                acc[0][0].add_large(q.x);
+                acc[0][1].add_large(q.y);
+                acc[1][0].add_large(q.z);
+                acc[1][1].add_large(q.w);
+            }
         }
         last = grid_reduce_f32<2, true, K, kNT, 2>(acc, rs, out, sh);
     } else {
