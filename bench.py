@@ -153,7 +153,7 @@ def bench_config(ne, nc):
                         f"{nc} cells), {sp.n_side * sp.n_side} stations, {nf} freqs "
                         f"{min(sp.freqs):g}-{max(sp.freqs):g} Hz, forward+adjoint+sensitivity gradient step "
                         f"({4 * nf} solves)",
-            "tol": TOL, "l2": "inputs larger than L2 (matrix alone 260 MB, K=16 FP32 vector 216 MB at C2)"}
+            "tol": TOL, "l2": "inputs larger than L2 (matrix alone 260 MB, K=16 FP32 vector 180 MB at C2)"}
 
 
 class ClockSampler:
@@ -401,7 +401,16 @@ def solver_params(args, plain):
     return p
 
 
-def solver_label(args, p, freqs):
+def multigrid_runs(p, leaves):
+    """Whether the mixed solve's preconditioner is geometric multigrid on these meshes (m3d_params.gradcorr)."""
+    from maple3dmt_gb300 import _loader
+    lib = _loader.load()
+    return bool(p["gradcorr"] and p["gradcorr_presmooth"] == 0 and p["ssor_relax"] == 1.0 and not p["coop_sweep"]
+                and not p["sweep_rows"] and all(lib.m3d_test_multigrid_levels(int(lv.level.min()), int(lv.level.max()))
+                                                for lv in leaves))
+
+
+def solver_label(args, p, freqs, leaves):
     if not p["precision"]:
         return {"arm": "plain FP64: one frequency per call, complex128 SSOR-BiCGStab, "
                        + ["csr", "staged"][p["row_kernels"]]
@@ -409,15 +418,18 @@ def solver_label(args, p, freqs):
     gc_all = p["gradcorr"] and p["gradcorr_fmax"] >= max(freqs)
     gc_none = not p["gradcorr"] or p["gradcorr_fmax"] < min(freqs)
     eis = "Eisenstat split form" if p["ssor_form"] else "right-preconditioned"
-    form = ("right-preconditioned (every batch carries the gradient-space term)" if gc_all
-            else eis if gc_none else f"right-preconditioned with the term, {eis} above {p['gradcorr_fmax']:g} Hz")
+    mg = multigrid_runs(p, leaves)
+    term = "multigrid" if mg else "the gradient-space term"
+    form = (f"right-preconditioned (every batch with {term})" if gc_all
+            else eis if gc_none else f"right-preconditioned with {term}, SSOR in {eis} above {p['gradcorr_fmax']:g} Hz")
     return {"arm": "batched", "precision": args.precision, "inner_tol_floor": p["inner_tol_floor"],
             "forward": args.forward, "row_kernels": ["csr", "staged"][p["row_kernels"]],
             "divcorr_precond": ["jacobi", "multigrid"][p["divcorr_precond"]],
             "divcorr_solve": ["fp64 pcg", "fp32 pcg in fp64 refinement"][p["divcorr_mixed"]],
             "ssor_form_run": form,
-            "gradcorr": (f"multigrid gradient-space term, V({p['gradcorr_presmooth']},1)"
-                         + (", V-cycle on a second stream" if p["gradcorr_overlap"] else "")) if p["gradcorr"]
+            "gradcorr": (("geometric multigrid: edge cycle V(1,1), node cycle V(0,1), two damped Jacobi steps" if mg else
+                          f"SSOR and multigrid gradient-space term, V({p['gradcorr_presmooth']},1)")
+                         + (", node cycle on a second stream" if p["gradcorr_overlap"] else "")) if p["gradcorr"]
             else "off",
             "residual_replacement": bool(p["residual_replacement"]),
             "sweep_rows": p["sweep_rows"], "coop_sweep": bool(p["coop_sweep"]), "ssor_relax": p["ssor_relax"],
@@ -583,7 +595,7 @@ def run_ours(args, rank, world, local_rank):
                  "ms_per_step": rp["t_dev"] * 1000.0 / args.plain_steps,
                  "rhs_at_tol": rp["stats"]["rhs_at_tol"], "rhs_reported": rp["stats"]["rhs_reported"],
                  "true_residual_max": rp["stats"]["true_residual_max"],
-                 "krylov_iterations_per_step": statistics.mean(rp["iters"]), **solver_label(args, pp, sv.freqs)}
+                 "krylov_iterations_per_step": statistics.mean(rp["iters"]), **solver_label(args, pp, sv.freqs, [sv.leaves])}
         sp_.close()
     learned = None
     if not plain_main and args.learned_steps > 0 and world == 1 and CONFIG == "c2":
@@ -621,7 +633,7 @@ def run_ours(args, rank, world, local_rank):
         "scaling": "strong", "vs_baseline": None, "dtype": "c128" if not p["precision"] else "c64+c128",
         "data": "synthetic",
         "config": bench_config(s.ne, s.nc),
-        "solver": {**solver_label(args, p, sv.freqs), "colours": s.n_colours,
+        "solver": {**solver_label(args, p, sv.freqs, [sv.leaves]), "colours": s.n_colours,
                    "parallelism": f"frequency groups x{world} (round-robin, one gradient SUM)"},
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         "plain": plain,
@@ -721,7 +733,7 @@ def run_c3(args, rank, world, local_rank):
                    "handles_at_once": args.c3_concurrent,
                    "timing": "host clock between device synchronisations (one stream per handle)",
                    "l2": "inputs larger than L2"},
-        "solver": {**solver_label(args, p, freqs), "parallelism": "handles run concurrently, one host thread and "
+        "solver": {**solver_label(args, p, freqs, [sv.leaves for sv in svs]), "parallelism": "handles run concurrently, one host thread and "
                                                                    "CUDA stream per handle"},
         "e2e": {"value": n_solves * args.steps / total, "unit": UNIT, "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},

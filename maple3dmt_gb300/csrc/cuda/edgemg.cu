@@ -1082,12 +1082,13 @@ void emg_coarse_k(const KrylovCtx<float>& c, const float2* r, float2* z0) {
     const GcDev& gc = *c.gc;
     Omegas om;
     for (int k = 0; k < kMaxRhs; ++k) om.v[k] = k < K ? (float)c.B.omega[k] : 0.0f;
-    const double nb = (double)c.n_rows * K * sizeof(float2), e0 = (double)emg_entries(g.lv[0].n) * K * sizeof(float2),
-                 nn = (double)gc.nn * K * sizeof(float2);
+    const double nb = (double)c.n_rows * K * sizeof(float2), nn = (double)gc.nn * K * sizeof(float2);
+    const double side = g.lv[0].n + 1, e0 = 3.0 * side * side * edge_planes(g.lv[0]) * K * sizeof(float2);
     // r gathered by both restrictions and read by the last kernel, z0 written;
-    // level-0 edge vectors b, x written and read, residual, x updated, y;
-    // octree node vectors b, t, out
-    const int th = c.timer ? c.timer->begin(kClsGradcorr, 4 * nb + 11 * e0 + 7 * nn, K) : -1;
+    // level-0 edge vectors: b, x written and read, the residual written and
+    // read, x updated, x, b read and y written, y read; octree node vectors: b
+    // written and read twice, t written and read, the result likewise
+    const int th = c.timer ? c.timer->begin(kClsGradcorr, 4 * nb + 12 * e0 + 7 * nn, K) : -1;
     if (c.gc_stream) {
         cudaEventRecord(c.gc_fork, c.stream);
         cudaStreamWaitEvent(c.gc_stream, c.gc_fork, 0);

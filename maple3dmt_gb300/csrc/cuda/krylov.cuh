@@ -151,7 +151,7 @@ struct KrylovCtx {
     long long* launches;   // host counter of kernel launches
     KernelTimer* timer;    // may be null
     long nnz;              // true off-diagonal entries (algorithmic bytes)
-    int n_rows;            // real edge rows
+    int n_rows;            // edge rows among them, without padding (bytes of the timed classes)
     int n_freq;            // distinct diagonals in use
     // slice-staged copy of A's off-diagonal part (see staged.cuh) and which
     // row kernels run: kRowsDirect (CSR rows read by the lanes) or

@@ -402,6 +402,8 @@ void GpuSolver::setup(const m3d_leaves* lv, const m3d_params* params) {
             }
         if (part == 0) n_free = (int)perm.size();
     }
+    n_free_edges = 0;
+    for (int e = 0; e < ne; ++e) n_free_edges += free_row(e);
     n_pad = (int)perm.size();
     n_slices = n_pad / dev::kSlice;
     iperm.assign(ne, -1);
@@ -1404,7 +1406,7 @@ KrylovCtx<float> GpuSolver::kctx32(int K, const int* fmap, bool free_rows) const
     f.launches = c.launches;
     f.timer = c.timer;
     f.nnz = c.nnz;
-    f.n_rows = c.n_rows;
+    f.n_rows = free_rows ? n_free_edges : c.n_rows;
     f.n_freq = c.n_freq;
     f.seg = seg32;
     f.row_kernels = c.row_kernels;

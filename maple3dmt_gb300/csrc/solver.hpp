@@ -165,6 +165,7 @@ private:
     std::vector<unsigned char> flags_ref;  // reference order
     int n_pad = 0, n_slices = 0;
     int n_free = 0;                     // the free rows are the first n_free (padding included)
+    int n_free_edges = 0;               // free rows without padding
     std::vector<int> hp_levels;         // dependency levels of the hanging pairs (ranges of md.hp)
 
     // device mesh
