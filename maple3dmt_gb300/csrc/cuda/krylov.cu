@@ -461,7 +461,7 @@ template <class R, int LPT> struct alignas(LPT * 2 * sizeof(R)) CVec {
 // so most gathers hit the SM's L1 (see tile_ring): at K = 8 on the 1.7 M-edge
 // mesh the pass over colour-sorted slices dealt out to the blocks in turn took
 // 200 us, bound by L2 gathers (13 rows of 64 bytes per row); now 110 us, 119 as
-// a damped Jacobi step (data once: 91 us).
+// a damped Jacobi step (data once: 64 us).
 template <class R, int K, int MODE>
 __global__ void __launch_bounds__(SpmvShape<R, K>::NT, 1)
     k_spmv_st(SegView<R> S, int n_slices, int T, int ring, DiagView<R> D, BatchView B, const cplx<R>* x,
