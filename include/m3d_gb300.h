@@ -131,7 +131,9 @@ typedef struct m3d_params {
                                  setting of the SSOR sweeps or of the aggregation cycle other than its
                                  default (ssor_relax, coop_sweep, sweep_rows, gradcorr_presmooth), by
                                  SSOR plus a gradient-space term G (i omega L)^-1 G^T (one multigrid V-cycle on
-                                 the divergence-correction Laplacian L); needs div_correction.
+                                 the divergence-correction Laplacian L); needs div_correction.  A
+                                 right-hand side that multigrid does not advance goes on with the
+                                 latter, for up to bicgstab_maxiter further iterations.
                                  Batches with such a right-hand side run the right-preconditioned
                                  form.  0: SSOR alone (the reference's preconditioner) */
     double gradcorr_fmax;     /* Hz */
